@@ -163,6 +163,26 @@ def test_gemm_f32_is_true_32_bit_and_rows_do_not_depend_on_the_batch(M, N, K):
     assert torch.allclose(nobias.cpu() + b, out.cpu(), atol=1e-5)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 130, 76), (2, 31, 64), (5, 33, 260), (16, 149, 1000), (16, 4737, 68), (17, 65, 260),
+                                   (33, 64, 1024), (64, 63, 1020), (65, 257, 1028), (130, 129, 4100), (777, 40, 16)])
+def test_gemm_f32_kernels_of_every_size_add_in_one_order(M, N, K):
+    """Few rows, tiles with and without a cluster, and rows that are not aligned to 16 bytes: the same sums, bit for bit, at
+    remainders of every tile; the bound is that of a chain of K additions."""
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w, b = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g), torch.randn(N, generator=g)
+    out, other = torch.full((M, N), 7.0, device="cuda"), torch.empty(M, N, device="cuda")
+    ops().gemm_f32(dev(a), dev(w), dev(b), out)
+    want = a.double() @ w.double().T + b.double()
+    assert (out.cpu().double() - want).abs().max() / want.abs().max() < 5e-7 * math.sqrt(K)
+    shifted = torch.empty(M * K + 1, device="cuda")[1:].view(M, K)
+    ops().gemm_f32(shifted.copy_(a), dev(w), dev(b), other)
+    assert torch.equal(out, other)
+    if M > 16:
+        few = torch.empty(3, N, device="cuda")
+        ops().gemm_f32(dev(a[5:8].contiguous()), dev(w), dev(b), few)
+        assert torch.equal(few, out[5:8])
+
+
 def rope_reference(x, positions, theta, rot):
     """x [T, heads, d]: rotate the first `rot` elements of every head (plain formula)."""
     y = x.copy()
