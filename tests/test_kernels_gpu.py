@@ -301,6 +301,30 @@ def test_paged_attention_ref(H, K, d, P, window, dtype):
     assert np.abs(out.float().cpu().numpy() - want).max() < tol * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("H,K,d,P", [(6, 2, 48, 16), (8, 2, 128, 64), (12, 1, 20, 48), (16, 16, 16, 16)])
+@pytest.mark.parametrize("window,chunk", [(0, None), (21, None), (0, 50)])
+def test_float32_attention_of_rows_together_is_that_of_rows_alone(H, K, d, P, window, chunk):
+    """Many rows (several of them to a block, runs of every length up to more than a block's) give the bits that each row
+    gives alone, and the plain result."""
+    lens, q_lens = [150, 1, 64, 333, 40, 41], [147, 1, 1, 330, 3, 5]
+    q, cache, bt, positions, seq_of, ks, vs = paged_case(H, K, d, P, lens, q_lens, "float32", seed=d + window, num_pages=64)
+    if d % 16:
+        cache = np.ascontiguousarray(cache.reshape(cache.shape[0], -1))       # (the form for heads of any size)
+    args = dict(chunk=chunk, kv_heads=K, page_tokens=P)
+    out = torch.empty(q.shape, device="cuda")
+    sink = torch.randn(H, generator=torch.Generator().manual_seed(d)).cuda()
+    ops().paged_attention_ref(dev(q), dev(cache), dev(bt), dev(seq_of), dev(positions), out, window, d ** -0.5, sink=sink, **args)
+    for t in list(range(0, 9)) + [146, 147, 148, 149, 477, 478, 479, 481, 482, len(q) - 1]:
+        one = torch.empty((1,) + q.shape[1:], device="cuda")
+        ops().paged_attention_ref(dev(q[t:t + 1]), dev(cache), dev(bt), dev(seq_of[t:t + 1]), dev(positions[t:t + 1]), one, window,
+                                  d ** -0.5, sink=sink, **args)
+        assert torch.equal(one[0], out[t]), t
+    if chunk is None:
+        ops().paged_attention_ref(dev(q), dev(cache), dev(bt), dev(seq_of), dev(positions), out, window, d ** -0.5, **args)
+        want = attention_reference(q, ks, vs, positions, seq_of, window)
+        assert np.abs(out.cpu().numpy() - want).max() < 2e-6 * max(1.0, np.abs(want).max())
+
+
 @pytest.mark.parametrize("far", [0, 15, 16, 17, 63, 64, 300, 447])
 def test_attention_finds_one_far_key_among_hundreds(far):
     """One key is made to match the query so that its score stands out: the output must be that
