@@ -1,5 +1,5 @@
-// The delta rule with a decay per key channel over whole portions of prompts, in chunks of 16 tokens whose rows are computed
-// side by side from the state ahead of them.  Per head, with k, q of length d (k, and q before its scale, of unit length),
+// The delta rule (with a decay per key channel, or one per head) and gated linear attention over whole portions of prompts, in
+// chunks of 16 tokens whose rows are computed side by side from the state ahead of them.  Per head, with k, q of length d (k, and q before its scale, of unit length),
 // g_t the decays and beta_t the step sizes, the recurrence is
 //
 //   S_t = diag(g_t) S_(t-1) + k_t u_t^T,   u_t = beta_t (v_t - (diag(g_t) S_(t-1))^T k_t),   o_t = S_t^T q_t.
@@ -13,6 +13,9 @@
 //   o_t  = (q_t exp(b_t)) S_0 + sum_(s <= t) p_ts u_s
 //   S    = diag(exp(b_last)) S_0 + sum_s (k_s exp(b_last - b_s)) u_s^T
 //
+// One decay per head is the same with equal b's: a and p are then plain products times exp(b_t - b_s).  Gated linear attention
+// is the same with u_t = v_t (q and k as they come, q times its scale): there is no a, W or X, and Y is v.
+//
 // delta_chunk_prepare_kernel   all that does not depend on the state, 32-bit on the CUDA cores, a block per chunk and head
 // delta_chunk_scan_kernel      the last three lines, a block per head, portion and 16 columns of the state.  The state's
 //                              columns are the rows of the tensor-core instruction (m16n8k8, TF32 operands, 32-bit sums), its
@@ -22,6 +25,10 @@
 //                              two TF32 numbers, hi + lo, and every product as lo hi + hi lo + hi hi, which keeps 21 bits of
 //                              the operands: what is left out is of the order of 32-bit rounding.  The next chunk's
 //                              numbers arrive by the copy engine, in two runs of bytes, while this one's are used.
+//
+// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 194 (prepare
+// 54, scan 140); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 87 (22 and 65).  Below 24 tokens the two
+// launches and a chunk's chain are no shorter than the tokens' own.
 //
 // What a row is depends on the state and the portion's tokens only.
 #include "common.cuh"
@@ -40,8 +47,10 @@ constexpr float DC_FLOOR = -60.f;   // a decay of 2^-60 is none: the logarithms'
 //   p    [16][16]     swizzled as the keys are
 //   Y^T  [dvp][16]    dvp: dv filled up to a multiple of 16 (zeros)
 // (in this arrangement four rows that a warp reads eight bytes at a time fall into different banks)
-template <int DP> struct DeltaChunk {
-    static constexpr int KEYS = 32 * DP, LAST = KEYS + DC * DP, P = LAST + DP, Y = P + DC * DC;
+// (gated linear attention has no W: rows [16][DP] are q exp b alone)
+enum { CHUNK_CHANNEL = 0, CHUNK_HEAD = 1, CHUNK_GLA = 2 };
+template <int DP, int MODE> struct DeltaChunk {
+    static constexpr int ROWS = MODE == CHUNK_GLA ? DC : 2 * DC, KEYS = ROWS * DP, LAST = KEYS + DC * DP, P = LAST + DP, Y = P + DC * DC;
 };
 __device__ __forceinline__ int dc_row_place(int t, int c) { return c ^ ((t & 3) << 3); }
 __device__ __forceinline__ int dc_key_place(int c, int t) { return t ^ (((c >> 1) & 1) << 3); }
@@ -50,17 +59,17 @@ struct DeltaChunkArgs {
     const float* q; int ldq;        // [T, ldq]: head g's d numbers at column g * d, before their unit length and scale
     const float* k; int ldk;
     const float* v; int ldv;        // [T, ldv]: head h's dv numbers at column h * dv
-    const float* decay; int ldd;    // [T, ldd]: d logits per head
-    const float* beta; int ldb;     // [T, ldb]: one logit per head
-    const float* a_log;             // [H]
-    const float* dt_bias;           // [H * d]
+    const float* decay; int ldd;    // [T, ldd]: d logits per head (HEAD: one)
+    const float* beta; int ldb;     // [T, ldb]: one logit per head (not GLA)
+    const float* a_log;             // [H] (not GLA)
+    const float* dt_bias;           // [H * d] (HEAD: [H]; not GLA)
     const int* chunks;              // [N, 2]: first row, tokens
     const int* portions;            // [L, 4]: first row, tokens, slot, first chunk
     float* scratch;                 // [N, H, stride]
     float* state;                   // [slots, H, d, dv]
     float* out;                     // [T, H, dv]
     int H, G, d, dv, dvp;
-    float q_scale, unit_eps;
+    float q_scale, unit_eps, inv_tau;
     long long stride;
     int* status;
 };
@@ -73,7 +82,7 @@ __device__ __forceinline__ float power_of_2(float x) {
     return y;
 }
 
-template <int DP>
+template <int DP, int MODE>
 __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_kernel(const DeltaChunkArgs p) {
     constexpr int ld = DP + 4, PER = DP / 32;
     extern __shared__ __align__(16) float smem[];
@@ -86,7 +95,7 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
     float* sk = smem;                       // [16][ld]
     float* sq = sk + DC * ld;
     float* sb = sq + DC * ld;               // the decays' logarithms to the base 2, then their sums
-    const float rate = -expf(p.a_log[h]) * 1.4426950408889634f;
+    const float rate = MODE == CHUNK_GLA ? -p.inv_tau * 1.4426950408889634f : -expf(p.a_log[h]) * 1.4426950408889634f;
     {   // a warp per two tokens: unit lengths, logarithms (both tokens' loads under way at once)
         float x[2][PER], y[2][PER], z[2][PER];
 #pragma unroll
@@ -98,7 +107,11 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
                 const bool in = t < n && c < d;
                 x[r][i] = in ? p.k[(size_t)(q0 + t) * p.ldk + g * d + c] : 0.f;
                 y[r][i] = in ? p.q[(size_t)(q0 + t) * p.ldq + g * d + c] : 0.f;
-                z[r][i] = in ? p.decay[(size_t)(q0 + t) * p.ldd + h * d + c] + p.dt_bias[h * d + c] : 0.f;
+                // (log sigmoid(z) = -softplus(-z))
+                z[r][i] = !in ? 0.f
+                    : MODE == CHUNK_GLA ? -p.decay[(size_t)(q0 + t) * p.ldd + h * d + c]
+                    : MODE == CHUNK_HEAD ? p.decay[(size_t)(q0 + t) * p.ldd + h] + p.dt_bias[h]
+                    : p.decay[(size_t)(q0 + t) * p.ldd + h * d + c] + p.dt_bias[h * d + c];
             }
         }
 #pragma unroll
@@ -111,13 +124,17 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
                 qs = fmaf(y[r][i], y[r][i], qs);
                 sb[t * ld + lane + 32 * i] = t < n && lane + 32 * i < d ? fmaxf(rate * softplus_1(z[r][i]), DC_FLOOR) : 0.f;
             }
-            const float kf = 1.f / sqrtf(warp_sum(ss) + p.unit_eps), qf = p.q_scale / sqrtf(warp_sum(qs) + p.unit_eps);
+            float kf = 1.f, qf = p.q_scale;
+            if (MODE != CHUNK_GLA) {
+                kf = 1.f / sqrtf(warp_sum(ss) + p.unit_eps);
+                qf = p.q_scale / sqrtf(warp_sum(qs) + p.unit_eps);
+            }
 #pragma unroll
             for (int i = 0; i < PER; ++i) {
                 sk[t * ld + lane + 32 * i] = x[r][i] * kf;
                 sq[t * ld + lane + 32 * i] = y[r][i] * qf;
             }
-            if (lane == 0) sbeta[t] = t < n ? 1.f / (1.f + expf(-p.beta[(size_t)(q0 + t) * p.ldb + h])) : 0.f;
+            if (MODE != CHUNK_GLA && lane == 0) sbeta[t] = t < n ? 1.f / (1.f + expf(-p.beta[(size_t)(q0 + t) * p.ldb + h])) : 0.f;
         }
     }
     __syncthreads();
@@ -129,7 +146,7 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
             sb[t * ld + tid] = sum;
         }
     }
-    using Place = DeltaChunk<DP>;
+    using Place = DeltaChunk<DP, MODE>;
     float* base = p.scratch + ((size_t)blockIdx.x * p.H + h) * p.stride;
     float* Pm = base + Place::P;
     {
@@ -166,8 +183,8 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
                     for (int e = 0; e < 4; ++e) {
                         float x = xb[r][e] - yb[s][e];
                         if (r < s) x = fminf(x, 0.f);      // (above the diagonal where i = j: not kept, but it may not overflow)
-                        const float w = yk[s][e] * power_of_2(x);
-                        a[r][s] = fmaf(xk[r][e], w, a[r][s]);
+                        const float w = MODE == CHUNK_HEAD ? yk[s][e] : yk[s][e] * power_of_2(x);
+                        if (MODE != CHUNK_GLA) a[r][s] = fmaf(xk[r][e], w, a[r][s]);
                         pq[r][s] = fmaf(xq[r][e], w, pq[r][s]);
                     }
         }
@@ -181,7 +198,12 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
                 pq[r][s] += __shfl_xor_sync(0xffffffffu, pq[r][s], 2);
                 const int t = 2 * i + r, u = 2 * j + s;
                 if (part == 0 && tid < 144 && u <= t) {
-                    sa[t][u] = u < t ? sbeta[t] * a[r][s] : 0.f;
+                    if (MODE == CHUNK_HEAD) {
+                        const float w = power_of_2(sb[t * ld] - sb[u * ld]);
+                        a[r][s] *= w;
+                        pq[r][s] *= w;
+                    }
+                    if (MODE != CHUNK_GLA) sa[t][u] = u < t ? sbeta[t] * a[r][s] : 0.f;
                     Pm[t * DC + dc_key_place(t, u)] = pq[r][s];
                 }
             }
@@ -200,7 +222,7 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
                 for (int i = 0; i < 4; ++i) {
                     const float b = sb[(t + i) * ld + j], k = sk[(t + i) * ld + j], e = power_of_2(b);
                     x[t + i] = k * e;
-                    base[(DC + t + i) * DP + dc_row_place(t + i, j)] = sq[(t + i) * ld + j] * e;
+                    base[(Place::ROWS - DC + t + i) * DP + dc_row_place(t + i, j)] = sq[(t + i) * ld + j] * e;
                     kv[i] = k * power_of_2(last - b);
                 }
                 store4(keys + dc_key_place(j, t), kv);
@@ -211,6 +233,8 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
 #pragma unroll
             for (int t = 0; t < DC; ++t) x[t] = t < n && c < p.dv ? p.v[(size_t)(q0 + t) * p.ldv + h * p.dv + c] : 0.f;
         }
+        if (MODE == CHUNK_GLA && j < DP) continue;
+        if (MODE != CHUNK_GLA)
 #pragma unroll
         for (int t = 0; t < DC; ++t) {
             float sum = sbeta[t] * x[t];
@@ -265,11 +289,12 @@ constexpr int DC_STAGES = 2;
 
 // A warp holds NJ tiles of 8 channels of the state, transposed: S[j] is (column g or g + 8 of the block) x (channels 8 j + 2 t,
 // 8 j + 2 t + 1), g = lane / 4, t = lane % 4.
-template <int DP>
+template <int DP, int MODE>
 __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const DeltaChunkArgs p) {
     constexpr int NJ = DP / (8 * DC_WARPS);
-    constexpr int STAGES = DC_STAGES, BUF = DeltaChunk<DP>::Y + DC * DC;      // floats of a buffer: the chunk's, and 16 columns of Y
-    using Place = DeltaChunk<DP>;
+    using Place = DeltaChunk<DP, MODE>;
+    constexpr int STAGES = DC_STAGES, BUF = Place::Y + DC * DC;      // floats of a buffer: the chunk's, and 16 columns of Y
+    constexpr int RG = Place::ROWS / 8;      // tiles of 8 rows of W and q
     extern __shared__ __align__(16) float smem[];
     __shared__ __align__(8) uint64_t full[STAGES];
     __shared__ int gave_up;
@@ -313,7 +338,7 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
     const int rows_at = g * DP + t2, swap = dc_key_place(g, 0);      // (of rows 8 j + g: the tile does not matter)
     float* mine = red + (warp * DC + g) * DC_RLD + t2;
     const int sum_c = tid >> 3, sum_t = 4 * (tid & 7);               // the four sums that this thread completes: column, rows
-    const float* sum_from = red + sum_c * DC_RLD + sum_t;
+    const float* sum_from = red + sum_c * DC_RLD + sum_t - (MODE == CHUNK_GLA && sum_t >= DC ? DC : 0);
     float* sum_to = (sum_t < DC ? UT : OT - DC) + sum_c * DC_ULD + sum_t;
     const int t0 = 8 * (warp & 1);                                   // warps 0 and 1: the tokens whose o they finish
     float* out = p.out + ((size_t)(row0 + t0 + t2) * p.H + h) * p.dv + col0 + g;
@@ -328,38 +353,40 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
             return;
         }
         if (tid == 0 && i + STAGES - 1 < chunks) stage(i + STAGES - 1);
-        float acc[4][4];
+        float acc[RG][4];
 #pragma unroll
-        for (int x = 0; x < 4; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f;
+        for (int x = 0; x < RG; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f;
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
             const Two a[4] = {two_of(S[j][0]), two_of(S[j][2]), two_of(S[j][1]), two_of(S[j][3])};
             const float* at = buf + rows_at + dc_row_place(g, r0 + 8 * j);
-            Two b[4][2];
+            Two b[RG][2];
 #pragma unroll
-            for (int x = 0; x < 4; ++x) two_pair(b[x], at + 8 * x * DP);
+            for (int x = 0; x < RG; ++x) two_pair(b[x], at + 8 * x * DP);
             // (the four sums in turn: a product does not wait for the one before it)
 #pragma unroll
-            for (int x = 0; x < 4; ++x) mma_tf32(acc[x], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[x][0].hi, b[x][1].hi);
+            for (int x = 0; x < RG; ++x) mma_tf32(acc[x], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[x][0].hi, b[x][1].hi);
 #pragma unroll
-            for (int x = 0; x < 4; ++x) mma_tf32(acc[x], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].lo, b[x][1].lo);
+            for (int x = 0; x < RG; ++x) mma_tf32(acc[x], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].lo, b[x][1].lo);
 #pragma unroll
-            for (int x = 0; x < 4; ++x) mma_tf32(acc[x], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].hi, b[x][1].hi);
+            for (int x = 0; x < RG; ++x) mma_tf32(acc[x], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].hi, b[x][1].hi);
         }
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
+        for (int x = 0; x < RG; ++x) {
             *reinterpret_cast<float2*>(mine + 8 * x) = make_float2(acc[x][0], acc[x][1]);
             *reinterpret_cast<float2*>(mine + 8 * DC_RLD + 8 * x) = make_float2(acc[x][2], acc[x][3]);
         }
         __syncthreads();
         {   // the warps' sums in order: U = Y - W S (rows 0 .. 15 of 32), o's first part (the others)
             float v[DC_WARPS][4];
+            if (MODE != CHUNK_GLA || sum_t >= DC)
 #pragma unroll
-            for (int w = 0; w < DC_WARPS; ++w) load4(sum_from + w * DC * DC_RLD, v[w]);
+                for (int w = 0; w < DC_WARPS; ++w) load4(sum_from + w * DC * DC_RLD, v[w]);
             float y[4] = {0.f, 0.f, 0.f, 0.f};
             if (sum_t < DC) load4(buf + Place::Y + sum_c * DC + sum_t, y);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
+                if (MODE == CHUNK_GLA && sum_t < DC) continue;            // (u is v)
                 const float sum = (v[0][e] + v[1][e]) + (v[2][e] + v[3][e]);
                 y[e] = sum_t < DC ? y[e] - sum : sum;
             }
@@ -421,19 +448,19 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
         }
 }
 
-template <int DP>
+template <int DP, int MODE>
 static int launch_delta_chunks(const DeltaChunkArgs& args, int N, int L, cudaStream_t stream) {
     DeltaChunkArgs a = args;
     a.dvp = (a.dv + 15) / 16 * 16;
-    a.stride = DeltaChunk<DP>::Y + (long long)DC * a.dvp;
+    a.stride = DeltaChunk<DP, MODE>::Y + (long long)DC * a.dvp;
     const size_t smem1 = sizeof(float) * 3 * DC * (DP + 4);
     if (smem1 > 44 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(delta_chunk_prepare_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+        cudaError_t e = cudaFuncSetAttribute(delta_chunk_prepare_kernel<DP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
         if (e != cudaSuccess) return (int)e;
     }
-    int rc = launch(delta_chunk_prepare_kernel<DP>, dim3(N, a.H), 256, smem1, stream, a);
+    int rc = launch(delta_chunk_prepare_kernel<DP, MODE>, dim3(N, a.H), 256, smem1, stream, a);
     if (rc) return rc;
-    size_t smem2 = sizeof(float) * (DC_STAGES * (DeltaChunk<DP>::Y + DC * DC) + DC_WARPS * DC * DC_RLD + 2 * DC * DC_ULD);
+    size_t smem2 = sizeof(float) * (DC_STAGES * (DeltaChunk<DP, MODE>::Y + DC * DC) + DC_WARPS * DC * DC_RLD + 2 * DC * DC_ULD);
     const dim3 grid(a.dvp / DC, a.H, L);
     // (as for the scan token by token: the blocks start when their predecessor has ended, and spread over the SMs)
     int sms = 148, dev = 0;
@@ -441,38 +468,49 @@ static int launch_delta_chunks(const DeltaChunkArgs& args, int N, int L, cudaStr
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long blocks = (long long)grid.x * grid.y * grid.z;
     if (blocks <= sms && smem2 < 120 * 1024) smem2 = 120 * 1024;
-    cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+    cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(DC_WARPS * 32);
     cfg.dynamicSmemBytes = smem2;
     cfg.stream = stream;
-    return (int)cudaLaunchKernelEx(&cfg, delta_chunk_scan_kernel<DP>, a);
+    return (int)cudaLaunchKernelEx(&cfg, delta_chunk_scan_kernel<DP, MODE>, a);
 }
 
 }  // namespace air
 
-// scratch: float32 [N, H, 49 DP + 256 + 16 dvp] with DP = d filled up to 32, 64, 128 or 256, dvp = dv to a multiple of 16.
-// Rows and slots as the lists say; d up to 256.
-AIR_API int air_delta_portions(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay,
-                               int ldd, const float* beta, int ldb, const float* a_log, const float* dt_bias, float* state,
-                               float* out, const int* portions, int L, const int* chunks, int N, float* scratch, int H, int G,
-                               int d, int dv, float q_scale, float unit_eps, int* status, cudaStream_t stream) {
+namespace air {
+template <int MODE> static int launch_chunks_of(const DeltaChunkArgs& a, int N, int L, cudaStream_t stream) {
+    if (a.d <= 32) return launch_delta_chunks<32, MODE>(a, N, L, stream);
+    if (a.d <= 64) return launch_delta_chunks<64, MODE>(a, N, L, stream);
+    if (a.d <= 128) return launch_delta_chunks<128, MODE>(a, N, L, stream);
+    return launch_delta_chunks<256, MODE>(a, N, L, stream);
+}
+}  // namespace air
+
+// mode 0: the delta rule with a decay per key channel, 1: with one per head, 2: gated linear attention (alpha =
+// sigmoid(decay)^inv_tau; no beta, a_log, dt_bias, unit lengths).  scratch: float32 [N, H, 49 DP + 256 + 16 dvp] (mode 2: 33
+// DP) with DP = d filled up to 32, 64, 128 or 256, dvp = dv to a multiple of 16.  Rows and slots as the lists say; d up to 256.
+AIR_API int air_delta_portions(int mode, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
+                               const float* decay, int ldd, const float* beta, int ldb, const float* a_log,
+                               const float* dt_bias, float* state, float* out, const int* portions, int L, const int* chunks,
+                               int N, float* scratch, int H, int G, int d, int dv, float q_scale, float unit_eps, float inv_tau,
+                               int* status, cudaStream_t stream) {
     using namespace air;
     if (L <= 0 || N <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || d > 256 || dv <= 0 || H > 65535 || L > 65535 || !scratch ||
-        ((uintptr_t)scratch & 15))
+        ((uintptr_t)scratch & 15) || mode < 0 || mode > 2 || (mode != CHUNK_GLA && (!beta || !a_log || !dt_bias)))
         return AIR_ERR_BAD_ARGUMENT;
     DeltaChunkArgs a;
     a.q = q; a.ldq = ldq; a.k = k; a.ldk = ldk; a.v = v; a.ldv = ldv; a.decay = decay; a.ldd = ldd; a.beta = beta; a.ldb = ldb;
     a.a_log = a_log; a.dt_bias = dt_bias; a.chunks = chunks; a.portions = portions; a.scratch = scratch; a.state = state;
     a.out = out; a.H = H; a.G = G; a.d = d; a.dv = dv; a.dvp = 0; a.q_scale = q_scale; a.unit_eps = unit_eps; a.stride = 0;
+    a.inv_tau = inv_tau;
     a.status = status;
-    if (d <= 32) return launch_delta_chunks<32>(a, N, L, stream);
-    if (d <= 64) return launch_delta_chunks<64>(a, N, L, stream);
-    if (d <= 128) return launch_delta_chunks<128>(a, N, L, stream);
-    return launch_delta_chunks<256>(a, N, L, stream);
+    if (mode == CHUNK_GLA) return launch_chunks_of<CHUNK_GLA>(a, N, L, stream);
+    if (mode == CHUNK_HEAD) return launch_chunks_of<CHUNK_HEAD>(a, N, L, stream);
+    return launch_chunks_of<CHUNK_CHANNEL>(a, N, L, stream);
 }
 
 AIR_API int air_trace_set_delta_chunks(unsigned long long* buffer) { return air::set_trace_here(buffer); }

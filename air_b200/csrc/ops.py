@@ -89,9 +89,9 @@ _SIGNATURES = {
                         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                         c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_float, c_void_p,
                         c_void_p, c_int, c_float, c_void_p],
-    "air_delta_portions": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
-                           c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
-                           c_int, c_float, c_float, c_void_p, c_void_p],
+    "air_delta_portions": [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int,
+                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int,
+                           c_int, c_int, c_float, c_float, c_float, c_void_p, c_void_p],
     "air_gated_rmsnorm": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float,
                           c_int, c_void_p],
     "air_polynorm": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_float,
@@ -1176,35 +1176,49 @@ DELTA_CHUNK = 16         # tokens of a chunk of delta_portions
 DELTA_MAX_D = 256        # key channels per head that it takes
 
 
-def delta_portions(q, k, v, decay, state, out, portions, chunks, q_scale, beta, a_log, dt_bias, unit_eps=1e-6,
-                   status=None):
-    """linear_scan's SCAN_CHANNEL_DELTA with unit lengths, for whole portions: the tokens of a chunk are computed side by side
-    from the state ahead of it (delta_chunks.cu).  portions int32 [L, 4] = (first row, tokens, slot, first chunk), chunks
-    int32 [N, 2] = (first row, tokens): a portion's tokens cut into chunks of DELTA_CHUNK.  State, decays and sums
-    are 32-bit; the products with the state run on the tensor cores, their 32-bit operands as two TF32 numbers each."""
+_CHUNK_MODES = {SCAN_CHANNEL_DELTA: 0, SCAN_DELTA: 1, SCAN_GLA: 2}
+
+
+def delta_portions(q, k, v, decay, state, out, portions, chunks, q_scale, beta=None, a_log=None, dt_bias=None, unit_eps=1e-6,
+                   status=None, mode=SCAN_CHANNEL_DELTA, tau=1.0):
+    """linear_scan's SCAN_CHANNEL_DELTA or SCAN_DELTA with unit lengths, or SCAN_GLA, for whole portions: the tokens of a chunk
+    are computed side by side from the state ahead of it (delta_chunks.cu).  portions int32 [L, 4] = (first row, tokens,
+    slot, first chunk), chunks int32 [N, 2] = (first row, tokens): a portion's tokens cut into chunks of DELTA_CHUNK.  State,
+    decays and sums are 32-bit; the products with the state run on the tensor cores, their 32-bit operands as two TF32
+    numbers each."""
     _, H, d, dv = state.shape
+    if mode not in _CHUNK_MODES:
+        raise KernelError(f"delta_portions: mode {mode}")
     _req(state, "state", (torch.float32,))
     T = out.shape[0]
     _req(out, "out", (torch.float32,), (T, H, dv))
-    (qp, ldq), (kp, ldk), (vp, ldv) = _columns(q, "q"), _columns(k, "k"), _columns(v, "v")
-    (dp, ldd), (bp, ldb) = _columns(decay, "decay"), _columns(beta, "beta")
-    if q.shape[1] % d or k.shape != q.shape or v.shape[1] != H * dv or decay.shape[1] != H * d or beta.shape[1] != H:
-        raise KernelError("delta_portions: q, k, v, decay or beta do not fit the state's shape")
+    (qp, ldq), (kp, ldk), (vp, ldv), (dp, ldd) = _columns(q, "q"), _columns(k, "k"), _columns(v, "v"), _columns(decay, "decay")
+    per_head = 1 if mode == SCAN_DELTA else d
+    if q.shape[1] % d or k.shape != q.shape or v.shape[1] != H * dv or decay.shape[1] != H * per_head:
+        raise KernelError("delta_portions: q, k, v or decay do not fit the state's shape")
     G = q.shape[1] // d
     if G == 0 or H % G or d > DELTA_MAX_D:
         raise KernelError(f"delta_portions: {H} heads over {G} heads of q and k, of {d} channels (up to {DELTA_MAX_D})")
-    _req(a_log, "a_log", (torch.float32,), (H,))
-    _req(dt_bias, "dt_bias", (torch.float32,), (H * d,))
+    bp, ldb = None, 0
+    if mode == SCAN_GLA:
+        if G != H:
+            raise KernelError("delta_portions: gated linear attention takes a head of q and k per head of v")
+    else:
+        bp, ldb = _columns(beta, "beta")
+        if beta.shape[1] != H:
+            raise KernelError("delta_portions: the delta rule takes one beta per head")
+        _req(a_log, "a_log", (torch.float32,), (H,))
+        _req(dt_bias, "dt_bias", (torch.float32,), (H * per_head,))
     _req(portions, "portions", _I32, (None, 4))
     _req(chunks, "chunks", _I32, (None, 2))
     N = chunks.shape[0]
     wide = next(w for w in (32, 64, 128, 256) if d <= w)
-    stride = 49 * wide + 256 + 16 * (-(-dv // 16) * 16)
+    stride = (33 if mode == SCAN_GLA else 49) * wide + 256 + 16 * (-(-dv // 16) * 16)
     scratch = torch.empty(N * H * stride, dtype=torch.float32, device=out.device)
     _check(_get("air_delta_portions")(
-        qp, ldq, kp, ldk, vp, ldv, dp, ldd, bp, ldb, a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), out.data_ptr(),
-        portions.data_ptr(), portions.shape[0], chunks.data_ptr(), N, scratch.data_ptr(), H, G, d, dv, float(q_scale),
-        float(unit_eps), _ptr(status), _stream()), "delta_portions")
+        _CHUNK_MODES[mode], qp, ldq, kp, ldk, vp, ldv, dp, ldd, bp, ldb, _ptr(a_log), _ptr(dt_bias), state.data_ptr(),
+        out.data_ptr(), portions.data_ptr(), portions.shape[0], chunks.data_ptr(), N, scratch.data_ptr(), H, G, d, dv,
+        float(q_scale), float(unit_eps), 1.0 / float(tau), _ptr(status), _stream()), "delta_portions")
     global launches
     launches += 1
     return out

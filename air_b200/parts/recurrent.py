@@ -47,8 +47,49 @@ class _StateMixer(Mixer):
         return ops.short_conv_silu(proj[:, :self.channels], self.conv_weight, state, y, ctx.q_start, ctx.slots, ctx.max_q_len)
 
 
+class _ChunkedMixer(_StateMixer):
+    """State mixers whose longer portions a bfloat16 engine takes in chunks whose rows are computed side by side
+    (ops.delta_portions); everything else goes token by token (ops.linear_scan)."""
+
+    PORTION = 24
+
+    def plan_key(self):
+        chunks = self.rt.dtype == torch.bfloat16 and self.head_dim <= ops.DELTA_MAX_D
+        return ("linear.chunks", self.PORTION) if chunks else None
+
+    def plan(self, batch: HostBatch) -> Plan:
+        """portions [L, 4] = (first row, tokens, slot, first chunk) of the entries of at least PORTION tokens, chunks [N, 2] =
+        (first row, tokens) of theirs; short_slots: the slot of every other entry, short_seq: of their rows, -1 elsewhere."""
+        portions, chunks, short_slots = [], [], []
+        short_seq = np.full(batch.q_start[-1], -1, dtype=np.int32)
+        for i, n in enumerate(batch.counts):
+            first = batch.q_start[i]
+            if n < self.PORTION:
+                short_slots.append(batch.slots[i])
+                short_seq[first:first + n] = batch.slots[i]
+                continue
+            short_slots.append(-1)
+            portions.append((first, n, batch.slots[i], len(chunks)))
+            chunks += [(first + at, min(ops.DELTA_CHUNK, n - at)) for at in range(0, n, ops.DELTA_CHUNK)]
+        return Plan(arrays={"portions": np.asarray(portions, dtype=np.int32).reshape(-1, 4),
+                            "chunks": np.asarray(chunks, dtype=np.int32).reshape(-1, 2),
+                            "short_slots": np.asarray(short_slots, dtype=np.int32), "short_seq": short_seq},
+                    values={"long": bool(portions), "short": len(portions) < len(batch.counts)})
+
+    def _scan(self, mode, q, k, v, decay, state, o, ctx, unit_lengths=True, **numbers):
+        bands = (q, k, v, decay, state, o)
+        unit = dict(unit=True, unit_eps=1e-6) if unit_lengths else {}
+        plan = ctx.plans.get(self.plan_key()) if self.plan_key() is not None else None
+        if plan is None or not plan.long:
+            ops.linear_scan(mode, *bands, ctx.q_start, ctx.slots, ctx.token_seq, **unit, **numbers)
+            return
+        if plan.short:
+            ops.linear_scan(mode, *bands, ctx.q_start, plan.short_slots, plan.short_seq, **unit, **numbers)
+        ops.delta_portions(*bands, plan.portions, plan.chunks, status=ctx.status, mode=mode, **numbers)
+
+
 @register_mixer("gated_delta")
-class GatedDeltaRule(_StateMixer):
+class GatedDeltaRule(_ChunkedMixer):
     """The gated delta rule.  q, k (kv_heads x head_dim) and v (heads x v_dim) are projections of the input followed by
     a short causal convolution over time per channel (`conv` taps, the last one the current token's) and SiLU; q and k
     are scaled to unit length per head (x / sqrt(sum x^2 + 1e-6)), q also by head_dim^-1/2; head h reads q/k head
@@ -108,14 +149,13 @@ class GatedDeltaRule(_StateMixer):
         proj = self.proj.f32(x)
         y = self._convolved(proj, tail, ctx)
         o = torch.empty((T, H, dv), dtype=torch.float32, device=x.device)
-        ops.linear_scan(ops.SCAN_DELTA, y[:, :G * d], y[:, G * d:2 * G * d], y[:, 2 * G * d:],
-                        self._band(proj, "a"), state.state, o, ctx.q_start, ctx.slots, ctx.token_seq, q_scale=d ** -0.5,
-                        beta=self._band(proj, "b"), a_log=self.a_log, dt_bias=self.dt_bias, unit=True, unit_eps=1e-6)
+        self._scan(ops.SCAN_DELTA, y[:, :G * d], y[:, G * d:2 * G * d], y[:, 2 * G * d:], self._band(proj, "a"), state.state, o,
+                   ctx, q_scale=d ** -0.5, beta=self._band(proj, "b"), a_log=self.a_log, dt_bias=self.dt_bias)
         return self._finish(o, self._band(proj, "g"), ctx)
 
 
 @register_mixer("channel_delta")
-class ChannelDeltaRule(_StateMixer):
+class ChannelDeltaRule(_ChunkedMixer):
     """The delta rule with a decay per key channel.  q, k, v, their convolutions, unit lengths and b as in GatedDeltaRule; the
     decay of channel c of head h is g = exp(-exp(A_log_h) * softplus(W_a2 (W_a1 x) + dt_bias)), a product through a narrow
     middle laid out heads x head_dim, and scales row c of the head's state:
@@ -203,31 +243,6 @@ class ChannelDeltaRule(_StateMixer):
             full[:rows, i * width:i * width + rank] = m
         return Linear(full, rt.status)
 
-    PORTION = 24
-
-    def plan_key(self):
-        chunks = self.rt.dtype == torch.bfloat16 and self.head_dim <= ops.DELTA_MAX_D
-        return ("channel_delta.chunks", self.PORTION) if chunks else None
-
-    def plan(self, batch: HostBatch) -> Plan:
-        """portions [L, 4] = (first row, tokens, slot, first chunk) of the entries of at least PORTION tokens, chunks [N, 2] =
-        (first row, tokens) of theirs; short_slots: the slot of every other entry, short_seq: of their rows, -1 elsewhere."""
-        portions, chunks, short_slots = [], [], []
-        short_seq = np.full(batch.q_start[-1], -1, dtype=np.int32)
-        for i, n in enumerate(batch.counts):
-            first = batch.q_start[i]
-            if n < self.PORTION:
-                short_slots.append(batch.slots[i])
-                short_seq[first:first + n] = batch.slots[i]
-                continue
-            short_slots.append(-1)
-            portions.append((first, n, batch.slots[i], len(chunks)))
-            chunks += [(first + at, min(ops.DELTA_CHUNK, n - at)) for at in range(0, n, ops.DELTA_CHUNK)]
-        return Plan(arrays={"portions": np.asarray(portions, dtype=np.int32).reshape(-1, 4),
-                            "chunks": np.asarray(chunks, dtype=np.int32).reshape(-1, 2),
-                            "short_slots": np.asarray(short_slots, dtype=np.int32), "short_seq": short_seq},
-                    values={"long": bool(portions), "short": len(portions) < len(batch.counts)})
-
     def _narrow(self, proj):
         """(decay logits [T, heads*head_dim], gate logits [T, heads*v_dim]), float32."""
         at, (ra, rg) = self.columns["a1"][0], self.middle
@@ -246,21 +261,13 @@ class ChannelDeltaRule(_StateMixer):
         y = self._convolved(proj, tail, ctx)
         decay, gate = self._narrow(proj)
         o = torch.empty((T, H, dv), dtype=torch.float32, device=x.device)
-        bands = (y[:, :G * d], y[:, G * d:2 * G * d], y[:, 2 * G * d:], decay, state.state, o)
-        numbers = dict(q_scale=d ** -0.5, beta=self._band(proj, "b"), a_log=self.a_log, dt_bias=self.dt_bias, unit_eps=1e-6)
-        plan = ctx.plans.get(self.plan_key()) if self.plan_key() is not None else None
-        if plan is None or not plan.long:
-            ops.linear_scan(ops.SCAN_CHANNEL_DELTA, *bands, ctx.q_start, ctx.slots, ctx.token_seq, unit=True, **numbers)
-        else:
-            if plan.short:
-                ops.linear_scan(ops.SCAN_CHANNEL_DELTA, *bands, ctx.q_start, plan.short_slots, plan.short_seq, unit=True,
-                                **numbers)
-            ops.delta_portions(*bands, plan.portions, plan.chunks, status=ctx.status, **numbers)
+        self._scan(ops.SCAN_CHANNEL_DELTA, y[:, :G * d], y[:, G * d:2 * G * d], y[:, 2 * G * d:], decay, state.state, o, ctx,
+                   q_scale=d ** -0.5, beta=self._band(proj, "b"), a_log=self.a_log, dt_bias=self.dt_bias)
         return self._finish(o, gate, ctx, sigmoid=True)
 
 
 @register_mixer("gla")
-class GatedLinearAttention(_StateMixer):
+class GatedLinearAttention(_ChunkedMixer):
     """Gated linear attention.  q = W_q x * head_dim^-1/2, k = W_k x (heads x head_dim), v = W_v x (heads x v_dim);
     a decay per key channel, alpha = sigmoid(W_a2 (W_a1 x) + b_a2)^(1/tau) (a product through a narrow middle);
     per head and token
@@ -309,8 +316,8 @@ class GatedLinearAttention(_StateMixer):
         z = torch.empty((T, H * d), dtype=torch.float32, device=x.device)
         ops.gemm_f32(self._band(proj, "a1").contiguous(), self.a2, self.a2_bias, z)
         o = torch.empty((T, H, dv), dtype=torch.float32, device=x.device)
-        ops.linear_scan(ops.SCAN_GLA, self._band(proj, "q"), self._band(proj, "k"), self._band(proj, "v"), z,
-                        state.state, o, ctx.q_start, ctx.slots, ctx.token_seq, q_scale=d ** -0.5, tau=self.tau)
+        self._scan(ops.SCAN_GLA, self._band(proj, "q"), self._band(proj, "k"), self._band(proj, "v"), z, state.state, o, ctx,
+                   unit_lengths=False, q_scale=d ** -0.5, tau=self.tau)
         return self._finish(o, self._band(proj, "g"), ctx)
 
 

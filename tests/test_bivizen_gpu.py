@@ -120,6 +120,71 @@ def test_gated_linear_attention_scan(H, d, dv, tau):
         assert float(state[0].min()) == 3.0              # other requests' states are not touched
 
 
+@pytest.mark.parametrize("mode,H,G,d,dv", [("delta", 4, 2, 24, 20), ("delta", 1, 1, 64, 33), ("delta", 2, 1, 130, 8),
+                                           ("delta", 2, 2, 128, 128), ("delta", 1, 1, 1, 1), ("gla", 2, 2, 24, 20),
+                                           ("gla", 1, 1, 64, 33), ("gla", 2, 2, 130, 8), ("gla", 2, 2, 128, 256), ("gla", 3, 3, 12, 18)])
+@pytest.mark.parametrize("decays", ["mixed", "slow", "fast"])
+def test_chunks_against_token_by_token(decays, mode, H, G, d, dv):
+    """Both roads of the gated delta rule and of gated linear attention against the 64-bit recurrence, from states that are not
+    empty, the states they leave behind among the results: portions of every length around a chunk's in one batch."""
+    from air_b200.csrc import ops
+    rng = np.random.default_rng(d + dv + (mode == "gla"))
+    tau, delta = 16.0, mode == "delta"
+    for counts in ([15, 16, 17], [1, 32, 200], [48, 31, 2]):
+        T = sum(counts)
+        start = np.concatenate([[0], np.cumsum(counts)])
+        slots = [2, 0, 3]
+        q, k, v = rng.normal(size=(T, G * d)), rng.normal(size=(T, G * d)), rng.normal(size=(T, H * dv))
+        k[T // 3:T // 3 + 6] = k[T // 3]                 # the same key several times
+        shift = {"mixed": 0.0, "slow": -8.0, "fast": 9.0}[decays]
+        z, b = rng.normal(size=(T, H if delta else H * d)) * 3, rng.normal(size=(T, H)) * 3
+        a_log, dt = rng.uniform(-2, 0.5, size=H), rng.normal(size=H) + shift
+        if not delta:
+            z = (z - shift) * 4
+        S0 = rng.normal(size=(4, H, d, dv))
+        chunks, portions = [], []
+        for i, n in enumerate(counts):
+            portions.append((start[i], n, slots[i], len(chunks)))
+            chunks += [(start[i] + a, min(ops.DELTA_CHUNK, n - a)) for a in range(0, n, ops.DELTA_CHUNK)]
+        wide = dev(np.concatenate([q, k, v], axis=1))          # bands of a wider matrix
+        bands = (wide[:, :G * d], wide[:, G * d:2 * G * d], wide[:, 2 * G * d:], dev(z))
+        kw = dict(q_scale=d ** -0.5, **(dict(beta=dev(b), a_log=dev(a_log), dt_bias=dev(dt)) if delta else dict(tau=tau)))
+        which = ops.SCAN_DELTA if delta else ops.SCAN_GLA
+        got = []
+        for road in ("tokens", "chunks"):
+            S, o = dev(S0), torch.full((T, H, dv), 9.0, device=DEV)
+            if road == "tokens":
+                ops.linear_scan(which, *bands, S, o, i32(start), i32(slots), i32(np.repeat(slots, counts)), unit=delta, **kw)
+            else:
+                ops.delta_portions(*bands, S, o, torch.tensor(np.array(portions), dtype=torch.int32, device=DEV),
+                                   torch.tensor(np.array(chunks), dtype=torch.int32, device=DEV), mode=which, **kw)
+            got.append((o.cpu().numpy(), S.cpu().numpy()))
+        assert np.array_equal(got[1][1][1], S0[1].astype(np.float32)), "another request's state is not touched"
+        if delta:
+            g = np.exp(-np.exp(a_log) * plain.softplus(z + dt))[:, :, None]
+            kk, qq = plain.unit(k.reshape(T, G, d)), plain.unit(q.reshape(T, G, d)) * d ** -0.5
+        else:
+            g = plain.sigmoid(z).reshape(T, H, d) ** (1.0 / tau)
+            kk, qq = k.reshape(T, G, d), q.reshape(T, G, d) * d ** -0.5
+        for i, n in enumerate(counts):
+            for h in range(H):
+                S = S0[slots[i], h].copy()
+                largest = np.abs(S).max()
+                for t in range(start[i], start[i] + n):
+                    S = g[t, h][:, None] * S
+                    u = v[t, h * dv:(h + 1) * dv]
+                    if delta:
+                        u = plain.sigmoid(b[t, h]) * (u - S.T @ kk[t, h // (H // G)])
+                    S = S + np.outer(kk[t, h // (H // G)], u)
+                    # (32-bit rounding of states that have grown: gated linear attention adds every value to them)
+                    largest = max(largest, np.abs(S).max())
+                    for road in range(2):
+                        bound = 5e-5 if delta else 5e-6 * largest * max(1.0, np.abs(qq[t, h]).sum())
+                        assert np.abs(got[road][0][t, h] - S.T @ qq[t, h // (H // G)]).max() < bound, (road, i, t)
+                for road in range(2):
+                    assert np.abs(got[road][1][slots[i], h] - S).max() < (5e-5 if delta else 5e-6) * max(1.0, largest), (road, i)
+
+
 def test_gated_norm_feed_forward_activation_and_scaled_sum():
     from air_b200.csrc import ops
     rng = np.random.default_rng(5)
