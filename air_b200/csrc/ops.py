@@ -66,7 +66,7 @@ _SIGNATURES = {
                         c_void_p, c_void_p],
     "air_masked_softmax": [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                            c_void_p, c_float, c_void_p, c_int, c_void_p],
-    "air_moe_route": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int,
+    "air_moe_route": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int,
                       c_int, c_int, c_float, c_float, c_void_p, c_void_p],
     "air_moe_identity": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "air_normed_add_norm": [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_float, c_void_p, c_void_p, c_int,
@@ -78,6 +78,9 @@ _SIGNATURES = {
                          c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_int,
                          c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float,
                          c_float, c_float, c_void_p],
+    "air_expert_stream": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                          c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_void_p, c_float, c_float, c_float, c_int,
+                          c_void_p, c_void_p],
     "air_rows_by_index": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "air_planes_by_index": [c_void_p, c_int, c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "air_qkv_prepare": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
@@ -884,14 +887,14 @@ def latent_prepare(q, c, c_weight, eps, freq, positions, token_seq, block_table,
 
 def moe_route(z, experts, top, expert_out, weight_out, gate_out=None, has_gate=False, score="sigmoid",
               renormalize=False, groups=0, keep=0, route_scale=1.0, norm_eps=0.0, choice_bias=None, mark="two"):
-    """z float32 [T, >= experts (+ 1)]: router logits.  expert_out int32 [T, top], weight_out float32 [T, top]: the
+    """z float32 [T, >= experts (+ 1)], or [parts, T, ..] partial sums to be added in order: router logits.  expert_out int32 [T, top], weight_out float32 [T, top]: the
     experts with the largest scores (sigmoid(z), or softmax(z)) and those scores (divided by their sum + norm_eps where
     renormalize), times route_scale; gate_out float32 [T] = sigmoid(z[:, experts]) where has_gate, else 1.  groups > 1:
     the experts are cut into `groups` runs of experts / groups consecutive indices, a run's mark is its best score plus
     its second best (mark "two"; "best": its best score alone), and only experts of the `keep` runs with the highest marks
     can be chosen.  choice_bias (float32
     [experts]): the experts are chosen by score + choice_bias; the weights stay the scores."""
-    T = z.shape[0]
+    parts, T = (1 if z.dim() == 2 else z.shape[0]), z.shape[-2]
     if choice_bias is not None:
         _req(choice_bias, "choice_bias", (torch.float32,), (experts,))
     _req(z, "z", (torch.float32,))
@@ -903,7 +906,7 @@ def moe_route(z, experts, top, expert_out, weight_out, gate_out=None, has_gate=F
         raise KernelError(f"moe_route: score {score!r}")
     if mark not in ("two", "best"):
         raise KernelError(f"moe_route: mark {mark!r}")
-    _check(_get("air_moe_route")(z.data_ptr(), z.shape[1], T, int(experts), int(top), 1 if score == "softmax" else 0,
+    _check(_get("air_moe_route")(z.data_ptr(), parts, z.shape[-1], T, int(experts), int(top), 1 if score == "softmax" else 0,
                                  1 if renormalize else 0, 1 if has_gate else 0, expert_out.data_ptr(),
                                  weight_out.data_ptr(), _ptr(gate_out), int(groups), int(keep),
                                  1 if mark == "best" else 0, float(route_scale),
@@ -976,6 +979,43 @@ def grouped_gemm(a, w, out, n, k, *, lda, ldo, groups, a_group_stride=0, o_group
         int(rows_per_group), _ptr(tiles), _ptr(num_tiles), tiles.shape[0] if tiles is not None else 0, int(groups),
         int(n), int(k), _DT[a.dtype], 2 if relu2 else (1 if silu_mul else 0), int(gate_block), _ptr(o_scale), int(o_scale_ld), float(act[0]),
         float(act[1]), float(act[2]), _stream()), "grouped_gemm")
+    return out
+
+
+def expert_stream_ok(x, w, gate_block, silu_mul):
+    """Whether expert_stream takes these rows and matrices (bfloat16, rows of whole 16-byte pieces, blocks of 128)."""
+    return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[2] % 8 == 0
+            and (not silu_mul or (gate_block == 128 and w.shape[1] % 256 == 0)) and w.shape[0] * w.shape[1] < 2 ** 31)
+
+
+def expert_stream(rows, w, out, start, tiles, num_tiles, most_rows, *, silu_mul=False, relu2=False, act=(1.0, 0.0, 0.0),
+                  o_index=None, o_div=1, splits=1, o_scale=None, lists_ready=False, status=None):
+    """The experts' products with the weights as the tensor cores' wide side (expert_stream.cu): rows bfloat16 [slots, K] in
+    moe_sort's order @ w[g]^T, w bfloat16 [groups, N, K].  No expert has more than most_rows slots.
+    silu_mul: out bfloat16 [slots, N / 2] = the gated activation `act` of blocks of 128 gate rows and 128 linear rows; relu2:
+    out bfloat16 [slots, N] = max(x, 0)^2; else out float32 [splits * o_div, T, N]: slot s goes to plane part * o_div +
+    o_index[s] % o_div, row o_index[s] // o_div, times o_scale[o_index[s]], one plane per part of k.  lists_ready: the kernel
+    launched right before is an expert_stream with the same lists and without lists_ready."""
+    slots, K = rows.shape
+    groups, N, _ = w.shape
+    _req(rows, "rows", (torch.bfloat16,))
+    _req(w, "w", (torch.bfloat16,), (groups, N, K))
+    for name, x in (("start", start), ("tiles", tiles), ("num_tiles", num_tiles)):
+        _req(x, name, _I32)
+    plane = ldo = 0
+    if silu_mul or relu2:
+        _req(out, "out", (torch.bfloat16,), (slots, N // 2 if silu_mul else N))
+    else:
+        _req(out, "out", (torch.float32,), (splits * o_div, None, N))
+        _req(o_index, "o_index", _I32, (slots,))
+        plane, ldo = out.shape[1] * N, N
+    if o_scale is not None:
+        _req(o_scale, "o_scale", (torch.float32,))
+    _check(_get("air_expert_stream")(
+        rows.data_ptr(), slots, w.data_ptr(), groups, N, K, start.data_ptr(), tiles.data_ptr(), num_tiles.data_ptr(),
+        tiles.shape[0], int(most_rows), 1 if silu_mul else 2 if relu2 else 0, out.data_ptr(), int(splits), _ptr(o_index),
+        int(o_div), plane, ldo, _ptr(o_scale), float(act[0]), float(act[1]), float(act[2]), 1 if lists_ready else 0,
+        _ptr(status), _stream()), "expert_stream")
     return out
 
 

@@ -7,7 +7,7 @@ from ..config.model_config import ConfigError
 from ..csrc import ops
 from ..weights.loader import TensorSpec
 from .base import FeedForward, GatedSum
-from .linear import Linear
+from .linear import Linear, SMS
 from .mlp import ClampedGLU, SwiGLU
 from .registry import register_feed_forward
 from .spec import PartSpec
@@ -51,11 +51,12 @@ class RoutedExperts(FeedForward):
     Everything happens on the device: a kernel picks the experts, one orders the (token, choice) pairs by expert, and
     two grouped products (gate and up with the activation; down) walk the experts' rows.  The outputs of a token's
     choices land in `top` planes that the norm behind the layer adds in order, so the sum does not depend on the
-    batch.  From LIBRARY_ROWS rows per expert (in the mean) on, a bfloat16 step hands the two products to the library's
+    batch.  In a bfloat16 engine the two products are a stream of the chosen experts' weights on the tcgen05 tensor cores
+    (ops.expert_stream; sizes that it does not take, and float32, run ops.grouped_gemm).  From LIBRARY_ROWS rows per expert (in the mean) on, a bfloat16 step hands the two products to the library's
     grouped product (which also takes the experts' bounds from the device): there the experts' outputs are rounded to
     bfloat16 before they are added up in 32-bit."""
 
-    LIBRARY_ROWS = 32
+    LIBRARY_ROWS = 64        # (measured, see csrc/expert_stream.cu)
 
     graph_safe = True
 
@@ -153,7 +154,7 @@ class RoutedExperts(FeedForward):
     def forward(self, x, ctx):
         T, E, F, n, top = x.shape[0], self.hidden, self.inter, self.experts, self.top
         dev = x.device
-        z = self.router.f32(x)
+        z = self.router.f32_sums(x)      # (few rows: a block per part of k instead of one for all of it)
         expert = torch.empty((T, top), dtype=torch.int32, device=dev)
         weight = torch.empty((T, top), dtype=torch.float32, device=dev)
         gate = torch.empty((T,), dtype=torch.float32, device=dev) if self.shared_gate else None
@@ -165,13 +166,26 @@ class RoutedExperts(FeedForward):
         ints = torch.empty(n + 1 + pairs + 2 * (pairs // ops.GROUP_TILE + n) + 1, dtype=torch.int32, device=dev)
         start, pair_of_slot = ints[:n + 1], ints[n + 1:n + 1 + pairs]
         tiles, num_tiles = ints[n + 1 + pairs:-1].view(-1, 2), ints[-1:]
+        by_library = x.dtype == torch.bfloat16 and pairs >= self.LIBRARY_ROWS * n and E % 16 == 0 and F % 16 == 0
+        streams = not by_library and ops.expert_stream_ok(x, self.gate_up, self.block, self.gated) and \
+            ops.expert_stream_ok(x, self.down, 0, False)
         ops.moe_sort(expert, n, start, pair_of_slot, tiles, num_tiles)
-        y = torch.empty((top, T, E), dtype=torch.float32, device=dev)
+        parts = self._parts(T) if streams else 1
+        y = torch.empty((parts * top, T, E), dtype=torch.float32, device=dev)
         if self.identity:
             # (pairs of an expert without matrices get no slot in the order by expert: their planes are written here)
             ops.moe_identity(x, expert, weight, n, y)
-        if x.dtype == torch.bfloat16 and pairs >= self.LIBRARY_ROWS * n and E % 16 == 0 and F % 16 == 0:
+        if by_library:
             self._experts_by_the_library(x, start, pair_of_slot, weight, y)
+        elif streams:
+            rows = ops.rows_by_index(x, pair_of_slot, top, weight.view(-1) if on_input else None,
+                                     torch.empty((pairs, E), dtype=x.dtype, device=dev))
+            act = torch.empty((pairs, F), dtype=x.dtype, device=dev)
+            lists = (start, tiles, num_tiles, T)       # (a token takes an expert once at most)
+            ops.expert_stream(rows, self.gate_up, act, *lists, silu_mul=self.gated, relu2=not self.gated, act=self.act,
+                              status=self.rt.status)
+            ops.expert_stream(act, self.down, y, *lists, o_index=pair_of_slot, o_div=top, splits=parts,
+                              o_scale=None if on_input else weight.view(-1), lists_ready=True, status=self.rt.status)
         else:
             act = torch.empty((pairs, F), dtype=x.dtype, device=dev)
             ops.grouped_gemm(x, self.gate_up, act, F, E, lda=E, ldo=F, groups=n, a_index=pair_of_slot, a_div=top,
@@ -184,6 +198,21 @@ class RoutedExperts(FeedForward):
         if self.shared is None:
             return y
         return GatedSum(y, self.shared.forward(x, ctx), gate)
+
+    def _parts(self, T):
+        """Parts of k of the second product in a step of few tokens: what shares the tiles of the experts that such a step
+        reaches (in the mean) most evenly over the SMs.  Every part has planes of its own, so not with identity experts,
+        which write a plane themselves, nor where the planes are many rows."""
+        k_tiles = -(-self.inter // 64)
+        if self.identity or T > 64:
+            return 1
+        reached = self.experts * (1.0 - (1.0 - self.top / self.outputs) ** T)
+        tiles = reached * -(-self.hidden // 128)
+
+        def even(s):
+            rounds = tiles * s / SMS
+            return rounds / -(-rounds // 1) - 0.02 * s
+        return max((s for s in (1, 2, 4) if s == 1 or k_tiles % s == 0 and k_tiles // s >= 8), key=even)
 
     def _experts_by_the_library(self, x, start, pair_of_slot, weight, y):
         """The road of steps with many rows per expert: the rows in the experts' order with their weights on them, the

@@ -152,7 +152,7 @@ def test_attention_sees_the_keys_inside_its_mask_and_no_other(kind, size, dtype)
                 out = torch.empty((m, H, dv), dtype=dtype, device=DEV)
                 kernel(dev(q[at:at + m], dtype), cache, table, i32([1] * m), i32(range(at, at + m)), out,
                        size if kind == "window" else None, scale, kv_heads=G, page_tokens=P,
-                       chunk=size if kind == "chunk" else None, sink=dev(sink), **more)
+                       chunk=size if kind == "chunk" else None, sink=dev(sink))
                 tol = 3e-4 if dtype == torch.float32 else 0.3          # (values up to 35: bfloat16 holds them to 0.125)
                 assert np.abs(out.float().cpu().numpy() - want[at:at + m]).max() < tol, (at, m, kernel.__name__)
             at += m
@@ -515,3 +515,47 @@ def test_trace_runner_program_and_command_line(capsys):
     assert cli.main(["cuda", tu.model_folder(name), ",".join(map(str, prompt)), "--tokens", "6", "--dtype", "float32",
                      "--no-stop-on-eos"]) == 0
     assert capsys.readouterr().out.strip() == ",".join(map(str, tu.plain_greedy(name, prompt, 6)))
+
+
+@pytest.mark.parametrize("T,top,n,E,F", [(1, 1, 3, 64, 128), (8, 2, 16, 200, 256), (16, 3, 5, 72, 384), (17, 2, 4, 136, 128),
+                                         (33, 2, 7, 264, 128), (64, 1, 2, 64, 640), (150, 2, 9, 128, 256)])
+@pytest.mark.parametrize("splits", [1, 2])
+def test_expert_stream_against_64_bit_products(T, top, n, E, F, splits):
+    """The experts' products as a stream of weights: one to more than 64 rows per expert, experts without rows, widths that are
+    not whole tiles, parts of k in planes of their own, every epilogue."""
+    from air_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    expert = torch.argsort(torch.rand(T, n - (n > 2), generator=g, device="cuda"), dim=1)[:, :top].int().contiguous()
+    if T == 150:
+        expert[:, 0], expert[:, 1] = 0, 1 + torch.arange(T, device="cuda") % 3      # 150 rows of one expert
+    pairs = T * top
+    i32 = lambda *s: torch.empty(s, dtype=torch.int32, device="cuda")
+    start, slot_pair, tiles, count = i32(n + 1), i32(pairs), i32(pairs // 64 + n, 2), i32(1)
+    ops.moe_sort(expert, n, start, slot_pair, tiles, count)
+    x, weight = rand(T, E).bfloat16(), torch.rand(T, top, generator=g, device="cuda")
+    up, down = (rand(n, 2 * F, E) * E ** -0.5).bfloat16(), (rand(n, E, F) * F ** -0.5).bfloat16()
+    rows = ops.rows_by_index(x, slot_pair, top, weight.view(-1), torch.empty(pairs, E, dtype=torch.bfloat16, device="cuda"))
+    lists = (start, tiles, count, T)
+    act = torch.empty(pairs, F, dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.expert_stream(rows, up, act, *lists, silu_mul=True, status=status)
+    if splits > 1 and (-(-F // 64) % 2 or F < 128):
+        splits = 1
+    y = torch.full((splits * top, T, E), 9.0, device="cuda")
+    ops.expert_stream(act, down, y, *lists, o_index=slot_pair, o_div=top, splits=splits, o_scale=weight.view(-1), lists_ready=True,
+                      status=status)
+    plain_up = torch.empty(pairs, 2 * F, dtype=torch.bfloat16, device="cuda")
+    ops.expert_stream(rows, up, plain_up, *lists, relu2=True, status=status)
+    assert status.item() == 0
+    for s, p in enumerate(slot_pair.tolist()):
+        t, c = divmod(p, top)
+        e = int(expert[t, c])
+        z = up[e].double() @ rows[s].double()
+        assert (plain_up[s].double() - z.clamp(min=0) ** 2).abs().max() <= 0.005 * (z ** 2).max()      # (bfloat16: 2^-8)
+        z = z.view(F // 128, 2, 128)
+        want = (torch.nn.functional.silu(z[:, 0]) * z[:, 1]).flatten()
+        assert (act[s].double() - want).abs().max() <= 0.005 * want.abs().max()
+        want = down[e].double() @ act[s].double() * weight[t, c].double()
+        got = y.view(splits, top, T, E)[:, c, t].double().sum(0)
+        assert (got - want).abs().max() <= 3e-6 * (down[e].double().abs() @ act[s].double().abs()).max()
