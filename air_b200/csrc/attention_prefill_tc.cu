@@ -36,6 +36,12 @@
 // from a tile's keys than the table reaches, that is one number more in the exponent's multiply-add; in the tiles near the
 // diagonal a lane looks up its row's numbers one key after the other, 32 neighbours per access.
 //
+// With DK > 0 the keys and values do not come from pages: they are the expansion of a request's compressed latents, worked out
+// for the portion ahead of this kernel.  kv [keys, H * 2 D] holds, per key (the first one is position key_origin) and head, D
+// numbers of the key and the D numbers of the value; where DK > D the last DK - D numbers of a key are the same for all heads
+// and lie in the latents' rows behind the latent (map_k2, column k2_column).  A query's last DK - D numbers come from q2 [T, H
+// * (DK - D)] in the same way.  A stage is then DK + D numbers wide, and three of them are what fits beside the queries.
+//
 // tiles, q, out, cache, block_table, window as in attention_prefill.cu; the list pads every request
 // to whole pairs of groups.  Head size 64 or 128; pages of a divisor or a multiple of 64 tokens.
 // Every wait on an mbarrier is bounded (tma.cuh); on giving up the block flags *status = 7.  A list
@@ -115,10 +121,13 @@ struct RowTile {
     int n;           // key tiles it takes
 };
 
-template <int D, bool BIAS>
+constexpr int at_stages(int d, int dk) { return dk > d ? 3 : AT_STAGES; }
+
+template <int D, bool BIAS, int DK>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_cache,
-                            const int* __restrict__ block_table, int max_blocks, const int* __restrict__ tiles,
+                            const __grid_constant__ CUtensorMap map_q2, const __grid_constant__ CUtensorMap map_k2,
+                            int key_origin, int k2_column, const int* __restrict__ block_table, int max_blocks, const int* __restrict__ tiles,
                             int n_pairs, const int* __restrict__ segments, int n_slots, float* __restrict__ part_o,
                             float2* __restrict__ part_ml, __nv_bfloat16* __restrict__ out, int H, int K, int P,
                             int window, float scale_log2, float cap, float cap_pre, int* __restrict__ status,
@@ -126,21 +135,24 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // sink (or null): float32 [H]; one more term exp(sink[h]) in the softmax's denominator, which has no key and no
     // value: it joins a row's sum where the row is normalised (here, or where its segments are merged)
     // cap > 0: a score s becomes cap * tanh(s * cap_pre) (cap_pre = scale / cap) and scale_log2 is log2(e) alone
-    constexpr int SUB = D / 64;                            // 64-column (128-byte) sub-tiles per row
-    constexpr int Q_BYTES = SUB * AT_BM * 128;             // one row tile of Q
+    constexpr bool EXPANDED = DK > 0;
+    constexpr int SUB = D / 64;                            // 64-column (128-byte) sub-tiles per row of V
+    constexpr int SUBK = EXPANDED ? DK / 64 : SUB;         // and of Q and K
+    constexpr int STAGES = at_stages(D, DK);
+    constexpr int Q_BYTES = SUBK * AT_BM * 128;            // one row tile of Q
     constexpr int KV_SUB = AT_BN * 128;                    // one sub-tile of K or V
-    constexpr int STAGE_BYTES = 2 * SUB * KV_SUB;          // K then V
+    constexpr int STAGE_BYTES = (SUBK + SUB) * KV_SUB;     // K then V
     constexpr uint32_t TMEM_COLS = 512;                    // S_A0 S_A1 | S_B0 S_B1 | O_A | O_B
     constexpr uint32_t O_COL = 2 * AT_ROW_TILES * AT_BN;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sq = smem;
     uint8_t* skv = sq + AT_ROW_TILES * Q_BYTES;
-    uint64_t* bars = (uint64_t*)(skv + AT_STAGES * STAGE_BYTES);
+    uint64_t* bars = (uint64_t*)(skv + STAGES * STAGE_BYTES);
     uint64_t* q_full = bars;
     uint64_t* kv_full = bars + 1;
-    uint64_t* kv_empty = kv_full + AT_STAGES;
-    uint64_t* s_full = kv_empty + AT_STAGES;     // [row tile][2]
+    uint64_t* kv_empty = kv_full + STAGES;
+    uint64_t* s_full = kv_empty + STAGES;     // [row tile][2]
     uint64_t* p_ready = s_full + 4;              // [row tile][2]
     uint64_t* pv_done = p_ready + 4;             // [row tile][2]: key tile j of a row tile completes [j & 1]
     uint32_t* tmem_slot = (uint32_t*)(pv_done + 4);
@@ -150,7 +162,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
-        for (int i = 0; i < AT_STAGES; ++i) {
+        for (int i = 0; i < STAGES; ++i) {
             mbar_init(&kv_full[i], 1);
             mbar_init(&kv_empty[i], AT_ROW_TILES);   // one arrival per issuer
         }
@@ -163,8 +175,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
-    if (P < AT_BN || window > 0) {   // rows that no copy fills must not hold NaN bits (see attention_decode_tma.cu)
-        for (int i = threadIdx.x; i < AT_STAGES * STAGE_BYTES / 16; i += AT_THREADS)
+    if (!EXPANDED && (P < AT_BN || window > 0)) {   // rows that no copy fills must not hold NaN bits (see attention_decode_tma.cu)
+        for (int i = threadIdx.x; i < STAGES * STAGE_BYTES / 16; i += AT_THREADS)
             reinterpret_cast<uint4*>(skv)[i] = make_uint4(0, 0, 0, 0);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -233,14 +245,29 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             mbar_expect_tx(q_full, (uint32_t)(Q_BYTES * (has_b ? 2 : 1)));
             for (int x = 0; x < (has_b ? 2 : 1); ++x)
 #pragma unroll
-                for (int s = 0; s < SUB; ++s)
-                    tma_load_2d(sq + x * Q_BYTES + s * AT_BM * 128, &map_q, h * D + 64 * s, tok0 + x * AT_BM, q_full);
+                for (int s = 0; s < SUBK; ++s) {
+                    uint8_t* dst = sq + x * Q_BYTES + s * AT_BM * 128;
+                    if (s < SUB) tma_load_2d(dst, &map_q, h * D + 64 * s, tok0 + x * AT_BM, q_full);
+                    else tma_load_2d(dst, &map_q2, h * (64 * (SUBK - SUB)) + 64 * (s - SUB), tok0 + x * AT_BM, q_full);
+                }
             const int box_rows = P < AT_BN ? P : AT_BN;
             const int boxes = AT_BN / box_rows;
             for (int it = 0; it < n_stream; ++it) {
-                const int stage = it % AT_STAGES;
-                if (it >= AT_STAGES && !mbar_wait(&kv_empty[stage], ((it / AT_STAGES) - 1) & 1, abort_flag)) break;
+                const int stage = it % STAGES;
+                if (it >= STAGES && !mbar_wait(&kv_empty[stage], ((it / STAGES) - 1) & 1, abort_flag)) break;
                 const int kbase = (tile0 + it) * AT_BN;
+                if constexpr (EXPANDED) {        // (rows beyond the last key come as zeros)
+                    mbar_expect_tx(&kv_full[stage], (uint32_t)STAGE_BYTES);
+                    uint8_t* to = skv + stage * STAGE_BYTES;
+                    const int row = kbase - key_origin;
+#pragma unroll
+                    for (int s = 0; s < SUBK + SUB; ++s, to += KV_SUB) {
+                        if (s < SUB) tma_load_2d(to, &map_cache, h * 2 * D + 64 * s, row, &kv_full[stage]);
+                        else if (s < SUBK) tma_load_2d(to, &map_k2, k2_column + 64 * (s - SUB), row, &kv_full[stage]);
+                        else tma_load_2d(to, &map_cache, h * 2 * D + D + 64 * (s - SUBK), row, &kv_full[stage]);
+                    }
+                    continue;
+                }
                 int valid = 0;
                 for (int b = 0; b < boxes; ++b) {
                     const int first = kbase + b * box_rows;
@@ -283,8 +310,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             bool ok = true;
             auto pass = [&](int from, int to) {   // key tiles that this row tile does not take
                 for (int t = from; t < to && ok; ++t) {
-                    const int stage = t % AT_STAGES;
-                    ok = __all_sync(0xffffffffu, mbar_wait(&kv_full[stage], (t / AT_STAGES) & 1, abort_flag));
+                    const int stage = t % STAGES;
+                    ok = __all_sync(0xffffffffu, mbar_wait(&kv_full[stage], (t / STAGES) & 1, abort_flag));
                     if (ok && elect_one()) mbar_arrive(&kv_empty[stage]);
                     __syncwarp();
                 }
@@ -298,15 +325,15 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 if (j < me.n) {
                     // S(j) = Q K(j)^T into S[j & 1] (which held P(j-2): the product that read it was
                     // issued before this one)
-                    const int t = me.first + j, stage = t % AT_STAGES;
-                    if (!mbar_try_wait(&kv_full[stage], (t / AT_STAGES) & 1))      // (mostly there already: one try)
-                        ok = __all_sync(0xffffffffu, mbar_wait(&kv_full[stage], (t / AT_STAGES) & 1, abort_flag));
+                    const int t = me.first + j, stage = t % STAGES;
+                    if (!mbar_try_wait(&kv_full[stage], (t / STAGES) & 1))      // (mostly there already: one try)
+                        ok = __all_sync(0xffffffffu, mbar_wait(&kv_full[stage], (t / STAGES) & 1, abort_flag));
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t kaddr = smem_u32(skv + stage * STAGE_BYTES);
                     if (elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < D / 16; ++kk)
+                        for (int kk = 0; kk < SUBK * 4; ++kk)
                             umma_bf16(s_cols + (j & 1) * AT_BN, umma_desc(qaddr + (kk / 4) * AT_BM * 128) + 2 * (kk % 4),
                                       umma_desc(kaddr + (kk / 4) * KV_SUB) + 2 * (kk % 4), idesc_qk, kk > 0 ? 1u : 0u);
                         umma_commit(&my_s_full[j & 1]);
@@ -315,11 +342,11 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 }
                 if (j >= 1) {
                     // O += P(j-1) V(j-1), P from tensor memory (where S(j-1) was)
-                    const int u = j - 1, t = me.first + u, stage = t % AT_STAGES;
+                    const int u = j - 1, t = me.first + u, stage = t % STAGES;
                     ok = __all_sync(0xffffffffu, mbar_wait(&my_p_ready[u & 1], (u >> 1) & 1, abort_flag));
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t vaddr = smem_u32(skv + stage * STAGE_BYTES + SUB * KV_SUB);
+                    const uint32_t vaddr = smem_u32(skv + stage * STAGE_BYTES + SUBK * KV_SUB);
                     if (elect_one()) {
 #pragma unroll
                         for (int ks = 0; ks < AT_BN / 16; ++ks)
@@ -623,21 +650,27 @@ static int make_map_2d(CUtensorMap* map, const void* base, long long rows, long 
     return tensor_map_2d(map, base, rows, cols, box_rows);
 }
 
-template <int D>
-int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mc, const int* block_table, int max_blocks,
+struct Expanded { CUtensorMap q2, k2; int key_origin, k2_column; };      // (DK > 0: see the head of this file)
+
+template <int D, int DK = 0>
+int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mc, const Expanded& ex, const int* block_table, int max_blocks,
                       const int* tiles, int n_tiles, const int* segments, int n_segments, const int* items, int n_items,
                       int n_slots, float* part_o, float* part_ml, void* out, int H, int K, int P, int window, float scale,
                       float softcap, int* status, cudaStream_t stream, const float* sink, const DistanceBias& bias) {
     // (more than half of an SM's shared memory, so that two blocks never share its tensor memory)
-    size_t smem = 1024 + (size_t)AT_ROW_TILES * (D / 64) * AT_BM * 128 +
-                  (size_t)AT_STAGES * 2 * (D / 64) * AT_BN * 128 + 256;
+    constexpr int SUBK = (DK ? DK : D) / 64;
+    size_t smem = 1024 + (size_t)AT_ROW_TILES * SUBK * AT_BM * 128 +
+                  (size_t)at_stages(D, DK) * (SUBK + D / 64) * AT_BN * 128 + 256;
     if (smem < 120 * 1024) smem = 120 * 1024;
-    auto kernel = bias.table ? prefill_attention_tc_kernel<D, true> : prefill_attention_tc_kernel<D, false>;
+    auto kernel = prefill_attention_tc_kernel<D, false, DK>;
+    if constexpr (DK == 0) {
+        if (bias.table) kernel = prefill_attention_tc_kernel<D, true, 0>;
+    }
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const int n_pairs = n_tiles / (AT_GROUP * AT_ROW_TILES);
     const dim3 grid = segments ? dim3(n_segments) : dim3(H, n_pairs);
-    int rc = launch(kernel, grid, AT_THREADS, smem, stream, mq, mc, block_table, max_blocks, tiles, n_pairs, segments,
+    int rc = launch(kernel, grid, AT_THREADS, smem, stream, mq, mc, ex.q2, ex.k2, ex.key_origin, ex.k2_column, block_table, max_blocks, tiles, n_pairs, segments,
                     n_slots, part_o, (float2*)part_ml, (__nv_bfloat16*)out, H, K, P, window,
                     (softcap > 0.f ? 1.f : scale) * 1.4426950408889634f, softcap > 0.f ? softcap : 0.f,
                     softcap > 0.f ? scale / softcap : 0.f, status, sink, bias);
@@ -672,10 +705,11 @@ static int prefill_attention_tc_any(const void* q, int T, const void* cache, lon
     if (rc) return rc;
     rc = make_map_2d(&mc, cache, pages * 2 * K * P, D, P < AT_BN ? P : AT_BN);
     if (rc) return rc;
+    const Expanded none{mq, mc, 0, 0};
     if (D == 64)
-        return launch_prefill_tc<64>(mq, mc, block_table, max_blocks, tiles, n_tiles, segments, n_segments, items, n_items,
+        return launch_prefill_tc<64>(mq, mc, none, block_table, max_blocks, tiles, n_tiles, segments, n_segments, items, n_items,
                                      n_slots, part_o, part_ml, out, H, K, P, window, scale, softcap, status, stream, sink, bias);
-    return launch_prefill_tc<128>(mq, mc, block_table, max_blocks, tiles, n_tiles, segments, n_segments, items, n_items,
+    return launch_prefill_tc<128>(mq, mc, none, block_table, max_blocks, tiles, n_tiles, segments, n_segments, items, n_items,
                                   n_slots, part_o, part_ml, out, H, K, P, window, scale, softcap, status, stream, sink, bias);
 }
 
@@ -700,6 +734,42 @@ AIR_API int air_prefill_attention_tc_sink(const void* q, int T, const void* cach
     return prefill_attention_tc_any(q, T, cache, pages, block_table, max_blocks, tiles, n_tiles, segments, n_segments,
                                     items, n_items, n_slots, part_o, part_ml, out, H, K, D, P, window, scale, softcap,
                                     status, sink, air::DistanceBias{bias, bias_n}, stream);
+}
+
+// Attention over the expansion of one request's latents: q [T, H, 128], q2 [T, H, rot] (rot 0 or 64), kv [keys, H * 256], rows
+// [keys, width] (their columns k2_column .. k2_column + rot are the keys' common part), all bf16; the first key is position
+// key_origin, a multiple of 64.  The rest as above.
+AIR_API int air_prefill_attention_expanded(const void* q, const void* q2, int T, const void* kv, const void* rows, int keys,
+                                           int width, int k2_column, int key_origin, const int* tiles, int n_tiles,
+                                           const int* segments, int n_segments, const int* items, int n_items, int n_slots,
+                                           float* part_o, float* part_ml, void* out, int H, int rot, int window, float scale,
+                                           const float* sink, int* status, cudaStream_t stream) {
+    using namespace air;
+    if (n_tiles <= 0) return 0;
+    if (segments && (n_segments <= 0 || n_items < 0 || n_slots < 0 || (n_items > 0 && !items) ||
+                     (n_slots > 0 && (!part_o || !part_ml || ((uintptr_t)part_o & 15) || ((uintptr_t)part_ml & 7)))))
+        return AIR_ERR_BAD_ARGUMENT;
+    if (!segments) n_items = n_slots = 0;
+    if (H <= 0 || keys <= 0 || (rot != 0 && rot != 64) || (rot && (!q2 || !rows || width % 8 || k2_column % 8 || k2_column + rot > width)) ||
+        key_origin < 0 || key_origin % AT_BN || n_tiles % (AT_GROUP * AT_ROW_TILES) || n_tiles / (AT_GROUP * AT_ROW_TILES) > 65535 ||
+        (((uintptr_t)q | (uintptr_t)q2 | (uintptr_t)kv | (uintptr_t)rows) & 15))
+        return AIR_ERR_BAD_ARGUMENT;
+    CUtensorMap mq, mkv;
+    int rc = make_map_2d(&mq, q, T, (long long)H * 128, AT_BM);
+    if (rc) return rc;
+    rc = make_map_2d(&mkv, kv, keys, (long long)H * 256, AT_BN);
+    if (rc) return rc;
+    Expanded ex{mq, mkv, key_origin, k2_column};
+    const DistanceBias bias{nullptr, 0};
+    if (rot == 0)
+        return launch_prefill_tc<128, 128>(mq, mkv, ex, nullptr, 0, tiles, n_tiles, segments, n_segments, items, n_items, n_slots,
+                                           part_o, part_ml, out, H, H, AT_BN, window, scale, 0.f, status, stream, sink, bias);
+    rc = make_map_2d(&ex.q2, q2, T, (long long)H * rot, AT_BM);
+    if (rc) return rc;
+    rc = make_map_2d(&ex.k2, rows, keys, width, AT_BN);
+    if (rc) return rc;
+    return launch_prefill_tc<128, 192>(mq, mkv, ex, nullptr, 0, tiles, n_tiles, segments, n_segments, items, n_items, n_slots, part_o,
+                                       part_ml, out, H, H, AT_BN, window, scale, 0.f, status, stream, sink, bias);
 }
 
 AIR_API int air_trace_set_attention_prefill_tc(unsigned long long* buffer) { return air::set_trace_here(buffer); }

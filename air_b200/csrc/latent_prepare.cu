@@ -8,7 +8,8 @@
 //   (i, i + rot/2) (pairing 0) or (2i, 2i + 1) (pairing 1);
 //   the row [c | kr] goes to the token's place in the pages ([P, R + rot] per page, no heads); the plain part of q goes
 //   to q_plain [T, H, d] (the matrix product that absorbs the key expansion reads it), the rotated part to
-//   q_full[t, h, R : R + rot] (float32; that product fills q_full[t, h, 0 : R]).  rot may be 0 (no rotated parts).
+//   q_full[t, h, R : R + rot] (float32; that product fills q_full[t, h, 0 : R]) and, rounded, to q_rot [T, H, rot] (either may
+//   be absent).  rot may be 0 (no rotated parts).
 //   Where the layer gates its heads, gate [T, ldg] holds one logit per head, and gate_out[t, h] = sigmoid(logit)
 //   (float32).
 //
@@ -27,7 +28,8 @@ latent_prepare_kernel(const float* __restrict__ q_in, int ldq, const float* __re
                       const float* __restrict__ gate_in, int ldg, const float* __restrict__ c_w, float eps, int pairing,
                       const double* __restrict__ freq, const int* __restrict__ positions,
                       const int* __restrict__ token_seq, const int* __restrict__ block_table, int max_blocks,
-                      TO* __restrict__ q_plain, float* __restrict__ q_full, TO* __restrict__ cache, int owns, int H,
+                      TO* __restrict__ q_plain, float* __restrict__ q_full, TO* __restrict__ q_rot,
+                      TO* __restrict__ cache, int owns, int H,
                       int d, int rot, int R, int P, float* __restrict__ gate_out, int* status, int vec_q, int vec_c) {
     __shared__ float cs[128], sn[128];
     __shared__ float scratch[32];
@@ -63,9 +65,17 @@ latent_prepare_kernel(const float* __restrict__ q_in, int ldq, const float* __re
         const int h = idx / half, j = idx % half;
         const int i0 = pairing ? 2 * j : j, i1 = pairing ? i0 + 1 : j + half;
         const float u = in[h * qw + d + i0], v = in[h * qw + d + i1];
-        float* dst = q_full + ((size_t)t * H + h) * (R + rot) + R;
-        dst[i0] = u * cs[j] - v * sn[j];
-        dst[i1] = v * cs[j] + u * sn[j];
+        const float a = u * cs[j] - v * sn[j], b = v * cs[j] + u * sn[j];
+        if (q_full) {
+            float* dst = q_full + ((size_t)t * H + h) * (R + rot) + R;
+            dst[i0] = a;
+            dst[i1] = b;
+        }
+        if (q_rot) {
+            TO* dst = q_rot + ((size_t)t * H + h) * rot;
+            dst[i0] = from_float<TO>(a);
+            dst[i1] = from_float<TO>(b);
+        }
     }
     if (gate_out)
         for (int h = threadIdx.x; h < H; h += blockDim.x)
@@ -150,7 +160,7 @@ band_rmsnorm_kernel(const float* __restrict__ x, int ld, const float* __restrict
 
 AIR_API int air_latent_prepare(const float* q, int ldq, const float* c, int ldc, const float* gate, int ldg, const float* c_w,
                                float eps, const double* freq, int pairing, const int* positions, const int* token_seq,
-                               const int* block_table, int max_blocks, void* q_plain, float* q_full, void* cache,
+                               const int* block_table, int max_blocks, void* q_plain, float* q_full, void* q_rot, void* cache,
                                int out_dtype, int owns, int T, int H, int d, int rot, int R, int P, float* gate_out,
                                int* status, cudaStream_t stream) {
     if (T <= 0) return 0;
@@ -161,7 +171,7 @@ AIR_API int air_latent_prepare(const float* q, int ldq, const float* c, int ldc,
     const int vec_c = R % 4 == 0 && rot % 4 == 0 && ldc % 4 == 0 && (((uintptr_t)c | (uintptr_t)c_w | (uintptr_t)cache) & 15) == 0;
     AIR_DISPATCH(out_dtype, TO, return air::launch(air::latent_prepare_kernel<TO>, T, 256, 0, stream, q, ldq, c, ldc, gate,
                                                    ldg, c_w, eps, pairing, freq, positions, token_seq, block_table,
-                                                   max_blocks, (TO*)q_plain, q_full, (TO*)cache, owns, H, d, rot, R, P,
+                                                   max_blocks, (TO*)q_plain, q_full, (TO*)q_rot, (TO*)cache, owns, H, d, rot, R, P,
                                                    gate_out, status, vec_q, vec_c));
     return 0;
 }

@@ -55,8 +55,11 @@ _SIGNATURES = {
                              [c_void_p, c_int, c_void_p, c_int] + [c_void_p] * 5 + [c_int] * 4 + [c_float] * 3 +
                              [c_void_p],
     "air_latent_prepare": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_void_p, c_int, c_void_p,
-                           c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                           c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                            c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
+    "air_prefill_attention_expanded": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int,
+                                       c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                                       c_int, c_float, c_void_p, c_void_p, c_void_p],
     "air_band_rmsnorm": [c_void_p, c_int, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "air_split_bands": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p],
     "air_grouped_attention": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -842,12 +845,13 @@ def mlstm_portions(x, z, columns, i_bias, f_bias, weight, S, n, m, out, portions
 
 
 def latent_prepare(q, c, c_weight, eps, freq, positions, token_seq, block_table, q_plain, q_full, cache, owns,
-                   status=None, gate=None, gate_out=None, pairing="half"):
+                   status=None, gate=None, gate_out=None, pairing="half", q_rot=None):
     """From the projections of a latent-attention layer, q float32 [T, H (d + rot)] and (where owns) c float32
     [T, R + rot] (both may be bands of columns), to q_plain [T, H, d] (the cache's type), the rotated parts in
     q_full[:, :, R:] (float32 [T, H, R + rot]) and, where owns, the row [rms(c) * c_weight | rotated kr] in the pages
     (cache [pages, P, R + rot]).  freq None: nothing is rotated (rot = 0); pairing "half": element i turns with i + rot/2,
-    "neighbours": 2i with 2i + 1.  gate_out float32 [T, H] = sigmoid(gate), gate float32 [T, H] (may be a band)."""
+    "neighbours": 2i with 2i + 1.  gate_out float32 [T, H] = sigmoid(gate), gate float32 [T, H] (may be a band).  q_rot (the
+    cache's type, [T, H, rot]): receives the rotated parts as well; q_full may then be None."""
     T, H, d = q_plain.shape
     P, width = cache.shape[1], cache.shape[2]
     rot = 2 * freq.numel() if freq is not None else 0
@@ -876,12 +880,17 @@ def latent_prepare(q, c, c_weight, eps, freq, positions, token_seq, block_table,
     _req(token_seq, "token_seq", _I32, (T,))
     _req(block_table, "block_table", _I32)
     _req(q_plain, "q_plain", _FLOATS)
-    _req(q_full, "q_full", (torch.float32,), (T, H, width))
+    if q_full is not None:
+        _req(q_full, "q_full", (torch.float32,), (T, H, width))
+    elif q_rot is None and rot:
+        raise KernelError("latent_prepare: nowhere to write the rotated parts")
+    if q_rot is not None:
+        _req(q_rot, "q_rot", (q_plain.dtype,), (T, H, rot))
     _req(cache, "cache", (q_plain.dtype,))
     _check(_get("air_latent_prepare")(
         qp, ldq, cp, ldc, gp, ldg, _ptr(c_weight), float(eps), _ptr(freq), 1 if pairing == "neighbours" else 0,
         positions.data_ptr(), token_seq.data_ptr(), block_table.data_ptr(), block_table.shape[1], q_plain.data_ptr(),
-        q_full.data_ptr(), cache.data_ptr(), _DT[q_plain.dtype], 1 if owns else 0, T, H, d, rot, R, P, _ptr(gate_out),
+        _ptr(q_full), _ptr(q_rot), cache.data_ptr(), _DT[q_plain.dtype], 1 if owns else 0, T, H, d, rot, R, P, _ptr(gate_out),
         _ptr(status), _stream()), "latent_prepare")
 
 
@@ -1743,4 +1752,44 @@ def prefill_attention_tc(q, cache, block_table, tiles, out, window, scale, statu
                "prefill_attention_tc")
     else:
         _check(_get("air_prefill_attention_tc")(*args, _stream()), "prefill_attention_tc")
+    return out
+
+
+def prefill_attention_expanded(q, q_rot, kv, rows, rank, key_origin, tiles, out, window, scale, status=None, segments=None,
+                               items=None, slots=0, scratch=None, sink=None):
+    """prefill_attention_tc over the expansion of one request's latents instead of pages: q bfloat16 [T, H, 128], q_rot [T, H, 64]
+    or None, kv [keys, H * 256] (per head 128 numbers of the key, then the value), rows [keys, width] the latents' rows, whose
+    columns rank .. rank + 64 are the part of the key that all heads share (with q_rot); the first key is position
+    key_origin, a multiple of 64.  The tile list, segments, items, scratch and sink as there."""
+    T, H, d = q.shape
+    keys = kv.shape[0]
+    rot = 0 if q_rot is None else q_rot.shape[2]
+    _req(q, "q", (torch.bfloat16,), (T, H, 128))
+    _req(kv, "kv", (torch.bfloat16,), (keys, H * 256))
+    _req(out, "out", (torch.bfloat16,), (T, H, 128))
+    _req(tiles, "tiles", _I32, (None, 4))
+    width = 0
+    if rot:
+        _req(q_rot, "q_rot", (torch.bfloat16,), (T, H, 64))
+        _req(rows, "rows", (torch.bfloat16,), (keys, None))
+        width = rows.shape[1]
+    if sink is not None:
+        _req(sink, "sink", (torch.float32,), (H,))
+    if tiles.shape[0] % TILE_PAIR:
+        raise KernelError("prefill_attention_expanded: the tile list must come in groups of 16 per request")
+    part_o = part_ml = None
+    n_items = 0
+    if segments is not None:
+        _req(segments, "segments", _I32, (None, 5))
+        if slots:
+            _req(items, "items", _I32, (None, 4))
+            n_items = items.shape[0]
+            part_o, part_ml = scratch if scratch is not None else prefill_attention_scratch(slots, d, q.device)
+            if part_o.shape[0] < slots or part_ml.shape[0] < slots:
+                raise KernelError("prefill_attention_expanded: the scratch tensors hold fewer slots than the segments name")
+    _check(_get("air_prefill_attention_expanded")(
+        q.data_ptr(), _ptr(q_rot), T, kv.data_ptr(), _ptr(rows) if rot else None, keys, width, int(rank), int(key_origin),
+        tiles.data_ptr(), tiles.shape[0], _ptr(segments), 0 if segments is None else segments.shape[0],
+        _ptr(items) if n_items else None, n_items, int(slots) if segments is not None else 0, _ptr(part_o), _ptr(part_ml),
+        out.data_ptr(), H, rot, int(window or 0), float(scale), _ptr(sink), _ptr(status), _stream()), "prefill_attention_expanded")
     return out

@@ -88,6 +88,25 @@ def plan_segments(key_tiles, heads: int, sms: int = 0):
     return segments, items, int(is_cut.sum())
 
 
+def portion_tiles(n: int, pos0: int, slot: int, row0: int, window):
+    """(int32 [16 * pairs, 4] = (slot, first row, its position, rows <= 16), the 64-key tiles of every pair's stream) of one
+    entry: its 16-token tiles, filled up with rows = 0 to whole pairs of row tiles (256 tokens)."""
+    pairs = -(-n // 256)
+    first = np.arange(pairs * 16, dtype=np.int32) * 16
+    rows = np.clip(n - first, 0, 16)
+    tile = np.zeros((pairs * 16, 4), dtype=np.int32)
+    tile[:, 0] = slot
+    tile[:, 1] = np.where(rows > 0, row0 + first, 0)
+    tile[:, 2] = np.where(rows > 0, pos0 + first, 0)
+    tile[:, 3] = rows
+    key_tiles = []
+    for g0 in range(0, n, 256):
+        # the pair's keys: from the first one that its first row sees to its last row's own
+        lowest = max(0, pos0 + g0 - window + 1) if window else 0
+        key_tiles.append((pos0 + min(n, g0 + 256) - 1) // 64 + 1 - lowest // 64)
+    return tile, key_tiles
+
+
 class TiledAttention:
     """What mixers that attend over paged keys and values of one size (PagedKV pages [2, K, P, d]) share: the plan of
     a step's tiles, worked out on the host once for all such layers, and the choice of the attention kernel.  The
@@ -113,20 +132,9 @@ class TiledAttention:
             prefix += 1
         tiles, key_tiles = [], []
         for i in range(prefix, len(batch.counts)):
-            n, pos0 = batch.counts[i], batch.lengths[i]
-            pairs = -(-n // 256)
-            first = np.arange(pairs * 16, dtype=np.int32) * 16          # the entry's 16-token tiles, pairs filled up
-            rows = np.clip(n - first, 0, 16)
-            tile = np.zeros((pairs * 16, 4), dtype=np.int32)
-            tile[:, 0] = batch.slots[i]
-            tile[:, 1] = np.where(rows > 0, batch.q_start[i] + first, 0)
-            tile[:, 2] = np.where(rows > 0, pos0 + first, 0)
-            tile[:, 3] = rows
+            tile, of_pairs = portion_tiles(batch.counts[i], batch.lengths[i], batch.slots[i], batch.q_start[i], self.window)
             tiles.append(tile)
-            for g0 in range(0, n, 256):
-                # the pair's keys: from the first one that its first row sees to its last row's own
-                lowest = max(0, pos0 + g0 - self.window + 1) if self.window else 0
-                key_tiles.append((pos0 + min(n, g0 + 256) - 1) // 64 + 1 - lowest // 64)
+            key_tiles += of_pairs
         tiles = np.concatenate(tiles) if tiles else np.zeros((0, 4), dtype=np.int32)
         arrays, values = {"tiles": tiles}, {"decode_prefix": prefix, "segments": None, "items": None, "slots": 0}
         cut = plan_segments(key_tiles, self.heads)

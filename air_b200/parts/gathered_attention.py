@@ -67,7 +67,7 @@ class PortionAttention:
         sinks = getattr(self, "sinks", None)
         softcap = float(getattr(self, "softcap", 0.0) or 0.0)
         bias = getattr(self, "bias_table", None)
-        plan = ctx.plans.get((self.PLAN,)) if not self.rt.is_fp32 else None
+        plan = ctx.plans.get(self.plan_key()) if not self.rt.is_fp32 else None
 
         def through_the_pages(token_seq):
             if (pages is not None and not latent and not self.chunk and q.dtype == torch.bfloat16
@@ -90,11 +90,13 @@ class PortionAttention:
             if gate is not None:
                 ops.sigmoid_gate(out.view(out.shape[0], -1), gate, token_seq)
 
-        if plan is None or not plan.portions:
+        if plan is None:
             through_the_pages(ctx.token_seq)
             return out
         if plan.small:
             through_the_pages(plan.small_seq)
+        if not plan.portions:
+            return out
         T, H, dk = q.shape
         dv, G = out.shape[2], kv_heads
         J = H // G

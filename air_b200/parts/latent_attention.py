@@ -6,7 +6,8 @@ import torch
 from ..config.model_config import ConfigError
 from ..csrc import ops
 from ..weights.loader import TensorSpec
-from .base import Mixer, PagedLatent
+from .attention import plan_segments, portion_tiles
+from .base import HostBatch, Mixer, PagedLatent, Plan
 from .gathered_attention import PortionAttention
 from .linear import Linear
 from .registry import register_mixer, POSITION_ENCODINGS
@@ -23,10 +24,16 @@ class LatentAttention(PortionAttention, Mixer):
     denominator has one more term exp(sink_h), a learned number per head without key or value.  With head_gate head
     h's output is multiplied by sigmoid(Wg x)_h, one more projection of the layer's input.
 
-    The key and value expansions are never applied to the cache: q_plain is carried through Wuk_h once per query
+    Single tokens and short portions never expand the cache: q_plain is carried through Wuk_h once per query
     (q'_h = Wuk_h^T q_plain_h, so that q_plain . Wuk_h c = q'_h . c), every head then attends over the same rows [c | kr]
     with the query [q'_h | q_rot_h] and sums the rows' first kv_rank elements, and Wuv_h expands that sum.  The two
     small products per head are one grouped product each.
+
+    In a bfloat16 engine a portion of EXPAND tokens or more is the other way round (heads of 128, a rotated part of 64 or none):
+    the request's latents that it sees are expanded once, [keys, heads x (key | value)], one library product, and the
+    tcgen05 attention kernel of the dense decoder takes keys of 128 + 64 and values of 128 from there.  A pair of a query and
+    a key then costs 128 + 64 + 128 multiply-adds per head instead of 512 + 64 + 512, which the expansion repays from a few dozen
+    queries on, and the scores stay in tensor memory.
 
     params: hidden, heads, head_dim, rot_dim, v_dim, kv_rank, q_rank (0: none), scale, window, eps, sink, head_gate, position (rope_live
     with rotary_dim = rot_dim; absent where rot_dim is 0), borrows (the layer has no Wdkv: its run reads the rows that another layer's run keeps), keep (the
@@ -37,6 +44,9 @@ class LatentAttention(PortionAttention, Mixer):
     hidden] where head_gate."""
 
     graph_safe = True
+
+    EXPAND = 64                  # tokens of a portion from which its keys are expanded
+    EXPANDED_BYTES = 1 << 30     # and the most that the expansion may take; longer contexts stay compressed
 
     def __init__(self, spec, prefix=""):
         super().__init__(spec, prefix)
@@ -104,6 +114,10 @@ class LatentAttention(PortionAttention, Mixer):
         # Wuk_h [d, R] is the product's [K, N]: the grouped product wants [N, K] per head
         self.uk_t = tensors[p + "uk"].view(H, d, R).transpose(1, 2).contiguous()
         self.uv = tensors[p + "uv"].view(H, self.v_dim, R).contiguous()
+        # both expansions head by head, [heads x (d + v_dim), R], for portions (a tuple: the matrices above once more)
+        self.expansion = ()
+        if self.expands:
+            self.expansion = (torch.cat([tensors[p + "uk"].view(H, d, R), self.uv], dim=1).reshape(-1, R).contiguous(),)
         self.o = Linear(tensors[p + "o"], rt.status)
         if self.position is not None:
             self.position.load(tensors, rt)
@@ -111,6 +125,55 @@ class LatentAttention(PortionAttention, Mixer):
                 raise ConfigError("unsupported", "latent attention takes a rotation with 64-bit frequencies and no magnitude")
             if self.position.rotary_dim != self.rot_dim:
                 raise ConfigError("data_error", "latent attention: the rotation covers the rotated part, all of it")
+
+    @property
+    def expands(self) -> bool:
+        return (self.rt.dtype == torch.bfloat16 and self.head_dim == 128 and self.v_dim == 128 and self.rot_dim in (0, 64)
+                and self.rank % 8 == 0)
+
+    def plan_key(self):
+        key = super().plan_key()
+        return key + ("expanded", self.heads, self.window) if key is not None and self.expands else key
+
+    def plan(self, batch: HostBatch) -> Plan:
+        """PortionAttention's plan; where this layer expands, the portions that it expands are in `expanded` instead: (first
+        row, tokens, first position, slot, number of slots of partial sums), their tile lists in tiles<i>, segments<i> and
+        items<i> as TiledAttention.plan has them.  rows: how many of the step's leading rows the other roads need (all of them
+        up to the last row that is not in an expanded portion)."""
+        plan = super().plan(batch)
+        if not self.expands:
+            return plan
+        expanded, kept = [], []
+        for r0, n, pos0, slot in plan.values["portions"]:
+            keys = pos0 + n - self.first_visible(pos0)
+            if n < self.EXPAND or keys * self.heads * 512 > self.EXPANDED_BYTES:
+                kept.append((r0, n, pos0, slot))
+                continue
+            tiles, key_tiles = portion_tiles(n, pos0, slot, r0, self.window)
+            cut = plan_segments(key_tiles, self.heads)
+            i, slots = len(expanded), 0
+            plan.arrays[f"tiles{i}"] = tiles
+            if cut is not None:
+                plan.arrays[f"segments{i}"], plan.arrays[f"items{i}"], slots = cut
+            expanded.append((r0, n, pos0, slot, slots))
+        taken = {r0 for r0, *_ in expanded}
+        rows = max((batch.q_start[i + 1] for i, r0 in enumerate(batch.q_start[:-1]) if r0 not in taken), default=0)
+        plan.values.update(portions=kept, expanded=expanded, rows=rows)
+        return plan
+
+    def _attend_expanded(self, plan, q, q_rot, latent, bt, ctx, out):
+        """out rows of the plan's expanded portions."""
+        for i, (r0, n, pos0, slot, slots) in enumerate(plan.expanded):
+            lo = self.first_visible(pos0) // 64 * 64
+            count = pos0 + n - lo
+            keys = -(-count // 16) * 16
+            rows = torch.empty((1, keys, self.rank + self.rot_dim), dtype=torch.bfloat16, device=q.device)
+            ops.gather_keys(latent.rows, bt[slot], lo, count, rows, None, latent=True)
+            kv = torch.mm(rows[0, :, :self.rank], self.expansion[0].t())
+            cut = getattr(plan, f"segments{i}", None)
+            ops.prefill_attention_expanded(q, q_rot, kv, rows[0], self.rank, lo, getattr(plan, f"tiles{i}"), out, self.window,
+                                           self.scale, status=ctx.status, segments=cut, items=getattr(plan, f"items{i}", None),
+                                           slots=slots, sink=self.sinks)
 
     @staticmethod
     def _expansion(w, rt):
@@ -141,20 +204,30 @@ class LatentAttention(PortionAttention, Mixer):
         dev = x.device
         bt = ctx.block_tables[latent.group]
         proj = self.proj.f32(x)
+        plan = ctx.plans.get(self.plan_key()) if self.expands else None
+        expanded = plan is not None and bool(plan.expanded)
+        rows = plan.rows if expanded else T         # of the step, from its first on, that the other roads need
         q_plain = torch.empty((T, H, d), dtype=rt.dtype, device=dev)
-        q_full = torch.empty((T, H, R + rot), dtype=torch.float32, device=dev)
+        q_full = torch.empty((T, H, R + rot), dtype=torch.float32, device=dev) if rows else None
+        q_rot = torch.empty((T, H, rot), dtype=rt.dtype, device=dev) if expanded and rot else None
         gate = torch.empty((T, H), dtype=torch.float32, device=dev) if self.head_gate else None
         pos = self.position
         ops.latent_prepare(self._queries(proj), proj[:, self.c_column:self.c_column + R + rot] if owns_cache else None,
                            self.c_weight, self.eps, pos.frequencies64() if pos is not None else None, ctx.positions,
                            ctx.token_seq, bt, q_plain, q_full, latent.rows, owns_cache, status=ctx.status,
                            gate=proj[:, self.gate_column:self.gate_column + H] if gate is not None else None,
-                           gate_out=gate, pairing=pos.pairing if pos is not None else "half")
-        ops.grouped_gemm(q_plain, self.uk_t, q_full, R, d, lda=H * d, ldo=H * (R + rot), groups=H, a_group_stride=d,
-                         o_group_stride=R + rot, a_local=True, o_local=True, rows_per_group=T)
-        summed = torch.empty((T, H, R), dtype=rt.dtype, device=dev)
-        self.attend(q_full, latent.rows, bt, ctx, summed, latent=True)
+                           gate_out=gate, pairing=pos.pairing if pos is not None else "half", q_rot=q_rot)
         out = torch.empty((T, H, dv), dtype=rt.dtype, device=dev)
-        ops.grouped_gemm(summed, self.uv, out, dv, R, lda=H * R, ldo=H * dv, groups=H, a_group_stride=R,
-                         o_group_stride=dv, a_local=True, o_local=True, rows_per_group=T, o_scale=gate, o_scale_ld=H)
+        if rows:
+            ops.grouped_gemm(q_plain, self.uk_t, q_full, R, d, lda=H * d, ldo=H * (R + rot), groups=H, a_group_stride=d,
+                             o_group_stride=R + rot, a_local=True, o_local=True, rows_per_group=rows)
+            summed = torch.empty((T, H, R), dtype=rt.dtype, device=dev)
+            self.attend(q_full, latent.rows, bt, ctx, summed, latent=True)
+            ops.grouped_gemm(summed, self.uv, out, dv, R, lda=H * R, ldo=H * dv, groups=H, a_group_stride=R,
+                             o_group_stride=dv, a_local=True, o_local=True, rows_per_group=rows, o_scale=gate, o_scale_ld=H)
+        if expanded:      # (behind the other roads' products, which write all of the leading rows)
+            self._attend_expanded(plan, q_plain, q_rot, latent, bt, ctx, out)
+            if gate is not None:
+                for r0, n, *_ in plan.expanded:
+                    ops.head_gate(out[r0:r0 + n], gate[r0:r0 + n], ctx.token_seq[r0:r0 + n])
         return self.o.f32_sums(out.view(T, H * dv))

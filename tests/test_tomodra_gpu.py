@@ -559,3 +559,45 @@ def test_expert_stream_against_64_bit_products(T, top, n, E, F, splits):
         want = down[e].double() @ act[s].double() * weight[t, c].double()
         got = y.view(splits, top, T, E)[:, c, t].double().sum(0)
         assert (got - want).abs().max() <= 3e-6 * (down[e].double().abs() @ act[s].double().abs()).max()
+
+
+@pytest.mark.parametrize("H,rot,window,n,pos0,sink", [(3, 64, None, 64, 0, False), (2, 64, None, 300, 0, True), (1, 0, None, 257, 100, True),
+                                                      (2, 64, 70, 200, 333, False), (4, 0, 130, 65, 0, False),
+                                                      (2, 64, None, 70, 6000, True), (2, 64, 2000, 129, 5000, False)])
+def test_attention_over_expanded_latents(H, rot, window, n, pos0, sink):
+    """A portion's attention over keys and values expanded from latents: tiles with remainders, a prefix, windows, the keys'
+    common part, sinks, and streams of keys that are cut into segments."""
+    from air_b200.csrc import ops
+    from air_b200.parts.attention import plan_segments, portion_tiles
+    g = torch.Generator(device="cuda").manual_seed(n + pos0)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    lo = max(0, pos0 - window + 1) // 64 * 64 if window else 0
+    keys, rank, row0 = pos0 + n - lo, 40, 5
+    kv, rows, q = rand(keys, H * 256), rand(keys, rank + rot), rand(row0 + n + 3, H, 128)
+    q_rot = rand(row0 + n + 3, H, rot) if rot else None
+    sinks = torch.randn(H, generator=g, device="cuda") * 3 if sink else None
+    tiles, key_tiles = portion_tiles(n, pos0, 0, row0, window)
+    cut = plan_segments(key_tiles, H)
+    assert (cut is not None) == (pos0 >= 5000), "the long prefixes are cut"
+    on = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    more = {} if cut is None else dict(segments=on(cut[0]), items=on(cut[1]), slots=cut[2])
+    out, status = torch.full((row0 + n + 3, H, 128), 7.0, device="cuda").bfloat16(), torch.zeros(1, dtype=torch.int32, device="cuda")
+    scale = (128 + rot) ** -0.5
+    ops.prefill_attention_expanded(q, q_rot, kv, rows, rank, lo, on(tiles), out, window, scale, status=status, sink=sinks, **more)
+    assert status.item() == 0
+    assert (out[:row0] == 7).all() and (out[row0 + n:] == 7).all(), "rows outside the portion are not touched"
+    position = torch.arange(pos0, pos0 + n, device="cuda")[:, None]
+    key = torch.arange(lo, pos0 + n, device="cuda")[None]
+    seen = (key <= position) & (key > position - window if window else True)
+    for h in range(H):
+        k, v = kv[:, h * 256:h * 256 + 128].double(), kv[:, h * 256 + 128:(h + 1) * 256].double()
+        s = q[row0:row0 + n, h].double() @ k.t()
+        if rot:
+            s += q_rot[row0:row0 + n, h].double() @ rows[:, rank:].double().t()
+        s = (s * scale).masked_fill(~seen, -float("inf"))
+        if sink:
+            s = torch.cat([s, sinks[h].double().expand(n, 1)], dim=1)
+            v = torch.cat([v, torch.zeros(1, 128, dtype=torch.float64, device="cuda")])
+        want = torch.softmax(s, dim=1) @ v
+        # (the weights are rounded to bfloat16 and so is the result: 2^-8 of sums of values of unit size)
+        assert (out[row0:row0 + n, h].double() - want).abs().max() < 0.01 * max(1.0, want.abs().max().item()), h
