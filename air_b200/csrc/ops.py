@@ -546,7 +546,9 @@ def grouped_attention(q, cache, block_table, token_seq, positions, out, window, 
         # float32: always the same number, so that a row's sums do not depend on what else is in the batch;
         # bfloat16: as many as fill the device
         blocks = T * G * -(-J // (16 if J > 4 else 4))
-        splits = 4 if cache.dtype == torch.float32 else max(1, min(16, 296 // max(1, blocks)))
+        # (rows of which a block's two stages of 64, and its queries, leave no room for a second block: one per SM)
+        wide = 256 * (d + 8 + (0 if latent else dv + 8)) + 64 * (d + 8) > 100 * 1024
+        splits = 4 if cache.dtype == torch.float32 else max(1, min(16, (148 if wide else 296) // max(1, blocks)))
     part = torch.empty((T, H, splits, dv + 2), dtype=torch.float32, device=q.device)
     _check(_get("air_grouped_attention")(
         q.data_ptr(), 1 if q.dtype == torch.float32 else 0, cache.data_ptr(), _DT[cache.dtype], block_table.data_ptr(),
