@@ -38,7 +38,8 @@ def choose_tile(out_features: int, in_features: int, may_split: bool = True):
                 continue
             blocks = -(-out_features // bn) * s
             eff = blocks / (-(-blocks // SMS) * SMS)
-            score = eff - 0.02 * s - (0.05 if bn == 32 else 0.0)
+            # (a share of what is gained, so that a matrix of one or two tiles, a router's, is split as far as it goes)
+            score = eff * (1.0 - 0.02 * s) - (0.05 if bn == 32 else 0.0)
             if best is None or score > best[0] + 1e-9:
                 best = (score, bn, s)
     return best[1], best[2]
