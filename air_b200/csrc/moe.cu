@@ -38,8 +38,12 @@ moe_route_kernel(const float* __restrict__ z, int parts, int ld, int T, int n, i
     // (the logits may be partial sums over parts of k, added in order: [parts, T, ld])
     const float* row = z + (size_t)t * ld;
     auto logit = [&](int e) {
-        float v = row[e];
-        for (int i = 1; i < parts; ++i) v += row[(size_t)i * T * ld + e];
+        float part[8], v = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[i] = i < parts ? row[(size_t)i * T * ld + e] : 0.f;      // (all under way at once)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v += part[i];
+        for (int i = 8; i < parts; ++i) v += row[(size_t)i * T * ld + e];
         return v;
     };
     float s[MOE_MAX_PER_LANE];

@@ -29,6 +29,7 @@ namespace air {
 
 constexpr int CONV_MAX_TAPS = 16;
 constexpr int CONV_THREADS = 128;
+constexpr int CONV_AHEAD = 8;
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.f + expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
@@ -69,8 +70,7 @@ short_conv_silu_kernel(const float* __restrict__ x, int ld, const float* __restr
             win[j] = idx >= 0 ? x[(size_t)(q0 + idx) * ld + c] : st[keep + idx];
         }
     }
-    for (int t = t0; t < t1; ++t) {
-        const float cur = x[(size_t)(q0 + t) * ld + c];
+    auto take = [&](int t, float cur) {
         float acc = wv[M - 1] * cur;
 #pragma unroll
         for (int j = 0; j < M - 1; ++j)
@@ -79,7 +79,17 @@ short_conv_silu_kernel(const float* __restrict__ x, int ld, const float* __restr
 #pragma unroll
         for (int j = 0; j < M - 2; ++j) win[j] = win[j + 1];
         win[M - 2] = cur;
+    };
+    // (CONV_AHEAD tokens' inputs are asked for before any of them is used: CONV_MEASURED)
+    int t = t0;
+    for (; t + CONV_AHEAD <= t1; t += CONV_AHEAD) {
+        float cur[CONV_AHEAD];
+#pragma unroll
+        for (int i = 0; i < CONV_AHEAD; ++i) cur[i] = x[(size_t)(q0 + t + i) * ld + c];
+#pragma unroll
+        for (int i = 0; i < CONV_AHEAD; ++i) take(t + i, cur[i]);
     }
+    for (; t < t1; ++t) take(t, x[(size_t)(q0 + t) * ld + c]);
     if (blockIdx.z == 0) {
         // The state after the portion: its last taps - 1 inputs.  A portion that this thread has taken whole leaves
         // them in the window (older ones from the state as it was included); a longer one has them all among its tokens
