@@ -236,7 +236,7 @@ grouped_attention_kernel(const void* __restrict__ q_any, int q_f32, const T* __r
 // of the queries from shared memory for every tile, 300 KB where the keys are 74, in one chain of 72 products: 9 us a tile.)
 // Weighted values: warp w takes the columns' eighth w; the values' fragments come transposed out of the staged rows
 // (ldmatrix.trans).  Where a row lies is worked out once per key, a tile ahead of its copies.
-// Measured, rows of 576 (values 512), 32 heads, 8 single tokens over 4,096 keys: 75 us + 17 for the merge -> 49 + 8.
+// Measured, rows of 576 (values 512), 32 heads, 8 single tokens over 4,096 keys: 75 us + 17 for the merge -> 43 + 8.
 constexpr int GT_MAX_NT = 16;      // 8-column tiles of the values per warp: dv up to 1024
 constexpr int GT_RLD = GA_KT + 8;  // (rows 8 numbers apart: the halves of a warp's 64-bit stores fall into different banks)
 
@@ -256,8 +256,10 @@ __device__ __forceinline__ void split_bf16(float v, __nv_bfloat16& hi, __nv_bflo
 }
 
 // MAX_NT: 8-column tiles of the values that a warp has room for; MAX_KS: its share of the steps of 16 of d
-template <int MAX_NT, int MAX_KS>
-__global__ void __launch_bounds__(256)
+// WARPS: 8, or 16 of which every eight take half of a tile's keys (a tile is some 1,400 instructions for each of 8 warps, of which
+// two to a scheduler hide little: 49 us with 8, 43 with 16, measured as above)
+template <int MAX_NT, int MAX_KS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __nv_bfloat16* __restrict__ cache,
                             const int* __restrict__ block_table, int max_blocks, const int* __restrict__ token_seq,
                             const int* __restrict__ positions, float* __restrict__ part, int H, int G, int d, int dv,
@@ -285,7 +287,7 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
     __nv_bfloat16* K0 = Pl + JB * PLD;                        // per stage: keys [64][kld], then values [64][vld]
     const int stage_elems = GA_KT * kld + (latent ? 0 : GA_KT * vld);
     if (tid < JB) { mrun[tid] = -INFINITY; lrun[tid] = 0.f; }
-    const int ntiles = (dv + 7) / 8, per_warp = (ntiles + 7) / 8;      // 8-column tiles of the values, and a warp's share
+    const int ntiles = (dv + 7) / 8, per_warp = (ntiles + WARPS - 1) / WARPS;      // 8-column tiles of the values, and a warp's share
     const int nt0 = warp * per_warp;
     float acc[MAX_NT][4];
 #pragma unroll
@@ -299,7 +301,9 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
     // ldmatrix.x4 of a 16 x 16 block of A (rows = heads): lane l gives the address of row l % 16, columns 8 (l / 16) ..
     const int a_row = lane & 15, a_col = (lane >> 4) * 8;
     // This warp's share of d, and its part of the queries: rows gq and gq + 8, columns 2 tq, 2 tq + 1 and 8 further on.
-    const int steps = d / 16, ks0 = steps * warp / 8, my_steps = steps * (warp + 1) / 8 - ks0;
+    const int share = warp & 7, steps = d / 16, ks0 = steps * share / 8, my_steps = steps * (share + 1) / 8 - ks0;
+    constexpr int KN = 8 / (WARPS / 8);                       // 8-key tiles of scores that a warp takes, from n0 on
+    const int n0 = (warp >> 3) * KN;
     uint32_t qh[MAX_KS][4], ql[MAX_KS][4];
 #pragma unroll
     for (int x = 0; x < MAX_KS; ++x)
@@ -330,14 +334,14 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
         __nv_bfloat16* Vt = Kt + GA_KT * kld;
         const long long* at = rows + list * GA_KT;
 #pragma unroll 4
-        for (int r = warp; r < GA_KT; r += 8) {
+        for (int r = warp; r < GA_KT; r += WARPS) {
             const bool in = at[r] >= 0;
             const __nv_bfloat16* row = cache + (in ? at[r] : 0);
             for (int c = lane; c < kchunks; c += 32) cp_async16(Kt + r * kld + c * 8, row + c * 8, in);
         }
         if (!latent)
 #pragma unroll 4
-            for (int r = warp; r < GA_KT; r += 8) {
+            for (int r = warp; r < GA_KT; r += WARPS) {
                 // (a page's keys [G, P, d], then its values [G, P, dv]: the row's index among the keys is its index there)
                 const bool in = at[r] >= 0;
                 const long long page = in ? at[r] / (long long)page_stride * (long long)page_stride : 0;
@@ -379,15 +383,15 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
         const uint32_t vt_addr = (uint32_t)__cvta_generic_to_shared(latent ? Kt : Kt + GA_KT * kld);
         {   // scores of all 64 keys over this warp's share of d: lane l gives the address of key l % 8 (+ 8 for the second pair of
             // matrices) at column 8 (l / 8 % 2) of the step
-            float c[8][4];
+            float c[KN][4];
 #pragma unroll
-            for (int n = 0; n < 8; ++n) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
-            const uint32_t mine = kt_addr + (((lane & 7) + 8 * (lane >> 4)) * kld + ks0 * 16 + ((lane >> 3) & 1) * 8) * 2;
+            for (int n = 0; n < KN; ++n) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
+            const uint32_t mine = kt_addr + ((8 * n0 + (lane & 7) + 8 * (lane >> 4)) * kld + ks0 * 16 + ((lane >> 3) & 1) * 8) * 2;
 #pragma unroll
             for (int x = 0; x < MAX_KS; ++x) {
                 if (x >= my_steps) break;
 #pragma unroll
-                for (int n = 0; n < 8; n += 2) {
+                for (int n = 0; n < KN; n += 2) {
                     uint32_t b[4];
                     ldmatrix_x4(b, mine + (8 * n * kld + 16 * x) * 2);
                     mma_bf16_16816(c[n], qh[x][0], qh[x][1], qh[x][2], qh[x][3], b[0], b[1]);
@@ -398,17 +402,17 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
                     }
                 }
             }
-            float* r0 = R + (warp * JB + gq) * GT_RLD + 2 * tq;
+            float* r0 = R + (share * JB + gq) * GT_RLD + 8 * n0 + 2 * tq;
 #pragma unroll
-            for (int n = 0; n < 8; ++n) {
+            for (int n = 0; n < KN; ++n) {
                 *reinterpret_cast<float2*>(r0 + 8 * n) = make_float2(c[n][0], c[n][1]);
                 *reinterpret_cast<float2*>(r0 + 8 * GT_RLD + 8 * n) = make_float2(c[n][2], c[n][3]);
             }
         }
         __syncthreads();
 #pragma unroll
-        for (int jj = 0; jj < JB / 8; ++jj) {              // (the heads' chains side by side)
-            const int j = warp + 8 * jj;
+        for (int jj = 0; jj < JB / WARPS; ++jj) {          // (the heads' chains side by side)
+            const int j = warp + WARPS * jj;
             const bool seen0 = key0 + lane >= lo && key0 + lane <= pos, seen1 = key0 + lane + 32 >= lo && key0 + lane + 32 <= pos;
             float s0 = 0.f, s1 = 0.f;
 #pragma unroll
@@ -594,11 +598,11 @@ AIR_API int air_grouped_attention(const void* q, int q_f32, const void* cache, i
         const int stages = fixed + 2 * stage <= 227 * 1024 ? 2 : 1;
         const size_t smem = fixed + stages * stage;
         if (smem <= 227 * 1024) {
-            auto kernel = dv <= 512 && d <= 640 ? air::grouped_attention_tc_kernel<8, 5>
-                                                : air::grouped_attention_tc_kernel<air::GT_MAX_NT, 10>;
+            const bool most = dv <= 512 && d <= 640;
+            auto kernel = most ? air::grouped_attention_tc_kernel<4, 5, 16> : air::grouped_attention_tc_kernel<air::GT_MAX_NT, 10, 8>;
             if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             dim3 grid(T, G * ((J + 15) / 16), splits);
-            rc = air::launch(kernel, grid, 256, smem, stream, q, q_f32, (const __nv_bfloat16*)cache, block_table,
+            rc = air::launch(kernel, grid, most ? 512 : 256, smem, stream, q, q_f32, (const __nv_bfloat16*)cache, block_table,
                              max_blocks, token_seq, positions, part, H, G, d, dv, P, window, mask_mode, scale, softcap, latent,
                              splits, stages, bias);
             if (rc) return rc;
