@@ -118,6 +118,14 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
     const int per = (tile1 - tile0 + splits - 1) / splits;
     const int begin = tile0 + split * per, end = min(tile1, begin + per);
     const int n_tiles = max(0, end - begin);
+    if (splits > 1 && n_tiles == 0) {
+        // No key of the request falls to this split (a captured step has as many splits as a long context wants): the merge
+        // hears so, and the q/k/v product's sums are left to the blocks that need them.
+        const int r = hb * 16 + threadIdx.x;
+        if (threadIdx.x < 16 && r < G)
+            *reinterpret_cast<float2*>(part_ml + (((size_t)t * H + kvh * G + r) * splits + split) * 2) = make_float2(-INFINITY, 0.f);
+        return;
+    }
 
     float o[NT][4];
 #pragma unroll
@@ -406,9 +414,8 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
                 sm_o[(warp * 16 + g + 8 * (e >> 1)) * D + 8 * n + 2 * tq + (e & 1)] = o[n][e];
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < 16 * D; idx += DT_THREADS) {
+    for (int idx = threadIdx.x; idx < min(16, G - hb * 16) * D; idx += DT_THREADS) {
         const int r = idx / D, col = idx % D;
-        if (hb * 16 + r >= G) continue;
         float mm = -INFINITY;
 #pragma unroll
         for (int w = 0; w < DT_CONSUMERS; ++w) mm = fmaxf(mm, sm_m[w * 16 + r]);
