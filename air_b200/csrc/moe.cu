@@ -261,6 +261,26 @@ planes_by_index_kernel(const T* __restrict__ rows, const int* __restrict__ index
     for (int i = threadIdx.x; i < E; i += blockDim.x) dst[i] = to_float(rows[(size_t)s * E + i]) * m;
 }
 
+// The same for bfloat16 rows of whole 16-byte pieces.
+__global__ void __launch_bounds__(256)
+planes_by_index_vec_kernel(const uint4* __restrict__ rows, const int* __restrict__ index, int div, size_t plane,
+                           const float* __restrict__ scale, float* __restrict__ out, int pieces) {
+    pdl_enter(TR_MOE_SORT);
+    const int s = blockIdx.x, p = index[s];
+    if (p < 0) return;
+    const float m = scale ? scale[p] : 1.f;
+    float* dst = out + (size_t)(p % div) * plane + (size_t)(p / div) * pieces * 8;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < pieces; i += 256) {
+        const uint4 v = rows[(size_t)s * pieces + i];
+        const __nv_bfloat162* two = reinterpret_cast<const __nv_bfloat162*>(&v);
+        const float a[4] = {__low2float(two[0]) * m, __high2float(two[0]) * m, __low2float(two[1]) * m, __high2float(two[1]) * m};
+        const float b[4] = {__low2float(two[2]) * m, __high2float(two[2]) * m, __low2float(two[3]) * m, __high2float(two[3]) * m};
+        store4(dst + 8 * i, a);
+        store4(dst + 8 * i + 4, b);
+    }
+}
+
 }  // namespace air
 
 AIR_API int air_rows_by_index(const void* x, int dtype, const int* index, int div, const float* scale, void* out,
@@ -279,6 +299,9 @@ AIR_API int air_planes_by_index(const void* rows, int dtype, const int* index, i
                                 const float* scale, float* out, int n, int E, cudaStream_t stream) {
     if (n <= 0) return 0;
     if (div <= 0) return AIR_ERR_BAD_ARGUMENT;
+    if (dtype == AIR_BF16 && E % 8 == 0 && plane % 4 == 0 && (((uintptr_t)rows | (uintptr_t)out) & 15) == 0)
+        return air::launch(air::planes_by_index_vec_kernel, n, 256, 0, stream, (const uint4*)rows, index, div, (size_t)plane, scale,
+                           out, E / 8);
     AIR_DISPATCH(dtype, TT, return air::launch(air::planes_by_index_kernel<TT>, n, 256, 0, stream, (const TT*)rows, index,
                                                div, (size_t)plane, scale, out, E));
     return 0;

@@ -163,7 +163,8 @@ class RoutedExperts(FeedForward):
                       norm_eps=self.norm_eps, choice_bias=self.correction, mark=self.group_mark)
         on_input = self.weight_on == "input"
         pairs = T * top
-        ints = torch.empty(n + 1 + pairs + 2 * (pairs // ops.GROUP_TILE + n) + 1, dtype=torch.int32, device=dev)
+        # (three numbers ahead of `start`, so that the experts' ends, start[1:], lie on a 16-byte boundary)
+        ints = torch.empty(3 + n + 1 + pairs + 2 * (pairs // ops.GROUP_TILE + n) + 1, dtype=torch.int32, device=dev)[3:]
         start, pair_of_slot = ints[:n + 1], ints[n + 1:n + 1 + pairs]
         tiles, num_tiles = ints[n + 1 + pairs:-1].view(-1, 2), ints[-1:]
         by_library = x.dtype == torch.bfloat16 and pairs >= self.LIBRARY_ROWS * n and E % 16 == 0 and F % 16 == 0
@@ -223,7 +224,7 @@ class RoutedExperts(FeedForward):
         on_input = self.weight_on == "input"
         rows = ops.rows_by_index(x, pair_of_slot, top, weight.view(-1) if on_input else None,
                                  torch.empty((pairs, E), dtype=x.dtype, device=x.device))
-        ends = start[1:].clone()
+        ends = start[1:]
         act = torch.empty((pairs, self.inter), dtype=x.dtype, device=x.device)
         hidden = torch._grouped_mm(rows, self.gate_up.transpose(1, 2), offs=ends)
         if self.activation == "clamped_glu":
