@@ -17,6 +17,9 @@
 //   EPI_F32 / EPI_BF16  store C
 //   EPI_SILU            HALVES = 2 and W holds, per 256 rows, 128 rows of the gate projection followed
 //                       by the 128 rows of the up projection for the same outputs: silu(gate) * up
+//   EPI_SILU, HALVES 1  the same with 64 gate rows and the 64 up rows for the same outputs in one tile of 128 (two copies a
+//                       stage): twice as many tiles, for matrices whose tiles of 256 leave more than half of the SMs idle.
+//                       The up half's warps hand their sums to the gate half's through shared memory
 //   EPI_RELU2           store max(C, 0)^2 as bfloat16 (the hidden layer of a feed-forward without a gate)
 //   EPI_PARTIAL         the k range is split over `splits` blocks; each writes C[split][T][N] (float32)
 // Rows of X beyond T and rows of W beyond N are zero-filled by TMA.
@@ -77,7 +80,7 @@ template <int NT, int EPI, int HALVES>
 __global__ void __launch_bounds__(TS_THREADS, 1)
 gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                      const TsArgs args) {
-    static_assert(EPI != TS_SILU || HALVES == 2, "the activation needs the gate half and the up half of a tile");
+    constexpr bool PAIRED = EPI == TS_SILU && HALVES == 1;      // 64 gate rows and 64 up rows to a tile
     constexpr int HALF_W = 128 * TS_BK * 2;           // 16 KB: 128 rows of W, 64 of k
     constexpr int STAGE_W = HALVES * HALF_W;
     constexpr int STAGE_X = NT * TS_BK * 2;
@@ -97,6 +100,13 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     float* row_scale = (float*)(tmem_slot + 2);       // [NT]
+    float* ups = row_scale + NT;                       // PAIRED: [NT][64]
+    // where a tile's rows of W lie (PAIRED: its gate rows; the up rows are 128 further on)
+    auto row_of = [](int tile) { return PAIRED ? tile / 2 * 256 + tile % 2 * 64 : tile * TILE_N; };
+    auto load_w = [&](int stage, int k, int n0) {
+        tma_load_2d(sw + stage * STAGE_W, &map_w, k, n0, &full[stage]);
+        if (PAIRED) tma_load_2d(sw + stage * STAGE_W + HALF_W / 2, &map_w, k, n0 + 128, &full[stage]);
+    };
 
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -132,7 +142,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             trace_point(TR_GEMM_TC + 100);   // when this block became resident
             for (int tile = blockIdx.x; tile < total && !*abort_flag; tile += gridDim.x) {
                 const int split = tile % args.splits;
-                const int n0 = (tile / args.splits) * TILE_N;
+                const int n0 = row_of(tile / args.splits);
                 const int k_begin = split * k_per, k_end = min(k_tiles, k_begin + k_per);
                 int kt = k_begin;
                 if (first) {
@@ -143,7 +153,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     const int pre = min(STAGES, k_end - k_begin);
                     for (int i = 0; i < pre; ++i) {
                         mbar_expect_tx(&full[i], bytes);
-                        tma_load_2d(sw + i * STAGE_W, &map_w, (k_begin + i) * TS_BK, n0, &full[i]);
+                        load_w(i, (k_begin + i) * TS_BK, n0);
                     }
                     // (Asking further k-tiles into L2 here, as gemm_tc.cu does, was measured to cost 1.7 % of a
                     // decode step with this kernel: the ring is deep, and the requests delay the loads of
@@ -157,7 +167,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 for (; kt < k_end; ++kt) {
                     if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) break;
                     mbar_expect_tx(&full[stage], bytes);
-                    tma_load_2d(sw + stage * STAGE_W, &map_w, kt * TS_BK, n0, &full[stage]);
+                    load_w(stage, kt * TS_BK, n0);
                     tma_load_2d(sx + stage * STAGE_X, &map_x, kt * TS_BK, 0, &full[stage]);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
@@ -225,14 +235,39 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
         uint32_t it = 0;
-        for (int tile = blockIdx.x; tile < total && !*abort_flag; tile += gridDim.x, ++it) {
+        // (PAIRED: the four warps meet at a barrier twice per tile, so all of them go through all tiles, also when a wait has
+        // run out: one that left would keep the others there for good)
+        for (int tile = blockIdx.x; tile < total && (PAIRED || !*abort_flag); tile += gridDim.x, ++it) {
             const int split = tile % args.splits;
             const int n0 = (tile / args.splits) * TILE_N;
             const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-            if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag)) break;
+            bool ok = mbar_wait(&acc_full[acc], acc_phase, abort_flag);
+            if constexpr (PAIRED) ok = __all_sync(0xffffffffu, ok);
+            else if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
-            if constexpr (EPI == TS_SILU) {
+            if constexpr (PAIRED) {
+                float v[NT];
+                if (ok) ts_load_row<NT>(taddr, v);
+                if (args.ss) {
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) v[t] *= row_scale[t];
+                }
+                if (ok && r >= 64) {
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) ups[t * 64 + r - 64] = v[t];
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (ok && r < 64) {
+                    __nv_bfloat16* out = (__nv_bfloat16*)args.out + (size_t)(tile / args.splits) * 64 + r;
+#pragma unroll
+                    for (int t = 0; t < NT; ++t)
+                        if (t < args.T)
+                            out[(size_t)t * (args.N / 2)] = __float2bfloat16_rn(
+                                gated_activation(v[t], ups[t * 64 + r], args.act_alpha, args.act_limit, args.act_shift));
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");      // (read before the next tile's are written)
+            } else if constexpr (EPI == TS_SILU) {
                 float gate[NT], up[NT];
                 ts_load_row<NT>(taddr, gate);
                 ts_load_row<NT>(taddr + NT, up);
@@ -284,7 +319,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[acc]);
+            if (lane == 0 && ok) mbar_arrive(&acc_empty[acc]);
         }
     }
 
@@ -313,7 +348,8 @@ static int ts_launch(const CUtensorMap& mw, const CUtensorMap& mx, const TsArgs&
     constexpr int STAGES = ts_stages(NT, HALVES);
     // always more than half of an SM's shared memory, so that two blocks never share an SM (and its
     // tensor memory)
-    const size_t smem = 1024 + (size_t)STAGES * (HALVES * 128 + NT) * TS_BK * 2 + 16 * STAGES + 256 + 4 * NT;
+    const size_t smem = 1024 + (size_t)STAGES * (HALVES * 128 + NT) * TS_BK * 2 + 16 * STAGES + 256 + 4 * NT +
+                        (EPI == TS_SILU && HALVES == 1 ? 256 * NT : 0);
     const size_t request = smem < 120 * 1024 ? 120 * 1024 : smem;
     auto kernel = gemm_tc_small_kernel<NT, EPI, HALVES>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)request);
@@ -327,9 +363,7 @@ static int ts_dispatch_epi(int epi, const CUtensorMap& mw, const CUtensorMap& mx
     switch (epi) {
         case TS_F32: return ts_launch<NT, TS_F32, HALVES>(mw, mx, args, blocks, stream);
         case TS_BF16: return ts_launch<NT, TS_BF16, HALVES>(mw, mx, args, blocks, stream);
-        case TS_SILU:
-            if constexpr (HALVES == 2) return ts_launch<NT, TS_SILU, HALVES>(mw, mx, args, blocks, stream);
-            return AIR_ERR_BAD_ARGUMENT;
+        case TS_SILU: return ts_launch<NT, TS_SILU, HALVES>(mw, mx, args, blocks, stream);
         case TS_PARTIAL: return ts_launch<NT, TS_F32, HALVES>(mw, mx, args, blocks, stream);
         case TS_RELU2: return ts_launch<NT, TS_RELU2, HALVES>(mw, mx, args, blocks, stream);
         default: return AIR_ERR_BAD_ARGUMENT;
@@ -365,15 +399,20 @@ AIR_API int air_gemm_tc_small(const void* x, const void* w, void* out, int T, in
     if (splits > k_tiles || (long long)(splits - 1) * ((k_tiles + splits - 1) / splits) >= k_tiles)
         return AIR_ERR_BAD_ARGUMENT;
     const int nt = T > 32 ? 64 : (T > 16 ? 32 : 16);
-    CUtensorMap mw, mx;
-    int rc = ts_make_map(&mw, w, N, K, tile_rows);
-    if (rc) return rc;
-    rc = ts_make_map(&mx, x, T, K, nt);
-    if (rc) return rc;
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (max_blocks > 0 && max_blocks < sms) sms = max_blocks;
+    // Gate and up rows by 64 where twice as many tiles still are one round of the SMs (16,384 x 2,048, 64 tiles: 13.9 -> 11.1 us
+    // inside a decode step of one token; 14,336 x 4,096, 56 tiles: 26 -> 21); beyond, two rounds of
+    // half tiles are no shorter than one of whole ones.
+    const bool paired = epi == TS_SILU && N / 256 * 2 <= sms;
+    if (paired) tile_rows = 128;
+    CUtensorMap mw, mx;
+    int rc = ts_make_map(&mw, w, N, K, paired ? 64 : tile_rows);
+    if (rc) return rc;
+    rc = ts_make_map(&mx, x, T, K, nt);
+    if (rc) return rc;
     const long long tiles = (long long)((N + tile_rows - 1) / tile_rows) * splits;
     const int blocks = (int)(tiles < sms ? tiles : sms);
     if (ss && ss_tiles < 1) return AIR_ERR_BAD_ARGUMENT;

@@ -160,3 +160,26 @@ def test_scale_per_row_from_sums_of_squares(T, epi):
     with pytest.raises(o.KernelError, match="up to 64 rows"):
         o.gemm_tc(torch.zeros(100, K, dtype=torch.bfloat16, device="cuda"), w.cuda(), torch.zeros(100, N, device="cuda"),
                   256, o.EPI_F32, row_ss=torch.zeros(tiles, 100, device="cuda"), eps=eps)
+
+
+@pytest.mark.parametrize("tiles", [1, 73, 74, 75, 150])
+@pytest.mark.parametrize("M", [1, 17, 64])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_silu_epilogue_in_half_and_in_whole_tiles(tiles, M, scaled):
+    """Few rows: up to 74 tiles of 256 rows of W the kernel takes them by 64 gate and 64 up rows, beyond whole; with and
+    without the scale per row.  (bfloat16 results: 2^-8 of their size.)"""
+    o = ops()
+    K, I = 136, 128 * tiles
+    g = torch.Generator(device="cuda").manual_seed(tiles + M)
+    a = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(2 * I, K, generator=g, device="cuda") * 0.1).bfloat16()
+    out, status = torch.full((M, I), 9.0, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    ss = torch.rand(1, M, generator=g, device="cuda") * K if scaled else None
+    o.gemm_tc(a, w, out, 256, o.EPI_SILU, status=status, **(dict(row_ss=ss, eps=1e-6) if scaled else {}))
+    assert status.item() == 0
+    z = a.double() @ w.double().t()
+    if scaled:
+        z = z * torch.rsqrt(ss[0].double() / K + 1e-6)[:, None]
+    z = z.view(M, tiles, 2, 128)
+    want = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, I)
+    assert (out.double() - want).abs().max() <= 0.005 * want.abs().max()
