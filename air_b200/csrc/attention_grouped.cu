@@ -256,9 +256,11 @@ __device__ __forceinline__ void split_bf16(float v, __nv_bfloat16& hi, __nv_bflo
 }
 
 // MAX_NT: 8-column tiles of the values that a warp has room for; MAX_KS: its share of the steps of 16 of d
-// WARPS: 8, or 16 of which every eight take half of a tile's keys (a tile is some 1,400 instructions for each of 8 warps, of which
-// two to a scheduler hide little: 49 us with 8, 43 with 16, measured as above)
-template <int MAX_NT, int MAX_KS, int WARPS>
+// WARPS: 8, or 16 for wide rows (a tile is then some 1,400 instructions for each of 8 warps, of which two to a scheduler hide
+// little: 49 us with 8, 43 with 16, measured as above)
+// SHARE: how many warps share d; the others take other keys of the tile (rows of up to 256 numbers need no more than two, and
+// leave room for a second block)
+template <int MAX_NT, int MAX_KS, int WARPS, int SHARE>
 __global__ void __launch_bounds__(WARPS * 32)
 grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __nv_bfloat16* __restrict__ cache,
                             const int* __restrict__ block_table, int max_blocks, const int* __restrict__ token_seq,
@@ -277,8 +279,8 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
     const int lo = window > 0 ? (mask_mode == 1 ? pos - pos % window : max(0, pos - window + 1)) : 0;
     const int* bt = block_table + (size_t)slot * max_blocks;
     const int kld = d + 8, vld = latent ? kld : dv + 8;      // elements per staged row: 16 bytes of padding
-    float* R = smem;                                          // [8 warps][16][GT_RLD] partial scores
-    float* corr = R + 8 * JB * GT_RLD;                        // [16], then the running maximum and sum
+    float* R = smem;                                          // [SHARE][16][GT_RLD] partial scores
+    float* corr = R + SHARE * JB * GT_RLD;                    // [16], then the running maximum and sum
     float* mrun = corr + JB;
     float* lrun = mrun + JB;
     long long* rows = reinterpret_cast<long long*>(lrun + JB);               // [2][64]: where a key's row lies, -1: not seen
@@ -301,9 +303,9 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
     // ldmatrix.x4 of a 16 x 16 block of A (rows = heads): lane l gives the address of row l % 16, columns 8 (l / 16) ..
     const int a_row = lane & 15, a_col = (lane >> 4) * 8;
     // This warp's share of d, and its part of the queries: rows gq and gq + 8, columns 2 tq, 2 tq + 1 and 8 further on.
-    const int share = warp & 7, steps = d / 16, ks0 = steps * share / 8, my_steps = steps * (share + 1) / 8 - ks0;
-    constexpr int KN = 8 / (WARPS / 8);                       // 8-key tiles of scores that a warp takes, from n0 on
-    const int n0 = (warp >> 3) * KN;
+    const int share = warp % SHARE, steps = d / 16, ks0 = steps * share / SHARE, my_steps = steps * (share + 1) / SHARE - ks0;
+    constexpr int KN = 8 / (WARPS / SHARE);                   // 8-key tiles of scores that a warp takes, from n0 on
+    const int n0 = warp / SHARE * KN;
     uint32_t qh[MAX_KS][4], ql[MAX_KS][4];
 #pragma unroll
     for (int x = 0; x < MAX_KS; ++x)
@@ -350,18 +352,23 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
             }
         cp_async_commit();
     };
-    auto look_up = [&](int key0, int list) {
+    // the page of this thread's key of a tile (-1: not seen), asked for a tile before it is used; and where its row lies
+    auto page_of = [&](int key0) {
+        const int key = key0 + tid;
+        return tid < GA_KT && key >= lo && key <= pos ? bt[key / P] : -1;
+    };
+    auto look_up = [&](int key0, int page, int list) {
         if (tid < GA_KT) {
-            const int key = key0 + tid;
-            long long at = -1;
-            if (key >= lo && key <= pos)
-                at = (long long)bt[key / P] * (long long)page_stride + (latent ? (long long)(key % P) * d : ((long long)g * P + key % P) * d);
-            rows[list * GA_KT + tid] = at;
+            const int at = (key0 + tid) % P;
+            rows[list * GA_KT + tid] = page < 0 ? -1 : (long long)page * (long long)page_stride + (latent ? (long long)at * d : ((long long)g * P + at) * d);
         }
     };
     const int kt_first = lo / GA_KT + split;
+    int page_next = -1;
     if (kt_first * GA_KT <= pos) {
-        look_up(kt_first * GA_KT, 0);
+        const int page = page_of(kt_first * GA_KT);
+        page_next = page_of((kt_first + splits) * GA_KT);
+        look_up(kt_first * GA_KT, page, 0);
         __syncthreads();
         bring(0, 0);
     }
@@ -369,7 +376,10 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
     for (int kt = kt_first; kt * GA_KT <= pos; kt += splits, ++turn) {
         const int key0 = kt * GA_KT, next = (kt + splits) * GA_KT;
         const int after = (turn & 1) ^ 1, buf = stages == 2 ? (turn & 1) : 0;
-        if (next <= pos) look_up(next, after);             // (the list that the turn before last was read from)
+        if (next <= pos) {                                 // (into the list that the turn before last was read from)
+            look_up(next, page_next, after);
+            page_next = page_of(next + splits * GA_KT);
+        }
         __syncthreads();
         if (stages == 2 && next <= pos) {
             bring(after, after);
@@ -416,7 +426,7 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
             const bool seen0 = key0 + lane >= lo && key0 + lane <= pos, seen1 = key0 + lane + 32 >= lo && key0 + lane + 32 <= pos;
             float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) {
+            for (int w = 0; w < SHARE; ++w) {
                 s0 += R[(w * JB + j) * GT_RLD + lane];
                 s1 += R[(w * JB + j) * GT_RLD + lane + 32];
             }
@@ -594,15 +604,23 @@ AIR_API int air_grouped_attention(const void* q, int q_f32, const void* cache, i
         // both products on the tensor cores
         const int kld = d + 8, vld = dv + 8;
         const size_t stage = 2 * ((size_t)air::GA_KT * kld + (latent ? 0 : (size_t)air::GA_KT * vld));
-        const size_t fixed = sizeof(float) * (8 * 16 * air::GT_RLD + 3 * 16) + 8 * 2 * air::GA_KT + 2 * 2 * 16 * (air::GA_KT + 8);
+        // (rows of up to 256: several blocks to an SM; up to 640: one of sixteen warps.  Measured, us: 32 tokens over 1,000
+        // keys, 32 heads of 128 over 8: 159 as wide rows are taken, 142 with warps that share the keys and read the queries
+        // from shared memory, 120 so; 20 over 500, 16 of 64 over 4: 35, 30, 27; 8 over 2,048, 16 of 256 over 4: 68 the second
+        // way, 62 so)
+        const int kind = d <= 128 && dv <= 128 ? 0 : d <= 256 && dv <= 256 ? 1 : d <= 640 && dv <= 512 ? 2 : 3;
+        const int share = kind < 2 ? 2 : 8;
+        const size_t fixed = sizeof(float) * (share * 16 * air::GT_RLD + 3 * 16) + 8 * 2 * air::GA_KT + 2 * 2 * 16 * (air::GA_KT + 8);
         const int stages = fixed + 2 * stage <= 227 * 1024 ? 2 : 1;
         const size_t smem = fixed + stages * stage;
         if (smem <= 227 * 1024) {
-            const bool most = dv <= 512 && d <= 640;
-            auto kernel = most ? air::grouped_attention_tc_kernel<4, 5, 16> : air::grouped_attention_tc_kernel<air::GT_MAX_NT, 10, 8>;
+            auto kernel = kind == 0 ? air::grouped_attention_tc_kernel<2, 4, 8, 2>
+                        : kind == 1 ? air::grouped_attention_tc_kernel<4, 8, 8, 2>
+                        : kind == 2 ? air::grouped_attention_tc_kernel<4, 5, 16, 8>
+                                    : air::grouped_attention_tc_kernel<air::GT_MAX_NT, 10, 8, 8>;
             if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             dim3 grid(T, G * ((J + 15) / 16), splits);
-            rc = air::launch(kernel, grid, most ? 512 : 256, smem, stream, q, q_f32, (const __nv_bfloat16*)cache, block_table,
+            rc = air::launch(kernel, grid, kind == 2 ? 512 : 256, smem, stream, q, q_f32, (const __nv_bfloat16*)cache, block_table,
                              max_blocks, token_seq, positions, part, H, G, d, dv, P, window, mask_mode, scale, softcap, latent,
                              splits, stages, bias);
             if (rc) return rc;
