@@ -26,54 +26,73 @@ namespace air {
 
 constexpr int MOE_MAX_PER_LANE = 16;      // up to 512 experts
 
+// PER_LANE: experts that a lane has room for.  A step of few tokens is one warp's chain of instructions, so that few experts should
+// not pay for 512.  Measured, us, 8 tokens, against room for 512 always: 8 experts 4.2 -> 2.1, 64 4.9 -> 2.8, 128 6.2 ->
+// 3.7, 256 6.1 -> 4.3, 512 5.7 and 5.9; 1,000 tokens by 64 6.6 -> 3.2.
+template <int PER_LANE>
 __global__ void __launch_bounds__(128)
 moe_route_kernel(const float* __restrict__ z, int parts, int ld, int T, int n, int top, int score, int renormalize,
                  int has_gate, int* __restrict__ expert, float* __restrict__ weight, float* __restrict__ gate,
                  int groups, int keep, int mark, float route_scale, float norm_eps, const float* __restrict__ bias) {
-    __shared__ float held[4][32 * MOE_MAX_PER_LANE], marks[4][32 * MOE_MAX_PER_LANE];
+    __shared__ float held[4][32 * PER_LANE], marks[4][32 * PER_LANE];
     pdl_enter(TR_MOE_ROUTE);
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= T) return;
     // (the logits may be partial sums over parts of k, added in order: [parts, T, ld])
     const float* row = z + (size_t)t * ld;
-    auto logit = [&](int e) {
-        float part[8], v = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) part[i] = i < parts ? row[(size_t)i * T * ld + e] : 0.f;      // (all under way at once)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v += part[i];
-        for (int i = 8; i < parts; ++i) v += row[(size_t)i * T * ld + e];
-        return v;
-    };
-    float s[MOE_MAX_PER_LANE];
+    // (some eight loads of a lane under way at once)
+    constexpr int AHEAD = PER_LANE >= 8 ? 1 : 8 / PER_LANE;
+    float s[PER_LANE];
     float zmax = -INFINITY;
 #pragma unroll
-    for (int c = 0; c < MOE_MAX_PER_LANE; ++c) {
-        const int e = lane + 32 * c;
-        s[c] = e < n ? logit(e) : -INFINITY;
+    for (int c = 0; c < PER_LANE; ++c) s[c] = 0.f;
+    for (int i0 = 0; i0 < parts; i0 += AHEAD) {
+        float part[AHEAD][PER_LANE];
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+#pragma unroll
+            for (int c = 0; c < PER_LANE; ++c)
+                part[i][c] = i0 + i < parts && lane + 32 * c < n ? row[(size_t)(i0 + i) * T * ld + lane + 32 * c] : 0.f;
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+#pragma unroll
+            for (int c = 0; c < PER_LANE; ++c) s[c] += part[i][c];
+    }
+    float open = 0.f;      // the gate's logit
+    if (gate && has_gate && lane == 0)
+        for (int i0 = 0; i0 < parts; i0 += 8) {
+            float part[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) part[i] = i0 + i < parts ? row[(size_t)(i0 + i) * T * ld + n] : 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) open += part[i];
+        }
+#pragma unroll
+    for (int c = 0; c < PER_LANE; ++c) {
+        if (lane + 32 * c >= n) s[c] = -INFINITY;
         zmax = fmaxf(zmax, s[c]);
     }
     if (score == 1) {
         zmax = warp_max(zmax);
         float sum = 0.f;
 #pragma unroll
-        for (int c = 0; c < MOE_MAX_PER_LANE; ++c) {
+        for (int c = 0; c < PER_LANE; ++c) {
             s[c] = lane + 32 * c < n ? expf(s[c] - zmax) : 0.f;
             sum += s[c];
         }
         sum = warp_sum(sum);
 #pragma unroll
-        for (int c = 0; c < MOE_MAX_PER_LANE; ++c) s[c] /= sum;
+        for (int c = 0; c < PER_LANE; ++c) s[c] /= sum;
     } else {
 #pragma unroll
-        for (int c = 0; c < MOE_MAX_PER_LANE; ++c) s[c] = 1.f / (1.f + expf(-s[c]));
+        for (int c = 0; c < PER_LANE; ++c) s[c] = 1.f / (1.f + expf(-s[c]));
     }
     // ch: what the experts are chosen by (the score, plus the bias where there is one); s stays the weight
     constexpr float NEVER = -3.0e38f;
-    float ch[MOE_MAX_PER_LANE];
+    float ch[PER_LANE];
 #pragma unroll
-    for (int c = 0; c < MOE_MAX_PER_LANE; ++c) {
+    for (int c = 0; c < PER_LANE; ++c) {
         const int e = lane + 32 * c;
         if (e >= n || !(s[c] == s[c])) {      // outside, or not a number: never preferred
             s[c] = 0.f;
@@ -87,7 +106,7 @@ moe_route_kernel(const float* __restrict__ z, int parts, int ld, int T, int n, i
         float* mk = marks[threadIdx.x >> 5];
         const int size = n / groups;
 #pragma unroll
-        for (int c = 0; c < MOE_MAX_PER_LANE; ++c)
+        for (int c = 0; c < PER_LANE; ++c)
             if (lane + 32 * c < n) my[lane + 32 * c] = ch[c] == NEVER ? -1.f : ch[c];
         __syncwarp();
         for (int g = lane; g < groups; g += 32) {
@@ -109,7 +128,7 @@ moe_route_kernel(const float* __restrict__ z, int parts, int ld, int T, int n, i
         }
         __syncwarp();
 #pragma unroll
-        for (int c = 0; c < MOE_MAX_PER_LANE; ++c) {
+        for (int c = 0; c < PER_LANE; ++c) {
             const int e = lane + 32 * c;
             if (e < n && my[e / size] == 0.f) ch[c] = NEVER;
         }
@@ -121,7 +140,7 @@ moe_route_kernel(const float* __restrict__ z, int parts, int ld, int T, int n, i
         float best = -INFINITY;
         int best_e = n;
 #pragma unroll
-        for (int c = 0; c < MOE_MAX_PER_LANE; ++c) {
+        for (int c = 0; c < PER_LANE; ++c) {
             const int e = lane + 32 * c;
             if (e < n && ch[c] > best) { best = ch[c]; best_e = e; }      // ascending e: the first of equals stays
         }
@@ -133,7 +152,7 @@ moe_route_kernel(const float* __restrict__ z, int parts, int ld, int T, int n, i
         }
         float own = 0.f;      // the chosen expert's score, held by the lane that has it
 #pragma unroll
-        for (int c = 0; c < MOE_MAX_PER_LANE; ++c)
+        for (int c = 0; c < PER_LANE; ++c)
             if (lane + 32 * c == best_e) {
                 own = s[c];
                 ch[c] = -INFINITY;      // taken
@@ -154,7 +173,7 @@ moe_route_kernel(const float* __restrict__ z, int parts, int ld, int T, int n, i
         expert[(size_t)t * top + lane] = mine_e;
         weight[(size_t)t * top + lane] = (renormalize ? mine / (total + norm_eps) : mine) * route_scale;
     }
-    if (gate && lane == 0) gate[t] = has_gate ? 1.f / (1.f + expf(-logit(n))) : 1.f;
+    if (gate && lane == 0) gate[t] = has_gate ? 1.f / (1.f + expf(-open)) : 1.f;
 }
 
 __global__ void __launch_bounds__(1024)
@@ -315,7 +334,9 @@ AIR_API int air_moe_route(const float* z, int parts, int ld, int T, int n, int t
         score < 0 || score > 1 || mark < 0 || mark > 1 || parts < 1)
         return AIR_ERR_BAD_ARGUMENT;
     if (groups > 1 && (n % groups || keep <= 0 || keep > groups || top > keep * (n / groups))) return AIR_ERR_BAD_ARGUMENT;
-    return air::launch(air::moe_route_kernel, (T + 3) / 4, 128, 0, stream, z, parts, ld, T, n, top, score, renormalize,
+    auto kernel = n <= 32 ? air::moe_route_kernel<1> : n <= 128 ? air::moe_route_kernel<4>
+                : n <= 256 ? air::moe_route_kernel<8> : air::moe_route_kernel<air::MOE_MAX_PER_LANE>;
+    return air::launch(kernel, (T + 3) / 4, 128, 0, stream, z, parts, ld, T, n, top, score, renormalize,
                        has_gate, expert, weight, gate, groups, keep, mark, route_scale, norm_eps, bias);
 }
 

@@ -253,6 +253,38 @@ def test_latent_attention_through_its_kernels(H, d, rot, R, dv, window, dtype):
         assert np.abs(row[:R] - c[t]).max() < tol and np.abs(row[R:] - kr[t]).max() < tol
 
 
+@pytest.mark.parametrize("n,top,groups", [(31, 4, 1), (32, 32, 4), (33, 4, 3), (128, 8, 8), (129, 32, 3),
+                                          (256, 8, 8), (257, 8, 1), (512, 8, 8)])
+def test_router_at_the_edges_of_its_lanes(n, top, groups):
+    """The numbers of experts at which a lane's room changes, with ties, with and without groups: the chosen experts are those
+    of a stable sort; a weight is a sigmoid in 32 bits (a few roundings of a number below 1)."""
+    from air_b200.csrc import ops
+    rng = np.random.default_rng(n)
+    T = 9
+    z = np.round(rng.normal(size=(T, n)) * 8) / 8              # many equal scores
+    z[2] = 0.5
+    z[3, n - 1] = 9.0                                          # the last lane's last expert
+    s = plain.sigmoid(z)
+    expert = torch.empty((T, top), dtype=torch.int32, device=DEV)
+    weight = torch.empty((T, top), device=DEV)
+    keep = max(1, -(-top * groups // n), groups - 1)
+    for g, k in ((1, 0), (groups, keep)):
+        chosen = s.copy()
+        if g > 1:
+            marks = np.sort(s.reshape(T, g, n // g), axis=-1)[:, :, -1]
+            out = np.argsort(-marks, axis=-1, kind="stable")[:, k:]
+            for t in range(T):
+                for group in out[t]:
+                    chosen[t, group * (n // g):(group + 1) * (n // g)] = -1
+        order = np.argsort(-chosen, axis=-1, kind="stable")[:, :top]
+        more = dict(groups=g, keep=k, mark="best") if g > 1 else {}
+        if top > (k * (n // g) if g > 1 else n):
+            continue
+        ops.moe_route(dev(z), n, top, expert, weight, None, **more)
+        assert np.array_equal(expert.cpu().numpy(), order)
+        assert np.abs(weight.cpu().numpy() - np.take_along_axis(s, order, -1)).max() < 1e-6
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("n,top,E,F,T", [(5, 2, 64, 48, 150), (3, 3, 96, 40, 7), (8, 1, 72, 64, 65), (130, 6, 32, 20, 40)])
 def test_router_and_experts(n, top, E, F, T, dtype):
