@@ -23,6 +23,12 @@
 // token's own position do not wait for that write to be visible to the copy engine: they put the two new
 // rows into the tile in shared memory once it has landed.  A decode step is then one launch shorter per
 // layer, and the keys start to stream as soon as the product has ended.
+//
+// alongside (a mixed step): the portions' tcgen05 kernel is launched first, with fewer blocks than SMs and no merge behind it,
+// and this kernel on the SMs that are left.  That kernel lets its successor start only when it has itself waited for
+// what is ahead of it, so everything that this one reads is complete when its first block starts, and it waits for nothing.
+// But what follows waits for this kernel alone: so its first block ends only when the portions' kernel has (one block:
+// the others leave their places to the blocks still to come).  What it gives: TiledAttention.beside (parts/attention.py).
 #include "common.cuh"
 #include "mma.cuh"
 #include "tma.cuh"
@@ -53,7 +59,8 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
                             const int* __restrict__ block_table, int max_blocks, const int* __restrict__ token_seq,
                             const int* __restrict__ positions, __nv_bfloat16* __restrict__ out,
                             float* __restrict__ part_o, float* __restrict__ part_ml, int H, int K, int P, int window,
-                            float scale_log2, float cap_log2, float cap_pre, int* status, const DistanceBias bias) {
+                            float scale_log2, float cap_log2, float cap_pre, int* status, const DistanceBias bias,
+                            int alongside) {
     // cap_log2 > 0: a score s becomes cap * tanh(s * cap_pre) with cap_pre = scale / cap, in units of log2 e
     constexpr int SUB = D / 64;                 // 64-column sub-tiles of a row
     constexpr int SUB_BYTES = DT_TILE * 128;    // 8 KB
@@ -101,12 +108,16 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
     // come from the copy (they are patched into the tile from shared memory).  So the first tiles of old keys
     // are on their way while the product's last blocks still run.  Without fresh.qkv the token's key and value
     // were written to the page by the predecessor itself, and everybody waits.
-    if (!(warp == DT_CONSUMERS && fresh.qkv)) pdl_wait();
+    // alongside: see the head of this file; the first block alone waits, at its end, for all of the grid.
+    if (!alongside && !(warp == DT_CONSUMERS && fresh.qkv)) pdl_wait();
+    auto leave = [&] {
+        if (alongside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
+    };
     trace_point(TR_ATT_DECODE);
 
     const int t = blockIdx.z;
     const int slot = token_seq[t];
-    if (slot < 0) return;
+    if (slot < 0) return leave();
     const int G = H / K;
     const int head_blocks = (G + 15) / 16;
     const int kvh = blockIdx.y / head_blocks, hb = blockIdx.y % head_blocks;
@@ -124,7 +135,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
         const int r = hb * 16 + threadIdx.x;
         if (threadIdx.x < 16 && r < G)
             *reinterpret_cast<float2*>(part_ml + (((size_t)t * H + kvh * G + r) * splits + split) * 2) = make_float2(-INFINITY, 0.f);
-        return;
+        return leave();
     }
 
     float o[NT][4];
@@ -398,7 +409,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
     if (*abort_flag) {
         for (int i = 0; i < 32; ++i) __nanosleep(2000);   // copies on their way may still land
         if (threadIdx.x == 0 && status) atomicExch(status, 5);
-        return;
+        return leave();
     }
     if (warp < DT_CONSUMERS) {
         if (tq == 0) {
@@ -438,13 +449,14 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
             }
         }
     }
+    leave();
 }
 
 template <int D>
 int launch_decode_tma(const CUtensorMap& map, const FreshQkv& fresh, const void* q, const int* block_table, int max_blocks,
                       const int* token_seq, const int* positions, void* out, float* part_o, float* part_ml, int T,
                       int H, int K, int P, int window, float scale, float softcap, int splits, int* status,
-                      const DistanceBias& bias, cudaStream_t stream) {
+                      const DistanceBias& bias, int alongside, cudaStream_t stream) {
     const int head_blocks = (H / K + 15) / 16;
     const size_t ring = (size_t)DT_STAGES * 2 * (D / 64) * DT_TILE * 128;
     const size_t merge = (size_t)(DT_CONSUMERS * 16 * D + 2 * DT_CONSUMERS * 16) * sizeof(float);
@@ -455,7 +467,7 @@ int launch_decode_tma(const CUtensorMap& map, const FreshQkv& fresh, const void*
     return launch(kernel, dim3(splits, K * head_blocks, T), DT_THREADS, smem, stream, map, fresh, (const __nv_bfloat16*)q,
                   block_table, max_blocks, token_seq, positions, (__nv_bfloat16*)out, part_o, part_ml, H, K, P, window,
                   scale * 1.4426950408889634f, softcap > 0.f ? softcap * 1.4426950408889634f : 0.f,
-                  softcap > 0.f ? scale / softcap : 0.f, status, bias);
+                  softcap > 0.f ? scale / softcap : 0.f, status, bias, alongside);
 }
 
 }  // namespace air
@@ -476,13 +488,14 @@ static int decode_attention_tma(const FreshQkv& fresh, const void* q, const void
                                 float scale, float softcap, int splits, int* status, cudaStream_t stream,
                                 const float* sink = nullptr, const float* gate = nullptr, int ldg = 0,
                                 const TurnBack& turn = TurnBack{nullptr, 0, 0, nullptr},
-                                const DistanceBias& bias = DistanceBias{nullptr, 0}) {
+                                const DistanceBias& bias = DistanceBias{nullptr, 0}, int alongside = 0) {
     if (T <= 0) return 0;
     if (bias.table && bias.n < 1) return AIR_ERR_BAD_ARGUMENT;
     if (H <= 0 || K <= 0 || H % K || P % 16 || (P < 64 ? 64 % P : P % 64) || splits < 1 || T > 65535 ||
         (splits > 1 && (!part_o || !part_ml)) || ((uintptr_t)cache & 15))
         return AIR_ERR_BAD_ARGUMENT;
     // a sink, gates or a turn back enter where the splits are merged: the keys are then split in two parts at least
+    if (alongside && fresh.qkv) return AIR_ERR_BAD_ARGUMENT;
     const bool extra = sink || gate || turn.freq;
     if (extra && splits < 2) return AIR_ERR_BAD_ARGUMENT;
     CUtensorMap map;
@@ -492,15 +505,15 @@ static int decode_attention_tma(const FreshQkv& fresh, const void* q, const void
     switch (D) {
         case 64:
             rc = launch_decode_tma<64>(map, fresh, q, block_table, max_blocks, token_seq, positions, out, part_o, part_ml,
-                                       T, H, K, P, window, scale, softcap, splits, status, bias, stream);
+                                       T, H, K, P, window, scale, softcap, splits, status, bias, alongside, stream);
             break;
         case 128:
             rc = launch_decode_tma<128>(map, fresh, q, block_table, max_blocks, token_seq, positions, out, part_o,
-                                        part_ml, T, H, K, P, window, scale, softcap, splits, status, bias, stream);
+                                        part_ml, T, H, K, P, window, scale, softcap, splits, status, bias, alongside, stream);
             break;
         case 256:
             rc = launch_decode_tma<256>(map, fresh, q, block_table, max_blocks, token_seq, positions, out, part_o,
-                                        part_ml, T, H, K, P, window, scale, softcap, splits, status, bias, stream);
+                                        part_ml, T, H, K, P, window, scale, softcap, splits, status, bias, alongside, stream);
             break;
         default:
             return AIR_ERR_BAD_ARGUMENT;
@@ -515,14 +528,17 @@ static int decode_attention_tma(const FreshQkv& fresh, const void* q, const void
 }  // namespace air
 
 // Arguments as air_decode_attention (attention_decode.cu), plus the number of pages of the cache
-// (its first dimension), a soft cap (> 0: score = softcap * tanh(scale * q.k / softcap)) and the status word.
+// (its first dimension), a soft cap (> 0: score = softcap * tanh(scale * q.k / softcap)), the status word, and whether the
+// launch right ahead is prefill_attention_tc_kernel's over other rows of the same step (alongside).
 AIR_API int air_decode_attention_tma(const void* q, const void* cache, long long pages, const int* block_table,
                                      int max_blocks, const int* token_seq, const int* positions, void* out,
                                      float* part_o, float* part_ml, int T, int H, int K, int D, int P, int window,
-                                     float scale, float softcap, int splits, int* status, cudaStream_t stream) {
+                                     float scale, float softcap, int splits, int* status, int alongside,
+                                     cudaStream_t stream) {
     return air::decode_attention_tma(air::FreshQkv{nullptr, 0, 0, nullptr, nullptr, nullptr}, q, cache, pages,
                                      block_table, max_blocks, token_seq, positions, out, part_o, part_ml, T, H, K, D, P,
-                                     window, scale, softcap, splits, status, stream);
+                                     window, scale, softcap, splits, status, stream, nullptr, nullptr, 0,
+                                     air::TurnBack{nullptr, 0, 0, nullptr}, air::DistanceBias{nullptr, 0}, alongside);
 }
 
 // The same with one more term exp(sink[h]) in every head's softmax denominator (sink float32 [H] or null) and the

@@ -158,7 +158,6 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     uint32_t* tmem_slot = (uint32_t*)(pv_done + 4);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
-    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -185,6 +184,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();
+    // (only now: a decode kernel that runs alongside takes it that what was ahead of this kernel has ended when it starts,
+    // see attention_decode_tma.cu)
+    pdl_trigger();
     trace_point(TR_ATT_PREFILL);
 
     // The block's two groups of the list (heavy ones first) and its head.  The second group has to go

@@ -116,7 +116,7 @@ _SIGNATURES = {
                           c_void_p, c_int, c_float, c_float, c_float, c_float, c_void_p],
     "air_decode_attention_tma": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p,
-                                 c_void_p],
+                                 c_int, c_void_p],
     "air_decode_attention_tma_sink": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
                                       c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
@@ -1487,7 +1487,8 @@ def decode_splits(tokens: int, heads: int, kv_heads: int) -> int:
 
 
 def decode_attention(q, cache, block_table, token_seq, positions, out, window, scale, splits=None, scratch=None,
-                     status=None, engine="tma", softcap=0.0, sink=None, gate=None, turn=None, bias=None):
+                     status=None, engine="tma", softcap=0.0, sink=None, gate=None, turn=None, bias=None,
+                     alongside=False):
     """bfloat16 attention for one query token per request.  softcap > 0: score = softcap * tanh(scale * q.k /
     softcap) (the copy-engine kernel only).  sink (float32 [H]): one more term exp(sink[h]) in the softmax's
     denominator; gate (float32 [T, H * d] logits, may be a band of columns): out is multiplied by sigmoid(gate) element
@@ -1495,7 +1496,9 @@ def decode_attention(q, cache, block_table, token_seq, positions, out, window, s
     does it; all enter where the key splits are merged (the copy-engine kernel only, two splits at least).  bias (float32
     [H, n]): a score gets bias[h, min(distance, n - 1)] (the copy-engine kernel only).  scratch: (float32 [T*H*splits*D], float32
     [T*H*splits*2]) or None to allocate.  engine "tma": keys and values by the copy engine into shared
-    memory (attention_decode_tma.cu); "ldg": by the warps' own loads (attention_decode.cu)."""
+    memory (attention_decode_tma.cu); "ldg": by the warps' own loads (attention_decode.cu).
+    alongside: the last launch on this stream was prefill_attention_tc, without items, over other rows of q and out, and
+    what is attended over was written before it: the two may run side by side (the copy-engine kernel only)."""
     T, H, d = q.shape
     K, P = cache.shape[2], cache.shape[3]
     _req(q, "q", (torch.bfloat16,))
@@ -1507,7 +1510,10 @@ def decode_attention(q, cache, block_table, token_seq, positions, out, window, s
     if d not in DECODE_HEAD_DIMS:
         raise KernelError(f"decode_attention takes head sizes {DECODE_HEAD_DIMS}, not {d}")
     if splits is None:
-        splits = decode_splits(T, H, K)
+        # (side by side, blocks of half the length: the last ones start on SMs that the other kernel has left late.  Measured, us,
+        # both kernels, with the usual splits and with twice as many: 32 requests of 8,192 at 8 key/value heads 204 and 194, at 4 118 and
+        # 103; 32 of 2,048 at 8 65 and 59; 20 of 8,192 at 4 74 and 77.)
+        splits = min(32, 2 * decode_splits(T, H, K)) if alongside else decode_splits(T, H, K)
     extra = sink is not None or gate is not None or turn is not None
     if extra:
         splits = max(2, splits)
@@ -1541,8 +1547,8 @@ def decode_attention(q, cache, block_table, token_seq, positions, out, window, s
         _check(_get("air_decode_attention_tma")(
             q.data_ptr(), cache.data_ptr(), cache.shape[0], block_table.data_ptr(), block_table.shape[1],
             token_seq.data_ptr(), positions.data_ptr(), out.data_ptr(), _ptr(po), _ptr(pm), T, H, K, d, P,
-            int(window or 0), float(scale), float(softcap or 0.0), splits, _ptr(status), _stream()),
-            "decode_attention_tma")
+            int(window or 0), float(scale), float(softcap or 0.0), splits, _ptr(status), 1 if alongside else 0,
+            _stream()), "decode_attention_tma")
     elif softcap:
         raise KernelError("decode_attention: a soft cap is taken by the copy-engine kernel only (pages that divide "
                           "or are multiples of 64 tokens)")

@@ -21,6 +21,10 @@ from .registry import register_mixer, POSITION_ENCODINGS
 # its own is as long.
 SEGMENT_COST = 8.0
 MIN_SEGMENT = 8
+# A block of the tcgen05 kernel takes this long for a key tile of its two row tiles, and keys and values stream at this rate
+# (microseconds, bytes a microsecond): how long a mixed step's two kernels take.
+KEY_TILE_US = 1.04
+STREAM_RATE = 6.5e6
 TO_THE_END = 1 << 30
 
 
@@ -120,13 +124,14 @@ class TiledAttention:
     def plan_key(self):
         return (self.PLAN, self.heads, self.window)
 
-    def plan(self, batch: HostBatch) -> Plan:
+    def plan(self, batch: HostBatch, alongside=True) -> Plan:
         """What the tile kernels want to know of a step, worked out once for all attention layers with this many
         heads and this window: `decode_prefix`, the number of leading entries that bring a single next token (they
         take the decode kernel), and for the tokens after them `tiles` [16n, 4] int32 = (slot, first row, its
         position, rows <= 16): 16-token tiles in groups of 16, filled up with rows = 0.  A group is a pair of row
         tiles, 256 consecutive tokens of a request on one stream of keys; `segments`, `items` and `slots` say which
-        block of the tcgen05 kernel takes which part of which pair's stream (plan_segments)."""
+        block of the tcgen05 kernel takes which part of which pair's stream (plan_segments).  `alongside`: the two kernels
+        run side by side (`beside`)."""
         prefix = 0
         while prefix < len(batch.counts) and batch.counts[prefix] == 1:
             prefix += 1
@@ -136,12 +141,31 @@ class TiledAttention:
             tiles.append(tile)
             key_tiles += of_pairs
         tiles = np.concatenate(tiles) if tiles else np.zeros((0, 4), dtype=np.int32)
-        arrays, values = {"tiles": tiles}, {"decode_prefix": prefix, "segments": None, "items": None, "slots": 0}
+        arrays, values = {"tiles": tiles}, {"decode_prefix": prefix, "segments": None, "items": None, "slots": 0, "alongside": False}
         cut = plan_segments(key_tiles, self.heads)
+        if alongside and prefix and key_tiles and self.beside(key_tiles, batch.lengths[:prefix], cut is not None):
+            cut, values["alongside"] = None, True
         if cut is not None:
             arrays["segments"], arrays["items"], values["slots"] = cut
             del values["segments"], values["items"]
         return Plan(arrays=arrays, values=values)
+
+    def beside(self, key_tiles, lengths, cut) -> bool:
+        """Whether a mixed step's two kernels had better run side by side: the portions' kernel with whole items (a merge behind
+        it would have to wait) on as many SMs, the single tokens' on the others.  That one is bound by memory and gets more
+        than its share of it from fewer SMs: a quarter more, up to some 0.8 of all.  One after the other they take what each of
+        them takes on all SMs.  Measured, us, one after the other and side by side: 512 tokens behind 3,840 at 40 heads over 8
+        beside 32 requests of 8,192 231 and 194, beside 8 of them 120 and 93; at 28 heads over 4 beside 32 141 and 103; 100 behind 4,000
+        beside 20 95 and 77; a prompt of 300 beside 16 requests of 2,000 31 and 27."""
+        items = len(key_tiles) * self.heads
+        if items > SMS - 16:
+            return False
+        whole = (max(key_tiles) + SEGMENT_COST) * KEY_TILE_US
+        spread = min(whole, (sum(key_tiles) * self.heads / SMS + 2.4 * SEGMENT_COST) * KEY_TILE_US) if cut else whole
+        keys = sum(min(n + 1, self.window or n + 1) for n in lengths)
+        single = keys * 4 * self.kv_heads * self.head_dim / STREAM_RATE
+        meanwhile = whole * min(0.8, 1.25 * (SMS - items) / SMS)
+        return whole + max(0.0, single - meanwhile) < spread + single
 
     def fast_attention(self, ctx, page_tokens: int) -> bool:
         """Whether this step's attention runs on the tensor-core kernels (bfloat16, a head size and a page size that
@@ -169,9 +193,16 @@ class TiledAttention:
         # prompt portions the tile kernels
         plan = ctx.plans[self.plan_key()]
         n = plan.decode_prefix
-        if n:
-            ops.decode_attention(q[:n], kv, bt, ctx.token_seq[:n], ctx.positions[:n], out[:n], self.window,
-                                 self.scale, softcap=self.softcap)
+        # (nothing between the two launches, and no memory that the first one reads is given back between them)
+        alongside = plan.alongside and d in ops.TC_ATTENTION_HEAD_DIMS
+
+        def decode():
+            if n:
+                ops.decode_attention(q[:n], kv, bt, ctx.token_seq[:n], ctx.positions[:n], out[:n], self.window,
+                                     self.scale, softcap=self.softcap, alongside=alongside)
+
+        if not alongside:
+            decode()
         if plan.tiles.shape[0] == 0:
             pass
         elif d in ops.TC_ATTENTION_HEAD_DIMS:     # both products on the tcgen05 tensor cores
@@ -183,6 +214,8 @@ class TiledAttention:
                                      scratch=getattr(plan, "scratch", None), softcap=self.softcap)
         else:
             ops.prefill_attention(q, kv, bt, plan.tiles, out, self.window, self.scale, status=ctx.status)
+        if alongside:
+            decode()
         return out
 
 

@@ -127,7 +127,7 @@ class NormedAttention(PortionAttention, Mixer):
         return TiledAttention.plan_key(self) if self.tiles_fit() else PortionAttention.plan_key(self)
 
     def plan(self, batch):
-        return TiledAttention.plan(self, batch) if self.tiles_fit() else PortionAttention.plan(self, batch)
+        return TiledAttention.plan(self, batch, alongside=False) if self.tiles_fit() else PortionAttention.plan(self, batch)
 
     def attend_tiles(self, q, kv, bt, ctx, out, plan, gate, turn=None):
         """The step's attention on the tile kernels: the single next tokens at the head of the batch through the

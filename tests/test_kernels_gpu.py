@@ -669,6 +669,42 @@ def test_prefill_attention_tc(H, K, d, P, window):
     assert np.abs(out.float().cpu().numpy() - want).max() < 1e-2 * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("H,K,d,P,n,portion,splits", [(8, 2, 128, 64, 1, 17, 1), (8, 2, 128, 64, 20, 300, 4), (28, 4, 128, 64, 3, 256, 1),
+                                                       (6, 2, 64, 16, 5, 1, None), (40, 8, 128, 64, 9, 512, 1)])
+def test_decode_and_portion_attention_side_by_side(H, K, d, P, n, portion, splits):
+    """The decode kernel launched alongside the portions' kernel gives the bits that the two give one after the other: what it
+    reads is written by the launch right ahead of the two, what they write is read by the one right behind, over and over
+    with new numbers.  The first row is padding in every second case."""
+    lens, q_lens = [200 + 7 * i for i in range(n)] + [portion + 90], [1] * n + [portion]
+    q, cache, bt, positions, seq_of, _, _ = paged_case(H, K, d, P, lens, q_lens, "bfloat16", seed=n + portion, num_pages=140)
+    cache, bt, seq, pos, tiles = dev(cache, torch.bfloat16), dev(bt), dev(seq_of), dev(positions), dev(tiles_for(lens, q_lens)[16 * n:])
+    if portion % 2:
+        seq[0] = -1
+    scale, status = d ** -0.5, torch.zeros(1, dtype=torch.int32, device="cuda")
+    queries = [dev(q) * (1 + i % 3) for i in range(6)]
+    rows = torch.empty(q.shape, dtype=torch.bfloat16, device="cuda")
+    out = torch.zeros(q.shape, dtype=torch.bfloat16, device="cuda")
+    more = dict(splits=splits, status=status)
+    want = []
+    for x in queries:
+        ops().convert(x, rows)
+        torch.cuda.synchronize()
+        ops().decode_attention(rows[:n], cache, bt, seq[:n], pos[:n], out[:n], 0, scale, **more)
+        torch.cuda.synchronize()
+        ops().prefill_attention_tc(rows, cache, bt, tiles, out, 0, scale, status=status)
+        want.append(out.float())
+    got = [torch.empty(q.shape, device="cuda") for _ in queries]
+    for _ in range(5):
+        for x, y in zip(queries, got):
+            ops().convert(x, rows)
+            ops().prefill_attention_tc(rows, cache, bt, tiles, out, 0, scale, status=status)
+            ops().decode_attention(rows[:n], cache, bt, seq[:n], pos[:n], out[:n], 0, scale, alongside=True, **more)
+            ops().convert(out, y)
+        for x, y in zip(want, got):
+            assert torch.equal(x, y)
+    assert status.item() == 0
+
+
 def streams_of(tiles, window):
     """Key tiles in the stream of every pair of a tile list (as the kernel counts them)."""
     out = []

@@ -382,3 +382,31 @@ def test_segments_cover_every_stream_exactly_once():
     # a whole prompt of 2,048 tokens: 224 items of graded length fill the SMs as they are; nothing to plan either
     assert plan_segments([4 * p + 4 for p in range(8)], 28) is None
     assert plan_segments([], 4) is None and plan_segments([2], 2) is None
+
+
+def test_which_mixed_steps_run_their_two_attention_kernels_side_by_side():
+    """Only with single tokens ahead of portions whose whole items leave SMs free, and where items that would have been cut
+    do not hold the step up for longer than that saves; then nothing is cut."""
+    from air_b200.parts.attention import TiledAttention
+    from air_b200.parts.base import HostBatch
+
+    def plan(heads, decoders, context, portion, prefix, window=None):
+        part = TiledAttention()
+        part.heads, part.kv_heads, part.head_dim, part.window = heads, 8, 128, window
+        counts = [1] * decoders + ([portion] if portion else [])
+        starts = [0]
+        for c in counts:
+            starts.append(starts[-1] + c)
+        batch = HostBatch(counts=counts, lengths=[context] * decoders + [prefix] * bool(portion), slots=list(range(len(counts))),
+                          q_start=starts)
+        return part.plan(batch)
+
+    for args, alongside, cut in (((40, 32, 8192, 512, 3840), True, False), ((40, 0, 0, 512, 3840), False, True),
+                                 ((40, 8, 8192, 512, 3840), True, False), ((40, 32, 20, 512, 3840), False, True),
+                                 ((40, 32, 8192, 1024, 3840), False, True), ((28, 2, 8192, 256, 32640), False, True),
+                                 ((40, 32, 8192, 512, 3840, 100), True, False), ((8, 2, 30, 17, 0), True, False),
+                                 ((8, 2, 30, 0, 0), False, False)):
+        p = plan(*args)
+        assert p.values["alongside"] == alongside, args
+        assert (p.arrays.get("segments") is not None) == cut, args
+        assert p.values["decode_prefix"] == args[1]
