@@ -32,6 +32,10 @@ class PortionAttention:
     def plan_key(self):
         return None if self.rt.is_fp32 else (self.PLAN,)
 
+    def portions_key(self):
+        """Where `attend` finds this class's plan (a mixer may plan some of its steps in another manner, under plan_key)."""
+        return PortionAttention.plan_key(self)
+
     def plan(self, batch: HostBatch) -> Plan:
         """portions: (first row, tokens, first position, slot) of the entries that the products take; small_seq
         [T] int32: the slot of every other row, -1 at the portions' rows (the 32-bit kernel skips those)."""
@@ -67,7 +71,7 @@ class PortionAttention:
         sinks = getattr(self, "sinks", None)
         softcap = float(getattr(self, "softcap", 0.0) or 0.0)
         bias = getattr(self, "bias_table", None)
-        plan = ctx.plans.get(self.plan_key()) if not self.rt.is_fp32 else None
+        plan = ctx.plans.get(self.portions_key()) if not self.rt.is_fp32 else None
 
         def through_the_pages(token_seq):
             if (pages is not None and not latent and not self.chunk and q.dtype == torch.bfloat16

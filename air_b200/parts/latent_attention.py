@@ -138,6 +138,9 @@ class LatentAttention(PortionAttention, Mixer):
         key = super().plan_key()
         return key + ("expanded", self.heads, self.window) if key is not None and self.expands else key
 
+    def portions_key(self):
+        return self.plan_key()
+
     def plan(self, batch: HostBatch) -> Plan:
         """PortionAttention's plan; where this layer expands, the portions that it expands are in `expanded` instead: (first
         row, tokens, first position, slot, number of slots of partial sums), their tile lists in tiles<i>, segments<i> and
