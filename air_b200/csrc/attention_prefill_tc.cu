@@ -39,7 +39,7 @@
 // With DK > 0 the keys and values do not come from pages: they are the expansion of a request's compressed latents, worked out
 // for the portion ahead of this kernel.  kv [keys, H * 2 D] holds, per key (the first one is position key_origin) and head, D
 // numbers of the key and the D numbers of the value; where DK > D the last DK - D numbers of a key are the same for all heads
-// and lie in the latents' rows behind the latent (map_k2, column k2_column).  A query's last DK - D numbers come from q2 [T, H
+// and lie in the latents' rows behind the latent (ex.k2, column k2_column).  A query's last DK - D numbers come from q2 [T, H
 // * (DK - D)] in the same way.  A stage is then DK + D numbers wide, and three of them are what fits beside the queries.
 //
 // tiles, q, out, cache, block_table, window as in attention_prefill.cu; the list pads every request
@@ -123,11 +123,14 @@ struct RowTile {
 
 constexpr int at_stages(int d, int dk) { return dk > d ? 3 : AT_STAGES; }
 
+// What the kernel needs beside its arguments where keys come from an expansion (DK > 0: see the head of this file).
+template <int DK> struct Expanded { CUtensorMap q2, k2; int key_origin, k2_column; };
+template <> struct Expanded<0> { int none; };
+
 template <int D, bool BIAS, int DK>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_cache,
-                            const __grid_constant__ CUtensorMap map_q2, const __grid_constant__ CUtensorMap map_k2,
-                            int key_origin, int k2_column, const int* __restrict__ block_table, int max_blocks, const int* __restrict__ tiles,
+                            const __grid_constant__ Expanded<DK> ex, const int* __restrict__ block_table, int max_blocks, const int* __restrict__ tiles,
                             int n_pairs, const int* __restrict__ segments, int n_slots, float* __restrict__ part_o,
                             float2* __restrict__ part_ml, __nv_bfloat16* __restrict__ out, int H, int K, int P,
                             int window, float scale_log2, float cap, float cap_pre, int* __restrict__ status,
@@ -250,7 +253,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 for (int s = 0; s < SUBK; ++s) {
                     uint8_t* dst = sq + x * Q_BYTES + s * AT_BM * 128;
                     if (s < SUB) tma_load_2d(dst, &map_q, h * D + 64 * s, tok0 + x * AT_BM, q_full);
-                    else tma_load_2d(dst, &map_q2, h * (64 * (SUBK - SUB)) + 64 * (s - SUB), tok0 + x * AT_BM, q_full);
+                    else if constexpr (EXPANDED) tma_load_2d(dst, &ex.q2, h * (64 * (SUBK - SUB)) + 64 * (s - SUB), tok0 + x * AT_BM, q_full);
                 }
             const int box_rows = P < AT_BN ? P : AT_BN;
             const int boxes = AT_BN / box_rows;
@@ -261,11 +264,11 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 if constexpr (EXPANDED) {        // (rows beyond the last key come as zeros)
                     mbar_expect_tx(&kv_full[stage], (uint32_t)STAGE_BYTES);
                     uint8_t* to = skv + stage * STAGE_BYTES;
-                    const int row = kbase - key_origin;
+                    const int row = kbase - ex.key_origin;
 #pragma unroll
                     for (int s = 0; s < SUBK + SUB; ++s, to += KV_SUB) {
                         if (s < SUB) tma_load_2d(to, &map_cache, h * 2 * D + 64 * s, row, &kv_full[stage]);
-                        else if (s < SUBK) tma_load_2d(to, &map_k2, k2_column + 64 * (s - SUB), row, &kv_full[stage]);
+                        else if (s < SUBK) tma_load_2d(to, &ex.k2, ex.k2_column + 64 * (s - SUB), row, &kv_full[stage]);
                         else tma_load_2d(to, &map_cache, h * 2 * D + D + 64 * (s - SUBK), row, &kv_full[stage]);
                     }
                     continue;
@@ -652,10 +655,9 @@ static int make_map_2d(CUtensorMap* map, const void* base, long long rows, long 
     return tensor_map_2d(map, base, rows, cols, box_rows);
 }
 
-struct Expanded { CUtensorMap q2, k2; int key_origin, k2_column; };      // (DK > 0: see the head of this file)
 
 template <int D, int DK = 0>
-int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mc, const Expanded& ex, const int* block_table, int max_blocks,
+int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mc, const Expanded<DK>& ex, const int* block_table, int max_blocks,
                       const int* tiles, int n_tiles, const int* segments, int n_segments, const int* items, int n_items,
                       int n_slots, float* part_o, float* part_ml, void* out, int H, int K, int P, int window, float scale,
                       float softcap, int* status, cudaStream_t stream, const float* sink, const DistanceBias& bias) {
@@ -672,7 +674,7 @@ int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mc, const Expand
     if (e != cudaSuccess) return (int)e;
     const int n_pairs = n_tiles / (AT_GROUP * AT_ROW_TILES);
     const dim3 grid = segments ? dim3(n_segments) : dim3(H, n_pairs);
-    int rc = launch(kernel, grid, AT_THREADS, smem, stream, mq, mc, ex.q2, ex.k2, ex.key_origin, ex.k2_column, block_table, max_blocks, tiles, n_pairs, segments,
+    int rc = launch(kernel, grid, AT_THREADS, smem, stream, mq, mc, ex, block_table, max_blocks, tiles, n_pairs, segments,
                     n_slots, part_o, (float2*)part_ml, (__nv_bfloat16*)out, H, K, P, window,
                     (softcap > 0.f ? 1.f : scale) * 1.4426950408889634f, softcap > 0.f ? softcap : 0.f,
                     softcap > 0.f ? scale / softcap : 0.f, status, sink, bias);
@@ -707,7 +709,7 @@ static int prefill_attention_tc_any(const void* q, int T, const void* cache, lon
     if (rc) return rc;
     rc = make_map_2d(&mc, cache, pages * 2 * K * P, D, P < AT_BN ? P : AT_BN);
     if (rc) return rc;
-    const Expanded none{mq, mc, 0, 0};
+    const Expanded<0> none{0};
     if (D == 64)
         return launch_prefill_tc<64>(mq, mc, none, block_table, max_blocks, tiles, n_tiles, segments, n_segments, items, n_items,
                                      n_slots, part_o, part_ml, out, H, K, P, window, scale, softcap, status, stream, sink, bias);
@@ -761,10 +763,10 @@ AIR_API int air_prefill_attention_expanded(const void* q, const void* q2, int T,
     if (rc) return rc;
     rc = make_map_2d(&mkv, kv, keys, (long long)H * 256, AT_BN);
     if (rc) return rc;
-    Expanded ex{mq, mkv, key_origin, k2_column};
+    Expanded<192> ex{mq, mkv, key_origin, k2_column};
     const DistanceBias bias{nullptr, 0};
     if (rot == 0)
-        return launch_prefill_tc<128, 128>(mq, mkv, ex, nullptr, 0, tiles, n_tiles, segments, n_segments, items, n_items, n_slots,
+        return launch_prefill_tc<128, 128>(mq, mkv, Expanded<128>{mq, mkv, key_origin, k2_column}, nullptr, 0, tiles, n_tiles, segments, n_segments, items, n_items, n_slots,
                                            part_o, part_ml, out, H, H, AT_BN, window, scale, 0.f, status, stream, sink, bias);
     rc = make_map_2d(&ex.q2, q2, T, (long long)H * rot, AT_BM);
     if (rc) return rc;

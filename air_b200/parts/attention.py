@@ -193,16 +193,11 @@ class TiledAttention:
         # prompt portions the tile kernels
         plan = ctx.plans[self.plan_key()]
         n = plan.decode_prefix
-        # (nothing between the two launches, and no memory that the first one reads is given back between them)
+        # (side by side: nothing between the two launches, and no memory that the first one reads is given back between them)
         alongside = plan.alongside and d in ops.TC_ATTENTION_HEAD_DIMS
-
-        def decode():
-            if n:
-                ops.decode_attention(q[:n], kv, bt, ctx.token_seq[:n], ctx.positions[:n], out[:n], self.window,
-                                     self.scale, softcap=self.softcap, alongside=alongside)
-
-        if not alongside:
-            decode()
+        if n and not alongside:
+            ops.decode_attention(q[:n], kv, bt, ctx.token_seq[:n], ctx.positions[:n], out[:n], self.window,
+                                 self.scale, softcap=self.softcap)
         if plan.tiles.shape[0] == 0:
             pass
         elif d in ops.TC_ATTENTION_HEAD_DIMS:     # both products on the tcgen05 tensor cores
@@ -215,7 +210,8 @@ class TiledAttention:
         else:
             ops.prefill_attention(q, kv, bt, plan.tiles, out, self.window, self.scale, status=ctx.status)
         if alongside:
-            decode()
+            ops.decode_attention(q[:n], kv, bt, ctx.token_seq[:n], ctx.positions[:n], out[:n], self.window,
+                                 self.scale, softcap=self.softcap, alongside=True)
         return out
 
 
