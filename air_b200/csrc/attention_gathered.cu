@@ -5,7 +5,8 @@
 //
 // gather_keys_kernel: keys lo .. lo + L of one request from its pages into dense blocks.  Paged keys and values: a
 //   page holds the keys [G, P, dk] and then the values [G, P, dv]; out: K [G, Lp, dk], V [G, Lp, dv].  Latent rows: a
-//   page is [P, dk]; out: K [1, Lp, dk] only (the values are its first columns).  Rows L .. Lp are zeroed.
+//   page is [P, dk]; out: K [1, Lp, dk] only (the values are its first columns).  Rows 0 .. ahead and L .. Lp are zeroed, and
+//   so is the row of a key whose page the request has given back (-1 in its table).
 //
 // masked_softmax_kernel: S [G, n * J, Lp] float32 (row (t, j): token t of the portion, head g * J + j) -> weights of the
 //   same shape in bfloat16.  Column c is the key at position lo + c; the query of token t stands at pos0 + t and sees
@@ -20,19 +21,18 @@ namespace air {
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-gather_keys_kernel(const T* __restrict__ cache, const int* __restrict__ block_table, int lo, int L, int Lp, int G,
-                   int dk, int dv, int P, int latent, T* __restrict__ K, T* __restrict__ V) {
+gather_keys_kernel(const T* __restrict__ cache, const int* __restrict__ block_table, int lo, int ahead, int L, int Lp,
+                   int G, int dk, int dv, int P, int latent, T* __restrict__ K, T* __restrict__ V) {
     pdl_enter(TR_GATHER_KEYS);
-    const int c = blockIdx.x;
-    if (c >= L) {
+    const int c = blockIdx.x, key = lo + c;
+    const int page = c < ahead || c >= L ? -1 : block_table[key / P];
+    if (page < 0) {
         for (int i = threadIdx.x; i < G * dk; i += blockDim.x) K[((size_t)(i / dk) * Lp + c) * dk + i % dk] = from_float<T>(0.f);
         if (V)
             for (int i = threadIdx.x; i < G * dv; i += blockDim.x)
                 V[((size_t)(i / dv) * Lp + c) * dv + i % dv] = from_float<T>(0.f);
         return;
     }
-    const int key = lo + c;
-    const int page = block_table[key / P];
     const int place = key % P;
     if (latent) {
         const T* src = cache + ((size_t)page * P + place) * dk;
@@ -89,12 +89,12 @@ masked_softmax_kernel(const float* __restrict__ S, __nv_bfloat16* __restrict__ W
 
 }  // namespace air
 
-AIR_API int air_gather_keys(const void* cache, int dtype, const int* block_table, int lo, int L, int Lp, int G, int dk,
-                            int dv, int P, int latent, void* K, void* V, cudaStream_t stream) {
+AIR_API int air_gather_keys(const void* cache, int dtype, const int* block_table, int lo, int ahead, int L, int Lp, int G,
+                            int dk, int dv, int P, int latent, void* K, void* V, cudaStream_t stream) {
     if (Lp <= 0) return 0;
-    if (L > Lp || lo < 0 || G <= 0 || (latent && G != 1) || (!latent && !V)) return AIR_ERR_BAD_ARGUMENT;
+    if (L > Lp || lo < 0 || ahead < 0 || G <= 0 || (latent && G != 1) || (!latent && !V)) return AIR_ERR_BAD_ARGUMENT;
     AIR_DISPATCH(dtype, TT, return air::launch(air::gather_keys_kernel<TT>, Lp, 128, 0, stream, (const TT*)cache,
-                                               block_table, lo, L, Lp, G, dk, dv, P, latent, (TT*)K, (TT*)V));
+                                               block_table, lo, ahead, L, Lp, G, dk, dv, P, latent, (TT*)K, (TT*)V));
     return 0;
 }
 

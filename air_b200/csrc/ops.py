@@ -65,8 +65,7 @@ _SIGNATURES = {
     "air_grouped_attention": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                               c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_int,
                               c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p],
-    "air_gather_keys": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
-                        c_void_p, c_void_p],
+    "air_gather_keys": [c_void_p, c_int, c_void_p] + [c_int] * 9 + [c_void_p, c_void_p, c_void_p],
     "air_masked_softmax": [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                            c_void_p, c_float, c_void_p, c_int, c_void_p],
     "air_moe_route": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int,
@@ -560,10 +559,10 @@ def grouped_attention(q, cache, block_table, token_seq, positions, out, window, 
     return out
 
 
-def gather_keys(cache, table_row, lo, count, keys, values, kv_heads=1, page_tokens=None, latent=False):
+def gather_keys(cache, table_row, lo, count, keys, values, kv_heads=1, page_tokens=None, latent=False, ahead=0):
     """The keys lo .. lo + count of the request whose block-table row is table_row, from the pages into keys
-    [G, Lp, dk] (and values [G, Lp, dv]; latent: cache [pages, P, dk], keys [1, Lp, dk], no values).  Rows count .. Lp
-    are zeroed."""
+    [G, Lp, dk] (and values [G, Lp, dv]; latent: cache [pages, P, dk], keys [1, Lp, dk], no values).  Rows 0 .. ahead and
+    count .. Lp are zeroed, and so are the rows of keys whose page the request has given back."""
     G, Lp, dk = keys.shape
     _req(keys, "keys", _FLOATS)
     _req(cache, "cache", (keys.dtype,))
@@ -574,8 +573,8 @@ def gather_keys(cache, table_row, lo, count, keys, values, kv_heads=1, page_toke
     else:
         _req(values, "values", (keys.dtype,), (G, Lp, None))
         dv, P = values.shape[2], int(page_tokens)
-    _check(_get("air_gather_keys")(cache.data_ptr(), _DT[keys.dtype], table_row.data_ptr(), int(lo), int(count), Lp,
-                                   int(kv_heads), dk, dv, P, 1 if latent else 0, keys.data_ptr(),
+    _check(_get("air_gather_keys")(cache.data_ptr(), _DT[keys.dtype], table_row.data_ptr(), int(lo), int(ahead),
+                                   int(count), Lp, int(kv_heads), dk, dv, P, 1 if latent else 0, keys.data_ptr(),
                                    None if latent else values.data_ptr(), _stream()), "gather_keys")
 
 

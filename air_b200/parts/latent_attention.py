@@ -167,14 +167,21 @@ class LatentAttention(PortionAttention, Mixer):
         plan.values.update(portions=kept, expanded=expanded, rows=rows)
         return plan
 
+    def expanded_keys(self, pos0: int, n: int):
+        """What is expanded for a portion of n tokens at pos0: (the first row's position, rows that stand ahead of the first
+        visible key, rows).  The attention kernel's tiles want the first row at a multiple of 64; the keys from there to the
+        first visible one may lie in pages that the request has given back, so their rows are zeros."""
+        first = self.first_visible(pos0)
+        origin = first // 64 * 64
+        return origin, first - origin, pos0 + n - origin
+
     def _attend_expanded(self, plan, q, q_rot, latent, bt, ctx, out):
         """out rows of the plan's expanded portions."""
         for i, (r0, n, pos0, slot, slots) in enumerate(plan.expanded):
-            lo = self.first_visible(pos0) // 64 * 64
-            count = pos0 + n - lo
+            lo, ahead, count = self.expanded_keys(pos0, n)
             keys = -(-count // 16) * 16
             rows = torch.empty((1, keys, self.rank + self.rot_dim), dtype=torch.bfloat16, device=q.device)
-            ops.gather_keys(latent.rows, bt[slot], lo, count, rows, None, latent=True)
+            ops.gather_keys(latent.rows, bt[slot], lo, count, rows, None, latent=True, ahead=ahead)
             kv = torch.mm(rows[0, :, :self.rank], self.expansion[0].t())
             cut = getattr(plan, f"segments{i}", None)
             ops.prefill_attention_expanded(q, q_rot, kv, rows[0], self.rank, lo, getattr(plan, f"tiles{i}"), out, self.window,

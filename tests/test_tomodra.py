@@ -114,3 +114,41 @@ def test_plain_mechanisms_against_closed_forms():
     s = plain.sigmoid(0.5)
     y = plain.mixture(u, w, "", dict(router=dict(experts=1, top=1)))
     assert np.allclose(y, plain.expert(s * u, w, "e0.")) and not np.allclose(y, s * plain.expert(u, w, "e0."))
+
+
+@pytest.mark.parametrize("page", [16, 32, 48, 64, 128])
+@pytest.mark.parametrize("window", [70, 1000, 4096])
+def test_an_expanded_portion_reads_pages_that_the_request_still_holds(window, page, monkeypatch):
+    """Portions of latent layers with a window behind every remainder of a tile of 64 keys: what is gathered from the pages
+    lies in blocks that the cache has not taken back, and the rows ahead of it are filled up to the tile."""
+    from types import SimpleNamespace
+    import torch
+    from air_b200.cache.manager import CacheManager
+    from air_b200.csrc import ops
+    from air_b200.parts.base import HostBatch, Runtime
+    from air_b200.parts.latent_attention import LatentAttention
+    from air_b200.parts.spec import PartSpec
+    n, R = 100, 8
+    part = LatentAttention(PartSpec("latent_attention", {
+        "hidden": 16, "heads": 1, "head_dim": 128, "rot_dim": 0, "v_dim": 128, "kv_rank": R, "scale": 0.1, "window": window}), "m.")
+    part.rt, part.expansion = Runtime(device=torch.device("cpu"), dtype=torch.bfloat16, page_tokens=page), (torch.zeros(256, R).bfloat16(),)
+    gathered = []
+    monkeypatch.setattr(ops, "gather_keys", lambda cache, table, lo, count, rows, *a, ahead=0, **k: gathered.append((lo, ahead, count)))
+    monkeypatch.setattr(ops, "prefill_attention_expanded", lambda *a, **k: None)
+    cache = CacheManager([part.cache_needs()], page, 400, 1, allocate=False)
+    seq = cache.open("r")
+    for behind in (4990, 10) + (1,) * 66:
+        cache.reserve([("r", behind)])
+        cache.commit("r", behind)
+        cache.reserve([("r", n)])                       # the portion's own pages
+        pos0 = seq.length
+        plan = part.plan(HostBatch(counts=[n], lengths=[pos0], slots=[0], q_start=[0, n]))
+        assert len(plan.values["expanded"]) == 1
+        part._attend_expanded(SimpleNamespace(**plan.values, **{k: None for k in plan.arrays}), torch.zeros(n, 1, 128), None,
+                              SimpleNamespace(rows=None), [None], SimpleNamespace(status=None), None)
+        lo, ahead, count = gathered.pop()
+        first = max(0, pos0 - window + 1)
+        assert lo % 64 == 0 and lo <= first < lo + 64 and lo + count == pos0 + n
+        assert lo + ahead <= first, "every key that a query sees is gathered"
+        assert all(seq.pages[0][key // page] >= 0 for key in range(lo + ahead, lo + count)), (pos0, lo, ahead)
+        cache.trim("r")

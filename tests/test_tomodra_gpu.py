@@ -533,6 +533,79 @@ def test_greedy_generation_through_the_service(name):
     engine.check_status()
 
 
+@pytest.mark.parametrize("page", [16, 48, 64])
+@pytest.mark.parametrize("W,reader_W,R", [(70, 100, 40), (200, 131, 64), (1000, 70, 512)])
+def test_latent_layers_in_portions_over_expanded_keys(W, reader_W, R, page):
+    """A latent layer with heads of 128 + 64 and values of 128 and one that reads its rows through another window, alone in a
+    bfloat16 engine: two requests in steps of portions that are expanded, shorter ones and single tokens, against the plain
+    function on each whole sequence.  Pages go back to the pool as the windows pass; what no token was written to is NaN."""
+    from air_b200.cache.manager import CacheManager
+    from air_b200.config import load_config
+    from air_b200.engine.batch import Entry, build_context
+    from air_b200.parts import registry
+    from air_b200.parts.base import Runtime
+    E, eps, H = 64, 1e-5, (2, 3)
+    layers = [tu.with_mlp(tu.latent(H[0], 128, 64, 128, R, W, 0.08)),
+              tu.with_mlp(tu.latent(H[1], 128, 64, 128, R, reader_W, 0.1, kv_from=0))]
+    cfg = tu.config(20, E, eps, 1.0, layers)
+    w = {n: a.astype(np.float64) for n, a in tu.draw_tensors(cfg, R + page).items()}
+    spec = registry.architecture("Tomodra").build_spec(load_config(cfg))
+    rt = Runtime(torch.device(DEV), torch.bfloat16, page, status=torch.zeros(1, dtype=torch.int32, device=DEV))
+    parts = []
+    for i in (0, 1):
+        part = registry.MIXERS.get("latent_attention")(spec.layers[i].parts["mixer"], f"l{i}.mix.")
+        part.load({n: dev(a, torch.float32 if n.endswith("norm") else torch.bfloat16) for n, a in w.items()}, rt)
+        assert part.expands
+        parts.append(part)
+    rng = np.random.default_rng(R + W)
+    streams = {"a": tu.bf16(rng.normal(size=(620, E))).astype(np.float64), "b": tu.bf16(rng.normal(size=(170, E))).astype(np.float64)}
+    want = {}
+    for r, x in streams.items():
+        at = np.arange(len(x))
+        kept = plain.latent_kv(x, w, "l0.mix.", layers[0]["mixer"], eps, at)
+        want[r] = [plain.latent_attention(x, w, f"l{i}.mix.", layers[i]["mixer"], eps, at, kept) for i in (0, 1)]
+    cache = CacheManager([parts[0].cache_needs()], page, 64, 3, dtype=torch.bfloat16, device=DEV)
+    (view,) = cache.views(0)
+    view.rows.fill_(float("nan"))
+    for r in ("other", "a", "b"):
+        cache.open(r)
+    done, expanded = {"a": 0, "b": 0}, 0
+    for step in ([("a", 200)], [("b", 1), ("a", 1)], [("a", 64), ("b", 65)], [("b", 1), ("a", 129)], [("a", 33), ("b", 2)], [("b", 64)],
+                 [("a", 1), ("b", 36)], [("a", 115), ("b", 1)], [("a", 77)]):
+        cache.reserve(step)
+        x = np.concatenate([streams[r][done[r]:done[r] + n] for r, n in step])
+        ctx = build_context([Entry(r, [0] * n, []) for r, n in step], cache, DEV, status=rt.status,
+                            planners=list({p.plan_key(): p for p in parts}.values()))
+        expanded += len(ctx.plans[parts[0].plan_key()].expanded)
+        for i, part in enumerate(parts):
+            y = part.forward(dev(x, torch.bfloat16), ctx, cache.views(0), i == 0)
+            y = (y.sum(0) if y.dim() == 3 else y).cpu().numpy()
+            at = 0
+            for r, n in step:
+                ref = want[r][i][done[r]:done[r] + n]
+                assert np.abs(y[at:at + n] - ref).max() < 4e-2 * max(1.0, np.abs(want[r][i]).max()), (i, step, r)
+                at += n
+        for r, n in step:
+            cache.commit(r, n)
+            done[r] += n
+    assert done == {"a": 620, "b": 170} and expanded == 7 and rt.status.item() == 0
+    assert max(W, reader_W) > 600 or min(cache.sequences["a"].pages[0]) == -1, "pages were given back"
+
+
+@pytest.mark.parametrize("page", [16, 48, 64])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_expanded_latents_and_wide_experts_in_every_schedule(dtype, page):
+    """Configuration D whole, in portions and in mixed steps: latents expanded for portions of 64 tokens and more behind windows,
+    gated experts as a stream of weights with planes per part of k through the norms, also in replayed decode steps."""
+    lengths = (2, 65, 230, 420, 131)
+    streams = streams_for("D", 90, lengths)
+    for steps, requests in ((util.trace_whole(streams), 4), (util.trace_bulk_tail(streams, tail=40), 4),
+                            (util.trace_portions(streams, sizes=(100, 1, 64, 65, 2, 33, 128)), 4),
+                            (util.trace_mixed(streams, seed=6, live=3, portions=(2, 70, 100, 33, 128)), 3)):
+        got, _ = replay("D", dtype, steps, page_tokens=page, max_requests=requests, peak_page=192)
+        tu.check(got, "D", streams, dtype)
+
+
 def test_trace_runner_program_and_command_line(capsys):
     """bin/trace_run as a program on a Tomodra folder (the class is chosen by config.json), and the command line."""
     name = "B"

@@ -44,6 +44,8 @@ def config(vocab, width, eps, alpha, layers):
 #    whole head rotated without stretching, every expert chosen (top == experts), a window wider than any prompt, a
 #    chunk of one page, a window of 1 (a token sees itself only).
 # C: heads of 64 and 128 with values of the same size, chunks of 64 and 128, a latent of 64 + 32, pages of 64.
+# D: latent heads of 128 + 64 with values of 128, whose longer portions are expanded, through windows that are no multiples of
+#    a tile, one of them over another layer's rows; experts wide enough for the stream of weights and its parts of k.
 CONFIGS = {
     "A": config(211, 64, 1e-5, 2.0, [
         with_mlp(latent(4, 24, 8, 20, 40, 48, 0.2), 5, 2, 48, 40),
@@ -61,8 +63,12 @@ CONFIGS = {
         with_mlp(latent(4, 64, 32, 64, 64, 100, 0.1), 6, 2, 64, 128),
         with_mlp(attention(2, 1, 128, 128, 128, 0.09, 128, 1e6), 6, 1, 64, 128),
         with_mlp(latent(2, 32, 32, 32, 64, 64, 0.12, kv_from=1), 6, 2, 64)]),
+    "D": config(200, 128, 1e-6, 3.0, [
+        with_mlp(latent(2, 128, 64, 128, 64, 100, 0.08), 6, 2, 1024, 128),
+        with_mlp(latent(2, 128, 64, 128, 64, 180, 0.07, kv_from=0)),
+        with_mlp(latent(3, 128, 64, 128, 72, 70, 0.09, base=1e6), 5, 1, 1024)]),
 }
-SEEDS = {"A": 21, "B": 22, "C": 23}
+SEEDS = {"A": 21, "B": 22, "C": 23, "D": 24}
 
 
 def random_config(seed):
