@@ -162,6 +162,14 @@ def test_latent_attention_without_positions_with_sink_and_gates(H, d, dv, R, pag
     assert np.abs(got - want).max() < tol * max(1.0, np.abs(want).max()), float(np.abs(got - want).max())
 
 
+@pytest.mark.parametrize("H,R,page", [(2, 40, 16), (3, 512, 64), (1, 8, 48)])
+def test_portions_over_expanded_latents_with_sink_and_gates(H, R, page):
+    """The same with heads and values of 128, whose portions of 64 tokens and more are expanded."""
+    from air_b200.parts.latent_attention import LatentAttention
+    assert LatentAttention.EXPAND == 64
+    test_latent_attention_without_positions_with_sink_and_gates(H, 128, 128, R, page, "bfloat16")
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_latent_attention_finds_a_key_far_away_and_at_page_borders(dtype):
     """Keys and queries are made by hand: the latent of tokens 0, 15, 16 and 200 each lies along an axis of its own,
