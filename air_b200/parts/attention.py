@@ -121,8 +121,10 @@ class TiledAttention:
     # ------------------------------------------------------------------ the step's plan
     PLAN = "attention.tiles"
 
-    def plan_key(self):
-        return (self.PLAN, self.heads, self.window)
+    def plan_key(self, alongside=True):
+        """All that the plan depends on, since layers of one key share it (`alongside` as in plan)."""
+        key = (self.PLAN, self.heads, self.window)
+        return key + (self.kv_heads, self.head_dim) if alongside else key
 
     def plan(self, batch: HostBatch, alongside=True) -> Plan:
         """What the tile kernels want to know of a step, worked out once for all attention layers with this many

@@ -124,7 +124,7 @@ class NormedAttention(PortionAttention, Mixer):
                 and self.head_dim in ops.TC_ATTENTION_HEAD_DIMS and ops.tile_pages(self.rt.page_tokens))
 
     def plan_key(self):
-        return TiledAttention.plan_key(self) if self.tiles_fit() else PortionAttention.plan_key(self)
+        return TiledAttention.plan_key(self, alongside=False) if self.tiles_fit() else PortionAttention.plan_key(self)
 
     def plan(self, batch):
         return TiledAttention.plan(self, batch, alongside=False) if self.tiles_fit() else PortionAttention.plan(self, batch)
@@ -259,7 +259,7 @@ class NormedAttention(PortionAttention, Mixer):
         out = torch.empty((T, H, dv), dtype=rt.dtype, device=x.device)
         gate = full[:, C:] if self.out_gate else None
         turn = None if self.v_freq is None else (self.v_freq, pos.pairing)
-        plan = ctx.plans.get(TiledAttention.plan_key(self)) if self.tiles_fit() and not ctx.all_decode else None
+        plan = ctx.plans.get(self.plan_key()) if self.tiles_fit() and not ctx.all_decode else None
         if plan is not None:
             self.attend_tiles(q, pages.kv, bt, ctx, out, plan, gate, turn)
         else:

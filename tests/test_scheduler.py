@@ -410,3 +410,32 @@ def test_which_mixed_steps_run_their_two_attention_kernels_side_by_side():
         assert p.values["alongside"] == alongside, args
         assert (p.arrays.get("segments") is not None) == cut, args
         assert p.values["decode_prefix"] == args[1]
+
+
+def test_layers_share_a_plan_only_where_it_is_the_same_for_both():
+    """A mixed step's plan depends on the bytes of a key and on whether a layer's kernels may run side by side: layers that
+    differ there, with equal heads and windows, have plans of their own."""
+    from air_b200.parts.attention import TiledAttention
+    from air_b200.parts.base import HostBatch
+    from air_b200.parts.normed_attention import NormedAttention
+
+    def layer(kv_heads, head_dim, cls=TiledAttention, **more):
+        part = cls.__new__(cls)
+        part.heads, part.kv_heads, part.head_dim, part.window = 40, kv_heads, head_dim, None
+        part.__dict__.update(more)
+        return part
+
+    from types import SimpleNamespace
+    import torch
+    normed = layer(8, 128, NormedAttention, v_dim=128, chunk=None, rt=SimpleNamespace(dtype=torch.bfloat16, page_tokens=64, is_fp32=False))
+    assert normed.tiles_fit()
+    layers = [layer(8, 128), layer(8, 64), layer(1, 128), layer(8, 128), normed]
+    batch = HostBatch(counts=[1] * 8 + [512], lengths=[8192] * 8 + [3840], slots=list(range(9)), q_start=list(range(9)) + [520])
+    for a in layers:
+        for b in layers:
+            if a.plan_key() == b.plan_key():
+                p, q = a.plan(batch), b.plan(batch)
+                assert p.values == q.values and sorted(p.arrays) == sorted(q.arrays)
+    plans = {p.plan_key(): p.plan(batch) for p in layers}
+    assert len(plans) == 4 and len({p.values["alongside"] for p in plans.values()}) == 2
+    assert "segments" in plans[normed.plan_key()].arrays, "a layer whose kernels run in turn is cut as before"
