@@ -167,7 +167,7 @@ constexpr int FEW_ROWS = 16, FEW_COLS = 32, FEW_K = 64, FEW_LD = PARTS * FEW_K +
 template <int RM>
 __global__ void __launch_bounds__(384)
 gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                    float* __restrict__ C, int M, int N, int K, int cols) {
+                    float* __restrict__ C, int M, int N, int K, int cols, int w_ready) {
     constexpr int RN = 2;
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, workers = blockDim.x - COPIERS;
@@ -196,13 +196,13 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, co
                 gf_copy16(to + (row - row0 + cols) * FEW_LD, in_k ? src : A, in_k);
         }
     };
-    // (W is written by no kernel: its first stages are asked for before the predecessor has ended)
-    if (copies)
+    // (w_ready, a model's weights: their first stages are asked for before the predecessor has ended)
+    if (copies && w_ready)
         for (int s = 0; s < min(FEW_STAGES - 1, steps); ++s) bring(s, true, false);
     pdl_enter(TR_GEMM_F32);
     if (copies)
         for (int s = 0; s < FEW_STAGES - 1; ++s) {
-            if (s < steps) bring(s, false, true);
+            if (s < steps) bring(s, !w_ready, true);
             gf_commit();
         }
     const int warp = tid >> 5, lane = tid & 31, part = lane >> 3;
@@ -356,13 +356,14 @@ static int launch_f32_tiles(const float* A, const float* W, const float* bias, f
 }
 
 template <int RM>
-static int launch_f32_few(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int cols, cudaStream_t stream) {
+static int launch_f32_few(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int cols, int w_ready,
+                          cudaStream_t stream) {
     const int smem = FEW_STAGES * (cols + M) * FEW_LD * 4;
     const int warps = (cols + 15) / 16 * ((M + RM - 1) / RM);
     cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<RM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     return launch(gemm_f32_few_kernel<RM>, dim3((N + cols - 1) / cols), warps * 32 + COPIERS, smem, stream, A, W, bias, C, M, N, K,
-                  cols);
+                  cols, w_ready);
 }
 
 // How many outputs, over all of k, the fullest SM takes.
@@ -373,7 +374,8 @@ static double fullest(int M, int N, int BM, int BN, int CL) {
 
 }  // namespace air
 
-AIR_API int air_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
+// w_ready: W was complete before the launch ahead of this one was made (a model's weights): it may be read before that one ends.
+AIR_API int air_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int w_ready,
                          cudaStream_t stream) {
     using namespace air;
     if (M <= 0 || N <= 0) return 0;
@@ -388,9 +390,9 @@ AIR_API int air_gemm_f32(const float* A, const float* W, const float* bias, floa
     // blocks at 1,024 columns.)
     if (M <= FEW_ROWS) {
         const int cols = max(1, min(FEW_COLS, (N + 147) / 148));
-        if (M == 1) return launch_f32_few<1>(A, W, bias, C, M, N, K, cols, stream);
-        if (M == 2) return launch_f32_few<2>(A, W, bias, C, M, N, K, cols, stream);
-        return launch_f32_few<4>(A, W, bias, C, M, N, K, cols, stream);
+        if (M == 1) return launch_f32_few<1>(A, W, bias, C, M, N, K, cols, w_ready, stream);
+        if (M == 2) return launch_f32_few<2>(A, W, bias, C, M, N, K, cols, w_ready, stream);
+        return launch_f32_few<4>(A, W, bias, C, M, N, K, cols, w_ready, stream);
     }
     // Tiles of 64 x 64 wherever they share out as evenly over the SMs as tiles of 32 x 64 do, whose outputs cost an eighth more
     // to feed.  (32 rows by 16,384 x 2,048: 77 us against 125; 300 by 3,072 x 2,048: 126 against 111.  Tiles of 128 columns or

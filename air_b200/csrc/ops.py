@@ -31,7 +31,7 @@ _SIGNATURES = {
                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "air_silu_mul": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "air_convert": [c_void_p, c_int, c_void_p, c_int, c_longlong, c_void_p],
-    "air_gemm_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+    "air_gemm_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "air_paged_attention_ref": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p,
                                 c_int, c_void_p, c_int, c_void_p],
@@ -414,8 +414,9 @@ def convert(src, out):
     return out
 
 
-def gemm_f32(a, w, bias, out):
-    """out[M, N] = a[M, K] @ w[N, K]^T + bias, all float32, on the CUDA cores."""
+def gemm_f32(a, w, bias, out, w_ready=False):
+    """out[M, N] = a[M, K] @ w[N, K]^T + bias, all float32, on the CUDA cores.  w_ready: w was complete before the launch ahead
+    of this one was made (a model's weights), so that it may be read while that one still runs."""
     M, K = a.shape
     N = w.shape[0]
     _req(a, "a", (torch.float32,))
@@ -423,8 +424,8 @@ def gemm_f32(a, w, bias, out):
     if bias is not None:
         _req(bias, "bias", (torch.float32,), (N,))
     _req(out, "out", (torch.float32,), (M, N))
-    _check(_get("air_gemm_f32")(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K, _stream()),
-           "gemm_f32")
+    _check(_get("air_gemm_f32")(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K,
+                              1 if w_ready else 0, _stream()), "gemm_f32")
     return out
 
 

@@ -136,7 +136,7 @@ class Linear:
             if x.dtype != torch.float32:
                 x = ops.convert(x, torch.empty(x.shape, dtype=torch.float32, device=x.device))
             out = torch.empty((x.shape[0], self.out_features), dtype=torch.float32, device=x.device)
-            ops.gemm_f32(x, w, bias, out)
+            ops.gemm_f32(x, w, bias, out, w_ready=True)
             if out_dtype != torch.float32:
                 out = ops.convert(out, torch.empty(out.shape, dtype=out_dtype, device=x.device))
             return out

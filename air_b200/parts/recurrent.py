@@ -314,7 +314,7 @@ class GatedLinearAttention(_ChunkedMixer):
         T, H, d, dv = x.shape[0], self.heads, self.head_dim, self.v_dim
         proj = self.proj.f32(x)
         z = torch.empty((T, H * d), dtype=torch.float32, device=x.device)
-        ops.gemm_f32(self._band(proj, "a1").contiguous(), self.a2, self.a2_bias, z)
+        ops.gemm_f32(self._band(proj, "a1").contiguous(), self.a2, self.a2_bias, z, w_ready=True)
         o = torch.empty((T, H, dv), dtype=torch.float32, device=x.device)
         self._scan(ops.SCAN_GLA, self._band(proj, "q"), self._band(proj, "k"), self._band(proj, "v"), z, state.state, o, ctx,
                    unit_lengths=False, q_scale=d ** -0.5, tau=self.tau)

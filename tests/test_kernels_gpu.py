@@ -301,6 +301,24 @@ def test_paged_attention_ref(H, K, d, P, window, dtype):
     assert np.abs(out.float().cpu().numpy() - want).max() < tol * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("M", [1, 4, 16])
+def test_gemm_f32_with_a_matrix_that_the_launches_ahead_write(M):
+    """Both operands come from the package's own kernels right ahead, over and over with new numbers: a matrix that is not a
+    model's weights is not read before it is there.  (Whole numbers: the products are exact.)"""
+    N, K = 5000, 1024
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randint(-3, 4, (M, K), generator=g, device="cuda").bfloat16()
+    ws = [torch.randint(-3, 4, (N, K), generator=g, device="cuda").bfloat16() for _ in range(4)]
+    w, x, outs = torch.empty(N, K, device="cuda"), torch.empty(M, K, device="cuda"), [torch.empty(M, N, device="cuda") for _ in ws]
+    for _ in range(10):
+        for b, out in zip(ws, outs):
+            ops().convert(b, w)
+            ops().convert(a, x)
+            ops().gemm_f32(x, w, None, out)
+        for b, out in zip(ws, outs):
+            assert torch.equal(out, a.float() @ b.float().T)
+
+
 @pytest.mark.parametrize("H,K,d,P", [(6, 2, 48, 16), (8, 2, 128, 64), (12, 1, 20, 48), (16, 16, 16, 16)])
 @pytest.mark.parametrize("window,chunk", [(0, None), (21, None), (0, 50)])
 def test_float32_attention_of_rows_together_is_that_of_rows_alone(H, K, d, P, window, chunk):
