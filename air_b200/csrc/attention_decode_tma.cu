@@ -28,7 +28,8 @@
 // and this kernel on the SMs that are left.  That kernel lets its successor start only when it has itself waited for
 // what is ahead of it, so everything that this one reads is complete when its first block starts, and it waits for nothing.
 // But what follows waits for this kernel alone: so its first block ends only when the portions' kernel has (one block:
-// the others leave their places to the blocks still to come).  What it gives: TiledAttention.beside (parts/attention.py).
+// the others leave their places to the blocks still to come).  Where the thread's last launch was another kernel, or was on
+// another stream, the request is ignored (last_launch) and every block waits as it does otherwise.  What it gives: TiledAttention.beside (parts/attention.py).
 #include "common.cuh"
 #include "mma.cuh"
 #include "tma.cuh"
@@ -496,6 +497,8 @@ static int decode_attention_tma(const FreshQkv& fresh, const void* q, const void
         return AIR_ERR_BAD_ARGUMENT;
     // a sink, gates or a turn back enter where the splits are merged: the keys are then split in two parts at least
     if (alongside && fresh.qkv) return AIR_ERR_BAD_ARGUMENT;
+    const LastLaunch& last = last_launch();
+    alongside = alongside && last.portions == last.count && last.stream == stream;
     const bool extra = sink || gate || turn.freq;
     if (extra && splits < 2) return AIR_ERR_BAD_ARGUMENT;
     CUtensorMap map;
@@ -528,8 +531,8 @@ static int decode_attention_tma(const FreshQkv& fresh, const void* q, const void
 }  // namespace air
 
 // Arguments as air_decode_attention (attention_decode.cu), plus the number of pages of the cache
-// (its first dimension), a soft cap (> 0: score = softcap * tanh(scale * q.k / softcap)), the status word, and whether the
-// launch right ahead is prefill_attention_tc_kernel's over other rows of the same step (alongside).
+// (its first dimension), a soft cap (> 0: score = softcap * tanh(scale * q.k / softcap)), the status word, and whether it
+// may run beside prefill_attention_tc_kernel over other rows of the same step (alongside), if that is the launch right ahead.
 AIR_API int air_decode_attention_tma(const void* q, const void* cache, long long pages, const int* block_table,
                                      int max_blocks, const int* token_seq, const int* positions, void* out,
                                      float* part_o, float* part_ml, int T, int H, int K, int D, int P, int window,

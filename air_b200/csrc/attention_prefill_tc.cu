@@ -678,6 +678,10 @@ int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mc, const Expand
                     n_slots, part_o, (float2*)part_ml, (__nv_bfloat16*)out, H, K, P, window,
                     (softcap > 0.f ? 1.f : scale) * 1.4426950408889634f, softcap > 0.f ? softcap : 0.f,
                     softcap > 0.f ? scale / softcap : 0.f, status, sink, bias);
+    if (rc == 0 && n_items <= 0) {
+        last_launch().portions = last_launch().count;      // (the single tokens' kernel may run beside this one)
+        last_launch().stream = stream;
+    }
     if (rc || !segments || n_items <= 0) return rc;
     return launch(prefill_combine_kernel<D>, dim3(n_items, AT_ROW_TILES * AT_BM / 8), 256, 0, stream, tiles, n_pairs,
                   items, n_slots, (const float*)part_o, (const float2*)part_ml, (__nv_bfloat16*)out, H, status, sink);

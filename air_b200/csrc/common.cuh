@@ -62,6 +62,20 @@ inline int set_trace_here(unsigned long long* buffer) {
 // 1: launches carry the programmatic-serialization attribute (set by air_set_pdl).
 int& pdl_enabled();
 
+// What the calling thread launched last: every launch counts, and the portions' attention notes which one it was where nothing
+// follows it in its own entry.  The single tokens' attention may run beside that launch, and only beside that one.
+struct LastLaunch {
+    unsigned long long count = 0, portions = ~0ull;
+    cudaStream_t stream = nullptr;      // of the portions
+};
+LastLaunch& last_launch();
+
+template <typename... KArgs, typename... Args>
+inline int launch_counted(const cudaLaunchConfig_t& cfg, void (*kernel)(KArgs...), Args... args) {
+    ++last_launch().count;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 template <typename... KArgs, typename... Args>
 inline int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
@@ -74,7 +88,7 @@ inline int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+    return launch_counted(cfg, kernel, args...);
 }
 
 __device__ __forceinline__ float to_float(float v) { return v; }

@@ -475,7 +475,7 @@ static int launch_delta_chunks(const DeltaChunkArgs& args, int N, int L, cudaStr
     cfg.blockDim = dim3(DC_WARPS * 32);
     cfg.dynamicSmemBytes = smem2;
     cfg.stream = stream;
-    return (int)cudaLaunchKernelEx(&cfg, delta_chunk_scan_kernel<DP, MODE>, a);
+    return launch_counted(cfg, delta_chunk_scan_kernel<DP, MODE>, a);
 }
 
 }  // namespace air

@@ -1030,6 +1030,10 @@ int& pdl_enabled() {
     static int enabled = 1;
     return enabled;
 }
+LastLaunch& last_launch() {
+    thread_local LastLaunch last;
+    return last;
+}
 }  // namespace air
 
 AIR_API int air_trace_set_elementwise(unsigned long long* buffer) { return air::set_trace_here(buffer); }

@@ -352,7 +352,7 @@ static int launch_f32_tiles(const float* A, const float* W, const float* bias, f
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    return (int)cudaLaunchKernelEx(&cfg, kernel, A, W, bias, C, M, N, K);
+    return launch_counted(cfg, kernel, A, W, bias, C, M, N, K);
 }
 
 template <int RM>

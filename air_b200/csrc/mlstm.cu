@@ -569,7 +569,7 @@ AIR_API int air_mlstm_portions(const float* x, int ldx, int cq, int ck, int cv, 
     cfg.blockDim = dim3(128);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    rc = (int)cudaLaunchKernelEx(&cfg, air::mlstm_states_kernel, c);
+    rc = air::launch_counted(cfg, air::mlstm_states_kernel, c);
     if (rc) return rc;
     AIR_DISPATCH(out_dtype, TO, {
         auto kernel = air::mlstm_outputs_kernel<TO>;

@@ -1498,7 +1498,8 @@ def decode_attention(q, cache, block_table, token_seq, positions, out, window, s
     [T*H*splits*2]) or None to allocate.  engine "tma": keys and values by the copy engine into shared
     memory (attention_decode_tma.cu); "ldg": by the warps' own loads (attention_decode.cu).
     alongside: the last launch on this stream was prefill_attention_tc, without items, over other rows of q and out, and
-    what is attended over was written before it: the two may run side by side (the copy-engine kernel only)."""
+    what is attended over was written before it: the two may run side by side (the copy-engine kernel only; behind any other
+    launch of this package it waits for that one, as it does without)."""
     T, H, d = q.shape
     K, P = cache.shape[2], cache.shape[3]
     _req(q, "q", (torch.bfloat16,))

@@ -496,7 +496,7 @@ static int launch_scan(const ScanPrepArgs& prep, const ScanArgs& a, int T, int S
         cfg.blockDim = dim3(SCAN_THREADS);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
-        return (int)cudaLaunchKernelEx(&cfg, kernel, p);
+        return launch_counted(cfg, kernel, p);
     };
     if (R == 32) return go(linear_scan_kernel<MODE, 32, 32>);
     switch (L) {

@@ -723,6 +723,40 @@ def test_decode_and_portion_attention_side_by_side(H, K, d, P, n, portion, split
     assert status.item() == 0
 
 
+@pytest.mark.parametrize("between", ["convert", "gemm_f32", "nothing"])
+def test_decode_attention_alongside_another_launch_waits_for_it(between):
+    """What the decode kernel reads is written by the launches right ahead of it, which are not the portions' kernel: although
+    it was asked to run alongside, it waits for them (over and over with new numbers)."""
+    H, K, d, P, n, portion = 8, 2, 128, 64, 5, 40
+    lens, q_lens = [300 + 7 * i for i in range(n)] + [portion + 90], [1] * n + [portion]
+    q, cache, bt, positions, seq_of, _, _ = paged_case(H, K, d, P, lens, q_lens, "bfloat16", seed=3, num_pages=140)
+    cache, bt, seq, pos, tiles = dev(cache, torch.bfloat16), dev(bt), dev(seq_of), dev(positions), dev(tiles_for(lens, q_lens)[16 * n:])
+    queries = [dev(q) * (1 + i % 3) for i in range(6)]
+    T, out, want = len(q), torch.zeros(q.shape, dtype=torch.bfloat16, device="cuda"), []
+    rows, wide, eye = torch.empty(q.shape, dtype=torch.bfloat16, device="cuda"), torch.empty(q.shape, device="cuda"), torch.eye(H * d, device="cuda")
+    for x in queries:
+        ops().convert(x, rows)
+        ops().decode_attention(rows[:n], cache, bt, seq[:n], pos[:n], out[:n], 0, d ** -0.5, splits=4)
+        want.append(out[:n].float())
+    for _ in range(5):
+        got = []
+        for x in queries:
+            if between == "nothing":
+                ops().convert(x, rows)
+            ops().prefill_attention_tc(rows, cache, bt, tiles, out, 0, d ** -0.5)
+            if between == "gemm_f32":
+                ops().gemm_f32(x.view(T, H * d), eye, None, wide.view(T, H * d))
+            if between in ("convert", "gemm_f32"):
+                ops().convert(wide if between == "gemm_f32" else x, rows)
+            ops().decode_attention(rows[:n], cache, bt, seq[:n], pos[:n], out[:n], 0, d ** -0.5, splits=4, alongside=True)
+            y = torch.empty((n, H, d), device="cuda")
+            ops().convert(out[:n], y)
+            got.append(y)
+        for x, y in zip(want, got):
+            assert torch.equal(x, y)
+
+
+
 def streams_of(tiles, window):
     """Key tiles in the stream of every pair of a tile list (as the kernel counts them)."""
     out = []
