@@ -152,7 +152,7 @@ def test_attention_sees_the_keys_inside_its_mask_and_no_other(kind, size, dtype)
                 out = torch.empty((m, H, dv), dtype=dtype, device=DEV)
                 kernel(dev(q[at:at + m], dtype), cache, table, i32([1] * m), i32(range(at, at + m)), out,
                        size if kind == "window" else None, scale, kv_heads=G, page_tokens=P,
-                       chunk=size if kind == "chunk" else None, sink=dev(sink))
+                       chunk=size if kind == "chunk" else None, sink=dev(sink), **more)
                 tol = 3e-4 if dtype == torch.float32 else 0.3          # (values up to 35: bfloat16 holds them to 0.125)
                 assert np.abs(out.float().cpu().numpy() - want[at:at + m]).max() < tol, (at, m, kernel.__name__)
             at += m
@@ -251,6 +251,52 @@ def test_latent_attention_through_its_kernels(H, d, rot, R, dv, window, dtype):
         row = kept[pages[t // P], t % P]
         tol = 2e-5 if dtype == torch.float32 else 3e-2
         assert np.abs(row[:R] - c[t]).max() < tol and np.abs(row[R:] - kr[t]).max() < tol
+
+
+@pytest.mark.parametrize("mask", [("all", None), ("window", 70), ("window", 450), ("chunk", 200)])
+@pytest.mark.parametrize("G,J,d,dv,latent,P", [(2, 5, 64, 48, False, 16), (1, 18, 128, 128, False, 64), (2, 16, 256, 200, False, 48),
+                                                (1, 20, 576, 512, True, 16), (1, 3, 512, 512, False, 64), (1, 16, 640, 128, True, 32),
+                                                (1, 17, 640, 600, True, 64)])
+def test_grouped_attention_over_many_tiles_of_keys(G, J, d, dv, latent, P, mask):
+    """Every shape of block (rows of up to 128, 256 and 640 numbers, one and two stages, values beyond 512), with so few splits
+    that a block walks several tiles, and with more splits than tiles: against the 64-bit softmax, at positions around the edges
+    of tiles; float32 and bfloat16 queries.  Keys that no query sees are NaN."""
+    from air_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(d + J)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    kind, size = mask
+    H, n, scale = G * J, 720, 2.5 * d ** -0.5
+    k = rand(n, G, d).bfloat16()
+    v = k[:, :, :dv] if latent else rand(n, G, dv).bfloat16()
+    blocks = -(-n // P)
+    table = torch.full((3, 64), -1, dtype=torch.int32, device="cuda")
+    pages = torch.randperm(64, generator=g, device="cuda")[:blocks]
+    table[2, :blocks] = pages.int()
+    cache = torch.full((64, P, d) if latent else (64, G * P * (d + dv)), float("nan"), dtype=torch.bfloat16, device="cuda")
+    at = torch.tensor([0, 63, 64, 127, 255, 384, 449, 450, 599, 600, 713], device="cuda")
+    last = int(at.max())
+    for t in range(last + 1):
+        page = cache[pages[t // P]]
+        if latent:
+            page[t % P] = k[t, 0]
+        else:
+            page[:G * P * d].view(G, P, d)[:, t % P] = k[t]
+            page[G * P * d:].view(G, P, dv)[:, t % P] = v[t]
+    key = torch.arange(last + 1, device="cuda")[None]
+    low = {"all": at * 0, "window": at - (size or 0) + 1, "chunk": at - at % (size or 1)}[kind]
+    seen = (key <= at[:, None]) & (key >= low[:, None])
+    sink = rand(H)
+    for q in (rand(len(at), H, d), rand(len(at), H, d).bfloat16()):
+        x = torch.einsum("tgjd,sgd->tgjs", q.double().view(len(at), G, J, d), k[:last + 1].double()) * scale
+        x = torch.cat([x.masked_fill(~seen[:, None, None], -float("inf")), sink.double().view(1, G, J, 1).expand(len(at), G, J, 1)], dim=-1)
+        want = torch.einsum("tgjs,sgv->tgjv", torch.softmax(x, dim=-1)[..., :-1], v[:last + 1].double()).reshape(len(at), H, dv)
+        for splits in (1, 2, 3, 16):
+            out = torch.empty((len(at), H, dv), dtype=torch.bfloat16, device="cuda")
+            ops.grouped_attention(q, cache, table, i32([2] * len(at)), at.int(), out, size if kind == "window" else None, scale, kv_heads=G,
+                                  page_tokens=P, chunk=size if kind == "chunk" else None, sink=sink, latent=latent, splits=splits)
+            # (a result rounded to the 8 bits of bfloat16: 2^-8 of it at most; the 32-bit queries and weights enter as two bfloat16
+            # numbers each, 2^-16 of them)
+            assert ((out.double() - want).abs() - want.abs() / 256).max() <= 1e-4 * max(1.0, want.abs().max().item()), splits
 
 
 @pytest.mark.parametrize("n,top,groups", [(31, 4, 1), (32, 32, 4), (33, 4, 3), (128, 8, 8), (129, 32, 3),
