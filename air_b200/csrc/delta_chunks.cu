@@ -30,6 +30,8 @@
 // 54, scan 140); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 87 (22 and 65).  Below 24 tokens the two
 // launches and a chunk's chain are no shorter than the tokens' own.
 //
+// An infinity or a NaN reaches what it reaches token by token, and nothing ahead of its token.
+//
 // What a row is depends on the state and the portion's tokens only.
 #include "common.cuh"
 #include "tma.cuh"
@@ -96,6 +98,10 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
     float* sq = sk + DC * ld;
     float* sb = sq + DC * ld;               // the decays' logarithms to the base 2, then their sums
     const float rate = MODE == CHUNK_GLA ? -p.inv_tau * 1.4426950408889634f : -expf(p.a_log[h]) * 1.4426950408889634f;
+    auto log_of = [&](float z) {            // (a NaN stays one)
+        const float x = rate * softplus_1(z);
+        return x < DC_FLOOR ? DC_FLOOR : x;
+    };
     {   // a warp per two tokens: unit lengths, logarithms (both tokens' loads under way at once)
         float x[2][PER], y[2][PER], z[2][PER];
 #pragma unroll
@@ -122,7 +128,7 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
             for (int i = 0; i < PER; ++i) {
                 ss = fmaf(x[r][i], x[r][i], ss);
                 qs = fmaf(y[r][i], y[r][i], qs);
-                sb[t * ld + lane + 32 * i] = t < n && lane + 32 * i < d ? fmaxf(rate * softplus_1(z[r][i]), DC_FLOOR) : 0.f;
+                sb[t * ld + lane + 32 * i] = t < n && lane + 32 * i < d ? log_of(z[r][i]) : 0.f;
             }
             float kf = 1.f, qf = p.q_scale;
             if (MODE != CHUNK_GLA) {
@@ -390,6 +396,11 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
                 const float sum = (v[0][e] + v[1][e]) + (v[2][e] + v[3][e]);
                 y[e] = sum_t < DC ? y[e] - sum : sum;
             }
+            if (i + 1 == chunks && sum_t < DC) {      // (of no token: nothing, also beside a state of infinities)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (i * DC + sum_t + e >= tokens) y[e] = 0.f;
+            }
             store4(sum_to, y);
         }
         __syncthreads();
@@ -413,26 +424,44 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
 #pragma unroll
             for (int j = 0; j < NJ; ++j)
                 two_pair(k[j], buf + Place::KEYS + (r0 + 8 * j + g) * DC + ((8 * x) ^ swap) + t2);
-            if (warp < 2) {                  // o: its products stand among the state's, which do not wait for them
-                if (x == 0) {
-                    const float2 lo = *reinterpret_cast<const float2*>(OT + g * DC_ULD + t0 + t2);
-                    const float2 hi = *reinterpret_cast<const float2*>(OT + (g + 8) * DC_ULD + t0 + t2);
-                    o[0] = lo.x; o[1] = lo.y; o[2] = hi.x; o[3] = hi.y;
-                }
-                two_pair(w, buf + Place::P + (t0 + g) * DC + ((8 * x) ^ swap) + t2);
-                mma_tf32(o, u[x][0].lo, u[x][1].lo, u[x][2].lo, u[x][3].lo, w[0].hi, w[1].hi);
+            if (warp == 1 && x == 0) {       // o of tokens 8 .. 15: what tokens 0 .. 7 add, among the state's products
+                two_pair(w, buf + Place::P + (8 + g) * DC + swap + t2);
+                mma_tf32(o, u[0][0].lo, u[0][1].lo, u[0][2].lo, u[0][3].lo, w[0].hi, w[1].hi);
             }
 #pragma unroll
             for (int j = 0; j < NJ; ++j) mma_tf32(S[j], u[x][0].lo, u[x][1].lo, u[x][2].lo, u[x][3].lo, k[j][0].hi, k[j][1].hi);
-            if (warp < 2) mma_tf32(o, u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, w[0].lo, w[1].lo);
+            if (warp == 1 && x == 0) mma_tf32(o, u[0][0].hi, u[0][1].hi, u[0][2].hi, u[0][3].hi, w[0].lo, w[1].lo);
 #pragma unroll
             for (int j = 0; j < NJ; ++j) mma_tf32(S[j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].lo, k[j][1].lo);
-            if (warp < 2) mma_tf32(o, u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, w[0].hi, w[1].hi);
+            if (warp == 1 && x == 0) mma_tf32(o, u[0][0].hi, u[0][1].hi, u[0][2].hi, u[0][3].hi, w[0].hi, w[1].hi);
 #pragma unroll
             for (int j = 0; j < NJ; ++j) mma_tf32(S[j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].hi, k[j][1].hi);
         }
         if (warp < 2) {
             float* to = out + (size_t)i * DC * out_row;
+            const float2 o_a = *reinterpret_cast<const float2*>(OT + g * DC_ULD + t0 + t2);
+            const float2 o_b = *reinterpret_cast<const float2*>(OT + (g + 8) * DC_ULD + t0 + t2);
+            const float first[4] = {o_a.x, o_a.y, o_b.x, o_b.y};
+            // what the eight tokens add to one another on the CUDA cores: only those up to a token itself, since a product with the
+            // zeros of p above the diagonal would carry a later token's infinity or NaN into this one's o
+            float pu[2][8], uu[2][8];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float* row = buf + Place::P + (t0 + t2 + e) * DC + dc_key_place(t0 + t2 + e, t0);
+                const float* col = UT + (g + 8 * e) * DC_ULD + t0;
+                load4(row, *reinterpret_cast<float(*)[4]>(&pu[e][0]));
+                load4(row + 4, *reinterpret_cast<float(*)[4]>(&pu[e][4]));
+                load4(col, *reinterpret_cast<float(*)[4]>(&uu[e][0]));
+                load4(col + 4, *reinterpret_cast<float(*)[4]>(&uu[e][4]));
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float sum = o[e];
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+                    if (s <= t2 + (e & 1)) sum = fmaf(pu[e & 1][s], uu[e >> 1][s], sum);
+                o[e] = first[e] + sum;
+            }
 #pragma unroll
             for (int e = 0; e < 4; ++e)
                 if (i * DC + t0 + t2 + (e & 1) < tokens && col0 + g + 8 * (e >> 1) < p.dv)

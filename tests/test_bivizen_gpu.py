@@ -185,6 +185,55 @@ def test_chunks_against_token_by_token(decays, mode, H, G, d, dv):
                     assert np.abs(got[road][1][slots[i], h] - S).max() < (5e-5 if delta else 5e-6) * max(1.0, largest), (road, i)
 
 
+@pytest.mark.parametrize("mode", ["delta", "gla", "channel"])
+@pytest.mark.parametrize("what,value", [("v", float("inf")), ("v", float("nan")), ("v", 3.4e38), ("k", float("nan")), ("k", float("-inf")),
+                                        ("q", float("inf")), ("z", float("nan")), ("z", float("inf")), ("b", float("nan")),
+                                        ("S", float("inf"))])
+def test_chunks_carry_infinities_and_nans_as_token_by_token_does(what, value, mode):
+    """An infinity or a NaN among a token's numbers (or in a state): the outputs and the places of the state that it reaches are
+    those that it reaches token by token, none of them of an earlier token, and all others have the same numbers."""
+    from air_b200.csrc import ops
+    H, d, dv, counts, slots = 2, 64, 40, (70, 33), (1, 2)
+    T, at = sum(counts), 41                      # (in the middle of the first portion's third chunk)
+    which = {"delta": ops.SCAN_DELTA, "gla": ops.SCAN_GLA, "channel": ops.SCAN_CHANNEL_DELTA}[mode]
+    per = H if mode == "delta" else H * d
+    g = torch.Generator(device=DEV).manual_seed(5)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    x = dict(q=rand(T, H * d), k=rand(T, H * d), v=rand(T, H * dv), z=rand(T, per), b=rand(T, H), S=rand(3, H, d, dv))
+    if what == "b" and mode == "gla":
+        return
+    if what == "S":
+        x["S"][1, 0, 7, 5] = value
+    else:
+        x[what][at, 0] = value
+    more = dict(tau=8.0) if mode == "gla" else dict(beta=x["b"], a_log=rand(H) / 2, dt_bias=rand(per))
+    start = np.concatenate([[0], np.cumsum(counts)])
+    portions, chunks = [], []
+    for i, n in enumerate(counts):
+        portions.append((start[i], n, slots[i], len(chunks)))
+        chunks += [(start[i] + a, min(16, n - a)) for a in range(0, n, 16)]
+    table = lambda rows: torch.tensor(np.array(rows), dtype=torch.int32, device=DEV)
+    got = []
+    for road in ("tokens", "chunks"):
+        S, o = x["S"].clone(), torch.empty((T, H, dv), device=DEV)
+        if road == "tokens":
+            ops.linear_scan(which, x["q"], x["k"], x["v"], x["z"], S, o, i32(start), i32(slots), i32(np.repeat(slots, counts)),
+                            q_scale=d ** -0.5, unit=mode != "gla", **more)
+        else:
+            ops.delta_portions(x["q"], x["k"], x["v"], x["z"], S, o, table(portions), table(chunks), d ** -0.5, mode=which, **more)
+        got.append((o, S))
+    # (the largest numbers overflow in k u where the scan takes one product after the other, and need not in p u: of them only that
+    # they, too, stay out of everything ahead of their token and beside it)
+    pieces = lambda o, S: [o[:at], o[counts[0]:], S[0], S[2]] + ([] if value == 3.4e38 else [o[at:counts[0]], S[1]])
+    for a, b in zip(pieces(*got[0]), pieces(*got[1])):
+        fine = torch.isfinite(a)
+        assert torch.equal(fine, torch.isfinite(b))
+        if fine.any():
+            assert (a[fine] - b[fine]).abs().max() < 5e-5 * max(1.0, float(a[fine].abs().max()))
+    if what != "S":
+        assert torch.isfinite(got[1][0][:at]).all(), "nothing runs backwards"
+
+
 def test_gated_norm_feed_forward_activation_and_scaled_sum():
     from air_b200.csrc import ops
     rng = np.random.default_rng(5)
