@@ -26,10 +26,14 @@
 //                              the operands: what is left out is of the order of 32-bit rounding.  The next chunk's
 //                              numbers arrive by the copy engine, in two runs of bytes, while this one's are used.
 //
-// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 194 (prepare
-// 54, scan 140); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 87 (22 and 65).  Below 24 tokens the two
+// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 196 (prepare
+// 49, scan 148); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 95 (25 and 70).  Below 24 tokens the two
 // launches and a chunk's chain are no shorter than the tokens' own.
 //
+// Errors against 64 bits (2-norm of the difference over that of the result, 2,048 tokens), token by token and here: one decay per
+// head, outputs 1.98e-7 and 1.97e-7, states 1.56e-7 and 1.59e-7; gated linear attention 1.60e-7 and 1.63e-7, 1.40e-7 and 1.14e-7; decays
+// near 1, where a token's own rounding adds up, 2.9e-6 and 2.5e-7.  (Operands cut instead of rounded to their upper half, the state
+// as the products' accumulator, sums of logarithms in one number and 2^x in one instruction: 8.8e-7 and 5.4e-7, at 191 and 86 us.)
 // An infinity or a NaN reaches what it reaches token by token, and nothing ahead of its token.
 //
 // What a row is depends on the state and the portion's tokens only.
@@ -40,7 +44,7 @@ namespace air {
 
 constexpr int DC = 16;              // tokens of a chunk, and columns of a block of the scan
 constexpr int DC_RLD = 40, DC_ULD = 24;      // strides of rows in shared memory: four rows fall into different banks
-constexpr float DC_FLOOR = -60.f;   // a decay of 2^-60 is none: the logarithms' sums stay small enough to be exact
+constexpr float DC_FLOOR = -110.f;   // (e^-110 is 0 in 32 bits; differences of the logarithms' sums stay numbers)
 
 // What a chunk and head leave in the scratch memory, DP the channels filled up to 32, 64, 128 or 256 (zeros), in floats:
 //   rows [32][DP]     W and q exp b; the eight channels from 8 i on of row t stand at 8 (i ^ (t & 3))
@@ -77,27 +81,24 @@ struct DeltaChunkArgs {
 };
 
 __device__ __forceinline__ float softplus_1(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
-// 2^x in one instruction (x <= 0 here; relative error about 2^-22)
-__device__ __forceinline__ float power_of_2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 template <int DP, int MODE>
 __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_kernel(const DeltaChunkArgs p) {
     constexpr int ld = DP + 4, PER = DP / 32;
     extern __shared__ __align__(16) float smem[];
     __shared__ __align__(16) float sa[DC][DC];
-    __shared__ float sbeta[DC];
+    __shared__ float sbeta[DC], slog[DC], skept[2][DC];       // (HEAD: a token's logarithm; what is left at it
+                                                                   // of the state ahead, and of it at the chunk's end)
     pdl_enter(TR_SCAN);
     const int h = blockIdx.y, g = h / (p.H / p.G), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int q0 = p.chunks[2 * blockIdx.x], n = p.chunks[2 * blockIdx.x + 1];
     const int d = p.d;
     float* sk = smem;                       // [16][ld]
     float* sq = sk + DC * ld;
-    float* sb = sq + DC * ld;               // the decays' logarithms to the base 2, then their sums
-    const float rate = MODE == CHUNK_GLA ? -p.inv_tau * 1.4426950408889634f : -expf(p.a_log[h]) * 1.4426950408889634f;
+    float* sg = sq + DC * ld;               // (not HEAD) the decays,
+    float* sb = sg + DC * ld;               // their logarithms, then the logarithms' sums,
+    float* sr = sb + DC * ld;               // and what rounding took from the sums
+    const float rate = MODE == CHUNK_GLA ? -p.inv_tau : -expf(p.a_log[h]);
     auto log_of = [&](float z) {            // (a NaN stays one)
         const float x = rate * softplus_1(z);
         return x < DC_FLOOR ? DC_FLOOR : x;
@@ -128,7 +129,10 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
             for (int i = 0; i < PER; ++i) {
                 ss = fmaf(x[r][i], x[r][i], ss);
                 qs = fmaf(y[r][i], y[r][i], qs);
-                sb[t * ld + lane + 32 * i] = t < n && lane + 32 * i < d ? log_of(z[r][i]) : 0.f;
+                if (MODE == CHUNK_HEAD) continue;
+                const float left = t < n && lane + 32 * i < d ? log_of(z[r][i]) : 0.f;
+                sb[t * ld + lane + 32 * i] = left;
+                sg[t * ld + lane + 32 * i] = expf(left);
             }
             float kf = 1.f, qf = p.q_scale;
             if (MODE != CHUNK_GLA) {
@@ -140,18 +144,29 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
                 sk[t * ld + lane + 32 * i] = x[r][i] * kf;
                 sq[t * ld + lane + 32 * i] = y[r][i] * qf;
             }
+            if (MODE == CHUNK_HEAD && lane == 0) slog[t] = t < n ? log_of(z[r][0]) : 0.f;
             if (MODE != CHUNK_GLA && lane == 0) sbeta[t] = t < n ? 1.f / (1.f + expf(-p.beta[(size_t)(q0 + t) * p.ldb + h])) : 0.f;
         }
     }
     __syncthreads();
-    if (tid < DP) {
-        float sum = 0.f;
+    // the logarithms' sums b_t, as two numbers each: b_t - b_s keeps the 24 bits that the decays between s and t have by
+    // themselves, also behind a token that forgets nearly everything
+    if (MODE != CHUNK_HEAD && tid < DP) {
+        float sum = 0.f, rest = 0.f;
 #pragma unroll
         for (int t = 0; t < DC; ++t) {
-            sum += sb[t * ld + tid];
+            const float x = sb[t * ld + tid], next = sum + x, from = next - sum;
+            rest += (sum - (next - from)) + (x - from);          // (what the addition has rounded away: Knuth)
+            sum = next;
             sb[t * ld + tid] = sum;
+            sr[t * ld + tid] = rest;
         }
     }
+    auto kept = [&](int s, int t) {                              // HEAD: what is left of token s at token t
+        float sum = 0.f;
+        for (int i = s + 1; i <= t; ++i) sum += slog[i];
+        return expf(sum);
+    };
     using Place = DeltaChunk<DP, MODE>;
     float* base = p.scratch + ((size_t)blockIdx.x * p.H + h) * p.stride;
     float* Pm = base + Place::P;
@@ -163,6 +178,10 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
         }
     }
     __syncthreads();
+    if (MODE == CHUNK_HEAD && tid >= 256 - 2 * DC) {
+        const int t = tid % DC, end = tid >= 256 - DC;
+        skept[end][t] = end ? kept(t, DC - 1) : kept(-1, t);
+    }
     // a and p: four threads (a quarter of the channels each) per square of 2 x 2 tokens on or below the diagonal, 36 squares
     if (tid < 160) {
         const int square = min(tid >> 2, 35), part = tid & 3;
@@ -172,27 +191,43 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
         float a[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, pq[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll 2
         for (int c = part * 4; c < DP; c += 16) {
-            float xk[2][4], xq[2][4], xb[2][4], yk[2][4], yb[2][4];
+            float xk[2][4], xq[2][4], yk[2][4], late[4], early[4], m[4];
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 load4(sk + (2 * i + r) * ld + c, xk[r]);
                 load4(sq + (2 * i + r) * ld + c, xq[r]);
-                load4(sb + (2 * i + r) * ld + c, xb[r]);
                 load4(sk + (2 * j + r) * ld + c, yk[r]);
-                load4(sb + (2 * j + r) * ld + c, yb[r]);
+            }
+            if (MODE != CHUNK_HEAD) {
+                // what is left of token 2 j + 1 at token 2 i, from there the other three by one decay more each
+                float b0[4], b1[4], r0[4], r1[4];
+                load4(sg + (2 * i + 1) * ld + c, late);
+                load4(sg + (2 * j + 1) * ld + c, early);
+                load4(sb + (2 * j + 1) * ld + c, b0);
+                load4(sb + 2 * i * ld + c, b1);
+                load4(sr + (2 * j + 1) * ld + c, r0);
+                load4(sr + 2 * i * ld + c, r1);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) m[e] = i == j ? 0.f : expf((b1[e] - b0[e]) + (r1[e] - r0[e]));
             }
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
+            for (int e = 0; e < 4; ++e) {
+                float w[2][2] = {{yk[0][e], yk[1][e]}, {yk[0][e], yk[1][e]}};
+                if (MODE != CHUNK_HEAD) {
+                    const float one = i == j ? 1.f : m[e] * early[e];      // (on the diagonal itself nothing has decayed)
+                    w[0][0] *= one;
+                    w[0][1] *= m[e];
+                    w[1][0] *= one * late[e];
+                    w[1][1] *= i == j ? 1.f : m[e] * late[e];
+                }
 #pragma unroll
-                for (int s = 0; s < 2; ++s)
+                for (int r = 0; r < 2; ++r)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        float x = xb[r][e] - yb[s][e];
-                        if (r < s) x = fminf(x, 0.f);      // (above the diagonal where i = j: not kept, but it may not overflow)
-                        const float w = MODE == CHUNK_HEAD ? yk[s][e] : yk[s][e] * power_of_2(x);
-                        if (MODE != CHUNK_GLA) a[r][s] = fmaf(xk[r][e], w, a[r][s]);
-                        pq[r][s] = fmaf(xq[r][e], w, pq[r][s]);
+                    for (int s = 0; s < 2; ++s) {
+                        if (MODE != CHUNK_GLA) a[r][s] = fmaf(xk[r][e], w[r][s], a[r][s]);
+                        pq[r][s] = fmaf(xq[r][e], w[r][s], pq[r][s]);
                     }
+            }
         }
 #pragma unroll
         for (int r = 0; r < 2; ++r)
@@ -205,7 +240,7 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
                 const int t = 2 * i + r, u = 2 * j + s;
                 if (part == 0 && tid < 144 && u <= t) {
                     if (MODE == CHUNK_HEAD) {
-                        const float w = power_of_2(sb[t * ld] - sb[u * ld]);
+                        const float w = kept(u, t);
                         a[r][s] *= w;
                         pq[r][s] *= w;
                     }
@@ -219,21 +254,21 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
     for (int j = tid; j < DP + p.dvp; j += 256) {
         float x[DC];
         if (j < DP) {
-            const float last = sb[(DC - 1) * ld + j];
             float* keys = base + Place::KEYS + j * DC;
 #pragma unroll
             for (int t = 0; t < DC; t += 4) {
                 float kv[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float b = sb[(t + i) * ld + j], k = sk[(t + i) * ld + j], e = power_of_2(b);
-                    x[t + i] = k * e;
-                    base[(Place::ROWS - DC + t + i) * DP + dc_row_place(t + i, j)] = sq[(t + i) * ld + j] * e;
-                    kv[i] = k * power_of_2(last - b);
+                    const int at = (t + i) * ld + j, end = (DC - 1) * ld + j;
+                    const float k = sk[at], here = MODE == CHUNK_HEAD ? skept[0][t + i] : expf(sb[at]);
+                    x[t + i] = k * here;
+                    base[(Place::ROWS - DC + t + i) * DP + dc_row_place(t + i, j)] = sq[at] * here;
+                    kv[i] = k * (MODE == CHUNK_HEAD ? skept[1][t + i] : expf((sb[end] - sb[at]) + (sr[end] - sr[at])));
+                    if (t + i == DC - 1) base[Place::LAST + j] = here;
                 }
                 store4(keys + dc_key_place(j, t), kv);
             }
-            base[Place::LAST + j] = power_of_2(last);
         } else {
             const int c = j - DP;
 #pragma unroll
@@ -268,10 +303,12 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_ke
     }
 }
 
-// A 32-bit number as two TF32 numbers: the instruction reads the upper 19 bits of an operand.
+// A 32-bit number as two TF32 numbers: the instruction reads the upper 19 bits of an operand.  The upper one is rounded, so that
+// the lower one has 12 bits and a sign of its own, and what it loses is 2^-23 of x at most, to either side.  (Where rounding
+// carries a NaN's bits into the sign, x - hi is a NaN all the same.)
 struct Two { uint32_t hi, lo; };
 __device__ __forceinline__ Two two_of(float x) {
-    const uint32_t hi = __float_as_uint(x) & 0xffffe000u;
+    const uint32_t hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
     return Two{hi, __float_as_uint(x - __uint_as_float(hi))};
 }
 // c += a b; with k in the order that the accumulators have: a holds (row g, k 2t), (g + 8, 2t), (g, 2t + 1), (g + 8, 2t + 1), b
@@ -359,9 +396,13 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
             return;
         }
         if (tid == 0 && i + STAGES - 1 < chunks) stage(i + STAGES - 1);
-        float acc[RG][4];
+        // (the tensor cores cut sums off instead of rounding them: a large product is summed from zero and added up in 32 bits, the
+        // small ones have sums of their own, and so has what is added to the state)
+        float acc[RG][4], low[RG][4];
 #pragma unroll
-        for (int x = 0; x < RG; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f;
+        for (int x = 0; x < RG; ++x)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[x][e] = low[x][e] = 0.f;
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
             const Two a[4] = {two_of(S[j][0]), two_of(S[j][2]), two_of(S[j][1]), two_of(S[j][3])};
@@ -369,18 +410,23 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
             Two b[RG][2];
 #pragma unroll
             for (int x = 0; x < RG; ++x) two_pair(b[x], at + 8 * x * DP);
-            // (the four sums in turn: a product does not wait for the one before it)
+            // (the sums in turn: a product does not wait for the one before it)
 #pragma unroll
-            for (int x = 0; x < RG; ++x) mma_tf32(acc[x], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[x][0].hi, b[x][1].hi);
+            for (int x = 0; x < RG; ++x) mma_tf32(low[x], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[x][0].hi, b[x][1].hi);
 #pragma unroll
-            for (int x = 0; x < RG; ++x) mma_tf32(acc[x], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].lo, b[x][1].lo);
+            for (int x = 0; x < RG; ++x) mma_tf32(low[x], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].lo, b[x][1].lo);
 #pragma unroll
-            for (int x = 0; x < RG; ++x) mma_tf32(acc[x], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].hi, b[x][1].hi);
+            for (int x = 0; x < RG; ++x) {
+                float part[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_tf32(part, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].hi, b[x][1].hi);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[x][e] += part[e];
+            }
         }
 #pragma unroll
         for (int x = 0; x < RG; ++x) {
-            *reinterpret_cast<float2*>(mine + 8 * x) = make_float2(acc[x][0], acc[x][1]);
-            *reinterpret_cast<float2*>(mine + 8 * DC_RLD + 8 * x) = make_float2(acc[x][2], acc[x][3]);
+            *reinterpret_cast<float2*>(mine + 8 * x) = make_float2(acc[x][0] + low[x][0], acc[x][1] + low[x][1]);
+            *reinterpret_cast<float2*>(mine + 8 * DC_RLD + 8 * x) = make_float2(acc[x][2] + low[x][2], acc[x][3] + low[x][3]);
         }
         __syncthreads();
         {   // the warps' sums in order: U = Y - W S (rows 0 .. 15 of 32), o's first part (the others)
@@ -392,9 +438,10 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
             if (sum_t < DC) load4(buf + Place::Y + sum_c * DC + sum_t, y);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                if (MODE == CHUNK_GLA && sum_t < DC) continue;            // (u is v)
-                const float sum = (v[0][e] + v[1][e]) + (v[2][e] + v[3][e]);
-                y[e] = sum_t < DC ? y[e] - sum : sum;
+                if (MODE != CHUNK_GLA || sum_t >= DC) {                   // (gated linear attention: u is v)
+                    const float sum = (v[0][e] + v[1][e]) + (v[2][e] + v[3][e]);
+                    y[e] = sum_t < DC ? y[e] - sum : sum;
+                }
             }
             if (i + 1 == chunks && sum_t < DC) {      // (of no token: nothing, also beside a state of infinities)
 #pragma unroll
@@ -412,12 +459,11 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
             two_pair(hi, UT + (g + 8) * DC_ULD + 8 * x + t2);
             u[x][0] = lo[0]; u[x][1] = hi[0]; u[x][2] = lo[1]; u[x][3] = hi[1];
         }
+        float more[NJ][4], less[NJ][4], o[4] = {0.f, 0.f, 0.f, 0.f}, o_low[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-            const float2 e = *reinterpret_cast<const float2*>(buf + Place::LAST + r0 + 8 * j + t2);
-            S[j][0] *= e.x; S[j][1] *= e.y; S[j][2] *= e.x; S[j][3] *= e.y;
-        }
-        float o[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) more[j][e] = less[j][e] = 0.f;
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             Two k[NJ][2], w[2];
@@ -426,16 +472,22 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
                 two_pair(k[j], buf + Place::KEYS + (r0 + 8 * j + g) * DC + ((8 * x) ^ swap) + t2);
             if (warp == 1 && x == 0) {       // o of tokens 8 .. 15: what tokens 0 .. 7 add, among the state's products
                 two_pair(w, buf + Place::P + (8 + g) * DC + swap + t2);
-                mma_tf32(o, u[0][0].lo, u[0][1].lo, u[0][2].lo, u[0][3].lo, w[0].hi, w[1].hi);
+                mma_tf32(o_low, u[0][0].lo, u[0][1].lo, u[0][2].lo, u[0][3].lo, w[0].hi, w[1].hi);
             }
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) mma_tf32(S[j], u[x][0].lo, u[x][1].lo, u[x][2].lo, u[x][3].lo, k[j][0].hi, k[j][1].hi);
-            if (warp == 1 && x == 0) mma_tf32(o, u[0][0].hi, u[0][1].hi, u[0][2].hi, u[0][3].hi, w[0].lo, w[1].lo);
+            for (int j = 0; j < NJ; ++j) mma_tf32(less[j], u[x][0].lo, u[x][1].lo, u[x][2].lo, u[x][3].lo, k[j][0].hi, k[j][1].hi);
+            if (warp == 1 && x == 0) mma_tf32(o_low, u[0][0].hi, u[0][1].hi, u[0][2].hi, u[0][3].hi, w[0].lo, w[1].lo);
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) mma_tf32(S[j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].lo, k[j][1].lo);
+            for (int j = 0; j < NJ; ++j) mma_tf32(less[j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].lo, k[j][1].lo);
             if (warp == 1 && x == 0) mma_tf32(o, u[0][0].hi, u[0][1].hi, u[0][2].hi, u[0][3].hi, w[0].hi, w[1].hi);
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) mma_tf32(S[j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].hi, k[j][1].hi);
+            for (int j = 0; j < NJ; ++j) mma_tf32(more[j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].hi, k[j][1].hi);
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const float2 w = *reinterpret_cast<const float2*>(buf + Place::LAST + r0 + 8 * j + t2);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) S[j][e] = fmaf(S[j][e], e & 1 ? w.y : w.x, more[j][e] + less[j][e]);
         }
         if (warp < 2) {
             float* to = out + (size_t)i * DC * out_row;
@@ -456,7 +508,7 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                float sum = o[e];
+                float sum = o[e] + o_low[e];
 #pragma unroll
                 for (int s = 0; s < 8; ++s)
                     if (s <= t2 + (e & 1)) sum = fmaf(pu[e & 1][s], uu[e >> 1][s], sum);
@@ -482,7 +534,7 @@ static int launch_delta_chunks(const DeltaChunkArgs& args, int N, int L, cudaStr
     DeltaChunkArgs a = args;
     a.dvp = (a.dv + 15) / 16 * 16;
     a.stride = DeltaChunk<DP, MODE>::Y + (long long)DC * a.dvp;
-    const size_t smem1 = sizeof(float) * 3 * DC * (DP + 4);
+    const size_t smem1 = sizeof(float) * (MODE == CHUNK_HEAD ? 2 : 5) * DC * (DP + 4);
     if (smem1 > 44 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(delta_chunk_prepare_kernel<DP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
         if (e != cudaSuccess) return (int)e;

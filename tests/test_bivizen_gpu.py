@@ -186,6 +186,48 @@ def test_chunks_against_token_by_token(decays, mode, H, G, d, dv):
 
 
 @pytest.mark.parametrize("mode", ["delta", "gla", "channel"])
+def test_chunks_are_as_precise_as_token_by_token(mode):
+    """The error of outputs and states against the 64-bit recurrence, over slow, usual and mixed decays and tokens that forget
+    nearly everything: the chunks' is not larger than the scan's (by more than a fifth, as the two differ from seed to seed) or
+    than 2^-22, what a product loses whose two operands are off by 2^-23 each."""
+    from air_b200.csrc import ops
+    H, d, dv, T, tau = 4, 128, 64, 400, 4.0
+    which = {"delta": ops.SCAN_DELTA, "gla": ops.SCAN_GLA, "channel": ops.SCAN_CHANNEL_DELTA}[mode]
+    per, errors = (H if mode == "delta" else H * d), {"tokens": [], "chunks": []}
+    chunks = torch.tensor([(t, min(16, T - t)) for t in range(0, T, 16)], dtype=torch.int32, device=DEV)
+    for seed, (mean, std) in enumerate([(-7.0, 1.0), (-3.0, 1.0), (0.0, 4.0), (-4.0, 1.0)]):
+        g = torch.Generator(device=DEV).manual_seed(seed)
+        rand = lambda *s: torch.randn(*s, generator=g, device=DEV)
+        q, k, v, z, b, a_log, S0 = rand(T, H * d), rand(T, H * d), rand(T, H * dv), rand(T, per) * std + mean, rand(T, H), rand(H) / 2, rand(1, H, d, dv)
+        if seed == 3:
+            z[::7] = 40.0                        # (what these tokens leave of the state is nothing)
+        z = -z if mode == "gla" else z
+        more = dict(tau=tau) if mode == "gla" else dict(beta=b, a_log=a_log, dt_bias=torch.zeros(per, device=DEV))
+        Q, K, V = q.double().view(T, H, d), k.double().view(T, H, d), v.double().view(T, H, dv)
+        if mode == "gla":
+            keep = torch.nn.functional.logsigmoid(z.double()).div(tau).exp().view(T, H, d)
+        else:
+            keep = (-a_log.double().exp()[:, None] * torch.nn.functional.softplus(z.double(), threshold=100).view(T, H, -1)).exp().expand(T, H, d)
+            Q, K = (x / (x * x).sum(-1, keepdim=True).add(1e-6).sqrt() for x in (Q, K))
+        S, want = S0[0].double(), []
+        for t in range(T):
+            S = S * keep[t][:, :, None]
+            u = V[t] if mode == "gla" else torch.sigmoid(b[t].double())[:, None] * (V[t] - torch.einsum("hdv,hd->hv", S, K[t]))
+            S = S + K[t][:, :, None] * u[:, None]
+            want.append(torch.einsum("hdv,hd->hv", S, Q[t] * d ** -0.5))
+        want = torch.stack(want)
+        for road in errors:
+            state, o = S0.clone(), torch.empty((T, H, dv), device=DEV)
+            if road == "tokens":
+                ops.linear_scan(which, q, k, v, z, state, o, i32([0, T]), i32([0]), i32([0] * T), q_scale=d ** -0.5, unit=mode != "gla", **more)
+            else:
+                ops.delta_portions(q, k, v, z, state, o, i32([0, T, 0, 0]).view(1, 4), chunks, d ** -0.5, mode=which, **more)
+            errors[road].append([float((o.double() - want).norm() / want.norm()), float((state[0].double() - S).norm() / S.norm())])
+    tokens, chunks = np.array(errors["tokens"]), np.array(errors["chunks"])
+    assert (chunks <= np.maximum(1.2 * tokens, 2.0 ** -22)).all(), (tokens.tolist(), chunks.tolist())
+
+
+@pytest.mark.parametrize("mode", ["delta", "gla", "channel"])
 @pytest.mark.parametrize("what,value", [("v", float("inf")), ("v", float("nan")), ("v", 3.4e38), ("k", float("nan")), ("k", float("-inf")),
                                         ("q", float("inf")), ("z", float("nan")), ("z", float("inf")), ("b", float("nan")),
                                         ("S", float("inf"))])
