@@ -9,14 +9,15 @@
 // x 64 tiles, steps of 32 of k by cp.async) streamed at half the copy rate.
 //   EPI 0  float32 rows to planes: p = o_index[slot], plane split * o_div + p % o_div, row p / o_div, times o_scale[p].  With
 //          `splits` parts of k every part has planes of its own, which the consumer adds in order: more and shorter tiles
-//          to deal out (10 experts of 4,096 x 3,584: 320 tiles for 148 SMs are 3 rounds, 640 halves 5)
+//          to deal out where few experts are reached (parts/experts.py)
 //   EPI 1  W_g holds, per 256 rows, 128 of the gate and 128 of the linear branch: bfloat16 [slots, N / 2]
 //   EPI 2  max(x, 0)^2 as bfloat16 [slots, N]
 // A tile of W may reach into the next expert's rows, a tile of X into the next expert's slots: what they give is not stored.
 // Measured, a whole mixture (router, lists, both products, a shared expert half as wide as the dense feed-forward) replayed as
 // a graph, us: width 4,096, 16 experts of 3,584, 8 tokens 331 -> 190 (its bytes at the copy rate: 169), 100 tokens 419 by the
 // library's grouped product -> 324, 300 tokens 418 -> 350; width 2,048, experts of 2,048: 8 tokens 94, 100 tokens 169 -> 129, 300
-// tokens 165 -> 140, 500 tokens 175 -> 182: from 64 rows per expert on the library's product is the faster one.
+// tokens 165 -> 140, 500 tokens 168 -> 178 (launched kernel by kernel, as such a step is: 196 and 195; where the library takes
+// over: RoutedExperts.LIBRARY_ROWS).
 // Every wait on an mbarrier is bounded; on giving up the block sets *status = 4 (as gemm_tc.cu).
 #include "common.cuh"
 #include "tma.cuh"

@@ -7,7 +7,7 @@ from ..config.model_config import ConfigError
 from ..csrc import ops
 from ..weights.loader import TensorSpec
 from .base import FeedForward, GatedSum
-from .linear import Linear, SMS
+from .linear import Linear, SMALL_ROWS
 from .mlp import ClampedGLU, SwiGLU
 from .registry import register_feed_forward
 from .spec import PartSpec
@@ -50,13 +50,17 @@ class RoutedExperts(FeedForward):
 
     Everything happens on the device: a kernel picks the experts, one orders the (token, choice) pairs by expert, and
     two grouped products (gate and up with the activation; down) walk the experts' rows.  The outputs of a token's
-    choices land in `top` planes that the norm behind the layer adds in order, so the sum does not depend on the
-    batch.  In a bfloat16 engine the two products are a stream of the chosen experts' weights on the tcgen05 tensor cores
+    choices land in `top` planes (times the parts of k, see _parts) that the norm behind the layer adds in order.  A
+    row's sum does not depend on the batch in float32; in bfloat16, below LIBRARY_ROWS rows per expert, it is the same in all
+    steps of up to SMALL_ROWS rows, and in all longer ones.  In a bfloat16 engine the two products are a stream of the chosen experts' weights on the tcgen05 tensor cores
     (ops.expert_stream; sizes that it does not take, and float32, run ops.grouped_gemm).  From LIBRARY_ROWS rows per expert (in the mean) on, a bfloat16 step hands the two products to the library's
     grouped product (which also takes the experts' bounds from the device): there the experts' outputs are rounded to
     bfloat16 before they are added up in 32-bit."""
 
-    LIBRARY_ROWS = 64        # (measured, see csrc/expert_stream.cu)
+    # (Measured, 16 experts, us by the library and by the stream of weights, launched kernel by kernel as steps of so many rows
+    # are, and replayed: width 2,048, 56 rows per expert 196 / 193 and 165 / 155, 62 rows 196 / 195 and 168 / 178, 80 rows 207 / 228 and 182 /
+    # 210; width 4,096, 62 rows 469 / 402 and 443 / 387, 80 rows 500 / 478 and 474 / 474, 96 rows 510 / 546 and 489 / 528.)
+    LIBRARY_ROWS = 64
 
     graph_safe = True
 
@@ -201,19 +205,15 @@ class RoutedExperts(FeedForward):
         return GatedSum(y, self.shared.forward(x, ctx), gate)
 
     def _parts(self, T):
-        """Parts of k of the second product in a step of few tokens: what shares the tiles of the experts that such a step
-        reaches (in the mean) most evenly over the SMs.  Every part has planes of its own, so not with identity experts,
-        which write a plane themselves, nor where the planes are many rows."""
+        """Parts of k of the second product: halves in a step of few rows, where they are 8 steps of the ring or more.  A step of
+        one or two tokens reaches so few experts that whole ranges leave SMs idle; every part has planes of its own, so not with
+        identity experts, which write a plane themselves, nor where the planes are many rows.  From the layer's sizes alone on
+        either side of SMALL_ROWS (where the dense products change their kernels as well), so that a row's sum does not depend
+        on how many others its step has.  Measured, a mixture of 16 experts with 1, 2 and 4 parts, us: width 2,048, one token 57.9, 55.5,
+        55.6; 16 tokens 99, 100, 103; 64 tokens 126, 129, 137; width 4,096, one token 99.7, 98.1, 98.3; 8 tokens 209, 211, 216; 64
+        tokens 315, 313, 329."""
         k_tiles = -(-self.inter // 64)
-        if self.identity or T > 64:
-            return 1
-        reached = self.experts * (1.0 - (1.0 - self.top / self.outputs) ** T)
-        tiles = reached * -(-self.hidden // 128)
-
-        def even(s):
-            rounds = tiles * s / SMS
-            return rounds / -(-rounds // 1) - 0.02 * s
-        return max((s for s in (1, 2, 4) if s == 1 or k_tiles % s == 0 and k_tiles // s >= 8), key=even)
+        return 1 if self.identity or T > SMALL_ROWS or k_tiles % 2 or k_tiles < 16 else 2
 
     def _experts_by_the_library(self, x, start, pair_of_slot, weight, y):
         """The road of steps with many rows per expert: the rows in the experts' order with their weights on them, the

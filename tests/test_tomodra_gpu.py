@@ -712,6 +712,39 @@ def test_expert_stream_against_64_bit_products(T, top, n, E, F, splits):
         assert (got - want).abs().max() <= 3e-6 * (down[e].double().abs() @ act[s].double().abs()).max()
 
 
+def test_a_rows_experts_do_not_depend_on_the_rows_beside_it():
+    """A mixture in bfloat16: a row's planes are the same, bit for bit, in every step of up to 64 rows, and in every longer one on
+    the stream of weights; their sums are those of the 64-bit experts."""
+    from types import SimpleNamespace
+    from air_b200.parts.base import Runtime
+    from air_b200.parts.experts import RoutedExperts
+    from air_b200.parts.spec import PartSpec
+    n, top, E, F = 16, 2, 4096, 1024
+    g = torch.Generator(device="cuda").manual_seed(8)
+    rand = lambda *s: (torch.randn(*s, generator=g, device="cuda") * s[-1] ** -0.5).bfloat16()
+    w = {"m.router": rand(n, E) * 4}
+    for e in range(n):
+        w.update({f"m.e{e}.gate": rand(F, E) * 2, f"m.e{e}.up": rand(F, E), f"m.e{e}.down": rand(E, F)})
+    part = RoutedExperts(PartSpec("routed_experts", dict(hidden=E, experts=n, top=top, intermediate=F, shared_intermediate=0,
+                                                         weight_on="output")), "m.")
+    part.load(w, Runtime(torch.device(DEV), torch.bfloat16, 64, status=torch.zeros(1, dtype=torch.int32, device=DEV)))
+    x = torch.randn(300, E, generator=g, device="cuda").bfloat16()
+    z = x.double() @ w["m.router"].double().T
+    kept = {}
+    for T in (64, 33, 17, 8, 3, 2, 1, 300, 130, 65):
+        y = part.forward(x[:T].contiguous(), SimpleNamespace(residual=None)).clone()
+        first = kept.setdefault(T <= 64, y)
+        assert y.shape[0] == first.shape[0] and torch.equal(y, first[:, :T]), T
+        for t in {0, T - 1}:
+            s, chosen = torch.sigmoid(z[t]).topk(top)
+            want = 0
+            for weight, e in zip(s, chosen.tolist()):
+                act = torch.nn.functional.silu(w[f"m.e{e}.gate"].double() @ x[t].double()) * (w[f"m.e{e}.up"].double() @ x[t].double())
+                want = want + weight * (w[f"m.e{e}.down"].double() @ act)
+            # (what the activation loses in bfloat16, 2^-8 of each of 1,024 numbers, averages out in the sum)
+            assert (y[:, t].double().sum(0) - want).abs().max() < 0.01 * want.abs().max(), T
+
+
 @pytest.mark.parametrize("H,rot,window,n,pos0,sink", [(3, 64, None, 64, 0, False), (2, 64, None, 300, 0, True), (1, 0, None, 257, 100, True),
                                                       (2, 64, 70, 200, 333, False), (4, 0, 130, 65, 0, False),
                                                       (2, 64, None, 70, 6000, True), (2, 64, 2000, 129, 5000, False)])
