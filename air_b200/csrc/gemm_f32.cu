@@ -36,8 +36,9 @@ template <int N> __device__ __forceinline__ void gf_wait() { asm volatile("cp.as
 // nothing is transposed.  Rows of TILE_K + 4 floats put the eight rows that a quarter of a warp reads into different banks.
 // A thread's rows and columns lie (BM / TM) and (BN / TN) apart.  (Staged transposed, and with 8 x 8 or 8 x 16 sums per
 // thread, the same product stayed within 5 %.)
-// CL 1: a block takes all ranges of k, one after the other, and adds their sums up in C.  CL PARTS: the blocks of a cluster
-// take a range each and add the sums up through one another's shared memory, a quarter of the tile each.
+// CL 1: a block takes all of k in one go and keeps the sum of the ranges that are done in shared memory (a number of its own per
+// thread).  CL PARTS: the blocks of a cluster take a range each and add the sums up through one another's shared memory, a
+// quarter of the tile each.
 constexpr int TILE_K = 16, TILE_LD = TILE_K + 4, TILE_STAGES = 4;
 
 template <int BM, int BN, int TM, int TN, int CL>
@@ -54,107 +55,111 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
     const int tid = threadIdx.x, tx = tid / 32 % (DX / 8) * 8 + tid % 8, ty = tid / 32 / (DX / 8) * 4 + tid % 32 / 8;
     const int rank = CL > 1 ? blockIdx.x % CL : 0;
     const int m0 = (blockIdx.x / CL) * BM, n0 = blockIdx.y * BN;        // (blocks beside one another share their weights)
-    const int Kp = part_of(K);
-    for (int part = CL > 1 ? rank : 0; part < (CL > 1 ? rank + 1 : PARTS); ++part) {
-        const int k_lo = part * Kp, k_hi = min(K, k_lo + Kp);
-        if (CL == 1 && part > 0 && k_lo >= K) break;
-        // this thread's pieces of a stage: the same rows at every step, TILE_K further on
-        const int k_mine = (tid % (TILE_K / 4)) * 4;
-        const float* src[COPIES];
+    const int Kp = part_of(K), k_lo = CL > 1 ? rank * Kp : 0, k_hi = CL > 1 ? min(K, k_lo + Kp) : K;
+    float* const done = smem + TILE_STAGES * ROWS * TILE_LD + threadIdx.x;      // CL 1: [TM * TN][THREADS]
+    // this thread's pieces of a stage: the same rows at every step, TILE_K further on
+    const int k_mine = (tid % (TILE_K / 4)) * 4;
+    const float* src[COPIES];
+#pragma unroll
+    for (int c = 0; c < COPIES; ++c) {
+        const int row = tid / (TILE_K / 4) + c * (THREADS / (TILE_K / 4)), r = row < BM ? m0 + row : n0 + row - BM;
+        src[c] = r < (row < BM ? M : N) ? (row < BM ? A : W) + (size_t)r * K + k_lo + k_mine : nullptr;
+    }
+    float* const dst = smem + (tid / (TILE_K / 4)) * TILE_LD + k_mine;
+    auto bring = [&](int step) {
+        float* to = dst + (step % TILE_STAGES) * ROWS * TILE_LD;
+        const bool in_k = k_lo + step * TILE_K + k_mine < k_hi;
 #pragma unroll
         for (int c = 0; c < COPIES; ++c) {
-            const int row = tid / (TILE_K / 4) + c * (THREADS / (TILE_K / 4)), r = row < BM ? m0 + row : n0 + row - BM;
-            src[c] = r < (row < BM ? M : N) ? (row < BM ? A : W) + (size_t)r * K + k_lo + k_mine : nullptr;
+            const bool in = in_k && src[c];
+            gf_copy16(to + c * (THREADS / (TILE_K / 4)) * TILE_LD, in ? src[c] + step * TILE_K : A, in);
         }
-        float* const dst = smem + (tid / (TILE_K / 4)) * TILE_LD + k_mine;
-        auto bring = [&](int step) {
-            float* to = dst + (step % TILE_STAGES) * ROWS * TILE_LD;
-            const bool in_k = k_lo + step * TILE_K + k_mine < k_hi;
+    };
+    float acc[TM][TN];
 #pragma unroll
-            for (int c = 0; c < COPIES; ++c) {
-                const bool in = in_k && src[c];
-                gf_copy16(to + c * (THREADS / (TILE_K / 4)) * TILE_LD, in ? src[c] + step * TILE_K : A, in);
-            }
-        };
-        float acc[TM][TN];
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int i = 0; i < TM; ++i)
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    const int steps = max(0, (k_hi - k_lo + TILE_K - 1) / TILE_K);
 #pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-        const int steps = max(0, (k_hi - k_lo + TILE_K - 1) / TILE_K);
-        if (CL == 1) __syncthreads();            // (everybody is done with the stages of the range before)
+    for (int s = 0; s < TILE_STAGES - 1; ++s) {
+        if (s < steps) bring(s);
+        gf_commit();
+    }
+    for (int step = 0; step < steps; ++step) {
+        gf_wait<TILE_STAGES - 2>();
+        __syncthreads();
+        if (step + TILE_STAGES - 1 < steps) bring(step + TILE_STAGES - 1);
+        gf_commit();
+        if (CL == 1 && step > 0 && step % (Kp / TILE_K) == 0) {       // a range is done
 #pragma unroll
-        for (int s = 0; s < TILE_STAGES - 1; ++s) {
-            if (s < steps) bring(s);
-            gf_commit();
-        }
-        for (int step = 0; step < steps; ++step) {
-            gf_wait<TILE_STAGES - 2>();
-            __syncthreads();
-            if (step + TILE_STAGES - 1 < steps) bring(step + TILE_STAGES - 1);
-            gf_commit();
-            const float* as = smem + (step % TILE_STAGES) * ROWS * TILE_LD + ty * TILE_LD;
-            const float* ws = smem + (step % TILE_STAGES) * ROWS * TILE_LD + (BM + tx) * TILE_LD;
-#pragma unroll
-            for (int k = 0; k < TILE_K; k += 4) {          // (beyond the range both operands hold zeros)
-                float a[TM][4], w[2][4];
-#pragma unroll
-                for (int i = 0; i < TM; ++i) load4(as + i * DY * TILE_LD + k, a[i]);
-                load4(ws + k, w[0]);
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) {
-                    if (j + 1 < TN) load4(ws + (j + 1) * DX * TILE_LD + k, w[(j + 1) & 1]);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-#pragma unroll
-                        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i][e], w[j & 1][e], acc[i][j]);
+                    float* sum = done + (i * TN + j) * THREADS;
+                    *sum = step > Kp / TILE_K ? *sum + acc[i][j] : acc[i][j];
+                    acc[i][j] = 0.f;
                 }
-            }
         }
-        gf_wait<0>();
-        if constexpr (CL == 1) {
-            const bool last = part + 1 == PARTS || k_lo + Kp >= K;
+        const float* as = smem + (step % TILE_STAGES) * ROWS * TILE_LD + ty * TILE_LD;
+        const float* ws = smem + (step % TILE_STAGES) * ROWS * TILE_LD + (BM + tx) * TILE_LD;
+#pragma unroll
+        for (int k = 0; k < TILE_K; k += 4) {          // (beyond the range both operands hold zeros)
+            float a[TM][4], w[2][4];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) load4(as + i * DY * TILE_LD + k, a[i]);
+            load4(ws + k, w[0]);
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
-                const int n = n0 + tx + j * DX;
-                if (n >= N) continue;
-                const float b = bias && last ? bias[n] : 0.f;
+                if (j + 1 < TN) load4(ws + (j + 1) * DX * TILE_LD + k, w[(j + 1) & 1]);
 #pragma unroll
-                for (int i = 0; i < TM; ++i) {
-                    const int m = m0 + ty + i * DY;
-                    if (m >= M) continue;
-                    float* to = C + (size_t)m * N + n;     // (of this thread alone)
-                    const float sum = part ? *to + acc[i][j] : acc[i][j];
-                    *to = last && bias ? sum + b : sum;
-                }
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i][e], w[j & 1][e], acc[i][j]);
             }
-        } else {
-            __syncthreads();                               // (the stages' memory takes the tile's sums)
-#pragma unroll
-            for (int j = 0; j < TN; ++j)
-#pragma unroll
-                for (int i = 0; i < TM; ++i) smem[(ty + i * DY) * BN + tx + j * DX] = acc[i][j];
-            cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-            cluster.sync();
-            const float* from[CL];
-#pragma unroll
-            for (int r = 0; r < CL; ++r) from[r] = cluster.map_shared_rank(smem, r);
-            for (int i = tid * 4; i < BM / CL * BN; i += THREADS * 4) {
-                const int at = rank * (BM / CL) * BN + i, m = m0 + at / BN, n = n0 + at % BN;
-                float v[CL][4];
-#pragma unroll
-                for (int r = 0; r < CL; ++r) load4(from[r] + at, v[r]);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    if (m >= M || n + e >= N) continue;
-                    float sum = v[0][e];
-#pragma unroll
-                    for (int r = 1; r < CL; ++r) sum += v[r][e];
-                    C[(size_t)m * N + n + e] = bias ? sum + bias[n + e] : sum;
-                }
-            }
-            cluster.sync();                                // (nobody leaves while its memory is read)
         }
+    }
+    gf_wait<0>();
+    if constexpr (CL == 1) {
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + tx + j * DX;
+            if (n >= N) continue;
+            const float b = bias ? bias[n] : 0.f;
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                const int m = m0 + ty + i * DY;
+                if (m >= M) continue;
+                const float sum = K > Kp ? done[(i * TN + j) * THREADS] + acc[i][j] : acc[i][j];
+                C[(size_t)m * N + n] = bias ? sum + b : sum;
+            }
+        }
+    } else {
+        __syncthreads();                               // (the stages' memory takes the tile's sums)
+#pragma unroll
+        for (int j = 0; j < TN; ++j)
+#pragma unroll
+            for (int i = 0; i < TM; ++i) smem[(ty + i * DY) * BN + tx + j * DX] = acc[i][j];
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        cluster.sync();
+        const float* from[CL];
+#pragma unroll
+        for (int r = 0; r < CL; ++r) from[r] = cluster.map_shared_rank(smem, r);
+        for (int i = tid * 4; i < BM / CL * BN; i += THREADS * 4) {
+            const int at = rank * (BM / CL) * BN + i, m = m0 + at / BN, n = n0 + at % BN;
+            float v[CL][4];
+#pragma unroll
+            for (int r = 0; r < CL; ++r) load4(from[r] + at, v[r]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (m >= M || n + e >= N) continue;
+                float sum = v[0][e];
+#pragma unroll
+                for (int r = 1; r < CL; ++r) sum += v[r][e];
+                C[(size_t)m * N + n + e] = bias ? sum + bias[n + e] : sum;
+            }
+        }
+        cluster.sync();                                // (nobody leaves while its memory is read)
     }
 }
 
@@ -275,28 +280,30 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, co
 constexpr int GB = 64;   // tile of C is GB x GB
 constexpr int GK = 16;   // k-step
 
-__global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                                                       const float* __restrict__ bias, float* __restrict__ C,
-                                                       int M, int N, int K) {
+__global__ void __launch_bounds__(256, 5)
+gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C, int M,
+                int N, int K) {
     __shared__ float sa[GK][GB + 4];
     __shared__ float sw[GK][GB + 4];
+    __shared__ float done[16][256];     // every thread's sums of the ranges that are done (in registers: a fifth slower in full waves)
     pdl_enter(TR_GEMM_F32);
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;          // 16 x 16 threads, 4 x 4 outputs each
     const int m0 = blockIdx.y * GB, n0 = blockIdx.x * GB;
     const int Kp = part_of(K);
-    float acc[4][4] = {}, total[4][4] = {};
+    float acc[4][4] = {};
     const int lr = tid >> 2;            // 0..63: row of the tile this thread loads
     const int lk = (tid & 3) * 4;       // 0,4,8,12: first k of its four elements
+    int next = Kp;
     for (int k0 = 0; k0 < K; k0 += GK) {
-        if (k0 && k0 % Kp == 0) {       // a range of k begins
+        if (k0 == next) {               // a range of k begins
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    total[i][j] = k0 == Kp ? acc[i][j] : total[i][j] + acc[i][j];
-                    acc[i][j] = 0.f;
-                }
+            for (int i = 0; i < 16; ++i) {
+                float& sum = acc[i / 4][i % 4];
+                done[i][tid] = k0 == Kp ? sum : done[i][tid] + sum;
+                sum = 0.f;
+            }
+            next += Kp;
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -327,7 +334,7 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + tx * 4 + j;
-            const float sum = K > Kp ? total[i][j] + acc[i][j] : acc[i][j];
+            const float sum = K > Kp ? done[4 * i + j][tid] + acc[i][j] : acc[i][j];
             if (n < N) C[(size_t)m * N + n] = bias ? sum + bias[n] : sum;
         }
     }
@@ -336,7 +343,7 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__
 template <int BM, int BN, int TM, int TN, int CL>
 static int launch_f32_tiles(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t stream) {
     auto kernel = gemm_f32_tile_kernel<BM, BN, TM, TN, CL>;
-    const int stages = TILE_STAGES * (BM + BN) * TILE_LD * 4, smem = CL > 1 ? max(stages, BM * BN * 4) : stages;
+    const int stages = TILE_STAGES * (BM + BN) * TILE_LD * 4, smem = CL > 1 ? max(stages, BM * BN * 4) : stages + BM * BN * 4;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
@@ -372,6 +379,14 @@ static double fullest(int M, int N, int BM, int BN, int CL) {
     return (double)((blocks + 147) / 148) * BM * BN / CL;
 }
 
+// What tiles of BM x 64 take for a short k, in steps of 16 of k of a tile of 64 x 64: the blocks that follow one another on the
+// fullest SM, and a block's own way through a step where it has the SM to itself; a cluster's exchange is one step more.
+static double tile_cost(int M, int N, int K, int BM, int CL) {
+    const long long blocks = (long long)((M + BM - 1) / BM) * ((N + 63) / 64) * CL;
+    const int steps = CL > 1 ? part_of(K) / TILE_K : (K + TILE_K - 1) / TILE_K;
+    return (steps + (CL > 1 ? 1 : 0)) * ((double)((blocks + 147) / 148) * (BM == 32 ? 0.5625 : 1.0) + (BM == 32 ? 0.7 : 1.0));
+}
+
 }  // namespace air
 
 // w_ready: W was complete before the launch ahead of this one was made (a model's weights): it may be read before that one ends.
@@ -385,24 +400,38 @@ AIR_API int air_gemm_f32(const float* A, const float* W, const float* bias, floa
         if (grid.y > 65535) return AIR_ERR_BAD_ARGUMENT;
         return launch(gemm_f32_kernel, grid, 256, 0, stream, A, W, bias, C, M, N, K);
     }
-    // A stream of weights up to 16 rows: as many columns to a block as put every SM to work.  (16 rows by 16,384 x 2,048: 80 us;
+    // A stream of weights up to 16 rows, unless k is so short that its blocks' ways in and out are all that it has: 4 rows by 4,096 x 16
+    // 2.8 us against 2.2 by half tiles, 16 rows by 4,096 x 32 4.3 and 2.6, by 16,384 x 64 14.7 and 6.4 (by 4,096 x 64 4.7 and 4.0, one row
+    // by 4,096 x 32 2.2 and 2.6).  As many columns to a block as put every SM to work.  (16 rows by 16,384 x 2,048: 80 us;
     // tiles of 32 rows, half of them empty, would take the 77 us of 32 rows there, and twice as long where N is small: 64
     // blocks at 1,024 columns.)
+    if (M <= FEW_ROWS && (K <= 16 || (K <= 32 && M > 8) || (K <= 64 && N > 148 * FEW_COLS)))
+        return launch_f32_tiles<32, 64, 4, 4, 1>(A, W, bias, C, M, N, K, stream);
     if (M <= FEW_ROWS) {
         const int cols = max(1, min(FEW_COLS, (N + 147) / 148));
         if (M == 1) return launch_f32_few<1>(A, W, bias, C, M, N, K, cols, w_ready, stream);
         if (M == 2) return launch_f32_few<2>(A, W, bias, C, M, N, K, cols, w_ready, stream);
         return launch_f32_few<4>(A, W, bias, C, M, N, K, cols, w_ready, stream);
     }
-    // Tiles of 64 x 64 wherever they share out as evenly over the SMs as tiles of 32 x 64 do, whose outputs cost an eighth more
-    // to feed.  (32 rows by 16,384 x 2,048: 77 us against 125; 300 by 3,072 x 2,048: 126 against 111.  Tiles of 128 columns or
-    // rows were within 3 % of 64 x 64 at 512 and 2,048 rows and slower below.)
-    if (fullest(M, N, 32, 64, PARTS) * 1.125 < fullest(M, N, 64, 64, PARTS))
-        return launch_f32_tiles<32, 64, 4, 4, PARTS>(A, W, bias, C, M, N, K, stream);
-    // A cluster's exchange costs what a few steps of k do: 777 rows by 2,048 x 16 take 10 us without, 25 with; from 64 steps on
-    // the cluster is ahead (300 by 2,048 x 2,048: 84 us against 150, 512 by 16,384 x 2,048: 838 against 860).
-    if (K < 1024) return launch_f32_tiles<64, 64, 4, 8, 1>(A, W, bias, C, M, N, K, stream);
-    return launch_f32_tiles<64, 64, 4, 8, PARTS>(A, W, bias, C, M, N, K, stream);
+    // From 64 steps of k on, a cluster with a block for every range: tiles of 64 x 64 wherever they share out as evenly over the
+    // SMs as tiles of 32 x 64 do, whose outputs cost an eighth more to feed.  (32 rows by 16,384 x 2,048: 72 us against 117; 300 by
+    // 3,072 x 2,048: 119 against 111.  Tiles of 128 columns or rows were within 3 % of 64 x 64 at 512 and 2,048 rows and slower
+    // below.)
+    if (K >= 1024) {
+        if (fullest(M, N, 32, 64, PARTS) * 1.125 < fullest(M, N, 64, 64, PARTS))
+            return launch_f32_tiles<32, 64, 4, 4, PARTS>(A, W, bias, C, M, N, K, stream);
+        return launch_f32_tiles<64, 64, 4, 8, PARTS>(A, W, bias, C, M, N, K, stream);
+    }
+    // Fewer steps: the quickest of the four by tile_cost.  Measured over 1,188 sizes (17 to 2,048 rows, 64 to 16,384 columns, k of
+    // 16 to 768): in the mean 2 % above the quickest of the four.  us, by blocks that began their ranges one after the other (17 rows: in
+    // a cluster), by the kernel of any width, and now: 2,048 rows by 8,192 x 64 173, 120, 74; 777 by 4,096 x 64 43, 28, 20; 300 by 2,048 x
+    // 512 65, 61, 28; 17 by 2,048 x 16 4.0, 2.4, 2.2.
+    const double whole = tile_cost(M, N, K, 64, 1), half = tile_cost(M, N, K, 32, 1), whole_cut = tile_cost(M, N, K, 64, PARTS),
+                 half_cut = tile_cost(M, N, K, 32, PARTS), least = min(min(whole, half), min(whole_cut, half_cut));
+    if (whole == least) return launch_f32_tiles<64, 64, 4, 8, 1>(A, W, bias, C, M, N, K, stream);
+    if (whole_cut == least) return launch_f32_tiles<64, 64, 4, 8, PARTS>(A, W, bias, C, M, N, K, stream);
+    if (half == least) return launch_f32_tiles<32, 64, 4, 4, 1>(A, W, bias, C, M, N, K, stream);
+    return launch_f32_tiles<32, 64, 4, 4, PARTS>(A, W, bias, C, M, N, K, stream);
 }
 
 AIR_API int air_trace_set_gemm_f32(unsigned long long* buffer) { return air::set_trace_here(buffer); }

@@ -301,6 +301,14 @@ def test_paged_attention_ref(H, K, d, P, window, dtype):
     assert np.abs(out.float().cpu().numpy() - want).max() < tol * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("M,N,K", [(17, 2048, 16), (31, 65, 1020), (33, 8192, 36), (70, 4097, 200), (70, 1024, 900), (130, 257, 64),
+                                   (300, 2047, 68), (777, 4095, 48), (1, 65, 16), (16, 301, 32), (3, 4800, 64), (9, 70, 17), (66, 130, 333), (2048, 1025, 132), (65, 16384, 20)])
+def test_gemm_f32_with_a_short_k(M, N, K):
+    """Whole and half tiles, with a cluster and without, with one to four ranges of k: the sums of the other kernels, at
+    remainders of every tile."""
+    test_gemm_f32_kernels_of_every_size_add_in_one_order(M, N, K)
+
+
 @pytest.mark.parametrize("M", [1, 4, 16])
 def test_gemm_f32_with_a_matrix_that_the_launches_ahead_write(M):
     """Both operands come from the package's own kernels right ahead, over and over with new numbers: a matrix that is not a
