@@ -9,7 +9,7 @@ from ..config.model_config import ConfigError
 from ..csrc import ops
 from ..weights.loader import TensorSpec
 from .base import HostBatch, Mixer, Plan, SlotState
-from .linear import Linear
+from .linear import Linear, SMS
 from .registry import register_mixer
 
 
@@ -51,20 +51,32 @@ class _ChunkedMixer(_StateMixer):
     """State mixers whose longer portions a bfloat16 engine takes in chunks whose rows are computed side by side
     (ops.delta_portions); everything else goes token by token (ops.linear_scan)."""
 
-    PORTION = 24
+    # Tokens from which a portion goes in chunks.  Their chain has a block per head, 16 columns of the state and portion, as the tokens'
+    # has, but two launches and a chain's beginning of its own, which wide heads repay from ALONE tokens on where one round of the SMs
+    # holds all blocks; beyond, and for narrow heads, from PORTION on.  Measured, us, token by token and in chunks: 16 heads of 128 x 128,
+    # one portion of 32, 48 and 64 tokens 11.1 / 12.9, 14.2 / 15.7, 17.5 / 17.0, four of 24 and 32 17.1 / 18.4, 20.0 / 18.6; 32 heads, one
+    # of 24 and 32 12.7 / 12.7, 14.2 / 12.7; gated linear attention, 8 heads of 128 x 256, one of 48 and 64 12.4 / 14.7, 15.1 / 15.7; 4 heads of
+    # 64 x 64, one of 24 and 32 8.8 / 9.5, 10.0 / 9.5.
+    PORTION, ALONE = 32, 64
 
     def plan_key(self):
         chunks = self.rt.dtype == torch.bfloat16 and self.head_dim <= ops.DELTA_MAX_D
-        return ("linear.chunks", self.PORTION) if chunks else None
+        return ("linear.chunks", self.heads * -(-self.v_dim // 16), self.head_dim > 64) if chunks else None
+
+    def least(self, counts):
+        """From how many tokens on the portions of a step of such entries go in chunks."""
+        blocks = sum(n >= self.PORTION for n in counts) * self.heads * -(-self.v_dim // 16)
+        return self.PORTION if self.head_dim <= 64 or blocks > SMS else self.ALONE
 
     def plan(self, batch: HostBatch) -> Plan:
-        """portions [L, 4] = (first row, tokens, slot, first chunk) of the entries of at least PORTION tokens, chunks [N, 2] =
+        """portions [L, 4] = (first row, tokens, slot, first chunk) of the entries that go in chunks (see least), chunks [N, 2] =
         (first row, tokens) of theirs; short_slots: the slot of every other entry, short_seq: of their rows, -1 elsewhere."""
         portions, chunks, short_slots = [], [], []
         short_seq = np.full(batch.q_start[-1], -1, dtype=np.int32)
+        least = self.least(batch.counts)
         for i, n in enumerate(batch.counts):
             first = batch.q_start[i]
-            if n < self.PORTION:
+            if n < least:
                 short_slots.append(batch.slots[i])
                 short_seq[first:first + n] = batch.slots[i]
                 continue
@@ -165,7 +177,7 @@ class ChannelDeltaRule(_ChunkedMixer):
     then o / sqrt(mean(o^2) + eps) * norm, times sigmoid(W_g2 (W_g1 x)) (laid out heads x v_dim), and the output
     projection.  S and the convolutions' last conv - 1 inputs are the request's state, 32-bit, zero at its start.
 
-    In a bfloat16 engine portions of PORTION tokens or more are taken in chunks whose rows are computed side by side
+    In a bfloat16 engine longer portions are taken in chunks whose rows are computed side by side
     (ops.delta_portions); everything else goes token by token (ops.linear_scan).
 
     The two products out of a narrow middle take its numbers as they left the first product: a float32 engine in 32-bit,

@@ -439,3 +439,34 @@ def test_layers_share_a_plan_only_where_it_is_the_same_for_both():
     plans = {p.plan_key(): p.plan(batch) for p in layers}
     assert len(plans) == 4 and len({p.values["alongside"] for p in plans.values()}) == 2
     assert "segments" in plans[normed.plan_key()].arrays, "a layer whose kernels run in turn is cut as before"
+
+
+def test_which_portions_of_a_recurrent_mixer_go_in_chunks():
+    """Short portions token by token where their blocks are one round of the SMs; a plan says so for all mixers of its key."""
+    from types import SimpleNamespace
+    import torch
+    from air_b200.parts.base import HostBatch
+    from air_b200.parts.recurrent import ChannelDeltaRule, GatedDeltaRule, GatedLinearAttention
+
+    def layer(cls, heads, head_dim, v_dim, dtype=torch.bfloat16):
+        part = cls.__new__(cls)
+        part.heads, part.head_dim, part.v_dim, part.rt = heads, head_dim, v_dim, SimpleNamespace(dtype=dtype)
+        return part
+
+    def chunked(part, counts):
+        starts = [0]
+        for c in counts:
+            starts.append(starts[-1] + c)
+        plan = part.plan(HostBatch(counts=counts, lengths=[0] * len(counts), slots=list(range(len(counts))), q_start=starts))
+        rows = plan.arrays["portions"][:, 1].tolist()
+        assert plan.values["long"] == bool(rows) and plan.values["short"] == (len(rows) < len(counts))
+        assert (plan.arrays["short_seq"] >= 0).sum() == sum(counts) - sum(rows)
+        return rows
+
+    for cls in (GatedDeltaRule, GatedLinearAttention, ChannelDeltaRule):
+        one, wide, narrow = layer(cls, 16, 128, 128), layer(cls, 32, 128, 128), layer(cls, 4, 64, 64)
+        assert chunked(one, [1, 63]) == [] and chunked(one, [1, 64]) == [64]
+        assert chunked(one, [32, 31, 33]) == [32, 33] and chunked(wide, [32]) == [32] and chunked(wide, [31, 1]) == []
+        assert chunked(narrow, [32, 5]) == [32] and chunked(narrow, [31]) == []
+        assert len({p.plan_key() for p in (one, wide, narrow)}) == 3 and layer(cls, 16, 96, 120).plan_key() == one.plan_key()
+        assert layer(cls, 16, 128, 128, torch.float32).plan_key() is None
