@@ -22,18 +22,19 @@
 //                              channels lie across the warps and stay in accumulators from the first chunk to the last:
 //                              as a result of one product they are the left operand of the next without a move (the
 //                              instruction's k may run in any order that both operands share).  Every 32-bit operand enters as
-//                              two TF32 numbers, hi + lo, and every product as lo hi + hi lo + hi hi, which keeps 21 bits of
-//                              the operands: what is left out is of the order of 32-bit rounding.  The next chunk's
+//                              two TF32 numbers, hi + lo, and every product as lo hi + hi lo + hi hi, which keeps the
+//                              operands to 2^-23: what is left out is of the order of 32-bit rounding.  The next chunk's
 //                              numbers arrive by the copy engine, in two runs of bytes, while this one's are used.
 //
-// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 196 (prepare
-// 49, scan 148); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 95 (25 and 70).  Which portions
-// come here: parts/recurrent.py (least).
+// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 197 (prepare
+// 49, scan 147); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 98 (24 and 73).  Which portions come here:
+// parts/recurrent.py (least).
 //
 // Errors against 64 bits (2-norm of the difference over that of the result, 2,048 tokens), token by token and here: one decay per
-// head, outputs 1.98e-7 and 1.97e-7, states 1.56e-7 and 1.59e-7; gated linear attention 1.60e-7 and 1.63e-7, 1.40e-7 and 1.14e-7; decays
+// head, outputs 1.98e-7 and 1.95e-7, states 1.56e-7 and 1.58e-7; gated linear attention 1.60e-7 and 1.60e-7, 1.40e-7 and 1.10e-7; decays
 // near 1, where a token's own rounding adds up, 2.9e-6 and 2.5e-7.  (Operands cut instead of rounded to their upper half, the state
-// as the products' accumulator, sums of logarithms in one number and 2^x in one instruction: 8.8e-7 and 5.4e-7, at 191 and 86 us.)
+// as the products' accumulator, sums of logarithms in one number and 2^x in one instruction: 8.8e-7 and 5.4e-7, at 191 and 86 us.
+// The state's update by multiply-adds on the CUDA cores: states 1.48e-7 and 1.01e-7, at 226 and 113 us.)
 // An infinity or a NaN reaches what it reaches token by token, and nothing ahead of its token.
 //
 // What a row is depends on the state and the portion's tokens only.
@@ -459,11 +460,11 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
             two_pair(hi, UT + (g + 8) * DC_ULD + 8 * x + t2);
             u[x][0] = lo[0]; u[x][1] = hi[0]; u[x][2] = lo[1]; u[x][3] = hi[1];
         }
-        float more[NJ][4], less[NJ][4], o[4] = {0.f, 0.f, 0.f, 0.f}, o_low[4] = {0.f, 0.f, 0.f, 0.f};
+        float more[2][NJ][4], less[NJ][4], o[4] = {0.f, 0.f, 0.f, 0.f}, o_low[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < NJ; ++j)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) more[j][e] = less[j][e] = 0.f;
+            for (int e = 0; e < 4; ++e) more[0][j][e] = more[1][j][e] = less[j][e] = 0.f;
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             Two k[NJ][2], w[2];
@@ -481,13 +482,13 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
             for (int j = 0; j < NJ; ++j) mma_tf32(less[j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].lo, k[j][1].lo);
             if (warp == 1 && x == 0) mma_tf32(o, u[0][0].hi, u[0][1].hi, u[0][2].hi, u[0][3].hi, w[0].hi, w[1].hi);
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) mma_tf32(more[j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].hi, k[j][1].hi);
+            for (int j = 0; j < NJ; ++j) mma_tf32(more[x][j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].hi, k[j][1].hi);
         }
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
             const float2 w = *reinterpret_cast<const float2*>(buf + Place::LAST + r0 + 8 * j + t2);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) S[j][e] = fmaf(S[j][e], e & 1 ? w.y : w.x, more[j][e] + less[j][e]);
+            for (int e = 0; e < 4; ++e) S[j][e] = fmaf(S[j][e], e & 1 ? w.y : w.x, more[0][j][e] + (more[1][j][e] + less[j][e]));
         }
         if (warp < 2) {
             float* to = out + (size_t)i * DC * out_row;
