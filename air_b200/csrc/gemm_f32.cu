@@ -346,6 +346,8 @@ static int launch_f32_tiles(const float* A, const float* W, const float* bias, f
     const int stages = TILE_STAGES * (BM + BN) * TILE_LD * 4, smem = CL > 1 ? max(stages, BM * BN * 4) : stages + BM * BN * 4;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
+    if constexpr (CL == 1)
+        return launch(kernel, dim3((M + BM - 1) / BM, (N + BN - 1) / BN), (BM / TM) * (BN / TN), smem, stream, A, W, bias, C, M, N, K);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((M + BM - 1) / BM * CL, (N + BN - 1) / BN);
     cfg.blockDim = dim3((BM / TM) * (BN / TN));
