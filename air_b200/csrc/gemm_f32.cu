@@ -1,5 +1,5 @@
-// True 32-bit matrix product on the CUDA cores: C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]).
-// No tensor cores and no reduced-precision mode.  The sum of an element of C is the same whatever kernel takes it: k is cut
+// True 32-bit matrix product on the CUDA cores: C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]), for matrices W that gemm_f32_tc.cu does not
+// take (short k, few columns, rows that are not whole aligned 16-byte pieces).  No reduced-precision mode.  The sum of an element of C is the same whatever kernel takes it: k is cut
 // into PARTS ranges of equal length (a multiple of 16), each accumulated in ascending order by one thread with fused
 // multiply-adds, and the ranges' sums are added in ascending order.  So a row of C does not depend on which other rows are
 // in the batch: the 32-bit path gives the same bits for a token whether it is computed alone, in a portion of a prompt or

@@ -7,8 +7,9 @@ keeps every SM streaming weights by splitting the k range and hands the partial 
 bfloat16 weights, many rows (prompts): the library's tensor-core product (cuBLAS through
 torch.mm), as AIR's engine calls cuBLAS for its dense products
 (src/cuda/cuda_backend.cu:1981-1989, 2037-2043); accumulation is 32-bit.
-float32 weights: this package's CUDA-core kernel with fused multiply-adds in a fixed order, no
-tensor cores and no reduced-precision mode; a bfloat16 input is widened first.
+float32 weights: this package's own 32-bit products in a fixed order and without a reduced-precision
+mode (csrc/gemm_f32_tc.cu: every number as three bfloat16 numbers that add up to it, on the tensor
+cores; csrc/gemm_f32.cu: fused multiply-adds, for small matrices); a bfloat16 input is widened first.
 """
 from __future__ import annotations
 
@@ -136,7 +137,7 @@ class Linear:
             if x.dtype != torch.float32:
                 x = ops.convert(x, torch.empty(x.shape, dtype=torch.float32, device=x.device))
             out = torch.empty((x.shape[0], self.out_features), dtype=torch.float32, device=x.device)
-            ops.gemm_f32(x, w, bias, out, w_ready=True)
+            ops.gemm_f32(x, w, bias, out, w_ready=True, status=self.status)
             if out_dtype != torch.float32:
                 out = ops.convert(out, torch.empty(out.shape, dtype=out_dtype, device=x.device))
             return out

@@ -309,6 +309,61 @@ def test_gemm_f32_with_a_short_k(M, N, K):
     test_gemm_f32_kernels_of_every_size_add_in_one_order(M, N, K)
 
 
+@pytest.mark.parametrize("N,K", [(1024, 2048), (1031, 2052), (1100, 3076), (2050, 4160), (37888, 2048)])
+def test_gemm_f32_on_the_tensor_cores(N, K):
+    """Remainders of tiles, chunks and eighths of k; every width of tile and every cluster gives a row the same bits, wherever it
+    stands and however it is aligned.  The bound is that of the additions: 24 truncated ones among the 64 k of a sum, a chain of
+    K / 512 sums, and eight totals."""
+    from air_b200.csrc import ops as o
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    w, b = torch.randn(N, K, generator=g, device="cuda") * 0.02, torch.randn(N, generator=g, device="cuda")
+    a = torch.randn(261, K, generator=g, device="cuda") * torch.exp2(torch.randint(-9, 9, (1, K), generator=g, device="cuda").float())
+    assert o.f32_on_tensor_cores(w)
+    want = a.double() @ w.double().T + b.double()
+    bound = (K / 512 + 8 + 2 * 24 + 1) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T + b.double().abs())
+    whole = torch.empty(261, N, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    o.gemm_f32(a, w, b, whole, status=status)
+    assert ((whole.double() - want).abs() <= bound).all()
+    for M in (1, 2, 8, 9, 16, 17, 33, 64, 65, 100, 128, 130):
+        out, shifted = torch.full((M, N), 7.0, device="cuda"), torch.empty(M * K + 1, device="cuda")[1:].view(M, K)
+        o.gemm_f32(a[261 - M:], w, b, out, w_ready=True, status=status)
+        assert torch.equal(out, whole[261 - M:]), M
+        o.gemm_f32(shifted.copy_(a[:M]), w, b, out, status=status)
+        assert torch.equal(out, whole[:M]), M
+    for width in (16, 32, 64, 96, 112, 128):
+        for cluster in (1, 4, 8):
+            out = torch.full_like(whole, 7.0)
+            o.gemm_f32(a, w, b, out, status=status, shape=(width, cluster))
+            assert torch.equal(out, whole), (width, cluster)
+    assert status.item() == 0
+
+
+@pytest.mark.parametrize("M", [3, 20, 200])
+def test_gemm_f32_on_the_tensor_cores_with_infinities_nan_and_the_largest_numbers(M):
+    """What multiply-adds give: infinities, NaN and finite sums of numbers that are infinite as bfloat16; other rows and columns
+    are what they are without them."""
+    N, K = 1030, 2048
+    g = torch.Generator().manual_seed(M)
+    a, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g) * 0.02
+    clean = torch.empty(M, N, device="cuda")
+    ops().gemm_f32(dev(a), dev(w), None, clean)
+    top = float(np.finfo(np.float32).max)
+    a[0, 5], a[0, 900], a[1, 77], a[2, 3], w[7, 3], w[7, 2000], w[8, 100], w[9, :] = math.inf, math.inf, math.nan, top, 1e-30, 0.0, -math.inf, 0.0
+    out = torch.empty(M, N, device="cuda")
+    ops().gemm_f32(dev(a), dev(w), None, out)
+    with np.errstate(all="ignore"):
+        want = (a.double() @ w.double().T)
+    want = torch.where(want.abs() > top, torch.full_like(want, math.inf) * want.sign(), want)
+    got = out.cpu().double()
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    assert torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
+    fine = torch.isfinite(want)
+    assert ((got - want).abs()[fine] <= 1e-5 * (want.abs()[fine] + 1)).all()
+    rows, cols = torch.arange(M) > 2, (torch.arange(N) < 7) | (torch.arange(N) > 9)
+    assert torch.equal(out.cpu()[rows][:, cols], clean.cpu()[rows][:, cols])
+
+
 @pytest.mark.parametrize("M", [1, 4, 16])
 def test_gemm_f32_with_a_matrix_that_the_launches_ahead_write(M):
     """Both operands come from the package's own kernels right ahead, over and over with new numbers: a matrix that is not a
