@@ -256,16 +256,35 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 // The kernel is a chain of latencies, so a thread asks for CHUNK splits' values at once (all of them, up
 // to 32; and for the token's slot beside them: a padding token has its place in the buffers too) and
 // folds them into a running maximum, sum and value, in the order of the splits.
+// With cut.positions only the splits that keys fall to are read (the others' numbers are nobody's), and a token whose keys are one
+// split's is finished already: a step of one token, 48 keys, 32 splits: 2.7 -> 1.5 us.
+struct KeySplits {
+    const int* positions;
+    int window, early;
+};
+
 template <int D, int CHUNK>
 __global__ void decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                       const int* __restrict__ token_seq, __nv_bfloat16* __restrict__ out, int H,
                                       int splits, const float* __restrict__ sink, const float* __restrict__ gate,
-                                      int ldg, const TurnBack turn) {
+                                      int ldg, const TurnBack turn, const KeySplits cut) {
     __shared__ float row[D];
-    pdl_enter(TR_ATT_COMBINE);
     const int t = blockIdx.y, h = blockIdx.x;
     const size_t base = ((size_t)t * H + h) * splits;
+    // (cut.early: the step's positions were there before its first kernel)
+    pdl_trigger();
+    if (!cut.early) pdl_wait();
     const int slot = token_seq[t];
+    if (cut.positions) {
+        // the splits that hold keys, as decode_attention_tma_kernel shares the tiles out; where it is one, that one's block has
+        // written the output
+        const int pos = cut.positions[t], tiles = pos / 64 + 1 - (cut.window > 0 ? max(0, pos - cut.window + 1) : 0) / 64;
+        const int per = (tiles + splits - 1) / splits;
+        splits = (tiles + per - 1) / per;
+    }
+    if (cut.early) pdl_wait();
+    trace_point(TR_ATT_COMBINE);
+    if (cut.positions && splits == 1) return;
     for (int col = threadIdx.x; col < D; col += blockDim.x) {
         float mm = -INFINITY, ll = 0.f, acc = 0.f;
         for (int s0 = 0; s0 < splits; s0 += CHUNK) {
@@ -324,16 +343,17 @@ __global__ void decode_combine_kernel(const float* __restrict__ part_o, const fl
 template <int D>
 int launch_combine(const float* part_o, const float* part_ml, const int* token_seq, __nv_bfloat16* out, int T, int H,
                    int splits, cudaStream_t stream, const float* sink = nullptr, const float* gate = nullptr,
-                   int ldg = 0, const TurnBack& turn = TurnBack{nullptr, 0, 0, nullptr}) {
+                   int ldg = 0, const TurnBack& turn = TurnBack{nullptr, 0, 0, nullptr},
+                   const KeySplits& cut = KeySplits{nullptr, 0, 0}) {
     const int threads = D >= 128 ? 128 : 64;
     if (splits <= 8)
         return launch(decode_combine_kernel<D, 8>, dim3(H, T), threads, 0, stream, part_o, part_ml, token_seq, out, H,
-                      splits, sink, gate, ldg, turn);
+                      splits, sink, gate, ldg, turn, cut);
     if (splits <= 16)
         return launch(decode_combine_kernel<D, 16>, dim3(H, T), threads, 0, stream, part_o, part_ml, token_seq, out, H,
-                      splits, sink, gate, ldg, turn);
+                      splits, sink, gate, ldg, turn, cut);
     return launch(decode_combine_kernel<D, 32>, dim3(H, T), threads, 0, stream, part_o, part_ml, token_seq, out, H,
-                  splits, sink, gate, ldg, turn);
+                  splits, sink, gate, ldg, turn, cut);
 }
 
 template <int D>
@@ -384,14 +404,17 @@ AIR_API int air_decode_attention(const void* q, const void* cache, const int* bl
     }
 }
 
-// The merge of the splits alone (used by the kernels that produce the partial results elsewhere).
-AIR_API int air_decode_combine(const float* part_o, const float* part_ml, const int* token_seq, void* out, int T,
-                               int H, int D, int splits, cudaStream_t stream) {
+// The merge of what decode_attention_tma_kernel leaves (KeySplits; that kernel finishes a token whose keys are one split's).
+AIR_API int air_decode_combine_split(const float* part_o, const float* part_ml, const int* token_seq, void* out, int T, int H, int D,
+                                     int splits, const int* positions, int window, int early, cudaStream_t stream) {
     using namespace air;
+    const KeySplits cut{positions, window, early};
+    const TurnBack turn{nullptr, 0, 0, nullptr};
+    __nv_bfloat16* to = (__nv_bfloat16*)out;
     switch (D) {
-        case 64: return launch_combine<64>(part_o, part_ml, token_seq, (__nv_bfloat16*)out, T, H, splits, stream);
-        case 128: return launch_combine<128>(part_o, part_ml, token_seq, (__nv_bfloat16*)out, T, H, splits, stream);
-        case 256: return launch_combine<256>(part_o, part_ml, token_seq, (__nv_bfloat16*)out, T, H, splits, stream);
+        case 64: return launch_combine<64>(part_o, part_ml, token_seq, to, T, H, splits, stream, nullptr, nullptr, 0, turn, cut);
+        case 128: return launch_combine<128>(part_o, part_ml, token_seq, to, T, H, splits, stream, nullptr, nullptr, 0, turn, cut);
+        case 256: return launch_combine<256>(part_o, part_ml, token_seq, to, T, H, splits, stream, nullptr, nullptr, 0, turn, cut);
         default: return AIR_ERR_BAD_ARGUMENT;
     }
 }

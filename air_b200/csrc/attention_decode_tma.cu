@@ -40,6 +40,8 @@ constexpr int DT_CONSUMERS = 4;
 constexpr int DT_THREADS = (DT_CONSUMERS + 1) * 32;
 constexpr int DT_TILE = 64;     // keys per stage
 constexpr int DT_STAGES = 3;
+constexpr int AHEAD = 2;        // ranges of memory that blocks without keys ask into L2 (Ahead), in pieces of
+constexpr unsigned AHEAD_PIECE = 4096;
 constexpr int FRESH_PARTS = 4;  // partial sums of the q/k/v product that a thread asks for at once
 
 // The token's new q, k and v as the product left them (see the head of the file); qkv == nullptr: q is read
@@ -53,15 +55,35 @@ struct FreshQkv {
     __nv_bfloat16* cache;    // where k and v are written (nullptr: another run has written them)
 };
 
+// What the kernels behind this one read and none writes (their weights), in the order in which they do.  A captured step has as many
+// splits as a long context wants; with a short one most blocks find no key, memory idles for the 15 us of the attention, its
+// merge, the output product and the norm, and those blocks ask for their share of these ranges into L2.
+// Short requests for L2 only: beyond some 24 MB nothing was gained (the products behind take what L2 and an SM's copies
+// deliver, 8.7 TB/s over all SMs, wherever the weights lie) and the next layer's were delayed.  A step of one token, 8
+// layers of width 2,048, us: nothing asked 361.6, 8 MB 359.6, 20 MB 348.4, 40 MB 351.4, 60 MB 355.5, 100 MB 369.0.
+struct Ahead {
+    const uint8_t* at[AHEAD];
+    unsigned pieces[AHEAD];
+};
+__device__ __forceinline__ void ask_ahead(const Ahead& ahead, int lane) {
+    const unsigned block = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), blocks = gridDim.x * gridDim.y * gridDim.z;
+#pragma unroll
+    for (int a = 0; a < AHEAD; ++a)
+        for (unsigned i = block + lane * blocks; i < ahead.pieces[a]; i += 32 * blocks)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(ahead.at[a] + (size_t)i * AHEAD_PIECE), "r"(AHEAD_PIECE)
+                         : "memory");
+}
+
 template <int D, bool BIAS>
-__global__ void __launch_bounds__(DT_THREADS)
-decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const FreshQkv fresh,
+__global__ void __launch_bounds__(DT_THREADS, 2)
+decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const FreshQkv fresh, const Ahead ahead,
                             const __nv_bfloat16* __restrict__ q,
                             const int* __restrict__ block_table, int max_blocks, const int* __restrict__ token_seq,
                             const int* __restrict__ positions, __nv_bfloat16* __restrict__ out,
                             float* __restrict__ part_o, float* __restrict__ part_ml, int H, int K, int P, int window,
                             float scale_log2, float cap_log2, float cap_pre, int* status, const DistanceBias bias,
-                            int alongside) {
+                            int alongside, int direct) {
+    // direct: where only one split has keys of a token, its block writes the output (the merge leaves such a token alone)
     // cap_log2 > 0: a score s becomes cap * tanh(s * cap_pre) with cap_pre = scale / cap, in units of log2 e
     constexpr int SUB = D / 64;                 // 64-column sub-tiles of a row
     constexpr int SUB_BYTES = DT_TILE * 128;    // 8 KB
@@ -110,31 +132,36 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
     // are on their way while the product's last blocks still run.  Without fresh.qkv the token's key and value
     // were written to the page by the predecessor itself, and everybody waits.
     // alongside: see the head of this file; the first block alone waits, at its end, for all of the grid.
-    if (!alongside && !(warp == DT_CONSUMERS && fresh.qkv)) pdl_wait();
+    // For the same reason everybody reads the token's place ahead of the wait then: two reads after one another that every
+    // block's way to its first sums of the product would begin with.
+    if (!alongside && !fresh.qkv) pdl_wait();
+    const int t = blockIdx.z;
+    const int slot = token_seq[t], pos = positions[t];
+    const int lo = window > 0 ? max(0, pos - window + 1) : 0;
+    const int* bt = block_table + (size_t)max(0, slot) * max_blocks;
+    const int own_page = fresh.qkv && slot >= 0 ? bt[pos / P] : 0;
+    if (fresh.qkv && warp != DT_CONSUMERS) pdl_wait();
     auto leave = [&] {
         if (alongside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
     };
     trace_point(TR_ATT_DECODE);
 
-    const int t = blockIdx.z;
-    const int slot = token_seq[t];
     if (slot < 0) return leave();
     const int G = H / K;
     const int head_blocks = (G + 15) / 16;
     const int kvh = blockIdx.y / head_blocks, hb = blockIdx.y % head_blocks;
     const int split = blockIdx.x, splits = gridDim.x;
-    const int pos = positions[t];
-    const int lo = window > 0 ? max(0, pos - window + 1) : 0;
-    const int* bt = block_table + (size_t)slot * max_blocks;
     const int tile0 = lo / DT_TILE, tile1 = pos / DT_TILE + 1;
     const int per = (tile1 - tile0 + splits - 1) / splits;
+    const bool alone = splits == 1 || (direct && tile1 - tile0 <= per);      // all of the token's keys are one split's
     const int begin = tile0 + split * per, end = min(tile1, begin + per);
     const int n_tiles = max(0, end - begin);
     if (splits > 1 && n_tiles == 0) {
         // No key of the request falls to this split (a captured step has as many splits as a long context wants): the merge
         // hears so, and the q/k/v product's sums are left to the blocks that need them.
+        if (warp == DT_CONSUMERS) ask_ahead(ahead, lane);
         const int r = hb * 16 + threadIdx.x;
-        if (threadIdx.x < 16 && r < G)
+        if (threadIdx.x < 16 && r < G && !alone)
             *reinterpret_cast<float2*>(part_ml + (((size_t)t * H + kvh * G + r) * splits + split) * 2) = make_float2(-INFINITY, 0.f);
         return leave();
     }
@@ -194,7 +221,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
             const float* cs = fresh.table + (size_t)pos * D;
             __nv_bfloat16* kdst = nullptr;
             if (patch && hb == 0) {
-                const int page = bt[pos / P];
+                const int page = own_page;
                 if (page < 0) {
                     if (threadIdx.x == 0 && status) atomicExch(status, 2);
                 } else {
@@ -439,7 +466,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
             ll += sm_l[w * 16 + r] * wgt;
         }
         const int h = kvh * G + hb * 16 + r;
-        if (splits == 1) {
+        if (alone) {
             out[((size_t)t * H + h) * D + col] = __float2bfloat16_rn(acc / ll);
         } else {
             const size_t pi = ((size_t)t * H + h) * splits + split;
@@ -457,7 +484,7 @@ template <int D>
 int launch_decode_tma(const CUtensorMap& map, const FreshQkv& fresh, const void* q, const int* block_table, int max_blocks,
                       const int* token_seq, const int* positions, void* out, float* part_o, float* part_ml, int T,
                       int H, int K, int P, int window, float scale, float softcap, int splits, int* status,
-                      const DistanceBias& bias, int alongside, cudaStream_t stream) {
+                      const DistanceBias& bias, int alongside, int direct, const Ahead& ahead, cudaStream_t stream) {
     const int head_blocks = (H / K + 15) / 16;
     const size_t ring = (size_t)DT_STAGES * 2 * (D / 64) * DT_TILE * 128;
     const size_t merge = (size_t)(DT_CONSUMERS * 16 * D + 2 * DT_CONSUMERS * 16) * sizeof(float);
@@ -465,10 +492,10 @@ int launch_decode_tma(const CUtensorMap& map, const FreshQkv& fresh, const void*
     auto kernel = bias.table ? decode_attention_tma_kernel<D, true> : decode_attention_tma_kernel<D, false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    return launch(kernel, dim3(splits, K * head_blocks, T), DT_THREADS, smem, stream, map, fresh, (const __nv_bfloat16*)q,
+    return launch(kernel, dim3(splits, K * head_blocks, T), DT_THREADS, smem, stream, map, fresh, ahead, (const __nv_bfloat16*)q,
                   block_table, max_blocks, token_seq, positions, (__nv_bfloat16*)out, part_o, part_ml, H, K, P, window,
                   scale * 1.4426950408889634f, softcap > 0.f ? softcap * 1.4426950408889634f : 0.f,
-                  softcap > 0.f ? scale / softcap : 0.f, status, bias, alongside);
+                  softcap > 0.f ? scale / softcap : 0.f, status, bias, alongside, direct);
 }
 
 }  // namespace air
@@ -478,8 +505,8 @@ extern "C" int air_decode_combine_sink(const float* part_o, const float* part_ml
                                        int H, int D, int splits, const float* sink, const float* gate, int ldg,
                                        const double* turn_freq, int turn_rot, int turn_pairing, const int* positions,
                                        cudaStream_t stream);
-extern "C" int air_decode_combine(const float* part_o, const float* part_ml, const int* token_seq, void* out, int T,
-                                  int H, int D, int splits, cudaStream_t stream);
+extern "C" int air_decode_combine_split(const float* part_o, const float* part_ml, const int* token_seq, void* out, int T, int H, int D,
+                                        int splits, const int* positions, int window, int early, cudaStream_t stream);
 
 namespace air {
 
@@ -489,7 +516,7 @@ static int decode_attention_tma(const FreshQkv& fresh, const void* q, const void
                                 float scale, float softcap, int splits, int* status, cudaStream_t stream,
                                 const float* sink = nullptr, const float* gate = nullptr, int ldg = 0,
                                 const TurnBack& turn = TurnBack{nullptr, 0, 0, nullptr},
-                                const DistanceBias& bias = DistanceBias{nullptr, 0}, int alongside = 0) {
+                                const DistanceBias& bias = DistanceBias{nullptr, 0}, int alongside = 0, const Ahead& ahead = Ahead{}) {
     if (T <= 0) return 0;
     if (bias.table && bias.n < 1) return AIR_ERR_BAD_ARGUMENT;
     if (H <= 0 || K <= 0 || H % K || P % 16 || (P < 64 ? 64 % P : P % 64) || splits < 1 || T > 65535 ||
@@ -500,6 +527,7 @@ static int decode_attention_tma(const FreshQkv& fresh, const void* q, const void
     const LastLaunch& last = last_launch();
     alongside = alongside && last.portions == last.count && last.stream == stream;
     const bool extra = sink || gate || turn.freq;
+    const int direct = !extra;
     if (extra && splits < 2) return AIR_ERR_BAD_ARGUMENT;
     CUtensorMap map;
     const int map_rc = tensor_map_2d(&map, cache, pages * 2 * K * P, D, P < DT_TILE ? P : DT_TILE);
@@ -508,15 +536,15 @@ static int decode_attention_tma(const FreshQkv& fresh, const void* q, const void
     switch (D) {
         case 64:
             rc = launch_decode_tma<64>(map, fresh, q, block_table, max_blocks, token_seq, positions, out, part_o, part_ml,
-                                       T, H, K, P, window, scale, softcap, splits, status, bias, alongside, stream);
+                                       T, H, K, P, window, scale, softcap, splits, status, bias, alongside, direct, ahead, stream);
             break;
         case 128:
             rc = launch_decode_tma<128>(map, fresh, q, block_table, max_blocks, token_seq, positions, out, part_o,
-                                        part_ml, T, H, K, P, window, scale, softcap, splits, status, bias, alongside, stream);
+                                        part_ml, T, H, K, P, window, scale, softcap, splits, status, bias, alongside, direct, ahead, stream);
             break;
         case 256:
             rc = launch_decode_tma<256>(map, fresh, q, block_table, max_blocks, token_seq, positions, out, part_o,
-                                        part_ml, T, H, K, P, window, scale, softcap, splits, status, bias, alongside, stream);
+                                        part_ml, T, H, K, P, window, scale, softcap, splits, status, bias, alongside, direct, ahead, stream);
             break;
         default:
             return AIR_ERR_BAD_ARGUMENT;
@@ -524,7 +552,8 @@ static int decode_attention_tma(const FreshQkv& fresh, const void* q, const void
     if (rc == 0 && splits > 1)
         rc = extra ? air_decode_combine_sink(part_o, part_ml, token_seq, out, T, H, D, splits, sink, gate, ldg, turn.freq,
                                              turn.rot, turn.pairing, positions, stream)
-                   : air_decode_combine(part_o, part_ml, token_seq, out, T, H, D, splits, stream);
+                   : air_decode_combine_split(part_o, part_ml, token_seq, out, T, H, D, splits, positions, window, fresh.qkv != nullptr,
+                                              stream);
     return rc;
 }
 
@@ -564,18 +593,24 @@ AIR_API int air_decode_attention_tma_sink(const void* q, const void* cache, long
 
 // The same from the q/k/v product's output instead of q: qkv float32 [parts][T][(H + 2 K) D] (partial sums that
 // are added in order), bias float32 or null, table float32 [positions][D] (cos | sin: all of a head is
-// rotated); write_kv = 0 where another run's layer has written this step's keys and values already.
+// rotated); write_kv = 0 where another run's layer has written this step's keys and values already.  ahead0, ahead1: memory of
+// bytes0 and bytes1 that the kernels behind read and none writes, or null (Ahead).
 AIR_API int air_decode_attention_tma_fresh(const float* qkv, int parts, const float* bias, const float* table,
                                            int write_kv, void* cache, long long pages, const int* block_table,
                                            int max_blocks, const int* token_seq, const int* positions, void* out,
                                            float* part_o, float* part_ml, int T, int H, int K, int D, int P,
-                                           int window, float scale, int splits, int* status, cudaStream_t stream) {
+                                           int window, float scale, int splits, int* status, const void* ahead0, long long bytes0,
+                                           const void* ahead1, long long bytes1, cudaStream_t stream) {
     if (!qkv || !table || parts < 1 || ((uintptr_t)qkv & 15) || ((uintptr_t)bias & 15) || ((uintptr_t)table & 15))
         return AIR_ERR_BAD_ARGUMENT;
     const air::FreshQkv fresh{qkv, parts, (size_t)T * (size_t)(H + 2 * K) * (size_t)D, bias, table,
                               write_kv ? (__nv_bfloat16*)cache : nullptr};
+    air::Ahead ahead{{(const uint8_t*)ahead0, (const uint8_t*)ahead1}, {0, 0}};
+    for (int a = 0; a < air::AHEAD; ++a)
+        if (ahead.at[a] && !((uintptr_t)ahead.at[a] & 15)) ahead.pieces[a] = (unsigned)((a ? bytes1 : bytes0) / air::AHEAD_PIECE);
     return air::decode_attention_tma(fresh, nullptr, cache, pages, block_table, max_blocks, token_seq, positions, out,
-                                     part_o, part_ml, T, H, K, D, P, window, scale, 0.f, splits, status, stream);
+                                     part_o, part_ml, T, H, K, D, P, window, scale, 0.f, splits, status, stream, nullptr, nullptr, 0,
+                                     air::TurnBack{nullptr, 0, 0, nullptr}, air::DistanceBias{nullptr, 0}, 0, ahead);
 }
 
 AIR_API int air_trace_set_attention_decode_tma(unsigned long long* buffer) { return air::set_trace_here(buffer); }

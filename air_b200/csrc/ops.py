@@ -124,7 +124,8 @@ _SIGNATURES = {
     "air_head_gate": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "air_decode_attention_tma_fresh": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_int,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                       c_int, c_int, c_float, c_int, c_void_p, c_void_p],
+                                       c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong,
+                                       c_void_p],
     "air_prefill_attention_tc": [c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int,
                                  c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int,
                                  c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p],
@@ -1590,12 +1591,16 @@ def decode_attention_fresh_ok(qkv, table, cache, head_dim) -> bool:
             and table.shape[1] == head_dim and cache.dtype == torch.bfloat16 and tile_pages(cache.shape[3]))
 
 
+AHEAD_BYTES = 24 << 20     # of what lies behind, that blocks of the attention without keys ask into L2 (attention_decode_tma.cu)
+
+
 def decode_attention_fresh(qkv, bias, table, cache, block_table, token_seq, positions, out, heads, window, scale,
-                           write_kv=True, splits=None, status=None):
+                           write_kv=True, splits=None, status=None, ahead=()):
     """bfloat16 attention for one query token per request, straight from the q/k/v product: qkv float32
     [T, (H + 2K) d] or [parts, T, (H + 2K) d] partial sums; the kernel adds the bias, rotates q and k by the
     table's row of each token's position, writes k and v to the pages (write_kv) and attends, which
-    qkv_rope_store followed by decode_attention do in two launches (attention_decode_tma.cu)."""
+    qkv_rope_store followed by decode_attention do in two launches (attention_decode_tma.cu).  ahead: up to two tensors that
+    the kernels behind read and none of them writes (their weights), in that order."""
     T, H = qkv.shape[-2], heads
     d, K, P = cache.shape[4], cache.shape[2], cache.shape[3]
     width = (H + 2 * K) * d
@@ -1617,11 +1622,17 @@ def decode_attention_fresh(qkv, bias, table, cache, block_table, token_seq, posi
     if splits > 1:
         po = torch.empty(T * H * splits * d, dtype=torch.float32, device=qkv.device)
         pm = torch.empty(T * H * splits * 2, dtype=torch.float32, device=qkv.device)
+    asked, left = [], AHEAD_BYTES
+    for w in ahead[:2]:
+        n = min(left, w.numel() * w.element_size()) if w.is_contiguous() else 0
+        asked += [w.data_ptr(), n]
+        left -= n
+    asked += [None, 0] * (2 - len(asked) // 2)
     _check(_get("air_decode_attention_tma_fresh")(
         qkv.data_ptr(), parts, _ptr(bias), table.data_ptr(), 1 if write_kv else 0, cache.data_ptr(), cache.shape[0],
         block_table.data_ptr(), block_table.shape[1], token_seq.data_ptr(), positions.data_ptr(), out.data_ptr(),
-        _ptr(po), _ptr(pm), T, H, K, d, P, int(window or 0), float(scale), splits, _ptr(status), _stream()),
-        "decode_attention_tma")
+        _ptr(po), _ptr(pm), T, H, K, d, P, int(window or 0), float(scale), splits, _ptr(status),
+        *asked, _stream()), "decode_attention_tma")
     if splits > 1:
         global launches
         launches += 1

@@ -394,6 +394,10 @@ class RowFilter(Part):
 
 
 class Mixer(Part):
+    # Weights that the parts behind this one read in a step of few rows, in that order (the block knows them): a kernel with
+    # memory to spare may ask for them ahead of time.
+    behind: Tuple[torch.Tensor, ...] = ()
+
     def cache_needs(self) -> Tuple[CacheNeed, ...]:
         return ()
 
@@ -402,5 +406,9 @@ class Mixer(Part):
 
 
 class FeedForward(Part):
+    def streams(self) -> Tuple[torch.Tensor, ...]:
+        """The weights that a step of few rows reads first, in that order."""
+        return ()
+
     def forward(self, x, ctx):
         raise NotImplementedError

@@ -79,6 +79,9 @@ class SwiGLU(FeedForward):
         self.gate_up = Linear(w.contiguous(), rt.status, gate_up_block=block if block != inter else 0)
         self.down = Linear(tensors[p + self.NAMES["down"]], rt.status)
 
+    def streams(self):
+        return (self.gate_up.weight,)
+
     def accepts_prenormed(self, ctx, owns_cache=True):
         return self.rt.dtype == torch.bfloat16 and self.gate_up.takes_prenormed(ctx.num_tokens, silu=True)
 

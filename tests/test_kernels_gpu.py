@@ -662,6 +662,38 @@ def test_decode_attention_from_the_product(H, K, d, P, window, splits):
     assert float((got2.float() - want.float())[keep].abs().max()) <= 2e-2 * max(1.0, float(want.float().abs().max()))
 
 
+@pytest.mark.parametrize("d,window", [(128, 0), (128, 40), (64, 0), (64, 70), (256, 0)])
+def test_decode_attention_with_more_splits_than_tiles(d, window):
+    """Tokens whose keys are one split's are finished by its block, others by the merge, which reads the splits that hold keys; blocks
+    without keys ask for memory ahead, of any size.  A token of one tile has the bits that one split gives it."""
+    from air_b200.parts.rope import RopeHalf
+    from air_b200.parts.spec import PartSpec
+    from air_b200.parts.base import Runtime
+    H, K, P = 8, 2, 64
+    lens = [1, 2, 63, 64, 65, 104, 105, 128, 129, 2047, 2048, 2049, 2300]
+    _, cache, bt, positions, seq_of, _, _ = paged_case(H, K, d, P, lens, [1] * len(lens), "bfloat16", seed=d, num_pages=160)
+    positions, seq_of = np.append(positions, 0).astype(np.int32), np.append(seq_of, -1).astype(np.int32)
+    T, width = len(positions), (H + 2 * K) * d
+    g = torch.Generator().manual_seed(d + window)
+    qkv = (torch.randn(2, T, width, generator=g) * 0.6).cuda()
+    pe = RopeHalf(PartSpec("rope_half", {"rotary_dim": d, "theta": 10000.0, "max_positions": 4096}))
+    pe.load({}, Runtime(torch.device("cuda"), torch.bfloat16, P))
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    o, outs = ops(), []
+    for splits, ahead in ((1, ()), (32, ()), (32, (torch.empty(4095, dtype=torch.uint8, device="cuda"),)),
+                          (32, (torch.empty(5 << 20, dtype=torch.uint8, device="cuda"), torch.empty(40 << 20, dtype=torch.uint8, device="cuda")))):
+        out = torch.full((T, H, d), 7.0, dtype=torch.bfloat16, device="cuda")
+        o.decode_attention_fresh(qkv, None, pe.table(), dev(cache, torch.bfloat16), dev(bt), dev(seq_of), dev(positions), out, H, window,
+                                 d ** -0.5, splits=splits, status=status, ahead=ahead)
+        outs.append(out)
+    one, cut = outs[:2]
+    assert status.item() == 0 and all(torch.equal(x, cut) for x in outs[2:])
+    assert float((cut.float() - one.float()).abs().max()) <= 2e-2 * max(1.0, float(one.float().abs().max()))
+    tiles = [n // 64 - (max(0, n - window + 1) // 64 if window else 0) + 1 for n in (m - 1 for m in lens)]
+    same = torch.tensor([i for i, n in enumerate(tiles) if n == 1] + [T - 1], device="cuda")
+    assert torch.equal(cut[same], one[same]) and (cut[T - 1] == 7.0).all()
+
+
 @pytest.mark.parametrize("far,n", [(0, 2048), (15, 2048), (16, 2048), (63, 2048), (64, 2048), (1000, 2048), (2047, 2048),
                                    (0, 32768), (20001, 32768), (32767, 32768)])
 def test_decode_attention_finds_one_far_key(far, n):
