@@ -138,10 +138,12 @@ struct RefArgs {
 };
 // Shared memory, in floats: the rows' queries, the warps' maxima and sums, then per warp 32 keys (rows of d + 4: eight that
 // lie beside one another cover the banks; behind the last block the warp's weighted values), 32 values and the weights.
+// SHARED: the values take the keys' memory once the scores are there.
 struct RefPlaces {
     int d, dv;
-    __host__ __device__ int keys() const { return max(32 * (d + 4), REF_QUERIES * dv); }
-    __host__ __device__ int of_warp() const { return keys() + 32 * dv + REF_QUERIES * 32; }
+    bool shared;
+    __host__ __device__ int keys() const { return max(max(32 * (d + 4), REF_QUERIES * dv), shared ? 32 * dv : 0); }
+    __host__ __device__ int of_warp() const { return keys() + (shared ? 0 : 32 * dv) + REF_QUERIES * 32; }
     __host__ __device__ int head() const { return REF_QUERIES * d + 2 * ATT_WARPS * REF_QUERIES; }
     __host__ __device__ size_t bytes() const { return sizeof(float) * (head() + ATT_WARPS * of_warp()); }
 };
@@ -158,7 +160,7 @@ template <int N> __device__ __forceinline__ void ref_wait() {
 // Rows t .. t + n - 1: positions pos .. pos + n - 1 of the request in row `seq` of the table.
 // D: the size of keys and values where it is known (the loops over it and the strides are then constants: 100 us against 126 for
 // 300 rows of 128), else 0.
-template <int N, int D>
+template <int N, int D, bool SHARED>
 __device__ __forceinline__ void ref_rows(const RefArgs& a, float* smem, int t, int n, int pos, int seq) {
     const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = D ? D : a.d, dv = D ? D : a.dv;
     const int kvh = (int)(((long long)h * a.K) / a.H);
@@ -169,13 +171,13 @@ __device__ __forceinline__ void ref_rows(const RefArgs& a, float* smem, int t, i
     auto first = [&](int p) { return a.window > 0 ? (a.mask_mode == 1 ? p - p % a.window : max(0, p - a.window + 1)) : 0; };
     for (int i = threadIdx.x; i < n * d; i += ATT_WARPS * 32) smem[i] = a.q[((size_t)(t + i / d) * a.H + h) * d + i % d];
     __syncthreads();
-    const RefPlaces places{d, dv};
+    const RefPlaces places{d, dv, SHARED};
     const float* sq = smem;
     float* sm = smem + REF_QUERIES * d;
     float* sl = sm + ATT_WARPS * REF_QUERIES;
     float* sk = smem + places.head() + warp * places.of_warp();
-    float* sv = sk + places.keys();
-    float* sp = sv + 32 * dv;
+    float* sv = SHARED ? sk : sk + places.keys();
+    float* sp = sk + places.keys() + (SHARED ? 0 : 32 * dv);
     const int kld = d + 4;
     const int last = pos + n - 1, lo = first(pos);       // (the lowest key of any row is the first row's)
     // lane j knows where key j of a block lies and where its value does; -1: no row sees it, it is not copied and not used
@@ -208,11 +210,11 @@ __device__ __forceinline__ void ref_rows(const RefArgs& a, float* smem, int t, i
     if (b * 32 <= last) {
         find(b);
         bring(k_at, sk, kld, d);
-        bring(v_at, sv, dv, dv);
+        if (!SHARED) bring(v_at, sv, dv, dv);
     }
     for (; b * 32 <= last; b += ATT_WARPS) {
         const int key = b * 32 + lane;
-        ref_wait<1>();                           // the keys are there
+        ref_wait<SHARED ? 0 : 1>();              // the keys are there
         float s[N];
 #pragma unroll
         for (int i = 0; i < N; ++i) s[i] = 0.f;
@@ -230,8 +232,9 @@ __device__ __forceinline__ void ref_rows(const RefArgs& a, float* smem, int t, i
         }
         __syncwarp();
         const bool more = (b + ATT_WARPS) * 32 <= last;
-        if (more) {
-            find(b + ATT_WARPS);
+        if (SHARED) bring(v_at, sv, dv, dv);
+        if (more) find(b + ATT_WARPS);
+        if (more && !SHARED) {
             bring(k_at, sk, kld, d);
         }
         float corr[N];
@@ -256,7 +259,7 @@ __device__ __forceinline__ void ref_rows(const RefArgs& a, float* smem, int t, i
             }
             sp[i * 32 + lane] = p;
         }
-        if (more) ref_wait<1>();                 // the values are there
+        if (more && !SHARED) ref_wait<1>();      // the values are there
         else ref_wait<0>();
         if (any) {
 #pragma unroll
@@ -282,7 +285,8 @@ __device__ __forceinline__ void ref_rows(const RefArgs& a, float* smem, int t, i
             }
         }
         __syncwarp();
-        if (more) bring(v_at, sv, dv, dv);
+        if (more && !SHARED) bring(v_at, sv, dv, dv);
+        if (more && SHARED) bring(k_at, sk, kld, d);
     }
     ref_wait<0>();
 #pragma unroll
@@ -310,8 +314,8 @@ __device__ __forceinline__ void ref_rows(const RefArgs& a, float* smem, int t, i
 }
 
 // A block takes `per_block` rows of the batch for one head: runs of consecutive tokens of a request among them together.
-template <int D>
-__global__ void __launch_bounds__(ATT_WARPS * 32) paged_attention_f32_kernel(const RefArgs a, int per_block) {
+template <int D, bool SHARED>
+__global__ void __launch_bounds__(ATT_WARPS * 32, SHARED ? 3 : 1) paged_attention_f32_kernel(const RefArgs a, int per_block) {
     extern __shared__ __align__(16) float smem[];
     pdl_enter(TR_ATT_REF);
     const int end = min(a.T, (int)(blockIdx.x + 1) * per_block);
@@ -320,9 +324,9 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) paged_attention_f32_kernel(con
         if (seq < 0) { ++t; continue; }          // padding
         int n = 1;
         while (n < REF_QUERIES && t + n < end && a.token_seq[t + n] == seq && a.positions[t + n] == pos + n) ++n;
-        if (n == 1) ref_rows<1, D>(a, smem, t, 1, pos, seq);
-        else if (n <= REF_QUERIES / 2) ref_rows<REF_QUERIES / 2, D>(a, smem, t, n, pos, seq);
-        else ref_rows<REF_QUERIES, D>(a, smem, t, n, pos, seq);
+        if (n == 1) ref_rows<1, D, SHARED>(a, smem, t, 1, pos, seq);
+        else if (n <= REF_QUERIES / 2) ref_rows<REF_QUERIES / 2, D, SHARED>(a, smem, t, n, pos, seq);
+        else ref_rows<REF_QUERIES, D, SHARED>(a, smem, t, n, pos, seq);
         t += n;
     }
 }
@@ -343,13 +347,18 @@ AIR_API int air_paged_attention_ref(const void* q, int q_f32, const void* cache,
     dim3 grid(T, H);
     if (dtype == AIR_F32 && d <= air::REF_D && dv <= air::REF_D && d % 4 == 0 && dv % 4 == 0 && ((uintptr_t)cache & 15) == 0) {
         // As many rows to a block, up to REF_QUERIES, as leave a block for every SM.  Measured, us, against the kernel above: 300
-        // rows of a prompt, 16 heads of 128: 473 -> 100; 512 rows behind 500: 3,315 -> 406; 4 single tokens over 1,000 keys, 28
-        // heads: 317 -> 33; one over 4,000: 1,217 -> 100; 64 over 2,000: 2,409 -> 768.
+        // rows of a prompt, 16 heads of 128: 473 -> 63; 512 rows behind 500: 3,315 -> 247; 4 single tokens over 1,000 keys, 28
+        // heads: 317 -> 32; one over 4,000: 1,217 -> 99; 64 over 2,000: 2,409 -> 488.
+        // Blocks of several rows are many and each waits for its own reads, its shared-memory loads and its chains of sums, one
+        // warp to a scheduler: with the values in the keys' memory three blocks share an SM instead of one (300 rows 101 -> 63, 512
+        // 401 -> 247, 64 single tokens 744 -> 488).  A block of one row keeps both, so that the next keys arrive meanwhile.
         const int per_block = (int)min((long long)air::REF_QUERIES, max(1ll, (long long)T * H / 148));
         const air::RefArgs args{(const float*)q, (const float*)cache, block_table, max_blocks, token_seq, positions, (float*)out,
                                 gate, T, H, K, d, dv, P, window, scale, softcap, mask_mode, sink, latent, db};
-        const size_t smem = air::RefPlaces{d, dv}.bytes();
-        auto kernel = d == 128 && dv == 128 ? air::paged_attention_f32_kernel<128> : air::paged_attention_f32_kernel<0>;
+        const bool shared = per_block > 1;
+        const size_t smem = air::RefPlaces{d, dv, shared}.bytes();
+        auto kernel = d == 128 && dv == 128 ? (shared ? air::paged_attention_f32_kernel<128, true> : air::paged_attention_f32_kernel<128, false>)
+                                            : (shared ? air::paged_attention_f32_kernel<0, true> : air::paged_attention_f32_kernel<0, false>);
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return (int)e;
