@@ -15,9 +15,11 @@
 // A tile of W may reach into the next expert's rows, a tile of X into the next expert's slots: what they give is not stored.
 // Measured, a whole mixture (router, lists, both products, a shared expert half as wide as the dense feed-forward) replayed as
 // a graph, us: width 4,096, 16 experts of 3,584, 8 tokens 331 -> 190 (its bytes at the copy rate: 169), 100 tokens 419 by the
-// library's grouped product -> 324, 300 tokens 418 -> 350; width 2,048, experts of 2,048: 8 tokens 94, 100 tokens 169 -> 129, 300
-// tokens 165 -> 140, 500 tokens 168 -> 178 (launched kernel by kernel, as such a step is: 196 and 195; where the library takes
-// over: RoutedExperts.LIBRARY_ROWS).
+// library's grouped product -> 324; width 2,048, experts of 2,048: 8 tokens 94, 100 tokens 169 -> 129.
+// What 300 and more tokens take now, and where the library takes over: RoutedExperts.  EPI 0's places and weights are worked out by
+// a thread per slot while the products run; row by row in the loop that stores, an index, two divisions and a weight stood
+// behind one another: a mixture of width 2,048 with 500 tokens 199 -> 163, with 64 145 -> 140, width 4,096 with 500 406 -> 378.
+// Tiles of 256 slots (one set of accumulators, three stages) were slower than the library at any number of rows.
 // Every wait on an mbarrier is bounded; on giving up the block sets *status = 4 (as gemm_tc.cu).
 #include "common.cuh"
 #include "tma.cuh"
@@ -27,13 +29,14 @@ namespace air {
 
 constexpr int XS_BK = 64;
 constexpr int XS_THREADS = 192;
-constexpr int XS_ROWS = 64;      // slots of a row tile (moe_sort_kernel's); tiles of 128 were no faster below 60 rows per expert
+constexpr int XS_ROWS = 64, XS_WIDE = 128;      // slots of a row tile (moe_sort_kernel's): few rows per expert, many
 
 struct XsArgs {
     void* out;
     int slots, N, K, splits;
     const int* start;            // [groups + 1]
-    const int* tiles;            // pairs (group, first slot), XS_ROWS slots to a tile
+    const int* tiles;            // pairs (group, first slot)
+    int tile_rows;               // slots to a tile
     const int* num_tiles;
     int lists_ready;             // the lists were complete before this kernel's predecessor let anything start
     const int* o_index; int o_div; long long o_part_stride; int ldo; const float* o_scale;
@@ -71,6 +74,8 @@ expert_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     uint64_t* acc_empty = bars + 2 * STAGES + 2;
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    long long* o_at = (long long*)(tmem_slot + 2);     // EPI 0: where a slot's row goes, and its weight
+    float* o_weight = (float*)(o_at + NT);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = (args.N + TILE_N - 1) / TILE_N;
@@ -191,11 +196,25 @@ expert_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         pdl_wait();   // nothing is written before the predecessor has completed
         const int quarter = warp & 3, r = quarter * 32 + lane;
         uint32_t it = 0;
-        for (int i = blockIdx.x; i < total && !*abort_flag; i += gridDim.x, ++it) {
+        // (EPI 0: the warps meet at a barrier, so all of them go through all tiles, also when a wait has run out)
+        for (int i = blockIdx.x; i < total && (EPI == 0 || !*abort_flag); i += gridDim.x, ++it) {
             const Item x = item_of(i);
-            const int rows = min(XS_ROWS, __ldcg(args.start + x.group + 1) - x.slot0);      // (up to NT: see air_expert_stream)
+            const int rows = min(args.tile_rows, __ldcg(args.start + x.group + 1) - x.slot0);      // (up to NT: see air_expert_stream)
             const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-            if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag)) break;
+            if constexpr (EPI == 0) {
+                // (worked out by a thread per slot while the products run, not row by row in the loop below)
+                asm volatile("bar.sync 1, 128;" ::: "memory");      // (the last tile's are read)
+                for (int t = threadIdx.x - 64; t < min(rows, NT); t += 128) {
+                    const int dst = __ldcg(args.o_index + x.slot0 + t);
+                    o_at[t] = (x.split * args.o_div + dst % args.o_div) * args.o_part_stride + (long long)(dst / args.o_div) * args.ldo;
+                    o_weight[t] = args.o_scale ? args.o_scale[dst] : 1.f;
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+            }
+            const bool ok = mbar_wait(&acc_full[acc], acc_phase, abort_flag);
+            if constexpr (EPI == 0) {
+                if (!__all_sync(0xffffffffu, ok)) continue;
+            } else if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
             // (16 slots at a time; a tile of an expert with few rows ends with them)
@@ -226,12 +245,7 @@ expert_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                         } else {
 #pragma unroll
                             for (int t = 0; t < 16; ++t)
-                                if (t < live) {
-                                    const int dst = __ldcg(args.o_index + x.slot0 + t0 + t);
-                                    const float scale = args.o_scale ? args.o_scale[dst] : 1.f;
-                                    ((float*)args.out)[(x.split * args.o_div + dst % args.o_div) * args.o_part_stride +
-                                                       (long long)(dst / args.o_div) * args.ldo + col] = v[t] * scale;
-                                }
+                                if (t < live) ((float*)args.out)[o_at[t0 + t] + col] = v[t] * o_weight[t0 + t];
                         }
                     }
                 }
@@ -261,7 +275,7 @@ template <int NT, int EPI, int HALVES>
 static int xs_launch(const CUtensorMap& mw, const CUtensorMap& mx, const XsArgs& args, int blocks, cudaStream_t stream) {
     constexpr int STAGES = xs_stages(NT, HALVES);
     // (more than half of an SM's shared memory: two blocks never share an SM and its tensor memory)
-    const size_t smem = 1024 + (size_t)STAGES * (HALVES * 128 + NT) * XS_BK * 2 + 16 * STAGES + 256;
+    const size_t smem = 1024 + (size_t)STAGES * (HALVES * 128 + NT) * XS_BK * 2 + 16 * STAGES + 256 + (EPI == 0 ? 12 * NT : 0);
     const size_t request = smem < 120 * 1024 ? 120 * 1024 : smem;
     auto kernel = expert_stream_kernel<NT, EPI, HALVES>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)request);
@@ -279,22 +293,22 @@ static int xs_dispatch(int epi, const CUtensorMap& mw, const CUtensorMap& mx, co
 }  // namespace air
 
 // x [slots, K] bf16 in slot order, w [groups, N, K] bf16, K % 8 == 0.  start [groups + 1], tiles and num_tiles as
-// moe_sort_kernel leaves them (64 slots to a tile); no expert has more than most_rows slots.  epi, out: see above (epi 1: N a
+// moe_sort_kernel leaves them (tile_rows slots to a tile, 64 or 128); no expert has more than most_rows slots.  epi, out: see above (epi 1: N a
 // multiple of 256).  lists_ready: the kernel launched right before this one is an expert_stream_kernel that was given the
 // same lists without it.
 AIR_API int air_expert_stream(const void* x, int slots, const void* w, int groups, int N, int K, const int* start,
-                              const int* tiles, const int* num_tiles, int max_tiles, int most_rows, int epi, void* out, int splits,
+                              const int* tiles, const int* num_tiles, int max_tiles, int tile_rows, int most_rows, int epi, void* out, int splits,
                               const int* o_index, int o_div, long long o_part_stride, int ldo, const float* o_scale, float alpha,
                               float limit, float shift, int lists_ready, int* status, cudaStream_t stream) {
     using namespace air;
     if (slots <= 0 || N <= 0 || groups <= 0 || max_tiles <= 0) return 0;
     if (K <= 0 || K % 8 || epi < 0 || epi > 2 || splits < 1 || (splits > 1 && epi) || (epi == 1 && N % 256) || !start || !tiles ||
         !num_tiles || (epi == 0 && (!o_index || o_div < 1)) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || most_rows < 1 ||
-        (long long)groups * N > 0x7fffffff)
+        (tile_rows != XS_ROWS && tile_rows != XS_WIDE) || (long long)groups * N > 0x7fffffff)
         return AIR_ERR_BAD_ARGUMENT;
     const int k_tiles = (K + XS_BK - 1) / XS_BK;
     if (splits > k_tiles || (long long)(splits - 1) * ((k_tiles + splits - 1) / splits) >= k_tiles) return AIR_ERR_BAD_ARGUMENT;
-    const int nt = most_rows > 32 ? 64 : most_rows > 16 ? 32 : 16;
+    const int nt = tile_rows == XS_WIDE ? XS_WIDE : most_rows > 32 ? 64 : most_rows > 16 ? 32 : 16;
     CUtensorMap mw, mx;
     int rc = tensor_map_2d(&mw, w, (long long)groups * N, K, epi == 1 ? 256 : 128);
     if (rc) return rc;
@@ -305,11 +319,12 @@ AIR_API int air_expert_stream(const void* x, int slots, const void* w, int group
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long most = (long long)max_tiles * ((N + (epi == 1 ? 255 : 127)) / (epi == 1 ? 256 : 128)) * splits;
     const int blocks = (int)(most < sms ? most : sms);
-    const XsArgs args{out, slots, N, K, splits, start, tiles, num_tiles, lists_ready, o_index, o_div, o_part_stride, ldo, o_scale,
+    const XsArgs args{out, slots, N, K, splits, start, tiles, tile_rows, num_tiles, lists_ready, o_index, o_div, o_part_stride, ldo, o_scale,
                       status, alpha, limit, shift};
     if (nt == 16) return xs_dispatch<16>(epi, mw, mx, args, blocks, stream);
     if (nt == 32) return xs_dispatch<32>(epi, mw, mx, args, blocks, stream);
-    return xs_dispatch<64>(epi, mw, mx, args, blocks, stream);
+    if (nt == 64) return xs_dispatch<64>(epi, mw, mx, args, blocks, stream);
+    return xs_dispatch<XS_WIDE>(epi, mw, mx, args, blocks, stream);
 }
 
 AIR_API int air_trace_set_expert_stream(unsigned long long* buffer) { return air::set_trace_here(buffer); }

@@ -81,7 +81,7 @@ _SIGNATURES = {
                          c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_int,
                          c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float,
                          c_float, c_float, c_void_p],
-    "air_expert_stream": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+    "air_expert_stream": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                           c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_void_p, c_float, c_float, c_float, c_int,
                           c_void_p, c_void_p],
     "air_rows_by_index": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p],
@@ -960,21 +960,21 @@ def moe_identity(x, expert, weight, real_experts, y):
     return y
 
 
-GROUP_TILE = 64      # rows of a tile of the grouped product
+GROUP_TILE, GROUP_WIDE = 64, 128      # rows of a tile of the grouped product; of expert_stream's for many rows per expert
 
 
-def moe_sort(expert, experts, start, pair_of_slot, tiles, num_tiles):
+def moe_sort(expert, experts, start, pair_of_slot, tiles, num_tiles, tile_rows=GROUP_TILE):
     """Orders the (token, choice) pairs of expert int32 [T, top] by expert: start int32 [experts + 1], pair_of_slot
-    int32 [T * top], the grouped product's row tiles (tiles int32 [max_tiles, 2], num_tiles int32 [1])."""
+    int32 [T * top], the grouped product's row tiles of tile_rows slots (tiles int32 [max_tiles, 2], num_tiles int32 [1])."""
     pairs = expert.numel()
     _req(expert, "expert", _I32)
     _req(start, "start", _I32, (experts + 1,))
     _req(pair_of_slot, "pair_of_slot", _I32, (pairs,))
     _req(tiles, "tiles", _I32, (None, 2))
-    if tiles.shape[0] < pairs // GROUP_TILE + experts:
+    if tiles.shape[0] < pairs // tile_rows + experts:
         raise KernelError("moe_sort: the tile list is too short")
     _req(num_tiles, "num_tiles", _I32, (1,))
-    _check(_get("air_moe_sort")(expert.data_ptr(), pairs, int(experts), GROUP_TILE, start.data_ptr(),
+    _check(_get("air_moe_sort")(expert.data_ptr(), pairs, int(experts), int(tile_rows), start.data_ptr(),
                                 pair_of_slot.data_ptr(), tiles.data_ptr(), num_tiles.data_ptr(), _stream()), "moe_sort")
 
 
@@ -1021,9 +1021,10 @@ def expert_stream_ok(x, w, gate_block, silu_mul):
 
 
 def expert_stream(rows, w, out, start, tiles, num_tiles, most_rows, *, silu_mul=False, relu2=False, act=(1.0, 0.0, 0.0),
-                  o_index=None, o_div=1, splits=1, o_scale=None, lists_ready=False, status=None):
+                  o_index=None, o_div=1, splits=1, o_scale=None, lists_ready=False, status=None, tile_rows=GROUP_TILE):
     """The experts' products with the weights as the tensor cores' wide side (expert_stream.cu): rows bfloat16 [slots, K] in
-    moe_sort's order @ w[g]^T, w bfloat16 [groups, N, K].  No expert has more than most_rows slots.
+    moe_sort's order @ w[g]^T, w bfloat16 [groups, N, K].  No expert has more than most_rows slots; the lists' tiles are of
+    tile_rows slots (GROUP_TILE, or GROUP_WIDE for many rows per expert).
     silu_mul: out bfloat16 [slots, N / 2] = the gated activation `act` of blocks of 128 gate rows and 128 linear rows; relu2:
     out bfloat16 [slots, N] = max(x, 0)^2; else out float32 [splits * o_div, T, N]: slot s goes to plane part * o_div +
     o_index[s] % o_div, row o_index[s] // o_div, times o_scale[o_index[s]], one plane per part of k.  lists_ready: the kernel
@@ -1045,7 +1046,7 @@ def expert_stream(rows, w, out, start, tiles, num_tiles, most_rows, *, silu_mul=
         _req(o_scale, "o_scale", (torch.float32,))
     _check(_get("air_expert_stream")(
         rows.data_ptr(), slots, w.data_ptr(), groups, N, K, start.data_ptr(), tiles.data_ptr(), num_tiles.data_ptr(),
-        tiles.shape[0], int(most_rows), 1 if silu_mul else 2 if relu2 else 0, out.data_ptr(), int(splits), _ptr(o_index),
+        tiles.shape[0], int(tile_rows), int(most_rows), 1 if silu_mul else 2 if relu2 else 0, out.data_ptr(), int(splits), _ptr(o_index),
         int(o_div), plane, ldo, _ptr(o_scale), float(act[0]), float(act[1]), float(act[2]), 1 if lists_ready else 0,
         _ptr(status), _stream()), "expert_stream")
     return out

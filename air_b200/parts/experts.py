@@ -51,16 +51,20 @@ class RoutedExperts(FeedForward):
     Everything happens on the device: a kernel picks the experts, one orders the (token, choice) pairs by expert, and
     two grouped products (gate and up with the activation; down) walk the experts' rows.  The outputs of a token's
     choices land in `top` planes (times the parts of k, see _parts) that the norm behind the layer adds in order.  A
-    row's sum does not depend on the batch in float32; in bfloat16, below LIBRARY_ROWS rows per expert, it is the same in all
+    row's sum does not depend on the batch in float32; in bfloat16, on the stream of weights, it is the same in all
     steps of up to SMALL_ROWS rows, and in all longer ones.  In a bfloat16 engine the two products are a stream of the chosen experts' weights on the tcgen05 tensor cores
-    (ops.expert_stream; sizes that it does not take, and float32, run ops.grouped_gemm).  From LIBRARY_ROWS rows per expert (in the mean) on, a bfloat16 step hands the two products to the library's
+    (ops.expert_stream; sizes that it does not take, and float32, run ops.grouped_gemm).  From so many rows per expert on (in the
+    mean; LIBRARY_ROWS, STREAM_HOLDS) a bfloat16 step hands the two products to the library's
     grouped product (which also takes the experts' bounds from the device): there the experts' outputs are rounded to
     bfloat16 before they are added up in 32-bit."""
 
-    # (Measured, 16 experts, us by the library and by the stream of weights, launched kernel by kernel as steps of so many rows
-    # are, and replayed: width 2,048, 56 rows per expert 196 / 193 and 165 / 155, 62 rows 196 / 195 and 168 / 178, 80 rows 207 / 228 and 182 /
-    # 210; width 4,096, 62 rows 469 / 402 and 443 / 387, 80 rows 500 / 478 and 474 / 474, 96 rows 510 / 546 and 489 / 528.)
-    LIBRARY_ROWS = 64
+    # Rows per expert from which the library takes over from ops.grouped_gemm, and how many times as many the stream of weights
+    # holds (144 rows).  From WIDE_ROWS on its tiles are of 128 slots: an expert's matrix then goes through the SMs once or twice
+    # instead of two or three times.  Measured, a mixture of 16 experts on the device, us, library / tiles of 64 / tiles of 128: width
+    # 2,048, 38 rows per expert 145 with either tile, 64 rows 196 / 163 / 159, 88 rows 213 / 187 / 175, 125 rows 229 / 214 / 206, 150 rows
+    # 231 / 241 / 230, 188 rows 248 / 257 / 250; width 4,096, 50 rows - / 374 / 381, 64 rows 469 / 390 / 394, 88 rows 501 / 458 / 427, 125
+    # rows 551 / 542 / 499, 150 rows 557 / 624 / 572, 188 rows 643 / 729 / 704.
+    LIBRARY_ROWS, STREAM_HOLDS, WIDE_ROWS = 64, 2.25, 64
 
     graph_safe = True
 
@@ -171,10 +175,12 @@ class RoutedExperts(FeedForward):
         ints = torch.empty(3 + n + 1 + pairs + 2 * (pairs // ops.GROUP_TILE + n) + 1, dtype=torch.int32, device=dev)[3:]
         start, pair_of_slot = ints[:n + 1], ints[n + 1:n + 1 + pairs]
         tiles, num_tiles = ints[n + 1 + pairs:-1].view(-1, 2), ints[-1:]
-        by_library = x.dtype == torch.bfloat16 and pairs >= self.LIBRARY_ROWS * n and E % 16 == 0 and F % 16 == 0
-        streams = not by_library and ops.expert_stream_ok(x, self.gate_up, self.block, self.gated) and \
-            ops.expert_stream_ok(x, self.down, 0, False)
-        ops.moe_sort(expert, n, start, pair_of_slot, tiles, num_tiles)
+        streams = ops.expert_stream_ok(x, self.gate_up, self.block, self.gated) and ops.expert_stream_ok(x, self.down, 0, False)
+        most = self.LIBRARY_ROWS * (self.STREAM_HOLDS if streams else 1) * n
+        by_library = x.dtype == torch.bfloat16 and pairs >= most and E % 16 == 0 and F % 16 == 0
+        streams = streams and not by_library
+        tile_rows = ops.GROUP_WIDE if streams and pairs >= self.WIDE_ROWS * n else ops.GROUP_TILE
+        ops.moe_sort(expert, n, start, pair_of_slot, tiles, num_tiles, tile_rows=tile_rows)
         parts = self._parts(T) if streams else 1
         y = torch.empty((parts * top, T, E), dtype=torch.float32, device=dev)
         if self.identity:
@@ -188,9 +194,10 @@ class RoutedExperts(FeedForward):
             act = torch.empty((pairs, F), dtype=x.dtype, device=dev)
             lists = (start, tiles, num_tiles, T)       # (a token takes an expert once at most)
             ops.expert_stream(rows, self.gate_up, act, *lists, silu_mul=self.gated, relu2=not self.gated, act=self.act,
-                              status=self.rt.status)
+                              status=self.rt.status, tile_rows=tile_rows)
             ops.expert_stream(act, self.down, y, *lists, o_index=pair_of_slot, o_div=top, splits=parts,
-                              o_scale=None if on_input else weight.view(-1), lists_ready=True, status=self.rt.status)
+                              o_scale=None if on_input else weight.view(-1), lists_ready=True, status=self.rt.status,
+                              tile_rows=tile_rows)
         else:
             act = torch.empty((pairs, F), dtype=x.dtype, device=dev)
             ops.grouped_gemm(x, self.gate_up, act, F, E, lda=E, ldo=F, groups=n, a_index=pair_of_slot, a_div=top,

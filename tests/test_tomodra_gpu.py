@@ -712,6 +712,47 @@ def test_expert_stream_against_64_bit_products(T, top, n, E, F, splits):
         assert (got - want).abs().max() <= 3e-6 * (down[e].double().abs() @ act[s].double().abs()).max()
 
 
+@pytest.mark.parametrize("T,top,n,E,F", [(70, 2, 3, 64, 128), (127, 1, 2, 136, 256), (128, 1, 1, 72, 128), (129, 2, 3, 264, 128),
+                                         (300, 2, 4, 200, 640)])
+def test_expert_stream_in_wide_tiles(T, top, n, E, F):
+    """Tiles of 128 slots: experts with fewer rows, just as many, one more, and several tiles; the rows' results are those of
+    tiles of 64, bit for bit, in every epilogue."""
+    from air_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    expert = torch.argsort(torch.rand(T, n, generator=g, device="cuda"), dim=1)[:, :top].int().contiguous()
+    expert[:, 0] = torch.where(torch.arange(T, device="cuda") < 65, 0, expert[:, 0]) if top == 1 else expert[:, 0]
+    pairs = T * top
+    i32 = lambda *s: torch.empty(s, dtype=torch.int32, device="cuda")
+    x, weight = rand(T, E).bfloat16(), torch.rand(T, top, generator=g, device="cuda")
+    up, down = (rand(n, 2 * F, E) * E ** -0.5).bfloat16(), (rand(n, E, F) * F ** -0.5).bfloat16()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    outs = []
+    for tile_rows in (ops.GROUP_TILE, ops.GROUP_WIDE):
+        start, slot_pair, tiles, count = i32(n + 1), i32(pairs), i32(pairs // tile_rows + n, 2), i32(1)
+        ops.moe_sort(expert, n, start, slot_pair, tiles, count, tile_rows=tile_rows)
+        rows = ops.rows_by_index(x, slot_pair, top, None, torch.empty(pairs, E, dtype=torch.bfloat16, device="cuda"))
+        lists, kw = (start, tiles, count, T), dict(status=status, tile_rows=tile_rows)
+        act, square = (torch.empty(pairs, k * F, dtype=torch.bfloat16, device="cuda") for k in (1, 2))
+        y = torch.full((top, T, E), 9.0, device="cuda")
+        ops.expert_stream(rows, up, square, *lists, relu2=True, **kw)
+        ops.expert_stream(rows, up, act, *lists, silu_mul=True, **kw)
+        ops.expert_stream(act, down, y, *lists, o_index=slot_pair, o_div=top, o_scale=weight.view(-1), lists_ready=True, **kw)
+        by_pair = torch.argsort(slot_pair)          # (the order of an expert's slots is not given)
+        outs.append((act[by_pair], square[by_pair], y))
+        sizes = (start[1:] - start[:-1]).tolist()
+        assert int(count) == sum(-(-s // tile_rows) for s in sizes)
+    assert status.item() == 0
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+    for t in (0, T // 2, T - 1):
+        for c in range(top):
+            e = int(expert[t, c])
+            z = (up[e].double() @ x[t].double()).view(F // 128, 2, 128)
+            want = down[e].double() @ (torch.nn.functional.silu(z[:, 0]) * z[:, 1]).flatten() * weight[t, c].double()
+            assert (outs[1][2][c, t].double() - want).abs().max() <= 0.01 * want.abs().max()
+
+
 def test_a_rows_experts_do_not_depend_on_the_rows_beside_it():
     """A mixture in bfloat16: a row's planes are the same, bit for bit, in every step of up to 64 rows, and in every longer one on
     the stream of weights; their sums are those of the 64-bit experts."""
