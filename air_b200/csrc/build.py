@@ -1,5 +1,5 @@
-"""Compiles the CUDA sources of this folder for sm_100a into one shared library and loads
-it with ctypes.  There is no fallback: without nvcc, or if a source does not compile, the
+"""Compiles the CUDA sources of this folder for sm_100a, and entry.cpp, into one shared library and loads it: an
+extension module whose functions are the launchers (entry), and through ctypes what else the library offers (library).  There is no fallback: without nvcc, or if a source does not compile, the
 import fails with the compiler's message.
 
 The library is built at the first call that needs it, into ``_build/`` beside the sources
@@ -16,9 +16,11 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import time
 from concurrent.futures import ThreadPoolExecutor
+from importlib import machinery, util
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -26,8 +28,10 @@ ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
               "--expt-relaxed-constexpr"]
 LIB_NAME = "libair_b200_kernels.so"
+ENTRY, ENTRY_MODULE = "entry.cpp", "air_b200_entry"
 
 _lib = None
+_entry = None
 
 
 def sources():
@@ -36,6 +40,26 @@ def sources():
 
 def _headers():
     return sorted(f for f in os.listdir(HERE) if f.endswith((".cuh", ".h")))
+
+
+def _entries() -> str:
+    """entries.inc: prototypes of the launchers, and their places in the module's table of methods."""
+    from . import ops
+    names = {ctypes.c_void_p: "void*", ctypes.c_int: "int", ctypes.c_longlong: "long long", ctypes.c_float: "float"}
+    lines = [f'extern "C" int {f}({", ".join(names[t] for t in types)});' for f, types in ops._SIGNATURES.items()]
+    return "\n".join(lines + ["#define AIR_ENTRIES \\"] +
+                     [f'    {{"{f}", (PyCFunction)(void (*)(void))Entry<{f}>::call, METH_FASTCALL, nullptr}}, \\' for f in ops._SIGNATURES] +
+                     ["", ""])
+
+
+def _entry_flags():
+    """How entry.cpp is compiled and linked: against Python's headers and torch's."""
+    import torch
+    root = os.path.dirname(torch.__file__)
+    compile_flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                     "-I", sysconfig.get_paths()["include"], "-I", os.path.join(root, "include"),
+                     "-I", os.path.join(root, "include", "torch", "csrc", "api", "include")]
+    return compile_flags, ["-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"], torch.__version__
 
 
 def _nvcc() -> str:
@@ -51,7 +75,10 @@ def _stamp() -> str:
     for f in sources() + _headers():
         with open(os.path.join(HERE, f), "rb") as fh:
             h.update(f.encode() + b"\0" + fh.read())
-    h.update(" ".join(ARCH_FLAGS + NVCC_FLAGS).encode())
+    with open(os.path.join(HERE, ENTRY), "rb") as fh:
+        h.update(fh.read())
+    flags, _, version = _entry_flags()
+    h.update(" ".join(ARCH_FLAGS + NVCC_FLAGS + flags + [version, sys.version]).encode() + _entries().encode())
     return h.hexdigest()
 
 
@@ -113,10 +140,26 @@ def build(force: bool = False, verbose: bool = False) -> str:
         _say(f"  nvcc {src} done in {time.time() - t:.1f} s")
         return obj
 
+    flags, libraries, _ = _entry_flags()
+
+    def compile_entry():
+        with open(os.path.join(out_dir, "entries.inc"), "w") as f:
+            f.write(_entries())
+        obj = os.path.join(out_dir, "entry.o")
+        t = time.time()
+        _say(f"  c++ {ENTRY} ...")
+        p = subprocess.run([os.environ.get("CXX", "g++")] + flags + ["-I", out_dir, "-c", os.path.join(HERE, ENTRY), "-o", obj],
+                           stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        if p.returncode != 0:
+            raise RuntimeError(f"air_b200: the C++ compiler failed on {ENTRY}:\n{p.stdout}")
+        _say(f"  c++ {ENTRY} done in {time.time() - t:.1f} s")
+        return obj
+
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 2)) as pool:
-        objs = list(pool.map(compile_one, srcs))
+        entry_obj = pool.submit(compile_entry)
+        objs = list(pool.map(compile_one, srcs)) + [entry_obj.result()]
     tmp = lib + f".tmp{os.getpid()}"
-    p = subprocess.run([nvcc] + ARCH_FLAGS + ["-shared", "-o", tmp] + objs + ["-lcudart"],
+    p = subprocess.run([nvcc] + ARCH_FLAGS + ["-shared", "-o", tmp] + objs + ["-lcudart"] + libraries,
                        stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if p.returncode != 0:
         raise RuntimeError(f"air_b200: linking {LIB_NAME} failed:\n{p.stdout}")
@@ -131,5 +174,18 @@ def library() -> ctypes.CDLL:
     """The loaded library (built first if needed)."""
     global _lib
     if _lib is None:
+        import torch  # noqa: F401  (the library is linked against it)
         _lib = ctypes.CDLL(build())
     return _lib
+
+
+def entry():
+    """The library as an extension module: a function per launcher (arguments as in ops._SIGNATURES; it returns the error code)."""
+    global _entry
+    if _entry is None:
+        loader = machinery.ExtensionFileLoader(ENTRY_MODULE, library()._name)
+        spec = util.spec_from_file_location(ENTRY_MODULE, library()._name, loader=loader)
+        module = util.module_from_spec(spec)
+        loader.exec_module(module)
+        _entry = module
+    return _entry

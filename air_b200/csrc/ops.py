@@ -29,7 +29,7 @@ _SIGNATURES = {
                         c_longlong, c_float, c_void_p],
     "air_qkv_rope_store": [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int,
                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
-    "air_silu_mul": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+    "air_silu_mul": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "air_convert": [c_void_p, c_int, c_void_p, c_int, c_longlong, c_void_p],
     "air_gemm_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "air_gemm_f32_tc": [c_void_p] * 5 + [c_int] * 6 + [c_void_p, c_void_p],
@@ -148,11 +148,7 @@ class KernelError(RuntimeError):
 def _get(name):
     f = _fn.get(name)
     if f is None:
-        lib = build.library()
-        f = getattr(lib, name)
-        f.argtypes = _SIGNATURES[name]
-        f.restype = c_int
-        _fn[name] = f
+        f = _fn[name] = getattr(build.entry(), name)
     return f
 
 
@@ -210,7 +206,8 @@ def _stream() -> int:
     return _raw_stream(_device_index)
 
 
-def _req(t: torch.Tensor, name: str, dtypes=None, shape=None):
+def _why_not(t: torch.Tensor, name: str, dtypes=None, shape=None):
+    """t, if it is a contiguous CUDA tensor of one of the types and of the shape (None: any size), else a KernelError."""
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise KernelError(f"{name} must be a CUDA tensor (there is no CPU implementation)")
     if not t.is_contiguous():
@@ -225,6 +222,25 @@ def _req(t: torch.Tensor, name: str, dtypes=None, shape=None):
             if s is not None and s != g:
                 raise KernelError(f"{name} has shape {tuple(got)}, expected {tuple(shape)}")
     return t
+
+
+def _req(*args, **kwargs):
+    """_why_not, by the library's own function from the first call on (without a device there is nothing that fits)."""
+    global _req
+    if not torch.cuda.is_available():
+        return _why_not(*args, **kwargs)
+    build.entry().set_say_why(_why_not)
+    _req = build.entry().require
+    return _req(*args, **kwargs)
+
+
+def empty(shape, dtype, device):
+    """torch.empty, by the library's own function from the first call on."""
+    global empty
+    if not torch.cuda.is_available():
+        return torch.empty(shape, dtype=dtype, device=device)
+    empty = build.entry().empty
+    return empty(shape, dtype, device)
 
 
 _FLOATS = (torch.float32, torch.bfloat16)
@@ -440,7 +456,7 @@ def gemm_f32(a, w, bias, out, w_ready=False, status=None, shape=(0, 0)):
         _req(bias, "bias", (torch.float32,), (N,))
     _req(out, "out", (torch.float32,), (M, N))
     if f32_on_tensor_cores(w):
-        planes = None if M <= F32_CUT_ROWS else torch.empty((3, M, -(-K // 64) * 64), dtype=torch.bfloat16, device=a.device)
+        planes = None if M <= F32_CUT_ROWS else empty((3, M, -(-K // 64) * 64), torch.bfloat16, a.device)
         width, cluster = shape
         _check(_get("air_gemm_f32_tc")(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), _ptr(planes), M, N, K,
                                        1 if w_ready else 0, width, cluster, _ptr(status), _stream()), "gemm_f32")
@@ -570,7 +586,7 @@ def grouped_attention(q, cache, block_table, token_seq, positions, out, window, 
         # (rows of which a block's two stages of 64, and its queries, leave no room for a second block: one per SM)
         wide = 256 * (d + 8 + (0 if latent else dv + 8)) + 64 * (d + 8) > 100 * 1024
         splits = 4 if cache.dtype == torch.float32 else max(1, min(16, (148 if wide else 296) // max(1, blocks)))
-    part = torch.empty((T, H, splits, dv + 2), dtype=torch.float32, device=q.device)
+    part = empty((T, H, splits, dv + 2), torch.float32, q.device)
     _check(_get("air_grouped_attention")(
         q.data_ptr(), 1 if q.dtype == torch.float32 else 0, cache.data_ptr(), _DT[cache.dtype], block_table.data_ptr(),
         block_table.shape[1], token_seq.data_ptr(), positions.data_ptr(), part.data_ptr(), out.data_ptr(), T, H, G, d,
@@ -851,14 +867,14 @@ def mlstm_portions(x, z, columns, i_bias, f_bias, weight, S, n, m, out, portions
     _req(portions, "portions", _I32, (None, 4))
     _req(chunks, "chunks", _I32, (None, 2))
     L, N = portions.shape[0], chunks.shape[0]
-    gates = torch.empty((5, H, T), dtype=torch.float32, device=dev)
-    chunk_S = torch.empty((N, H, d, dv), dtype=torch.float32, device=dev)
-    chunk_n = torch.empty((N, H, d), dtype=torch.float32, device=dev)
-    o = torch.empty((T, H, dv), dtype=torch.float32, device=dev) if dv > 128 else None
+    gates = empty((5, H, T), torch.float32, dev)
+    chunk_S = empty((N, H, d, dv), torch.float32, dev)
+    chunk_n = empty((N, H, d), torch.float32, dev)
+    o = empty((T, H, dv), torch.float32, dev) if dv > 128 else None
     lists = (portions.data_ptr(), L, chunks.data_ptr(), N, gates.data_ptr(), chunk_S.data_ptr())
     sizes = (chunk_n.data_ptr(), _ptr(o), T, H, d, dv, float(cap), float(q_scale), float(eps), _stream())
     if x.dtype == torch.bfloat16:
-        planes = torch.empty((N, H, 2, d, dv), dtype=torch.bfloat16, device=dev)
+        planes = empty((N, H, 2, d, dv), torch.bfloat16, dev)
         _check(_get("air_mlstm_portions_tc")(x.data_ptr(), *xs, *rest, *lists, planes.data_ptr(), *sizes), "mlstm_portions")
         launches += 1
     else:
@@ -1231,9 +1247,9 @@ def linear_scan(mode, q, k, v, decay, state, out, q_start, slots, token_seq, q_s
     lanes = 1
     while lanes * rows < d:
         lanes *= 2
-    kq = torch.empty((T, G, 2, lanes * rows), dtype=torch.float32, device=out.device)
+    kq = empty((T, G, 2, lanes * rows), torch.float32, out.device)
     dec = None if mode == SCAN_RETENTION else \
-        torch.empty((T, H, {SCAN_DELTA: 2, SCAN_CHANNEL_DELTA: lanes * rows + 4}.get(mode, lanes * rows)), dtype=torch.float32, device=out.device)
+        empty((T, H, {SCAN_DELTA: 2, SCAN_CHANNEL_DELTA: lanes * rows + 4}.get(mode, lanes * rows)), torch.float32, out.device)
     _check(_get("air_linear_scan")(
         int(mode), qp, ldq, kp, ldk, vp, ldv, dp, ldd, bp, ldb, _ptr(a_log), _ptr(dt_bias), state.data_ptr(),
         out.data_ptr(), q_start.data_ptr(), slots.data_ptr(), token_seq.data_ptr(), kq.data_ptr(), _ptr(dec),
@@ -1287,7 +1303,7 @@ def delta_portions(q, k, v, decay, state, out, portions, chunks, q_scale, beta=N
     N = chunks.shape[0]
     wide = next(w for w in (32, 64, 128, 256) if d <= w)
     stride = (33 if mode == SCAN_GLA else 49) * wide + 256 + 16 * (-(-dv // 16) * 16)
-    scratch = torch.empty(N * H * stride, dtype=torch.float32, device=out.device)
+    scratch = empty(N * H * stride, torch.float32, out.device)
     _check(_get("air_delta_portions")(
         _CHUNK_MODES[mode], qp, ldq, kp, ldk, vp, ldv, dp, ldd, bp, ldb, _ptr(a_log), _ptr(dt_bias), state.data_ptr(),
         out.data_ptr(), portions.data_ptr(), portions.shape[0], chunks.data_ptr(), N, scratch.data_ptr(), H, G, d, dv,
@@ -1322,8 +1338,8 @@ def split_bands(x, first, second):
     xp, ld = _columns(x, "x")
     if x.shape[1] != first + second:
         raise KernelError(f"split_bands: {x.shape[1]} columns, not {first} + {second}")
-    a = torch.empty((T, 2 * first), dtype=torch.bfloat16, device=x.device)
-    b = torch.empty((T, 2 * second), dtype=torch.bfloat16, device=x.device)
+    a = empty((T, 2 * first), torch.bfloat16, x.device)
+    b = empty((T, 2 * second), torch.bfloat16, x.device)
     _check(_get("air_split_bands")(xp, ld, int(first), int(second), a.data_ptr(), b.data_ptr(), T, _stream()), "split_bands")
     return a, b
 
@@ -1545,8 +1561,8 @@ def decode_attention(q, cache, block_table, token_seq, positions, out, window, s
     po = pm = None
     if splits > 1:
         if scratch is None:
-            scratch = (torch.empty(T * H * splits * d, dtype=torch.float32, device=q.device),
-                       torch.empty(T * H * splits * 2, dtype=torch.float32, device=q.device))
+            scratch = (empty(T * H * splits * d, torch.float32, q.device),
+                       empty(T * H * splits * 2, torch.float32, q.device))
         po, pm = scratch
         _req(po, "scratch[0]", (torch.float32,))
         _req(pm, "scratch[1]", (torch.float32,))
@@ -1621,8 +1637,8 @@ def decode_attention_fresh(qkv, bias, table, cache, block_table, token_seq, posi
         splits = decode_splits(T, H, K)
     po = pm = None
     if splits > 1:
-        po = torch.empty(T * H * splits * d, dtype=torch.float32, device=qkv.device)
-        pm = torch.empty(T * H * splits * 2, dtype=torch.float32, device=qkv.device)
+        po = empty(T * H * splits * d, torch.float32, qkv.device)
+        pm = empty(T * H * splits * 2, torch.float32, qkv.device)
     asked, left = [], AHEAD_BYTES
     for w in ahead[:2]:
         n = min(left, w.numel() * w.element_size()) if w.is_contiguous() else 0
@@ -1740,8 +1756,8 @@ TC_ATTENTION_HEAD_DIMS = (64, 128)
 
 def prefill_attention_scratch(slots: int, head_dim: int, device):
     """Where the segments of cut items leave their partial sums: (float32 [slots, 256, d], float32 [slots, 256, 2])."""
-    return (torch.empty((slots, 2 * TILE_GROUP * 16, head_dim), dtype=torch.float32, device=device),
-            torch.empty((slots, 2 * TILE_GROUP * 16, 2), dtype=torch.float32, device=device))
+    return (empty((slots, 2 * TILE_GROUP * 16, head_dim), torch.float32, device),
+            empty((slots, 2 * TILE_GROUP * 16, 2), torch.float32, device))
 
 
 def prefill_attention_tc(q, cache, block_table, tiles, out, window, scale, status=None, segments=None, items=None,

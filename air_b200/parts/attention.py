@@ -315,14 +315,14 @@ class Attention(TiledAttention, Mixer):
                 and ops.decode_attention_fresh_ok(qkv, table, pages.kv, d)):
             # single next tokens only: the attention kernel itself adds the bias, rotates, writes the new keys
             # and values and attends (one launch less, and the keys stream as soon as the product has ended)
-            out = torch.empty((T, H, d), dtype=rt.dtype, device=x.device)
+            out = ops.empty((T, H, d), rt.dtype, x.device)
             ops.decode_attention_fresh(qkv, self.bias, table, pages.kv, bt, ctx.token_seq, ctx.positions, out, H,
                                        self.window, self.scale, write_kv=owns_cache, status=ctx.status,
                                        ahead=(self.o.weight, *self.behind))
             return self._project(out.view(T, H * d), ctx)
         if isinstance(x, PreNormed):
             raise ops.KernelError("attention: rows without their norm's scale reached a road that does not apply it")
-        q = torch.empty((T, H, d), dtype=rt.dtype, device=x.device)
+        q = ops.empty((T, H, d), rt.dtype, x.device)
         ops.qkv_rope_store(qkv, self.bias, table, ctx.positions, ctx.token_seq, bt, q, pages.kv,
                            H, K, d, write_kv=owns_cache, status=ctx.status)
         out = torch.empty_like(q)

@@ -333,7 +333,7 @@ class Norm(Part):
             from ..csrc import ops
             if isinstance(delta, StreamSum):
                 S = delta.out.shape[0]
-                full = h if h.dim() == 3 else torch.empty((S,) + tuple(h.shape), dtype=h.dtype, device=h.device)
+                full = h if h.dim() == 3 else ops.empty((S,) + tuple(h.shape), h.dtype, h.device)
                 ops.stream_norm(h, S, None, None, 0.0, None, term=delta.term, mix=delta.mix, out_weights=delta.out,
                                 h_out=full)
                 return full

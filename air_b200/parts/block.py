@@ -177,7 +177,7 @@ class SandwichBlock(Block):
         if isinstance(delta, (GatedSum, ScaledSum, NormedSum)) or delta is None:
             raise ops.KernelError("sandwich: the sub-layer must return its output as a tensor or as partial sums")
         if delta.dtype != torch.float32:
-            delta = ops.convert(delta, torch.empty(delta.shape, dtype=torch.float32, device=delta.device))
+            delta = ops.convert(delta, ops.empty(delta.shape, torch.float32, delta.device))
         return NormedSum(delta, norm.weight_f32(), norm.eps)
 
     def forward(self, h, pending, ctx, cache, owns_cache=True):
@@ -295,7 +295,7 @@ class PostNormBlock(Block):
             x = None
         if x is None:
             rt = self.mixer.rt
-            x = h if rt.is_fp32 else ops.convert(h, torch.empty(h.shape, dtype=rt.dtype, device=h.device))
+            x = h if rt.is_fp32 else ops.convert(h, ops.empty(h.shape, rt.dtype, h.device))
         x = self.mixer_norm.forward(h, self.mixer.forward(x, ctx, cache, owns_cache))
         if self.ff_norm is not None:
             x = self.ff_norm.forward(h, self.feed_forward.forward(x, ctx) if self.feed_forward is not None else None)
@@ -374,7 +374,7 @@ class StreamsBlock(Block):
         if y is None or isinstance(y, (GatedSum, ScaledSum, NormedSum, StreamSum)):
             raise ops.KernelError("streams: the sub-layer must return its output as a tensor or as partial sums")
         if y.dtype != torch.float32:
-            y = ops.convert(y, torch.empty(y.shape, dtype=torch.float32, device=y.device))
+            y = ops.convert(y, ops.empty(y.shape, torch.float32, y.device))
         return StreamSum(y, numbers[1], numbers[2])
 
     def forward(self, h, pending, ctx, cache, owns_cache=True, kept=()):

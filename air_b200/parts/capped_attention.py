@@ -106,12 +106,12 @@ class CappedAttention(TiledAttention, Mixer):
         rt = self.rt
         P = rt.page_tokens
         proj = self.proj.f32(x)
-        q = torch.empty((T, H, dk), dtype=rt.dtype, device=x.device)
-        gate = torch.empty((T, H), dtype=torch.float32, device=x.device) if self.head_gate else None
+        q = ops.empty((T, H, dk), rt.dtype, x.device)
+        gate = ops.empty((T, H), torch.float32, x.device) if self.head_gate else None
         v_mode, v_first = 0, None
         if self.v_mix == "first":
             v_mode = 1
-            v_first = ctx.shared[self.v_stream] = torch.empty((T, G * dv), dtype=torch.float32, device=x.device)
+            v_first = ctx.shared[self.v_stream] = ops.empty((T, G * dv), torch.float32, x.device)
         elif self.v_mix == "mix":
             v_mode, v_first = 2, ctx.shared.get(self.v_stream)
             if v_first is None:
@@ -120,7 +120,7 @@ class CappedAttention(TiledAttention, Mixer):
         kv = pages.kv.view(pages.kv.shape[0], -1)
         ops.qkv_prepare(proj, self.bias, self.position.frequencies(), ctx.positions, ctx.token_seq, bt, q, kv, G, dv,
                         P, gate_out=gate, v_first=v_first, v_mode=v_mode, v_lambda=self.v_lambda, status=ctx.status)
-        out = torch.empty((T, H, dv), dtype=rt.dtype, device=x.device)
+        out = ops.empty((T, H, dv), rt.dtype, x.device)
         if dk == dv and self.fast_attention(ctx, P):
             self.attend(q, pages.kv, bt, ctx, out)
             if gate is not None:

@@ -26,7 +26,7 @@ class TokenEmbedding(Embedding):
         self.multiplier = float(self.spec.get("multiplier", 1.0))
 
     def forward(self, ctx, cache, copies=1):
-        h = torch.empty((ctx.num_tokens, self.spec["hidden"]), dtype=torch.float32, device=self.rt.device)
+        h = ops.empty((ctx.num_tokens, self.spec["hidden"]), torch.float32, self.rt.device)
         ops.embedding(self.table, ctx.token_ids, h, status=ctx.status, last_token=ctx.last_token,
                       multiplier=self.multiplier)
         return (h,) + tuple(ops.convert(h, torch.empty_like(h)) for _ in range(copies - 1))
@@ -70,11 +70,11 @@ class BigramHashEmbedding(Embedding):
     def forward(self, ctx, cache, copies=1):
         (previous,) = cache
         dev = self.rt.device
-        h = torch.empty((ctx.num_tokens, self.hidden), dtype=torch.float32, device=dev)
+        h = ops.empty((ctx.num_tokens, self.hidden), torch.float32, dev)
         more = tuple(torch.empty_like(h) for _ in range(copies - 1))
         if len(more) > 1:
             raise ops.KernelError("bigram embedding: at most two copies")
-        resolved = torch.empty((ctx.num_tokens,), dtype=torch.int32, device=dev)
+        resolved = ops.empty((ctx.num_tokens,), torch.int32, dev)
         ops.bigram_embedding(self.table, self.pairs, ctx.token_ids, ctx.positions, ctx.token_seq, previous.state, h,
                              more[0] if more else None, resolved, self.buckets, self.mul_prev, self.mul_cur,
                              status=ctx.status, last_token=ctx.last_token)

@@ -163,16 +163,16 @@ class RoutedExperts(FeedForward):
         T, E, F, n, top = x.shape[0], self.hidden, self.inter, self.experts, self.top
         dev = x.device
         z = self.router.f32_sums(x)      # (few rows: a block per part of k instead of one for all of it)
-        expert = torch.empty((T, top), dtype=torch.int32, device=dev)
-        weight = torch.empty((T, top), dtype=torch.float32, device=dev)
-        gate = torch.empty((T,), dtype=torch.float32, device=dev) if self.shared_gate else None
+        expert = ops.empty((T, top), torch.int32, dev)
+        weight = ops.empty((T, top), torch.float32, dev)
+        gate = ops.empty((T,), torch.float32, dev) if self.shared_gate else None
         ops.moe_route(z, self.outputs, top, expert, weight, gate, has_gate=self.shared_gate, score=self.score,
                       renormalize=self.renormalize, groups=self.groups, keep=self.keep, route_scale=self.route_scale,
                       norm_eps=self.norm_eps, choice_bias=self.correction, mark=self.group_mark)
         on_input = self.weight_on == "input"
         pairs = T * top
         # (three numbers ahead of `start`, so that the experts' ends, start[1:], lie on a 16-byte boundary)
-        ints = torch.empty(3 + n + 1 + pairs + 2 * (pairs // ops.GROUP_TILE + n) + 1, dtype=torch.int32, device=dev)[3:]
+        ints = ops.empty(3 + n + 1 + pairs + 2 * (pairs // ops.GROUP_TILE + n) + 1, torch.int32, dev)[3:]
         start, pair_of_slot = ints[:n + 1], ints[n + 1:n + 1 + pairs]
         tiles, num_tiles = ints[n + 1 + pairs:-1].view(-1, 2), ints[-1:]
         streams = ops.expert_stream_ok(x, self.gate_up, self.block, self.gated) and ops.expert_stream_ok(x, self.down, 0, False)
@@ -182,7 +182,7 @@ class RoutedExperts(FeedForward):
         tile_rows = ops.GROUP_WIDE if streams and pairs >= self.WIDE_ROWS * n else ops.GROUP_TILE
         ops.moe_sort(expert, n, start, pair_of_slot, tiles, num_tiles, tile_rows=tile_rows)
         parts = self._parts(T) if streams else 1
-        y = torch.empty((parts * top, T, E), dtype=torch.float32, device=dev)
+        y = ops.empty((parts * top, T, E), torch.float32, dev)
         if self.identity:
             # (pairs of an expert without matrices get no slot in the order by expert: their planes are written here)
             ops.moe_identity(x, expert, weight, n, y)
@@ -190,8 +190,8 @@ class RoutedExperts(FeedForward):
             self._experts_by_the_library(x, start, pair_of_slot, weight, y)
         elif streams:
             rows = ops.rows_by_index(x, pair_of_slot, top, weight.view(-1) if on_input else None,
-                                     torch.empty((pairs, E), dtype=x.dtype, device=dev))
-            act = torch.empty((pairs, F), dtype=x.dtype, device=dev)
+                                     ops.empty((pairs, E), x.dtype, dev))
+            act = ops.empty((pairs, F), x.dtype, dev)
             lists = (start, tiles, num_tiles, T)       # (a token takes an expert once at most)
             ops.expert_stream(rows, self.gate_up, act, *lists, silu_mul=self.gated, relu2=not self.gated, act=self.act,
                               status=self.rt.status, tile_rows=tile_rows)
@@ -199,7 +199,7 @@ class RoutedExperts(FeedForward):
                               o_scale=None if on_input else weight.view(-1), lists_ready=True, status=self.rt.status,
                               tile_rows=tile_rows)
         else:
-            act = torch.empty((pairs, F), dtype=x.dtype, device=dev)
+            act = ops.empty((pairs, F), x.dtype, dev)
             ops.grouped_gemm(x, self.gate_up, act, F, E, lda=E, ldo=F, groups=n, a_index=pair_of_slot, a_div=top,
                              a_scale=weight.view(-1) if on_input else None, start=start, tiles=tiles,
                              num_tiles=num_tiles, silu_mul=self.gated, gate_block=self.block if self.gated else 0,
@@ -230,9 +230,9 @@ class RoutedExperts(FeedForward):
         pairs = T * top
         on_input = self.weight_on == "input"
         rows = ops.rows_by_index(x, pair_of_slot, top, weight.view(-1) if on_input else None,
-                                 torch.empty((pairs, E), dtype=x.dtype, device=x.device))
+                                 ops.empty((pairs, E), x.dtype, x.device))
         ends = start[1:]
-        act = torch.empty((pairs, self.inter), dtype=x.dtype, device=x.device)
+        act = ops.empty((pairs, self.inter), x.dtype, x.device)
         hidden = torch._grouped_mm(rows, self.gate_up.transpose(1, 2), offs=ends)
         if self.activation == "clamped_glu":
             ops.glu(hidden, act, block=self.block, alpha=self.act[0], limit=self.act[1], shift=self.act[2])

@@ -105,15 +105,15 @@ class PortionAttention:
         dv, G = out.shape[2], kv_heads
         J = H // G
         dev = q.device
-        q16 = q if q.dtype == torch.bfloat16 else ops.convert(q, torch.empty(q.shape, dtype=torch.bfloat16, device=dev))
+        q16 = q if q.dtype == torch.bfloat16 else ops.convert(q, ops.empty(q.shape, torch.bfloat16, dev))
         for r0, n, pos0, slot in plan.portions:
             for b0 in range(0, n, self.BLOCK):
                 nb, p0 = min(self.BLOCK, n - b0), pos0 + b0
                 lo = self.first_visible(p0)
                 L = p0 + nb - lo
                 Lp = -(-L // 16) * 16
-                keys = torch.empty((G, Lp, dk), dtype=torch.bfloat16, device=dev)
-                values = None if latent else torch.empty((G, Lp, dv), dtype=torch.bfloat16, device=dev)
+                keys = ops.empty((G, Lp, dk), torch.bfloat16, dev)
+                values = None if latent else ops.empty((G, Lp, dv), torch.bfloat16, dev)
                 ops.gather_keys(cache, bt[slot], lo, L, keys, values, kv_heads=G, page_tokens=page_tokens, latent=latent)
                 rows = q16[r0 + b0:r0 + b0 + nb]
                 if G == 1:
@@ -121,13 +121,13 @@ class PortionAttention:
                 else:      # rows of one key/value head together: (token, query head of the group)
                     rows = rows.view(nb, G, J, dk).permute(1, 0, 2, 3).reshape(G, nb * J, dk)
                 # (one library product per key/value head: the batched call with a 32-bit result is far slower)
-                scores = torch.empty((G, nb * J, Lp), dtype=torch.float32, device=dev)
+                scores = ops.empty((G, nb * J, Lp), torch.float32, dev)
                 for g in range(G):
                     torch.mm(rows[g], keys[g].t(), out_dtype=torch.float32, out=scores[g])
-                weights = torch.empty(scores.shape, dtype=torch.bfloat16, device=dev)
+                weights = ops.empty(scores.shape, torch.bfloat16, dev)
                 ops.masked_softmax(scores, weights, J, lo, L, p0, self.scale, window=self.window, chunk=self.chunk,
                                    sink=sinks, softcap=softcap, bias=bias)
-                summed = torch.empty((G, nb * J, dv), dtype=torch.bfloat16, device=dev)
+                summed = ops.empty((G, nb * J, dv), torch.bfloat16, dev)
                 for g in range(G):
                     torch.mm(weights[g], keys[g, :, :dv] if latent else values[g], out=summed[g])
                 dst = out[r0 + b0:r0 + b0 + nb]

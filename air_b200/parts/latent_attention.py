@@ -180,7 +180,7 @@ class LatentAttention(PortionAttention, Mixer):
         for i, (r0, n, pos0, slot, slots) in enumerate(plan.expanded):
             lo, ahead, count = self.expanded_keys(pos0, n)
             keys = -(-count // 16) * 16
-            rows = torch.empty((1, keys, self.rank + self.rot_dim), dtype=torch.bfloat16, device=q.device)
+            rows = ops.empty((1, keys, self.rank + self.rot_dim), torch.bfloat16, q.device)
             ops.gather_keys(latent.rows, bt[slot], lo, count, rows, None, latent=True, ahead=ahead)
             kv = torch.mm(rows[0, :, :self.rank], self.expansion[0].t())
             cut = getattr(plan, f"segments{i}", None)
@@ -204,7 +204,7 @@ class LatentAttention(PortionAttention, Mixer):
         width = self.heads * (self.head_dim + self.rot_dim)
         if not self.q_rank:
             return proj[:, :width]
-        latent = torch.empty((proj.shape[0], self.q_up.in_features), dtype=self.rt.dtype, device=proj.device)
+        latent = ops.empty((proj.shape[0], self.q_up.in_features), self.rt.dtype, proj.device)
         ops.band_rmsnorm(proj[:, :self.q_rank], self.q_weight, self.eps, latent)
         return self.q_up.f32(latent)[:, :width]
 
@@ -220,21 +220,21 @@ class LatentAttention(PortionAttention, Mixer):
         plan = ctx.plans.get(self.plan_key()) if self.expands else None
         expanded = plan is not None and bool(plan.expanded)
         rows = plan.rows if expanded else T         # of the step, from its first on, that the other roads need
-        q_plain = torch.empty((T, H, d), dtype=rt.dtype, device=dev)
-        q_full = torch.empty((T, H, R + rot), dtype=torch.float32, device=dev) if rows else None
-        q_rot = torch.empty((T, H, rot), dtype=rt.dtype, device=dev) if expanded and rot else None
-        gate = torch.empty((T, H), dtype=torch.float32, device=dev) if self.head_gate else None
+        q_plain = ops.empty((T, H, d), rt.dtype, dev)
+        q_full = ops.empty((T, H, R + rot), torch.float32, dev) if rows else None
+        q_rot = ops.empty((T, H, rot), rt.dtype, dev) if expanded and rot else None
+        gate = ops.empty((T, H), torch.float32, dev) if self.head_gate else None
         pos = self.position
         ops.latent_prepare(self._queries(proj), proj[:, self.c_column:self.c_column + R + rot] if owns_cache else None,
                            self.c_weight, self.eps, pos.frequencies64() if pos is not None else None, ctx.positions,
                            ctx.token_seq, bt, q_plain, q_full, latent.rows, owns_cache, status=ctx.status,
                            gate=proj[:, self.gate_column:self.gate_column + H] if gate is not None else None,
                            gate_out=gate, pairing=pos.pairing if pos is not None else "half", q_rot=q_rot)
-        out = torch.empty((T, H, dv), dtype=rt.dtype, device=dev)
+        out = ops.empty((T, H, dv), rt.dtype, dev)
         if rows:
             ops.grouped_gemm(q_plain, self.uk_t, q_full, R, d, lda=H * d, ldo=H * (R + rot), groups=H, a_group_stride=d,
                              o_group_stride=R + rot, a_local=True, o_local=True, rows_per_group=rows)
-            summed = torch.empty((T, H, R), dtype=rt.dtype, device=dev)
+            summed = ops.empty((T, H, R), rt.dtype, dev)
             self.attend(q_full, latent.rows, bt, ctx, summed, latent=True)
             ops.grouped_gemm(summed, self.uv, out, dv, R, lda=H * R, ldo=H * dv, groups=H, a_group_stride=R,
                              o_group_stride=dv, a_local=True, o_local=True, rows_per_group=rows, o_scale=gate, o_scale_ld=H)

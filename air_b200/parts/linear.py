@@ -50,6 +50,7 @@ class Linear:
     def __init__(self, weight: torch.Tensor, status: Optional[torch.Tensor] = None, gate_up_block: int = 0):
         assert weight.dim() == 2
         self.weight = weight
+        self.transposed = weight.t()             # (a view, as the library's product wants it)
         self.status = status
         self.out_features, self.in_features = weight.shape
         self.gate_up_block = gate_up_block       # > 0: rows are blocks of gate rows and up rows in turn
@@ -85,7 +86,7 @@ class Linear:
     def partial(self, x) -> torch.Tensor:
         """float32 [parts, rows, out]: partial sums over parts of k, for a consumer that adds them."""
         x, scale = self._scaled(x)
-        out = torch.empty((self.parts, x.shape[0], self.out_features), dtype=torch.float32, device=x.device)
+        out = ops.empty((self.parts, x.shape[0], self.out_features), torch.float32, x.device)
         return ops.gemm_tc(x, self.weight, out, self.tile, ops.EPI_PARTIAL, splits=self.parts, status=self.status,
                            **scale)
 
@@ -93,21 +94,21 @@ class Linear:
         """float32 [rows, out] in one pass of the tcgen05 kernel."""
         x, scale = self._scaled(x)
         bn, _ = choose_tile(self.out_features, self.in_features, may_split=False)
-        out = torch.empty((x.shape[0], self.out_features), dtype=torch.float32, device=x.device)
+        out = ops.empty((x.shape[0], self.out_features), torch.float32, x.device)
         return ops.gemm_tc(x, self.weight, out, bn, ops.EPI_F32, status=self.status, **scale)
 
     def silu_mul(self, x, act=ops.SILU) -> torch.Tensor:
         """bfloat16 [rows, out / 2] = silu(gate) * up, in the epilogue of the tcgen05 kernel; with act = (alpha,
         limit, shift) the gated activation that ops.gemm_tc describes."""
         x, scale = self._scaled(x)
-        out = torch.empty((x.shape[0], self.out_features // 2), dtype=torch.bfloat16, device=x.device)
+        out = ops.empty((x.shape[0], self.out_features // 2), torch.bfloat16, x.device)
         return ops.gemm_tc(x, self.weight, out, 2 * self.gate_up_block, ops.EPI_SILU, status=self.status, act=act,
                            **scale)
 
     def relu2(self, x) -> torch.Tensor:
         """bfloat16 [rows, out] = max(x W^T, 0)^2, in the epilogue of the tcgen05 kernel."""
         bn, _ = choose_tile(self.out_features, self.in_features, may_split=False)
-        out = torch.empty((x.shape[0], self.out_features), dtype=torch.bfloat16, device=x.device)
+        out = ops.empty((x.shape[0], self.out_features), torch.bfloat16, x.device)
         return ops.gemm_tc(x, self.weight, out, bn, ops.EPI_RELU2, status=self.status)
 
     def f32(self, x: torch.Tensor) -> torch.Tensor:
@@ -129,17 +130,17 @@ class Linear:
     def add_into(self, x: torch.Tensor, residual: torch.Tensor) -> None:
         """residual += x W^T, the sum taken in 32-bit in the library product's epilogue (the product is not
         rounded to 16 bits first, and is not written and read again by the norm that follows)."""
-        torch.addmm(residual, x, self.weight.t(), out_dtype=torch.float32, out=residual)
+        torch.addmm(residual, x, self.transposed, out_dtype=torch.float32, out=residual)
 
     def __call__(self, x: torch.Tensor, out_dtype: torch.dtype, bias=None) -> torch.Tensor:
         w = self.weight
         if w.dtype == torch.float32:
             if x.dtype != torch.float32:
-                x = ops.convert(x, torch.empty(x.shape, dtype=torch.float32, device=x.device))
-            out = torch.empty((x.shape[0], self.out_features), dtype=torch.float32, device=x.device)
+                x = ops.convert(x, ops.empty(x.shape, torch.float32, x.device))
+            out = ops.empty((x.shape[0], self.out_features), torch.float32, x.device)
             ops.gemm_f32(x, w, bias, out, w_ready=True, status=self.status)
             if out_dtype != torch.float32:
-                out = ops.convert(out, torch.empty(out.shape, dtype=out_dtype, device=x.device))
+                out = ops.convert(out, ops.empty(out.shape, out_dtype, x.device))
             return out
         if x.dtype != w.dtype:
             raise ops.KernelError(f"Linear: input {x.dtype} with weight {w.dtype}")
@@ -147,4 +148,4 @@ class Linear:
             raise ops.KernelError("Linear: a bias with 16-bit weights is added by the consumer's kernel")
         if not x.is_cuda:
             raise ops.KernelError("Linear: input must be a CUDA tensor")
-        return torch.mm(x, w.t(), out_dtype=out_dtype)
+        return torch.mm(x, self.transposed, out_dtype=out_dtype)

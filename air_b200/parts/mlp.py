@@ -93,7 +93,7 @@ class SwiGLU(FeedForward):
             act = self.gate_up.silu_mul(x, act=self.ACT)
         else:
             gu = self.gate_up(x, torch.float32 if self.rt.is_fp32 else self.rt.dtype)
-            act = torch.empty((x.shape[0], self.intermediate), dtype=self.rt.dtype, device=x.device)
+            act = ops.empty((x.shape[0], self.intermediate), self.rt.dtype, x.device)
             ops.silu_mul(gu, act, block=self.block, relu=self.ACT is ops.RELU)
         if self.down.small(act):
             return self.down.partial(act)
@@ -134,7 +134,7 @@ class ClampedGLU(SwiGLU):
             act = self.gate_up.silu_mul(x, act=shape)
         else:
             gu = self.gate_up(x, torch.float32 if self.rt.is_fp32 else self.rt.dtype)
-            act = torch.empty((x.shape[0], self.intermediate), dtype=self.rt.dtype, device=x.device)
+            act = ops.empty((x.shape[0], self.intermediate), self.rt.dtype, x.device)
             ops.glu(gu, act, block=self.block, alpha=shape[0], limit=shape[1], shift=shape[2])
         return self.down.f32_sums(act)
 
@@ -174,7 +174,7 @@ class PolyNormMLP(FeedForward):
 
     def forward(self, x, ctx):
         z = self.up.f32(x)
-        act = torch.empty((x.shape[0], self.padded), dtype=self.rt.dtype, device=x.device)
+        act = ops.empty((x.shape[0], self.padded), self.rt.dtype, x.device)
         ops.polynorm(z, self.up_bias, self.coefficients, self.eps, act, self.intermediate)
         return self.down.f32_sums(act)
 
@@ -207,5 +207,5 @@ class Relu2MLP(FeedForward):
             act = self.up.relu2(x)
         else:
             z = self.up(x, torch.float32 if self.rt.is_fp32 else self.rt.dtype)
-            act = ops.relu2(z, torch.empty(z.shape, dtype=self.rt.dtype, device=x.device))
+            act = ops.relu2(z, ops.empty(z.shape, self.rt.dtype, x.device))
         return self.down.f32_sums(act)

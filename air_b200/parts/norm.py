@@ -48,7 +48,7 @@ class RMSNorm(Norm):
 
     def forward(self, h, delta, rows=None):
         n = h.shape[0] if rows is None else rows.shape[0]
-        out = torch.empty((n, h.shape[1]), dtype=self.rt.dtype, device=h.device)
+        out = ops.empty((n, h.shape[1]), self.rt.dtype, h.device)
         delta = self._as_terms(delta)
         if isinstance(delta, GatedSum):
             if rows is not None:
@@ -80,8 +80,8 @@ class RMSNorm(Norm):
         if isinstance(delta, (ScaledSum, GatedSum, NormedSum)):
             self.add_delta(h, delta)
             delta = None
-        xg = torch.empty((T, E), dtype=torch.bfloat16, device=h.device)
-        ss = torch.empty((-(-E // ops.PRENORM_CHUNK), T), dtype=torch.float32, device=h.device)
+        xg = ops.empty((T, E), torch.bfloat16, h.device)
+        ss = ops.empty((-(-E // ops.PRENORM_CHUNK), T), torch.float32, h.device)
         ops.add_prenorm(h, delta, self.weight, xg, ss)
         return PreNormed(xg, ss, self.eps)
 
@@ -126,8 +126,8 @@ class PostRMSNorm(Norm):
             raise ops.KernelError("rms_after: sums with a scale per column are not offered")
         a, b, gate = (delta.a, delta.b, delta.gate) if isinstance(delta, GatedSum) else (delta, None, None)
         if a is not None and a.dtype != torch.float32:
-            a = ops.convert(a, torch.empty(a.shape, dtype=torch.float32, device=a.device))
-        out = None if self.rt.is_fp32 else torch.empty(h.shape, dtype=self.rt.dtype, device=h.device)
+            a = ops.convert(a, ops.empty(a.shape, torch.float32, a.device))
+        out = None if self.rt.is_fp32 else ops.empty(h.shape, self.rt.dtype, h.device)
         ops.post_norm(h, self.alpha, a, b, gate, self.weight, self.eps, out)
         return h if out is None else out
 
@@ -162,7 +162,7 @@ class LayerNorm(Norm):
         if isinstance(delta, StreamSum) or h.dim() == 3:
             return self.forward_streams(h, delta, None, rows=rows)[1]
         n = h.shape[0] if rows is None else rows.shape[0]
-        out = torch.empty((n, h.shape[1]), dtype=self.rt.dtype, device=h.device)
+        out = ops.empty((n, h.shape[1]), self.rt.dtype, h.device)
         terms = row_terms(delta)
         if terms is None:
             if rows is not None:
@@ -183,7 +183,7 @@ class LayerNorm(Norm):
             return h, ops.stream_norm(h, S, self.weight, self.bias, self.eps, out, read=read, rows=rows, conv=conv)
         full = None
         if rows is None:
-            full = h if h.dim() == 3 else torch.empty((S,) + tuple(h.shape), dtype=torch.float32, device=h.device)
+            full = h if h.dim() == 3 else ops.empty((S,) + tuple(h.shape), torch.float32, h.device)
         ops.stream_norm(h, S, self.weight, self.bias, self.eps, out, term=delta.term, mix=delta.mix, out_weights=delta.out,
                         read=read, h_out=full, rows=rows, conv=conv)
         return (h if full is None else full), out

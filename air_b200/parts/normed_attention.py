@@ -244,11 +244,11 @@ class NormedAttention(PortionAttention, Mixer):
             tail = cache[1].state if self.taps > 1 else torch.empty((ctx.slots.shape[0], C, 0), dtype=torch.float32,
                                                                     device=x.device)
             proj = ops.short_conv_silu(full[:, :C], self.conv_weight, tail,
-                                       torch.empty((T, C), dtype=torch.float32, device=x.device), ctx.q_start,
+                                       ops.empty((T, C), torch.float32, x.device), ctx.q_start,
                                        ctx.slots, ctx.max_q_len, act=False)
         elif self.out_gate:
             proj = full[:, :C]
-        q = torch.empty((T, H, dk), dtype=rt.dtype, device=x.device)
+        q = ops.empty((T, H, dk), rt.dtype, x.device)
         bt = ctx.block_tables[pages.group]
         kv = pages.kv.view(pages.kv.shape[0], -1)
         pos = self.position
@@ -256,7 +256,7 @@ class NormedAttention(PortionAttention, Mixer):
                               pos.magnitude, ctx.positions, ctx.token_seq, bt, q, kv, G, dv, P, status=ctx.status,
                               bias=self.bias, whole=self.norm_whole, q_scale=self.temp, v_freq=self.v_freq,
                               write_kv=owns_cache)
-        out = torch.empty((T, H, dv), dtype=rt.dtype, device=x.device)
+        out = ops.empty((T, H, dv), rt.dtype, x.device)
         gate = full[:, C:] if self.out_gate else None
         turn = None if self.v_freq is None else (self.v_freq, pos.pairing)
         plan = ctx.plans.get(self.plan_key()) if self.tiles_fit() and not ctx.all_decode else None

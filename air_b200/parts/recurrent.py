@@ -36,13 +36,13 @@ class _StateMixer(Mixer):
     def _finish(self, o, gate, ctx, sigmoid=False):
         """norm over each head's read-out, times the weight and silu(gate) (or sigmoid(gate)), then the output projection"""
         T = o.shape[0]
-        y = torch.empty((T, self.heads * self.v_dim), dtype=self.rt.dtype, device=o.device)
+        y = ops.empty((T, self.heads * self.v_dim), self.rt.dtype, o.device)
         ops.gated_rmsnorm(o, gate, self.norm_weight, self.eps, y, ctx.token_seq, sigmoid=sigmoid)
         return self.o.f32_sums(y)
 
     def _convolved(self, proj, tail, ctx):
         """The first `channels` columns of proj behind the short convolution and SiLU; tail: the state of its last inputs."""
-        y = torch.empty((proj.shape[0], self.channels), dtype=torch.float32, device=proj.device)
+        y = ops.empty((proj.shape[0], self.channels), torch.float32, proj.device)
         state = tail.state if self.taps > 1 else tail.state[:, :, :0].contiguous()
         return ops.short_conv_silu(proj[:, :self.channels], self.conv_weight, state, y, ctx.q_start, ctx.slots, ctx.max_q_len)
 
@@ -160,7 +160,7 @@ class GatedDeltaRule(_ChunkedMixer):
         T, H, G, d, dv = x.shape[0], self.heads, self.kv_heads, self.head_dim, self.v_dim
         proj = self.proj.f32(x)
         y = self._convolved(proj, tail, ctx)
-        o = torch.empty((T, H, dv), dtype=torch.float32, device=x.device)
+        o = ops.empty((T, H, dv), torch.float32, x.device)
         self._scan(ops.SCAN_DELTA, y[:, :G * d], y[:, G * d:2 * G * d], y[:, 2 * G * d:], self._band(proj, "a"), state.state, o,
                    ctx, q_scale=d ** -0.5, beta=self._band(proj, "b"), a_log=self.a_log, dt_bias=self.dt_bias)
         return self._finish(o, self._band(proj, "g"), ctx)
@@ -272,7 +272,7 @@ class ChannelDeltaRule(_ChunkedMixer):
         proj = self.proj.f32(x)
         y = self._convolved(proj, tail, ctx)
         decay, gate = self._narrow(proj)
-        o = torch.empty((T, H, dv), dtype=torch.float32, device=x.device)
+        o = ops.empty((T, H, dv), torch.float32, x.device)
         self._scan(ops.SCAN_CHANNEL_DELTA, y[:, :G * d], y[:, G * d:2 * G * d], y[:, 2 * G * d:], decay, state.state, o, ctx,
                    q_scale=d ** -0.5, beta=self._band(proj, "b"), a_log=self.a_log, dt_bias=self.dt_bias)
         return self._finish(o, gate, ctx, sigmoid=True)
@@ -325,9 +325,9 @@ class GatedLinearAttention(_ChunkedMixer):
         (state,) = cache
         T, H, d, dv = x.shape[0], self.heads, self.head_dim, self.v_dim
         proj = self.proj.f32(x)
-        z = torch.empty((T, H * d), dtype=torch.float32, device=x.device)
+        z = ops.empty((T, H * d), torch.float32, x.device)
         ops.gemm_f32(self._band(proj, "a1").contiguous(), self.a2, self.a2_bias, z, w_ready=True)
-        o = torch.empty((T, H, dv), dtype=torch.float32, device=x.device)
+        o = ops.empty((T, H, dv), torch.float32, x.device)
         self._scan(ops.SCAN_GLA, self._band(proj, "q"), self._band(proj, "k"), self._band(proj, "v"), z, state.state, o, ctx,
                    unit_lengths=False, q_scale=d ** -0.5, tau=self.tau)
         return self._finish(o, self._band(proj, "g"), ctx)
@@ -378,11 +378,11 @@ class HGRN2(_StateMixer):
         (state,) = cache
         T, H, dv = x.shape[0], self.heads, self.v_dim
         proj = self.proj.f32(x)
-        o = torch.empty((T, H, dv), dtype=torch.float32, device=x.device)
+        o = ops.empty((T, H, dv), torch.float32, x.device)
         ops.linear_scan(ops.SCAN_HGRN, self._band(proj, "q"), None, self._band(proj, "v"), self._band(proj, "f"),
                         state.state, o, ctx.q_start, ctx.slots, ctx.token_seq, lower=self.lower,
                         gate_bias=self.gate_bias)
-        y = torch.empty((T, H * dv), dtype=self.rt.dtype, device=o.device)
+        y = ops.empty((T, H * dv), self.rt.dtype, o.device)
         ops.gated_rmsnorm(o, None, self.norm_weight, self.eps, y, ctx.token_seq)
         return self.o.f32_sums(y)
 
@@ -446,7 +446,7 @@ class Retention(_StateMixer):
         (state,) = cache
         T, H, d, dv = x.shape[0], self.heads, self.head_dim, self.v_dim
         proj = self.proj.f32(x)
-        o = torch.empty((T, H, dv), dtype=torch.float32, device=x.device)
+        o = ops.empty((T, H, dv), torch.float32, x.device)
         ops.linear_scan(ops.SCAN_RETENTION, self._band(proj, "q"), self._band(proj, "k"), self._band(proj, "v"),
                         self.decays, state.state, o, ctx.q_start, ctx.slots, ctx.token_seq, positions=ctx.positions,
                         freq=self.freq, k_scale=d ** -0.5)
@@ -543,7 +543,7 @@ class MLSTM(_StateMixer):
         else:
             proj = self.proj.f32(x)
             qkvg, logits = proj[:, :gates], proj[:, gates:]
-        y = torch.empty((x.shape[0], self.heads * self.v_dim), dtype=self.rt.dtype, device=x.device)
+        y = ops.empty((x.shape[0], self.heads * self.v_dim), self.rt.dtype, x.device)
         args = (qkvg, logits, self.starts, self.i_bias, self.f_bias, self.norm_weight, memory.state, key_sum.state,
                 level.state, y)
         numbers = (self.cap, self.head_dim ** -0.5, self.eps)

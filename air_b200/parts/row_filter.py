@@ -38,5 +38,5 @@ class ResidualConvolution(RowFilter):
         return (self.weight, self._state(cache), ctx.token_seq) if ctx.all_decode else None
 
     def forward(self, x, ctx, cache):
-        out = torch.empty(x.shape, dtype=self.rt.dtype, device=x.device)
+        out = ops.empty(x.shape, self.rt.dtype, x.device)
         return ops.residual_conv(x, self.weight, self._state(cache), out, ctx.q_start, ctx.slots, ctx.max_q_len)

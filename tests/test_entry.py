@@ -1,0 +1,66 @@
+"""The library's own way in: its list of launchers is that of the sources, and its checks are those of ops._why_not."""
+import ctypes
+import glob
+import os
+import re
+
+import pytest
+import torch
+
+from air_b200.csrc import build, ops
+
+
+def test_signatures_are_those_of_the_sources():
+    kinds = {ctypes.c_void_p: "pointer", ctypes.c_int: "int", ctypes.c_longlong: "long long", ctypes.c_float: "float"}
+    found = {}
+    for path in glob.glob(os.path.join(build.HERE, "*.cu")):
+        with open(path) as f:
+            source = f.read()
+        for name, arguments in re.findall(r"AIR_API\s+int\s+(air_\w+)\(([^)]*)\)\s*{", source):
+            found[name] = ["pointer" if "*" in a or "cudaStream_t" in a else a.rsplit(None, 1)[0].replace("const ", "").strip()
+                           for a in arguments.split(",")]
+    for name, types in ops._SIGNATURES.items():
+        assert [kinds[t] for t in types] == found[name], name
+
+
+@pytest.mark.gpu
+def test_a_tensor_is_checked_as_in_python():
+    t = torch.zeros(3, 4, device="cuda")
+    fits = [((t, "t"), {}), ((t, "t", (torch.float32,)), {}), ((t, "t", (torch.bfloat16, torch.float32), (3, None)), {}),
+            ((t, "t", None, (3, 4)), {}), ((t, "t", None, t.shape), {}), ((t, "t"), {"shape": (3, 4)}),
+            ((t[:0], "t", None, (0, 4)), {}), ((t[0, 0], "t", None, ()), {}), ((torch.nn.Parameter(t), "t"), {})]
+    for args, names in fits:
+        assert ops._req(*args, **names) is args[0] and ops._why_not(*args, **names) is args[0]
+    for args, names in [((t.cpu(), "t"), {}), ((t.t(), "t"), {}), ((t, "t", (torch.int32,)), {}), ((t, "t", None, (3, 4, 1)), {}),
+                        ((t, "t", None, (4, 4)), {}), ((t, "t"), {"shape": (None, 5)}), ((None, "t"), {}), (([1.0], "t"), {})]:
+        said = []
+        for check in (ops._req, ops._why_not):
+            with pytest.raises(ops.KernelError) as e:
+                check(*args, **names)
+            said.append(str(e.value))
+        assert said[0] == said[1]
+
+
+@pytest.mark.gpu
+def test_new_tensors_and_launches():
+    dev = torch.device("cuda:0")
+    ops.empty(1, torch.float32, dev)
+    for shape in ((2, 3), (0, 5), (), 7, torch.Size((4,))):
+        a, b = ops.empty(shape, torch.bfloat16, dev), torch.empty(shape, dtype=torch.bfloat16, device=dev)
+        assert a.shape == b.shape and a.dtype == b.dtype and a.device == b.device and a.is_contiguous()
+    with pytest.raises(RuntimeError):
+        ops.empty((-1,), torch.float32, dev)
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        ops.empty((1 << 45,), torch.float32, dev)
+    f = build.entry().air_add_parts
+    for wrong in ((), (0,) * 5, (None, None, "x", 0, 0, None), (None, None, 0.5, 0, 0, None)):
+        with pytest.raises(TypeError):
+            f(*wrong)
+    # a launch on the stream that is current
+    h, d = torch.zeros(1, 1 << 20, device=dev), torch.ones(1, 1 << 20, device=dev)
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        ops.add_parts(h, d)
+    s.synchronize()
+    assert float(h.sum()) == 1 << 20
