@@ -75,7 +75,7 @@ __device__ __forceinline__ void ask_ahead(const Ahead& ahead, int lane) {
 }
 
 template <int D, bool BIAS>
-__global__ void __launch_bounds__(DT_THREADS, 2)
+__global__ void __launch_bounds__(DT_THREADS, D <= 128 ? 2 : 1)
 decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const FreshQkv fresh, const Ahead ahead,
                             const __nv_bfloat16* __restrict__ q,
                             const int* __restrict__ block_table, int max_blocks, const int* __restrict__ token_seq,
