@@ -21,6 +21,11 @@
 //                       stage): twice as many tiles, for matrices whose tiles of 256 leave more than half of the SMs idle.
 //                       The up half's warps hand their sums to the gate half's through shared memory
 //   EPI_RELU2           store max(C, 0)^2 as bfloat16 (the hidden layer of a feed-forward without a gate)
+//   EPI_F32, joined     matrices of few tiles, whose sums are wanted complete: a cluster of two or four blocks shares a tile, a part
+//                       of the k range each, and adds the parts up, in order, through one another's shared memory.  A block's
+//                       copies bring 65 GB/s whatever the tile, so 53 tiles leave half of the memory's rate unused:
+//                       8 rows by 6,720 x 4,096 (two blocks) 16.4 -> 13.5 us, by 4,096 x 4,096 (four) 15.2 -> 10.0, by 3,648 x
+//                       2,048 (four) 8.7 -> 6.7, 64 rows by 6,720 x 4,096 18.4 -> 15.6.  Tiles of 64 or 32 rows: 20 and 29.
 //   EPI_PARTIAL         the k range is split over `splits` blocks; each writes C[split][T][N] (float32)
 // Rows of X beyond T and rows of W beyond N are zero-filled by TMA.
 // Every wait on an mbarrier is bounded; on giving up the block sets *status = 4 (as gemm_tc.cu).
@@ -28,12 +33,15 @@
 #include "tma.cuh"
 #include "umma.cuh"
 
+#include <cooperative_groups.h>
+
 namespace air {
 
 constexpr int TS_BK = 64;
 constexpr int TS_THREADS = 192;
 
-enum { TS_F32 = 0, TS_BF16 = 1, TS_SILU = 2, TS_PARTIAL = 3, TS_RELU2 = 4 };   // as in gemm_tc.cu
+enum { TS_F32 = 0, TS_BF16 = 1, TS_SILU = 2, TS_PARTIAL = 3, TS_RELU2 = 4,   // as in gemm_tc.cu
+       TS_JOINED = 5 };
 
 struct TsArgs {
     void* out;          // F32/PARTIAL: float [splits][T][N]; BF16: bf16 [T][N]; SILU: bf16 [T][N/2]
@@ -81,6 +89,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
 gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                      const TsArgs args) {
     constexpr bool PAIRED = EPI == TS_SILU && HALVES == 1;      // 64 gate rows and 64 up rows to a tile
+    constexpr bool JOINED = EPI == TS_JOINED;                    // (a block is one part of one tile)
+    static_assert(!JOINED || HALVES == 1, "a cluster shares a tile of 128 rows");
     constexpr int HALF_W = 128 * TS_BK * 2;           // 16 KB: 128 rows of W, 64 of k
     constexpr int STAGE_W = HALVES * HALF_W;
     constexpr int STAGE_X = NT * TS_BK * 2;
@@ -246,7 +256,13 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             else if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
-            if constexpr (PAIRED) {
+            if constexpr (JOINED) {
+                float v[NT];
+                ts_load_row<NT>(taddr, v);
+                float* mine = (float*)smem;               // [NT][128]: every copy has landed and every product is done
+#pragma unroll
+                for (int t = 0; t < NT; ++t) mine[t * 128 + r] = v[t];
+            } else if constexpr (PAIRED) {
                 float v[NT];
                 if (ok) ts_load_row<NT>(taddr, v);
                 if (args.ss) {
@@ -336,6 +352,55 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         tc_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
+    if constexpr (JOINED) {
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        cluster.sync();
+        if (warp >= 2) {                                  // the parts in order; the tokens are shared out among the blocks
+            // (a warp takes a token's 128 features at once, a lane four of them)
+            const int col = (int)blockIdx.x / args.splits * TILE_N + 4 * lane;
+            const bool whole = args.N % 4 == 0;
+            const float* from[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) from[q] = cluster.map_shared_rank((float*)smem, q < args.splits ? q : 0) + 4 * lane;
+#pragma unroll 4
+            for (int t = (int)blockIdx.x % args.splits + args.splits * (warp & 3); t < args.T; t += 4 * args.splits) {
+                float v[4][4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (q < args.splits) load4(from[q] + t * 128, v[q]);
+                float* to = (float*)args.out + (size_t)t * args.N + col;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float sum = v[0][e] + v[1][e];
+                    if (args.splits == 4) sum = (sum + v[2][e]) + v[3][e];
+                    if (args.ss) sum *= row_scale[t];
+                    v[0][e] = sum;
+                    if (!whole && col + e < args.N) to[e] = sum;
+                }
+                if (whole && col < args.N) store4(to, v[0]);
+            }
+        }
+        cluster.sync();                                   // (nobody leaves while its memory is read)
+    }
+}
+
+// Blocks that share a tile of complete sums, by what a product takes, us: a block's copies (a step of k is 16 KB at 65 GB/s) or
+// the whole matrix at 6.5 TB/s, whichever is longer, and the exchange.  Every block has an SM to itself and eight steps of k or
+// more; clusters of four do not fit on all SMs (a cluster stands in one GPC).
+static int ts_joined_parts(int n_tiles, int k_tiles, int sms) {
+    int best = 1;
+    double least = 0.95 * max(k_tiles * 0.25, n_tiles * k_tiles * 0.0025);
+    for (int parts = 2; parts <= 4; parts *= 2) {
+        if (n_tiles * parts > (parts == 4 ? sms - sms / 8 : sms) || k_tiles < 8 * parts ||
+            (parts - 1) * ((k_tiles + parts - 1) / parts) >= k_tiles)
+            continue;
+        const double us = max(k_tiles * 0.25 / parts, n_tiles * k_tiles * 0.0025) + 3;
+        if (us < least) {
+            best = parts;
+            least = us;
+        }
+    }
+    return best;
 }
 
 // A tensor map of a row-major bf16 matrix [rows, cols] with boxes of box_rows x 64 and 128-byte swizzle.
@@ -354,6 +419,22 @@ static int ts_launch(const CUtensorMap& mw, const CUtensorMap& mx, const TsArgs&
     auto kernel = gemm_tc_small_kernel<NT, EPI, HALVES>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)request);
     if (e != cudaSuccess) return (int)e;
+    if constexpr (EPI == TS_JOINED) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(TS_THREADS);
+        cfg.dynamicSmemBytes = request;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = args.splits;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = pdl_enabled() ? 2 : 1;
+        return launch_counted(cfg, kernel, mw, mx, args);
+    }
     return launch(kernel, blocks, TS_THREADS, request, stream, mw, mx, args);
 }
 
@@ -361,6 +442,9 @@ template <int NT, int HALVES>
 static int ts_dispatch_epi(int epi, const CUtensorMap& mw, const CUtensorMap& mx, const TsArgs& args, int blocks,
                            cudaStream_t stream) {
     switch (epi) {
+        case TS_JOINED:
+            if constexpr (HALVES == 1) return ts_launch<NT, TS_JOINED, 1>(mw, mx, args, blocks, stream);
+            return AIR_ERR_BAD_ARGUMENT;
         case TS_F32: return ts_launch<NT, TS_F32, HALVES>(mw, mx, args, blocks, stream);
         case TS_BF16: return ts_launch<NT, TS_BF16, HALVES>(mw, mx, args, blocks, stream);
         case TS_SILU: return ts_launch<NT, TS_SILU, HALVES>(mw, mx, args, blocks, stream);
@@ -408,12 +492,20 @@ AIR_API int air_gemm_tc_small(const void* x, const void* w, void* out, int T, in
     // half tiles are no shorter than one of whole ones.
     const bool paired = epi == TS_SILU && N / 256 * 2 <= sms;
     if (paired) tile_rows = 128;
+    // (by the matrix alone, so that a row's sum does not depend on how many there are)
+    if (epi == TS_F32 && tile_rows == 128) {
+        const int parts = ts_joined_parts((N + 127) / 128, k_tiles, sms);
+        if (parts > 1) {
+            epi = TS_JOINED;
+            splits = parts;
+        }
+    }
     CUtensorMap mw, mx;
     int rc = ts_make_map(&mw, w, N, K, paired ? 64 : tile_rows);
     if (rc) return rc;
     rc = ts_make_map(&mx, x, T, K, nt);
     if (rc) return rc;
-    const long long tiles = (long long)((N + tile_rows - 1) / tile_rows) * splits;
+    const long long tiles = (long long)((N + tile_rows - 1) / tile_rows) * splits;     // (joined: at most one to a block)
     const int blocks = (int)(tiles < sms ? tiles : sms);
     if (ss && ss_tiles < 1) return AIR_ERR_BAD_ARGUMENT;
     TsArgs args{out, T, N, K, splits, status, ss, ss_tiles, eps, act_alpha, act_limit, act_shift};

@@ -183,3 +183,24 @@ def test_silu_epilogue_in_half_and_in_whole_tiles(tiles, M, scaled):
     z = z.view(M, tiles, 2, 128)
     want = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, I)
     assert (out.double() - want).abs().max() <= 0.005 * want.abs().max()
+
+
+@pytest.mark.parametrize("N,K", [(3648, 2048), (132, 2056), (256, 2104), (300, 8200), (6720, 4096), (5000, 2112)])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_complete_sums_by_clusters_along_k(N, K, scaled):
+    """Matrices of few tiles whose sums are wanted complete: two or four blocks share a tile.  Remainders of tiles and of k, every
+    width of tile of tokens, the scale per row; a row's bits do not depend on how many rows there are."""
+    o = ops()
+    a, w, want = inputs(64, N, K, N + K)
+    ss = torch.rand(3, 64, generator=torch.Generator().manual_seed(K)).cuda() * K
+    if scaled:
+        want = want * torch.rsqrt(ss.cpu().double().sum(0) / K + 1e-6)[:, None]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    kept = None
+    for T in (64, 33, 32, 17, 16, 7, 1):
+        out = torch.full((T, N), 9.0, device="cuda")
+        scale = dict(row_ss=ss[:, :T].contiguous(), eps=1e-6) if scaled else {}
+        o.gemm_tc(a[:T].contiguous(), w, out, 128, o.EPI_F32, status=status, **scale)
+        kept = out if kept is None else kept
+        assert close(out, want[:T], K) and torch.equal(out, kept[:T]), T
+    assert status.item() == 0
