@@ -26,8 +26,8 @@
 //                              operands to 2^-23: what is left out is of the order of 32-bit rounding.  The next chunk's
 //                              numbers arrive by the copy engine, in two runs of bytes, while this one's are used.
 //
-// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 197 (prepare
-// 49, scan 147); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 98 (24 and 73).  Which portions come here:
+// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 193 (prepare
+// 46, scan 147); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 98 (24 and 73).  Which portions come here:
 // parts/recurrent.py (least).
 //
 // Errors against 64 bits (2-norm of the difference over that of the result, 2,048 tokens), token by token and here: one decay per
@@ -83,8 +83,10 @@ struct DeltaChunkArgs {
 
 __device__ __forceinline__ float softplus_1(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 
+// (four blocks to an SM: a block is a chain of short phases between barriers.  With three 49.7 us for 128 chunks of 16 heads, 51.7 with
+// a decay per channel and 94 chunks; with four 45.7 and 48.5 for a few spilled registers; five 45.3 and 57.5)
 template <int DP, int MODE>
-__global__ void __launch_bounds__(256, DP <= 128 ? 3 : 2) delta_chunk_prepare_kernel(const DeltaChunkArgs p) {
+__global__ void __launch_bounds__(256, DP <= 128 ? 4 : 2) delta_chunk_prepare_kernel(const DeltaChunkArgs p) {
     constexpr int ld = DP + 4, PER = DP / 32;
     extern __shared__ __align__(16) float smem[];
     __shared__ __align__(16) float sa[DC][DC];
