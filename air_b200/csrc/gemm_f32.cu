@@ -10,7 +10,7 @@
 //   gemm_f32_tile_kernel   more rows: tiles of C in registers, a block for all ranges or a cluster with a block for each
 //   gemm_f32_kernel        rows that are not whole aligned 16-byte pieces, at any number of rows
 //
-// Measured, us, from memory, against tiles of 64 x 64 with scalar reads at every size: 4 rows by 4,608 x 3,584 281 -> 23, by
+// Measured, us, from memory, against tiles of 64 x 64 with scalar reads at every size (also at sizes that gemm_f32_tc.cu takes now): 4 rows by 4,608 x 3,584 281 -> 23, by
 // 37,888 x 3,584 631 -> 135 (4.0 TB/s), by 3,584 x 18,944 1,485 -> 74; 300 rows by 2,048 x 2,048 223 -> 83, by 16,384 x 2,048 886
 // -> 533 (38 TFLOP/s), by 2,048 x 8,192 870 -> 295; 2,048 rows by 16,384 x 2,048 5,368 -> 3,297 (42 TFLOP/s; the multiply-add
 // pipe alone gives 72).
