@@ -1,8 +1,9 @@
-"""Compiles the CUDA sources of this folder for sm_100a, and entry.cpp, into one shared library and loads it: an
-extension module whose functions are the launchers (entry), and through ctypes what else the library offers (library).  There is no fallback: without nvcc, or if a source does not compile, the
-import fails with the compiler's message.
+"""Compiles the CUDA sources of this folder for sm_100a into a shared library of C functions, which wants the CUDA runtime and
+nothing else and which any program may load, and entry.cpp into an extension module over it, whose functions are the launchers
+(entry); what else the library offers is called through ctypes (library).  There is no fallback: without nvcc, or if a source
+does not compile, the import fails with the compiler's message.
 
-The library is built at the first call that needs it, into ``_build/`` beside the sources
+Both are built at the first call that needs them, into ``_build/`` beside the sources
 (or into $AIR_B200_BUILD_DIR, or a per-user temporary folder if the package folder cannot
 be written).  A stamp of the sources' contents and the flags decides whether it is rebuilt.
 Each translation unit is compiled by its own nvcc process, a few at a time, and a line is
@@ -29,6 +30,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompil
               "--expt-relaxed-constexpr"]
 LIB_NAME = "libair_b200_kernels.so"
 ENTRY, ENTRY_MODULE = "entry.cpp", "air_b200_entry"
+ENTRY_NAME = ENTRY_MODULE + ".so"
 
 _lib = None
 _entry = None
@@ -53,13 +55,14 @@ def _entries() -> str:
 
 
 def _entry_flags():
-    """How entry.cpp is compiled and linked: against Python's headers and torch's."""
+    """How entry.cpp is compiled and linked: against Python's headers and torch's, and the library beside it."""
     import torch
     root = os.path.dirname(torch.__file__)
     compile_flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
                      "-I", sysconfig.get_paths()["include"], "-I", os.path.join(root, "include"),
                      "-I", os.path.join(root, "include", "torch", "csrc", "api", "include")]
-    return compile_flags, ["-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"], torch.__version__
+    libraries = ["-l:" + LIB_NAME, "-Wl,-rpath,$ORIGIN", "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
+    return compile_flags, libraries, torch.__version__
 
 
 def _nvcc() -> str:
@@ -77,8 +80,8 @@ def _stamp() -> str:
             h.update(f.encode() + b"\0" + fh.read())
     with open(os.path.join(HERE, ENTRY), "rb") as fh:
         h.update(fh.read())
-    flags, _, version = _entry_flags()
-    h.update(" ".join(ARCH_FLAGS + NVCC_FLAGS + flags + [version, sys.version]).encode() + _entries().encode())
+    flags, libraries, version = _entry_flags()
+    h.update(" ".join(ARCH_FLAGS + NVCC_FLAGS + flags + libraries + [version, sys.version]).encode() + _entries().encode())
     return h.hexdigest()
 
 
@@ -112,12 +115,12 @@ def _say(msg: str) -> None:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Builds the library if its stamp is stale; returns its path."""
+    """Builds the library and the module over it if their stamp is stale; returns the library's path."""
     out_dir = build_dir()
-    lib = os.path.join(out_dir, LIB_NAME)
+    lib, module = os.path.join(out_dir, LIB_NAME), os.path.join(out_dir, ENTRY_NAME)
     stamp_file = os.path.join(out_dir, "stamp.txt")
     stamp = _stamp()
-    if not force and os.path.exists(lib) and os.path.exists(stamp_file):
+    if not force and os.path.exists(lib) and os.path.exists(module) and os.path.exists(stamp_file):
         with open(stamp_file) as f:
             if f.read().strip() == stamp:
                 return lib
@@ -155,15 +158,18 @@ def build(force: bool = False, verbose: bool = False) -> str:
         _say(f"  c++ {ENTRY} done in {time.time() - t:.1f} s")
         return obj
 
+    def link(command, name, to):
+        tmp = to + f".tmp{os.getpid()}"
+        p = subprocess.run(command + ["-shared", "-o", tmp], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        if p.returncode != 0:
+            raise RuntimeError(f"air_b200: linking {name} failed:\n{p.stdout}")
+        os.replace(tmp, to)
+
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 2)) as pool:
         entry_obj = pool.submit(compile_entry)
-        objs = list(pool.map(compile_one, srcs)) + [entry_obj.result()]
-    tmp = lib + f".tmp{os.getpid()}"
-    p = subprocess.run([nvcc] + ARCH_FLAGS + ["-shared", "-o", tmp] + objs + ["-lcudart"] + libraries,
-                       stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
-    if p.returncode != 0:
-        raise RuntimeError(f"air_b200: linking {LIB_NAME} failed:\n{p.stdout}")
-    os.replace(tmp, lib)
+        objs = list(pool.map(compile_one, srcs))
+    link([nvcc] + ARCH_FLAGS + objs + ["-Xlinker", "-soname=" + LIB_NAME, "-lcudart"], LIB_NAME, lib)
+    link([os.environ.get("CXX", "g++"), entry_obj.result(), "-L" + out_dir] + libraries, ENTRY_NAME, module)
     with open(stamp_file, "w") as f:
         f.write(stamp + "\n")
     _say(f"built {LIB_NAME} in {time.time() - t0:.1f} s")
@@ -174,17 +180,18 @@ def library() -> ctypes.CDLL:
     """The loaded library (built first if needed)."""
     global _lib
     if _lib is None:
-        import torch  # noqa: F401  (the library is linked against it)
         _lib = ctypes.CDLL(build())
     return _lib
 
 
 def entry():
-    """The library as an extension module: a function per launcher (arguments as in ops._SIGNATURES; it returns the error code)."""
+    """The extension module over the library: a function per launcher (arguments as in ops._SIGNATURES; it returns the error code)."""
     global _entry
     if _entry is None:
-        loader = machinery.ExtensionFileLoader(ENTRY_MODULE, library()._name)
-        spec = util.spec_from_file_location(ENTRY_MODULE, library()._name, loader=loader)
+        import torch  # noqa: F401  (the module is linked against it)
+        path = os.path.join(os.path.dirname(library()._name), ENTRY_NAME)
+        loader = machinery.ExtensionFileLoader(ENTRY_MODULE, path)
+        spec = util.spec_from_file_location(ENTRY_MODULE, path, loader=loader)
         module = util.module_from_spec(spec)
         loader.exec_module(module)
         _entry = module

@@ -3,6 +3,7 @@ import ctypes
 import glob
 import os
 import re
+import subprocess
 
 import pytest
 import torch
@@ -21,6 +22,26 @@ def test_signatures_are_those_of_the_sources():
                            for a in arguments.split(",")]
     for name, types in ops._SIGNATURES.items():
         assert [kinds[t] for t in types] == found[name], name
+
+
+def test_the_library_is_one_of_c_functions(tmp_path):
+    """A program without Python and torch loads the library and calls a launcher (which refuses the arguments: no device is needed)."""
+    source, program = tmp_path / "host.c", str(tmp_path / "host")
+    source.write_text("""
+#include <dlfcn.h>
+#include <stdio.h>
+int main(int n, char** a) {
+    void* lib = dlopen(a[1], RTLD_NOW);
+    if (!lib) return puts(dlerror()), 2;
+    int (*f)(const float*, const float*, const float*, float*, int, int, int, int, void*) = dlsym(lib, "air_gemm_f32");
+    if (!f) return puts(dlerror()), 3;
+    printf("%d %d\\n", f(0, 0, 0, 0, 1, 1, -1, 0, 0), f(0, 0, 0, 0, 0, 1, 1, 0, 0));
+    return 0;
+}
+""")
+    subprocess.run(["gcc", str(source), "-o", program, "-ldl"], check=True)
+    done = subprocess.run([program, build.build()], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    assert (done.returncode, done.stdout.split()) == (0, ["100001", "0"]), done.stdout
 
 
 @pytest.mark.gpu
