@@ -404,6 +404,18 @@ AIR_API int air_decode_attention(const void* q, const void* cache, const int* bl
     }
 }
 
+// The merge of the splits alone, for partial results from elsewhere.
+AIR_API int air_decode_combine(const float* part_o, const float* part_ml, const int* token_seq, void* out, int T,
+                               int H, int D, int splits, cudaStream_t stream) {
+    using namespace air;
+    switch (D) {
+        case 64: return launch_combine<64>(part_o, part_ml, token_seq, (__nv_bfloat16*)out, T, H, splits, stream);
+        case 128: return launch_combine<128>(part_o, part_ml, token_seq, (__nv_bfloat16*)out, T, H, splits, stream);
+        case 256: return launch_combine<256>(part_o, part_ml, token_seq, (__nv_bfloat16*)out, T, H, splits, stream);
+        default: return AIR_ERR_BAD_ARGUMENT;
+    }
+}
+
 // The merge of what decode_attention_tma_kernel leaves (KeySplits; that kernel finishes a token whose keys are one split's).
 AIR_API int air_decode_combine_split(const float* part_o, const float* part_ml, const int* token_seq, void* out, int T, int H, int D,
                                      int splits, const int* positions, int window, int early, cudaStream_t stream) {

@@ -595,12 +595,12 @@ AIR_API int air_decode_attention_tma_sink(const void* q, const void* cache, long
 // are added in order), bias float32 or null, table float32 [positions][D] (cos | sin: all of a head is
 // rotated); write_kv = 0 where another run's layer has written this step's keys and values already.  ahead0, ahead1: memory of
 // bytes0 and bytes1 that the kernels behind read and none writes, or null (Ahead).
-AIR_API int air_decode_attention_tma_fresh(const float* qkv, int parts, const float* bias, const float* table,
-                                           int write_kv, void* cache, long long pages, const int* block_table,
-                                           int max_blocks, const int* token_seq, const int* positions, void* out,
-                                           float* part_o, float* part_ml, int T, int H, int K, int D, int P,
-                                           int window, float scale, int splits, int* status, const void* ahead0, long long bytes0,
-                                           const void* ahead1, long long bytes1, cudaStream_t stream) {
+AIR_API int air_decode_attention_tma_fresh_ahead(const float* qkv, int parts, const float* bias, const float* table,
+                                                 int write_kv, void* cache, long long pages, const int* block_table,
+                                                 int max_blocks, const int* token_seq, const int* positions, void* out,
+                                                 float* part_o, float* part_ml, int T, int H, int K, int D, int P,
+                                                 int window, float scale, int splits, int* status, const void* ahead0,
+                                                 long long bytes0, const void* ahead1, long long bytes1, cudaStream_t stream) {
     if (!qkv || !table || parts < 1 || ((uintptr_t)qkv & 15) || ((uintptr_t)bias & 15) || ((uintptr_t)table & 15))
         return AIR_ERR_BAD_ARGUMENT;
     const air::FreshQkv fresh{qkv, parts, (size_t)T * (size_t)(H + 2 * K) * (size_t)D, bias, table,
@@ -611,6 +611,15 @@ AIR_API int air_decode_attention_tma_fresh(const float* qkv, int parts, const fl
     return air::decode_attention_tma(fresh, nullptr, cache, pages, block_table, max_blocks, token_seq, positions, out,
                                      part_o, part_ml, T, H, K, D, P, window, scale, 0.f, splits, status, stream, nullptr, nullptr, 0,
                                      air::TurnBack{nullptr, 0, 0, nullptr}, air::DistanceBias{nullptr, 0}, 0, ahead);
+}
+AIR_API int air_decode_attention_tma_fresh(const float* qkv, int parts, const float* bias, const float* table,
+                                           int write_kv, void* cache, long long pages, const int* block_table,
+                                           int max_blocks, const int* token_seq, const int* positions, void* out,
+                                           float* part_o, float* part_ml, int T, int H, int K, int D, int P,
+                                           int window, float scale, int splits, int* status, cudaStream_t stream) {
+    return air_decode_attention_tma_fresh_ahead(qkv, parts, bias, table, write_kv, cache, pages, block_table, max_blocks, token_seq,
+                                                positions, out, part_o, part_ml, T, H, K, D, P, window, scale, splits, status,
+                                                nullptr, 0, nullptr, 0, stream);
 }
 
 AIR_API int air_trace_set_attention_decode_tma(unsigned long long* buffer) { return air::set_trace_here(buffer); }

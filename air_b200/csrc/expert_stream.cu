@@ -199,7 +199,7 @@ expert_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         // (EPI 0: the warps meet at a barrier, so all of them go through all tiles, also when a wait has run out)
         for (int i = blockIdx.x; i < total && (EPI == 0 || !*abort_flag); i += gridDim.x, ++it) {
             const Item x = item_of(i);
-            const int rows = min(args.tile_rows, __ldcg(args.start + x.group + 1) - x.slot0);      // (up to NT: see air_expert_stream)
+            const int rows = min(args.tile_rows, __ldcg(args.start + x.group + 1) - x.slot0);      // (up to NT: see air_expert_stream_tiles)
             const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
             if constexpr (EPI == 0) {
                 // (worked out by a thread per slot while the products run, not row by row in the loop below)
@@ -296,10 +296,11 @@ static int xs_dispatch(int epi, const CUtensorMap& mw, const CUtensorMap& mx, co
 // moe_sort_kernel leaves them (tile_rows slots to a tile, 64 or 128); no expert has more than most_rows slots.  epi, out: see above (epi 1: N a
 // multiple of 256).  lists_ready: the kernel launched right before this one is an expert_stream_kernel that was given the
 // same lists without it.
-AIR_API int air_expert_stream(const void* x, int slots, const void* w, int groups, int N, int K, const int* start,
-                              const int* tiles, const int* num_tiles, int max_tiles, int tile_rows, int most_rows, int epi, void* out, int splits,
-                              const int* o_index, int o_div, long long o_part_stride, int ldo, const float* o_scale, float alpha,
-                              float limit, float shift, int lists_ready, int* status, cudaStream_t stream) {
+AIR_API int air_expert_stream_tiles(const void* x, int slots, const void* w, int groups, int N, int K, const int* start,
+                                    const int* tiles, const int* num_tiles, int max_tiles, int tile_rows, int most_rows, int epi,
+                                    void* out, int splits, const int* o_index, int o_div, long long o_part_stride, int ldo,
+                                    const float* o_scale, float alpha, float limit, float shift, int lists_ready, int* status,
+                                    cudaStream_t stream) {
     using namespace air;
     if (slots <= 0 || N <= 0 || groups <= 0 || max_tiles <= 0) return 0;
     if (K <= 0 || K % 8 || epi < 0 || epi > 2 || splits < 1 || (splits > 1 && epi) || (epi == 1 && N % 256) || !start || !tiles ||
@@ -325,6 +326,14 @@ AIR_API int air_expert_stream(const void* x, int slots, const void* w, int group
     if (nt == 32) return xs_dispatch<32>(epi, mw, mx, args, blocks, stream);
     if (nt == 64) return xs_dispatch<64>(epi, mw, mx, args, blocks, stream);
     return xs_dispatch<XS_WIDE>(epi, mw, mx, args, blocks, stream);
+}
+// The same with 64 slots to a tile.
+AIR_API int air_expert_stream(const void* x, int slots, const void* w, int groups, int N, int K, const int* start,
+                              const int* tiles, const int* num_tiles, int max_tiles, int most_rows, int epi, void* out, int splits,
+                              const int* o_index, int o_div, long long o_part_stride, int ldo, const float* o_scale, float alpha,
+                              float limit, float shift, int lists_ready, int* status, cudaStream_t stream) {
+    return air_expert_stream_tiles(x, slots, w, groups, N, K, start, tiles, num_tiles, max_tiles, air::XS_ROWS, most_rows, epi, out,
+                                   splits, o_index, o_div, o_part_stride, ldo, o_scale, alpha, limit, shift, lists_ready, status, stream);
 }
 
 AIR_API int air_trace_set_expert_stream(unsigned long long* buffer) { return air::set_trace_here(buffer); }

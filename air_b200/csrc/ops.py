@@ -81,7 +81,7 @@ _SIGNATURES = {
                          c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_int,
                          c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float,
                          c_float, c_float, c_void_p],
-    "air_expert_stream": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+    "air_expert_stream_tiles": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                           c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_void_p, c_float, c_float, c_float, c_int,
                           c_void_p, c_void_p],
     "air_rows_by_index": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p],
@@ -122,7 +122,7 @@ _SIGNATURES = {
                                       c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
                                       c_int, c_void_p],
     "air_head_gate": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
-    "air_decode_attention_tma_fresh": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_int,
+    "air_decode_attention_tma_fresh_ahead": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_int,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                        c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong,
                                        c_void_p],
@@ -1060,7 +1060,7 @@ def expert_stream(rows, w, out, start, tiles, num_tiles, most_rows, *, silu_mul=
         plane, ldo = out.shape[1] * N, N
     if o_scale is not None:
         _req(o_scale, "o_scale", (torch.float32,))
-    _check(_get("air_expert_stream")(
+    _check(_get("air_expert_stream_tiles")(
         rows.data_ptr(), slots, w.data_ptr(), groups, N, K, start.data_ptr(), tiles.data_ptr(), num_tiles.data_ptr(),
         tiles.shape[0], int(tile_rows), int(most_rows), 1 if silu_mul else 2 if relu2 else 0, out.data_ptr(), int(splits), _ptr(o_index),
         int(o_div), plane, ldo, _ptr(o_scale), float(act[0]), float(act[1]), float(act[2]), 1 if lists_ready else 0,
@@ -1645,7 +1645,7 @@ def decode_attention_fresh(qkv, bias, table, cache, block_table, token_seq, posi
         asked += [w.data_ptr(), n]
         left -= n
     asked += [None, 0] * (2 - len(asked) // 2)
-    _check(_get("air_decode_attention_tma_fresh")(
+    _check(_get("air_decode_attention_tma_fresh_ahead")(
         qkv.data_ptr(), parts, _ptr(bias), table.data_ptr(), 1 if write_kv else 0, cache.data_ptr(), cache.shape[0],
         block_table.data_ptr(), block_table.shape[1], token_seq.data_ptr(), positions.data_ptr(), out.data_ptr(),
         _ptr(po), _ptr(pm), T, H, K, d, P, int(window or 0), float(scale), splits, _ptr(status),

@@ -11,8 +11,8 @@ import torch
 from air_b200.csrc import build, ops
 
 
-def test_signatures_are_those_of_the_sources():
-    kinds = {ctypes.c_void_p: "pointer", ctypes.c_int: "int", ctypes.c_longlong: "long long", ctypes.c_float: "float"}
+def prototypes():
+    """The kinds of the arguments of every launcher, by its name."""
     found = {}
     for path in glob.glob(os.path.join(build.HERE, "*.cu")):
         with open(path) as f:
@@ -20,8 +20,44 @@ def test_signatures_are_those_of_the_sources():
         for name, arguments in re.findall(r"AIR_API\s+int\s+(air_\w+)\(([^)]*)\)\s*{", source):
             found[name] = ["pointer" if "*" in a or "cudaStream_t" in a else a.rsplit(None, 1)[0].replace("const ", "").strip()
                            for a in arguments.split(",")]
+    return found
+
+
+def test_signatures_are_those_of_the_sources():
+    kinds = {ctypes.c_void_p: "pointer", ctypes.c_int: "int", ctypes.c_longlong: "long long", ctypes.c_float: "float"}
+    found = prototypes()
     for name, types in ops._SIGNATURES.items():
         assert [kinds[t] for t in types] == found[name], name
+
+
+def test_functions_that_c_programs_call_keep_their_arguments():
+    """Functions with more arguments stand beside the ones that were there, under names of their own."""
+    p, i, l, f = "pointer", "int", "long long", "float"
+    were = {"air_decode_combine": [p, p, p, p, i, i, i, i, p],
+            "air_decode_attention_tma_fresh": [p, i, p, p, i, p, l, p, i, p, p, p, p, p, i, i, i, i, i, i, f, i, p, p],
+            "air_expert_stream": [p, i, p, i, i, i, p, p, p, i, i, i, p, i, p, i, l, i, p, f, f, f, i, p, p]}
+    found, lib = prototypes(), build.library()
+    for name, arguments in were.items():
+        assert found[name] == arguments and hasattr(lib, name), name
+    assert lib.air_decode_combine(None, None, None, None, 1, 1, 7, 2, None) == 100001
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,splits", [(64, 1), (128, 7), (256, 32)])
+def test_the_merge_alone(D, splits):
+    """air_decode_combine against the same merge in 64 bits; a padding token's row stays as it is."""
+    T, H = 3, 5
+    g = torch.Generator().manual_seed(D)
+    o, m, n = torch.randn(T, H, splits, D, generator=g), torch.randn(T, H, splits, generator=g) * 4, torch.rand(T, H, splits, generator=g) + 1
+    ml, slots = torch.stack([m, n], dim=-1).cuda(), torch.tensor([0, -1, 4], dtype=torch.int32, device="cuda")
+    out, parts = torch.full((T, H, D), 7.0, dtype=torch.bfloat16, device="cuda"), o.cuda()
+    f = build.library().air_decode_combine
+    f.argtypes = [ctypes.c_void_p] * 4 + [ctypes.c_int] * 4 + [ctypes.c_void_p]
+    assert f(parts.data_ptr(), ml.data_ptr(), slots.data_ptr(), out.data_ptr(), T, H, D, splits, torch.cuda.current_stream().cuda_stream) == 0
+    w = torch.exp2(m.double() - m.double().amax(-1, keepdim=True))
+    want = (o.double() * w[..., None]).sum(2) / (n.double() * w).sum(-1)[..., None]
+    got = out.cpu().double()
+    assert (got[1] == 7).all() and ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5)[[0, 2]].all()
 
 
 def test_the_library_is_one_of_c_functions(tmp_path):
