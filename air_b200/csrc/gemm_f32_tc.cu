@@ -10,8 +10,8 @@
 // The sum of an element is the same whatever M is and wherever its row stands, as in gemm_f32.cu; which of the two files
 // takes a product depends on the matrix W alone.
 //
-// A result that is not finite (an infinity or NaN among the operands, or a number that rounds to infinity as bfloat16) is
-// worked out again by multiply-adds from memory, so that such operands give what they always gave.
+// A result that is not finite (an infinity among the operands, or a number that rounds to infinity as bfloat16) is worked out
+// again by multiply-adds from memory, in the order of gemm_f32.cu, so that such operands give what they give there.
 //
 //   split_rows_kernel      for more than eight rows: A -> planes of bfloat16 [3][M][Kp], Kp = K up to a multiple of 64
 //   gemm_f32_tc_kernel     one block, or a cluster of four or eight blocks that share out the eighths of k, per tile of 128
@@ -136,22 +136,111 @@ __device__ __forceinline__ void ft_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                  : "memory");
 }
 
-// A result that is not finite, by multiply-adds from memory.
-__device__ __noinline__ void ft_again(const float* x, const float* w, const float* bias, float* c, int K) {
-    if (isfinite(*c)) return;
-    float sum = 0.f;
-    for (int k = 0; k < K && !isnan(sum); ++k) sum = fmaf(x[k], w[k], sum);
-    *c = bias ? sum + *bias : sum;
+// The results of rows m_lo .. m_hi - 1 and columns n0 .. n0 + 127 that are not finite, by multiply-adds from memory in the order of
+// gemm_f32.cu, by all threads of the block: R rows at a time (few where registers are few), a thread half of them by one column,
+// both operands through a ring of stages of 32 k in shared memory.  A row of A with a NaN is left as it is (its results are NaN).
+// 300 rows by 16,384 x 2,048, us: no such results 155, NaN in every row 198, an infinity in one row 460, in every row 2,350 (gemm_f32.cu
+// 532 in all cases); 8 rows 34, 36, 134, 135 (47).  Result after result by the thread that had it: 155, 70,700, 548, 70,100.
+constexpr int FT_AGAIN_K = 32, FT_AGAIN_LD = FT_AGAIN_K + 4, FT_AGAIN_STAGES = 3;
+__host__ __device__ constexpr int ft_again_rows(int nt) { return nt <= 32 ? 16 : 32; }
+__host__ __device__ constexpr int ft_again_stage(int r) { return (r + FT_BM) * FT_AGAIN_LD; }        // in numbers
+__host__ __device__ constexpr int ft_again_bytes(int nt) {
+    return (FT_AGAIN_STAGES * ft_again_stage(ft_again_rows(nt)) + ft_again_rows(nt)) * 4;
+}
+
+template <int BYTES> __device__ __forceinline__ void ft_copy(float* to, const float* from, bool in) {
+    const int bytes = in ? BYTES : 0;                // (0: zeros, nothing is read)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(smem_u32(to)), "l"(from), "n"(BYTES), "r"(bytes) : "memory");
+}
+
+template <int R>
+__device__ __noinline__ void ft_again(const FtArgs& args, int m_lo, int m_hi, int n0, float* smem) {
+    constexpr int LD = FT_AGAIN_LD, PARTS = 4, STAGES = FT_AGAIN_STAGES, STAGE = ft_again_stage(R);
+    const float *const A = args.a, *const W = args.w;
+    const int K = args.K, N = args.N, Kp = ((K + PARTS - 1) / PARTS + 15) / 16 * 16, steps_per_part = (Kp + FT_AGAIN_K - 1) / FT_AGAIN_K;
+    const int tid = threadIdx.x, lane = tid & 31, col = tid & (FT_BM - 1), row0 = tid / FT_BM * (R / 2);
+    int* nan_row = (int*)(smem + STAGES * STAGE);
+    for (int m = m_lo; m < m_hi; m += R) {
+        const int rows = min(R, m_hi - m), mine = min(R / 2, rows - row0);
+        for (int i = tid >> 5; i < rows; i += blockDim.x >> 5) {
+            bool none = false;
+            for (int k = lane; k < K; k += 32) none |= isnan(A[(size_t)(m + i) * K + k]);
+            none = __any_sync(0xffffffffu, none);
+            if (lane == 0) nan_row[i] = none;
+        }
+        __syncthreads();
+        unsigned wrong = 0;
+        if (n0 + col < N)
+            for (int i = 0; i < mine; ++i)
+                if (!nan_row[row0 + i] && !isfinite(args.c[(size_t)(m + row0 + i) * N + n0 + col])) wrong |= 1u << i;
+        if (!__syncthreads_or(wrong)) continue;
+        // step s: 32 k of part s / steps_per_part; zeros beyond the part and beyond the rows and columns
+        const int steps = (K + Kp - 1) / Kp * steps_per_part;
+        auto bring = [&](int s) {
+            float* to = smem + s % STAGES * STAGE;
+            const int part = s / steps_per_part, k0 = part * Kp + s % steps_per_part * FT_AGAIN_K, k_hi = min(K, (part + 1) * Kp);
+            for (int j = tid; j < R * FT_AGAIN_K; j += blockDim.x) {
+                const int r = j / FT_AGAIN_K, k = j % FT_AGAIN_K;
+                const bool in = s < steps && r < rows && k0 + k < k_hi;
+                ft_copy<4>(to + r * LD + k, in ? A + (size_t)(m + r) * K + k0 + k : A, in);
+            }
+            for (int j = tid; j < FT_BM * FT_AGAIN_K / 4; j += blockDim.x) {
+                const int r = j / (FT_AGAIN_K / 4), k = j % (FT_AGAIN_K / 4) * 4;
+                const bool in = s < steps && n0 + r < N && k0 + k < k_hi;       // (K % 4 == 0)
+                ft_copy<16>(to + (R + r) * LD + k, in ? W + (size_t)(n0 + r) * K + k0 + k : W, in);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        for (int s = 0; s < STAGES - 1; ++s) bring(s);
+        float sum[R / 2], acc[R / 2];
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) acc[i] = sum[i] = 0.f;
+        for (int s = 0; s < steps; ++s) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+            __syncthreads();
+            bring(s + STAGES - 1);
+            const float* at = smem + s % STAGES * STAGE;
+            auto multiply = [&](auto whole) {
+#pragma unroll 1
+                for (int k = 0; k < FT_AGAIN_K; k += 4) {
+                    float w[4], x[4];
+                    load4(at + (R + col) * LD + k, w);
+#pragma unroll
+                    for (int i = 0; i < R / 2; ++i) {
+                        if (!decltype(whole)::value && i >= mine) break;
+                        load4(at + (row0 + i) * LD + k, x);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[i] = fmaf(x[e], w[e], acc[i]);
+                    }
+                }
+            };
+            if (mine == R / 2) multiply(std::true_type());      // (reads that need not wait for a row's count)
+            else if (mine > 0) multiply(std::false_type());
+            if ((s + 1) % steps_per_part == 0) {
+#pragma unroll
+                for (int i = 0; i < R / 2; ++i) {
+                    sum[i] = s >= steps_per_part ? sum[i] + acc[i] : acc[i];
+                    acc[i] = 0.f;
+                }
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i)
+            if (wrong >> i & 1) args.c[(size_t)(m + row0 + i) * N + n0 + col] = args.bias ? sum[i] + args.bias[n0 + col] : sum[i];
+        __syncthreads();
+    }
 }
 
 template <int NT>
 __global__ void __launch_bounds__(FT_THREADS, NT <= 32 ? 2 : 1)
-gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const FtArgs args) {
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ FtArgs args) {
     constexpr int WS = ft_w_stages(NT), XS = ft_x_stages(NT), XSTAGE = ft_x_stage(NT), XPLANE = XSTAGE / 3, HALF = NT / 2;
     constexpr int TMEM_COLS = ft_tmem_cols(NT);
     constexpr bool DONE_IN_SMEM = ft_done_in_smem(NT);
     static_assert(NT % 16 == 0 && 2 * FT_A_COLS + 2 * NT <= 512, "two sets of accumulators beside two buffers of planes");
     static_assert(WS >= 3 && WS * FT_BOX + XS * XSTAGE >= NT * FT_BM * 4 * 2, "the stages' memory takes a tile's sums twice");
+    static_assert(WS * FT_BOX + XS * XSTAGE >= ft_again_bytes(NT), "and what ft_again stages");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sw = smem;
@@ -401,10 +490,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const float* const bias = args.bias;
     const int M = args.M, N = args.N;
     bool odd = false;                                // a result that is not finite was stored
-    auto again = [&](int m, int n) {
-        if (m < M && n < N)
-            ft_again(args.a + (size_t)m * args.K, args.w + (size_t)n * args.K, bias ? bias + n : nullptr, C + (size_t)m * N + n, args.K);
-    };
     auto done_at = [&](int i) -> float {
         if constexpr (DONE_IN_SMEM) return done_smem[i * FT_WORKERS];
         else return done[i];
@@ -424,9 +509,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     to[(size_t)i * N] = sum;
                 }
             }
-            if (odd)
-                for (int i = 0; i < HALF; ++i) again(m1 + i, n0 + r);
         }
+        if (__syncthreads_or(odd)) ft_again<ft_again_rows(NT)>(args, m0, min(M, m0 + NT), n0, (float*)smem);
         return;
     }
     // A block of several hands on the sum of its eighths if it is the first, else (two of them) one and the other.
@@ -476,15 +560,15 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 }
             }
             if (whole) store4(to, v[0]);
-            if (odd)
-                for (int e = 0; e < 4; ++e) again(m, n + e);
         }
     };
     if (warp < 8 && !gave_up) {
         if (args.cluster == FT_PARTS) add_up(std::integral_constant<int, FT_PARTS>());
         else add_up(std::integral_constant<int, 4>());
     }
-    cluster.sync();                                  // (nobody leaves while its memory is read)
+    cluster.sync();                                  // (nobody's memory is read any more)
+    const int m1 = m0 + rank * (NT / args.cluster);
+    if (__syncthreads_or(odd)) ft_again<ft_again_rows(NT)>(args, m1, min(M, m1 + NT / args.cluster), n0, (float*)smem);
 }
 
 // A tensor map of a row-major float32 matrix [rows, cols] with boxes of 128 rows x 32 numbers and the 128-byte swizzle.

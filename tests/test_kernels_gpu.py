@@ -364,6 +364,35 @@ def test_gemm_f32_on_the_tensor_cores_with_infinities_nan_and_the_largest_number
     assert torch.equal(out.cpu()[rows][:, cols], clean.cpu()[rows][:, cols])
 
 
+@pytest.mark.parametrize("M,shape", [(1, (0, 0)), (5, (16, 1)), (20, (0, 0)), (20, (32, 4)), (45, (64, 8)), (200, (0, 0)), (130, (112, 8)), (130, (96, 1)),
+                                     (261, (128, 1))])
+def test_gemm_f32_on_the_tensor_cores_works_out_again_in_the_order_of_the_multiply_adds(M, shape):
+    """Finite sums of numbers that are infinite as bfloat16 have gemm_f32.cu's bits, every one of them and in every shape of the
+    kernel; a NaN elsewhere in the batch changes nothing for the other rows."""
+    from air_b200.csrc import build
+    N, K = 1157, 2072
+    g = torch.Generator().manual_seed(M)
+    a, w, b = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g) * 0.02, torch.randn(N, generator=g)
+    big = torch.rand(M, generator=g) < 0.5
+    big[0] = True
+    at = torch.randint(0, K, (M,), generator=g)
+    a[big, at[big]] = float(np.finfo(np.float32).max)
+    w = torch.where(torch.rand(N, K, generator=g) < 0.5, w, torch.zeros(())) * 1e-3
+    if M > 3:
+        a[3, K - 1] = math.nan
+    x, w, b = dev(a), dev(w), dev(b)
+    out, want = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    ops().gemm_f32(x, w, b, out, shape=shape)
+    assert build.entry().air_gemm_f32(x.data_ptr(), w.data_ptr(), b.data_ptr(), want.data_ptr(), M, N, K, 0,
+                                      torch.cuda.current_stream().cuda_stream) == 0
+    rows = torch.tensor([m for m in range(M) if big[m] and m != 3], device="cuda")
+    assert torch.isfinite(want[rows]).all() and torch.equal(out[rows], want[rows])
+    if M > 3:
+        assert torch.isnan(out[3]).all()
+    rest = torch.tensor([m for m in range(M) if not big[m] and m != 3], dtype=torch.long, device="cuda")
+    assert ((out[rest] - want[rest]).abs() <= 1e-6).all()
+
+
 @pytest.mark.parametrize("M", [1, 4, 16])
 def test_gemm_f32_with_a_matrix_that_the_launches_ahead_write(M):
     """Both operands come from the package's own kernels right ahead, over and over with new numbers: a matrix that is not a
