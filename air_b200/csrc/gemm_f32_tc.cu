@@ -1,17 +1,19 @@
 // 32-bit matrix product on the fifth-generation tensor cores: C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]), float32 in and out.
 //
-// Nothing is computed at a lower precision than by fused multiply-adds: a float32 number is cut into three bfloat16 numbers
-// that add up to it exactly (x = x1 + x2 + x3, each the rest rounded to nearest: 3 x 8 bits hold the 24), a product of two
-// bfloat16 numbers is exact in 32 bits, and of the nine products per pair the six down to 2^-17 of the largest are taken
-// (the others together are below 2^-25 of it, without a bias).  The tensor cores add up 64 numbers of k, the small products
-// first; every such sum is then added to a 32-bit total in registers, in ascending order over an eighth of k, and the eighths'
-// totals are added in ascending order.  So the chain of roundings is K/512 additions of sums of 64 where the multiply-add
-// kernels (gemm_f32.cu) have K/4 additions of one product.
+// Nothing is computed at a lower precision than by fused multiply-adds: a float32 number, times 2^24, is cut into three bfloat16
+// numbers that add up to it exactly (x = x1 + x2 + x3, each the rest rounded to nearest: 3 x 8 bits hold the 24, and the factor
+// keeps the last of them within bfloat16's range down to the smallest number that 32 bits hold; without it bits were lost below
+// 2^-110), a product of two bfloat16 numbers is exact in 32 bits, and of the nine products per pair the six down to 2^-17 of the
+// largest are taken (the others together are below 2^-24 of it, without a bias).  The tensor cores add up 64 numbers of k, the small
+// products first; every such sum is then added to a 32-bit total in registers, in ascending order over an eighth of k, and the
+// eighths' totals are added in ascending order; their sum is multiplied by 2^-48.  So the chain of roundings is K/512 additions of
+// sums of 64 where the multiply-add kernels (gemm_f32.cu) have K/4 additions of one product.
 // The sum of an element is the same whatever M is and wherever its row stands, as in gemm_f32.cu; which of the two files
 // takes a product depends on the matrix W alone.
 //
-// A result that is not finite (an infinity among the operands, or a number that rounds to infinity as bfloat16) is worked out
-// again by multiply-adds from memory, in the order of gemm_f32.cu, so that such operands give what they give there.
+// A result that is not finite (an infinity among the operands, a number from 2^104 or a sum from 2^80 on, which the factors take
+// out of range) is worked out again by multiply-adds from memory, in the order of gemm_f32.cu, so that such operands give what they
+// give there.
 //
 //   split_rows_kernel      for more than eight rows: A -> planes of bfloat16 [3][M][Kp], Kp = K up to a multiple of 64
 //   gemm_f32_tc_kernel     one block, or a cluster of four or eight blocks that share out the eighths of k, per tile of 128
@@ -85,8 +87,12 @@ __device__ __forceinline__ void ft_less(float& x, float& y, uint32_t p) {
     asm("{\n\t.reg .b16 l, h, m;\n\tmov.b16 m, 0xBF80;\n\tmov.b32 {l, h}, %2;\n\tfma.rn.f32.bf16 %0, l, m, %0;\n\tfma.rn.f32.bf16 %1, h, m, %1;\n\t}"
         : "+f"(x), "+f"(y) : "r"(p));
 }
-// Two neighbouring numbers as three pairs of bfloat16, the first in the low half.
+// Two neighbouring numbers times FT_SCALE as three pairs of bfloat16, the first in the low half.  (The factor costs 300 rows by
+// 16,384 x 2,048 138.5 -> 140.8 us, few rows nothing; as two multiplications one row lost 2 % as well.)
+constexpr float FT_SCALE = 0x1p24f, FT_UNSCALE = 0x1p-48f;      // (of a number, of a product of two)
 __device__ __forceinline__ void ft_split(float x, float y, uint32_t (&p)[3]) {
+    asm("{\n\t.reg .b64 v, f;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 f, {%2, %2};\n\tmul.rn.f32x2 v, v, f;\n\tmov.b64 {%0, %1}, v;\n\t}"
+        : "+f"(x), "+f"(y) : "f"(FT_SCALE));
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const __nv_bfloat162 b = __floats2bfloat162_rn(x, y);
@@ -502,7 +508,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             float* to = C + (size_t)m1 * N + n0 + r;
 #pragma unroll
             for (int i = 0; i < HALF; ++i) {
-                float sum = several ? done_at(i) + total[i] : total[i];
+                float sum = (several ? done_at(i) + total[i] : total[i]) * FT_UNSCALE;
                 if (bias) sum += b;
                 if (i < rows) {
                     odd |= !isfinite(sum);
@@ -552,6 +558,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 float sum = v[0][e];
 #pragma unroll
                 for (int q = 1; q < VALUES; ++q) sum += v[q][e];
+                sum *= FT_UNSCALE;
                 if (n + e < N) {
                     if (bias) sum += bias[n + e];
                     odd |= !isfinite(sum);

@@ -364,6 +364,27 @@ def test_gemm_f32_on_the_tensor_cores_with_infinities_nan_and_the_largest_number
     assert torch.equal(out.cpu()[rows][:, cols], clean.cpu()[rows][:, cols])
 
 
+@pytest.mark.parametrize("M", [2, 12, 70, 300])
+@pytest.mark.parametrize("small,large", [(1e-36, 1.0), (1e-40, 1e6), (3e-45, 1e10), (1e-19, 1e-19), (1e-37, 1e37), (1e-30, 1e30)])
+def test_gemm_f32_on_the_tensor_cores_with_small_numbers(M, small, large):
+    """Numbers down to the smallest that 32 bits hold, in the rows or in the matrix, keep their 24 bits (or what they have of them):
+    the bound is that of the additions (as above), and half of the smallest number for a result that is as small.  Beside numbers of
+    1e37 the multiply-adds work the results out: K/4 roundings in a row, each of half a unit at most and of either sign."""
+    N, K = 1040, 2176
+    g = torch.Generator(device="cuda").manual_seed(M)
+    for a_size, w_size in ((small, large), (large, small)):
+        a = (torch.randn(M, K, generator=g, device="cuda").double() * a_size).float()
+        w = (torch.randn(N, K, generator=g, device="cuda").double() * w_size).float()
+        out = torch.empty(M, N, device="cuda")
+        ops().gemm_f32(a, w, None, out)
+        want = a.double() @ w.double().T
+        bound = (K / 512 + 8 + 2 * 24 + 1) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T) + 2.0 ** -149
+        assert ((out.double() - want).abs() <= bound).all()
+        rms = ((out.double() - want).norm() / want.norm()).item()
+        limit = 2e-7 if large <= 1e30 else 2.0 ** -25 * (K / 4) ** 0.5
+        assert rms <= limit + 2.0 ** -149 / want.abs().mean().item(), rms
+
+
 @pytest.mark.parametrize("M,shape", [(1, (0, 0)), (5, (16, 1)), (20, (0, 0)), (20, (32, 4)), (45, (64, 8)), (200, (0, 0)), (130, (112, 8)), (130, (96, 1)),
                                      (261, (128, 1))])
 def test_gemm_f32_on_the_tensor_cores_works_out_again_in_the_order_of_the_multiply_adds(M, shape):
