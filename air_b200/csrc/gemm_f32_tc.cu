@@ -16,21 +16,22 @@
 // give there.
 //
 //   split_rows_kernel      for more than eight rows: A -> planes of bfloat16 [3][M][Kp], Kp = K up to a multiple of 64
-//   gemm_f32_tc_kernel     one block, or a cluster of four or eight blocks that share out the eighths of k, per tile of 128
-//                          rows of W by NT rows of A; 384
-//                          threads a block:
+//   gemm_f32_tc_kernel     one block, or several that share out the eighths of k, per tile of 128 rows of W by NT rows of A: a cluster of
+//                          four or eight, or (up to eight rows) two, four or eight that leave the eighths' totals in memory;
+//                          384 threads a block:
 //     warps 0-7   the 128 rows of W (float32, brought by TMA in boxes of 32 k) are cut into planes by the thread that owns
 //                 the row and put into tensor memory as the M side of the product, 64 k at a time, two buffers; the same
 //                 threads add the finished sums to their totals (warps 0-3 one half of k and of the columns, 4-7 the other);
 //     warps 8, 10 issue the copies of W (ahead of the end of the launch before this one where it is a model's weight) and A
 //                 (up to eight rows: warps 10 and 11 cut them themselves);
 //     warp 9      issues tcgen05.mma, A from tensor memory, B (the planes of the rows of A) from shared memory.
+//   ft_add_kernel          adds up the totals that are in memory
 // The planes of W stay out of shared memory, which for few rows would be the bound: 32 KB of W would be written, read,
 // written as 48 KB and read six times.
 // Measured, us a product in a chain of products with different matrices, by gemm_f32.cu and here: 4 rows by 37,888 x 3,584 122
-// and 83 (6.5 TB/s: bound by the bytes of W), by 3,584 x 18,944 69 and 49, by 3,584 x 3,584 15.7 and 14.0, by 4,608 x 3,584 16.2 and
-// 20 (36 tiles: 36 clusters of eight do not fit at a time); one row by 2,048 x 2,048 6.9 and 8.3, by 16,384 x 2,048 30 and 32;
-// 16 rows by 37,888 x 3,584 230 and 86; 64 rows by 16,384 x 2,048 122 and 33; 300 rows by 2,048 x 2,048 81 and 41, by 16,384 x 2,048
+// and 83 (6.5 TB/s: bound by the bytes of W), by 3,584 x 18,944 69 and 48, by 3,584 x 3,584 15.6 and 13.1, by 4,608 x 3,584 16.4 and
+// 14.9, by 16,384 x 2,048 40 and 26.5; one row by 16,384 x 2,048 30 and 25.8, by 2,048 x 8,192 18.8 and 16.5, by 2,048 x 2,048 6.2 and 6.9;
+// 16 rows by 37,888 x 3,584 230 and 86; 64 rows by 16,384 x 2,048 122 and 33; 300 rows by 2,048 x 2,048 81 and 33, by 16,384 x 2,048
 // 529 and 144 (140 TFLOP/s of float32 products, 840 of bfloat16 ones: the tensor pipe, three rounds of 2.6 full), by 37,888 x
 // 3,584 2,034 and 445.  Errors against 64 bits (2-norm), normal numbers: k 2,048 2.7e-7 and 7.4e-8, k 18,944 1.2e-6 and 1.8e-7;
 // numbers of one sign (truncation inside the tensor cores adds up) 1.7e-7 and 9.1e-8, 4.7e-7 and 1.1e-7.
@@ -59,8 +60,9 @@ struct FtArgs {
     const float* bias;
     float* c;
     int M, N, K, w_ready;
-    int cluster;        // blocks that share a tile: 1, 4 or 8
+    int cluster;        // blocks that share a tile: 1, 4 or 8 (a cluster), or 2, 4 or 8 that leave their sums in memory (APART)
     int* status;
+    float* sums;        // APART: [FT_PARTS][M][N], the eighths' totals, for ft_add_kernel
 };
 
 // Up to 32 rows of A two blocks share an SM; up to FT_CUT rows a warp of the block cuts them into planes itself.  The sum of the eighths that are done is kept in registers where there is room
@@ -147,12 +149,11 @@ __device__ __forceinline__ void ft_ld8(uint32_t taddr, uint32_t (&r)[8]) {
 // both operands through a ring of stages of 32 k in shared memory.  A row of A with a NaN is left as it is (its results are NaN).
 // 300 rows by 16,384 x 2,048, us: no such results 155, NaN in every row 198, an infinity in one row 460, in every row 2,350 (gemm_f32.cu
 // 532 in all cases); 8 rows 34, 36, 134, 135 (47).  Result after result by the thread that had it: 155, 70,700, 548, 70,100.
-constexpr int FT_AGAIN_K = 32, FT_AGAIN_LD = FT_AGAIN_K + 4, FT_AGAIN_STAGES = 3;
+constexpr int FT_AGAIN_K = 32, FT_AGAIN_LD = FT_AGAIN_K + 4;
 __host__ __device__ constexpr int ft_again_rows(int nt) { return nt <= 32 ? 16 : 32; }
+__host__ __device__ constexpr int ft_again_stages(int r) { return r <= 16 ? 2 : 3; }
 __host__ __device__ constexpr int ft_again_stage(int r) { return (r + FT_BM) * FT_AGAIN_LD; }        // in numbers
-__host__ __device__ constexpr int ft_again_bytes(int nt) {
-    return (FT_AGAIN_STAGES * ft_again_stage(ft_again_rows(nt)) + ft_again_rows(nt)) * 4;
-}
+__host__ __device__ constexpr int ft_again_numbers(int r) { return ft_again_stages(r) * ft_again_stage(r) + r; }
 
 template <int BYTES> __device__ __forceinline__ void ft_copy(float* to, const float* from, bool in) {
     const int bytes = in ? BYTES : 0;                // (0: zeros, nothing is read)
@@ -161,7 +162,7 @@ template <int BYTES> __device__ __forceinline__ void ft_copy(float* to, const fl
 
 template <int R>
 __device__ __noinline__ void ft_again(const FtArgs& args, int m_lo, int m_hi, int n0, float* smem) {
-    constexpr int LD = FT_AGAIN_LD, PARTS = 4, STAGES = FT_AGAIN_STAGES, STAGE = ft_again_stage(R);
+    constexpr int LD = FT_AGAIN_LD, PARTS = 4, STAGES = ft_again_stages(R), STAGE = ft_again_stage(R);
     const float *const A = args.a, *const W = args.w;
     const int K = args.K, N = args.N, Kp = ((K + PARTS - 1) / PARTS + 15) / 16 * 16, steps_per_part = (Kp + FT_AGAIN_K - 1) / FT_AGAIN_K;
     const int tid = threadIdx.x, lane = tid & 31, col = tid & (FT_BM - 1), row0 = tid / FT_BM * (R / 2);
@@ -238,7 +239,11 @@ __device__ __noinline__ void ft_again(const FtArgs& args, int m_lo, int m_hi, in
     }
 }
 
-template <int NT>
+// APART: the blocks of a tile leave every eighth's totals in memory and ft_add_kernel adds them up: up to FT_CUT rows, where the totals
+// are few.  Such blocks need not stand in one GPC, and the SMs take one each before any takes two, which a cluster's do not wait for:
+// 4 rows by 4,608 x 3,584 19.3 -> 15.3 us, by 2,048 x 8,192 21.0 -> 17.1, by 16,384 x 2,048 (two blocks) 32.2 -> 27.1; of 9 rows and
+// more the second launch and the totals cost what that saves.
+template <int NT, bool APART>
 __global__ void __launch_bounds__(FT_THREADS, NT <= 32 ? 2 : 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ FtArgs args) {
     constexpr int WS = ft_w_stages(NT), XS = ft_x_stages(NT), XSTAGE = ft_x_stage(NT), XPLANE = XSTAGE / 3, HALF = NT / 2;
@@ -246,7 +251,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     constexpr bool DONE_IN_SMEM = ft_done_in_smem(NT);
     static_assert(NT % 16 == 0 && 2 * FT_A_COLS + 2 * NT <= 512, "two sets of accumulators beside two buffers of planes");
     static_assert(WS >= 3 && WS * FT_BOX + XS * XSTAGE >= NT * FT_BM * 4 * 2, "the stages' memory takes a tile's sums twice");
-    static_assert(WS * FT_BOX + XS * XSTAGE >= ft_again_bytes(NT), "and what ft_again stages");
+    static_assert(WS * FT_BOX + XS * XSTAGE >= ft_again_numbers(ft_again_rows(NT)) * 4, "and what ft_again stages");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sw = smem;
@@ -289,10 +294,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    float total[HALF], done[DONE_IN_SMEM ? 1 : HALF];
+    float total[HALF], done[DONE_IN_SMEM || APART ? 1 : HALF];
 #pragma unroll
     for (int i = 0; i < HALF; ++i) total[i] = 0.f;
-    if constexpr (!DONE_IN_SMEM)
+    if constexpr (!DONE_IN_SMEM && !APART)
 #pragma unroll
         for (int i = 0; i < HALF; ++i) done[i] = 0.f;
     const int quarter = warp & 3, half = warp >> 2, r = quarter * 32 + lane;   // (workers: a row of W, half of k and of the columns)
@@ -314,7 +319,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
         }
     } else if (warp >= 10) {
-        if (NT == 16 && args.M <= FT_CUT) {
+        if (NT == 16 && (APART || args.M <= FT_CUT)) {
             // ------------------------------------------------ the rows of A, cut here: two warps take the
             // chunks in turn, 16 lanes a row's 64 k
             pdl_wait();
@@ -427,7 +432,19 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 }
             }
             tc_fence_before();
-            if (--left == 0 && c + 1 < chunks) {     // (the last eighth stays in total)
+            if constexpr (APART) {
+                if (--left > 0 && c + 1 < chunks) return true;
+                if (first_part) pdl_wait();          // (the memory may be what the predecessor reads)
+                const int m1 = m0 + half * HALF, rows = n0 + r < args.N ? args.M - m1 : 0;
+                float* to = args.sums + ((size_t)(rank * (FT_PARTS / args.cluster) + c / chunks_per_part) * args.M + m1) * args.N + n0 + r;
+#pragma unroll
+                for (int i = 0; i < HALF; ++i) {
+                    if (i < rows) to[(size_t)i * args.N] = total[i];
+                    total[i] = 0.f;
+                }
+                left = chunks_per_part;
+                first_part = false;
+            } else if (--left == 0 && c + 1 < chunks) {     // (the last eighth stays in total)
 #pragma unroll
                 for (int i = 0; i < HALF; ++i) {
                     if constexpr (DONE_IN_SMEM) done_smem[i * FT_WORKERS] = first_part ? total[i] : done_smem[i * FT_WORKERS] + total[i];
@@ -492,6 +509,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
 
     // ---------------------------------------------------------- the eighths' totals
+    if constexpr (APART) return;                     // (they are in memory)
+    else {
     float* const C = args.c;
     const float* const bias = args.bias;
     const int M = args.M, N = args.N;
@@ -576,6 +595,47 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     cluster.sync();                                  // (nobody's memory is read any more)
     const int m1 = m0 + rank * (NT / args.cluster);
     if (__syncthreads_or(odd)) ft_again<ft_again_rows(NT)>(args, m1, min(M, m1 + NT / args.cluster), n0, (float*)smem);
+    }
+}
+
+// The eighths' totals of up to FT_CUT rows: 128 columns to a block, a thread four columns of a row.
+__global__ void __launch_bounds__(256) ft_add_kernel(const __grid_constant__ FtArgs args) {
+    __shared__ __align__(16) float smem[ft_again_numbers(16)];
+    pdl_enter(TR_GEMM_F32);
+    const int M = args.M, N = args.N, n0 = blockIdx.x * FT_BM, n = n0 + (threadIdx.x & 31) * 4, m = threadIdx.x >> 5;
+    const int part = ft_part(args.K), parts = (args.K + part - 1) / part;
+    const size_t eighth = (size_t)M * N;
+    const bool whole = N % 4 == 0 && ((uintptr_t)args.c & 15) == 0;
+    bool odd = false;
+    if (m < M && n < N) {
+        const float* from = args.sums + (size_t)m * N + n;
+        float* to = args.c + (size_t)m * N + n;
+        float v[FT_PARTS][4];
+#pragma unroll
+        for (int p = 0; p < FT_PARTS; ++p) {
+            if (p >= parts) continue;
+            if (N % 4 == 0) load4(from + p * eighth, v[p]);
+            else
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[p][e] = n + e < N ? from[p * eighth + e] : 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float sum = v[0][e];
+#pragma unroll
+            for (int p = 1; p < FT_PARTS; ++p)
+                if (p < parts) sum += v[p][e];
+            sum *= FT_UNSCALE;
+            if (n + e < N) {
+                if (args.bias) sum += args.bias[n + e];
+                odd |= !isfinite(sum);
+                if (!whole) to[e] = sum;
+            }
+            v[0][e] = sum;
+        }
+        if (whole) store4(to, v[0]);
+    }
+    if (__syncthreads_or(odd)) ft_again<16>(args, 0, M, n0, smem);
 }
 
 // A tensor map of a row-major float32 matrix [rows, cols] with boxes of 128 rows x 32 numbers and the 128-byte swizzle.
@@ -591,13 +651,17 @@ static int ft_map_w(CUtensorMap* map, const float* base, long long rows, long lo
     return r == CUDA_SUCCESS ? 0 : 200000 + (int)r;
 }
 
-template <int NT>
+template <int NT, bool APART = false>
 static int ft_launch(const CUtensorMap& mw, const CUtensorMap& mx, const FtArgs& args, cudaStream_t stream) {
-    auto kernel = gemm_f32_tc_kernel<NT>;
+    auto kernel = gemm_f32_tc_kernel<NT, APART>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ft_smem(NT));
     if (e != cudaSuccess) return (int)e;
     const unsigned blocks = (unsigned)((args.N + FT_BM - 1) / FT_BM) * ((args.M + NT - 1) / NT) * args.cluster;
     if (args.cluster == 1) return launch(kernel, blocks, FT_THREADS, ft_smem(NT), stream, mw, mx, args);
+    if constexpr (APART) {
+        const int rc = launch(kernel, blocks, FT_THREADS, ft_smem(NT), stream, mw, mx, args);
+        return rc ? rc : launch(ft_add_kernel, (args.N + FT_BM - 1) / FT_BM, 32 * FT_CUT, 0, stream, args);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(FT_THREADS);
@@ -617,46 +681,78 @@ static int ft_launch(const CUtensorMap& mw, const CUtensorMap& mx, const FtArgs&
 // Width of a tile and blocks that share it, by what they were measured to take, us: a chunk of 64 k (with all SMs at work; tensor
 // pipe, power and L2 at widths of 96 and more, the cutting of W below), and the way into and out of a block.  A grid of more
 // blocks than fit takes another round; a cluster wants its SMs in one GPC, so that fewer blocks fit.  W itself arrives at 6.3 TB/s.
-struct FtShape { int width, cluster; };
+struct FtShape { int width, cluster, apart; };
+// Up to FT_CUT rows: `blocks` blocks of `chunks` chunks.  A block that has an SM to itself takes 0.8 us a chunk, two on one 1.15,
+// and 6.3 TB/s are 0.0052 a block.  Measured in a chain of products of one row and here, us: 4,096 x 2,048 8 blocks apart 9.0 (9.3); 2,048 x 8,192
+// 16.4 (16.8); 4,608 x 3,584 14.5 (14.5); 16,384 x 2,048 one block to a tile 32.6, two apart 25.9 (25.3); 37,888 x 3,584 82 (89), 87 (93).
+// Clusters of eight: their blocks stand two to an SM from some 74 on, and 232 fit.  They are taken where each has its SM (1,024
+// x 2,048 5.6 against 5.8 apart), and where they fill the chip, so that there is nothing to spread (a layer of width 3,584 with one
+// request, the output product's 224 blocks 176 against 183, its whole; 2 to 8 requests +-1); between (2,048 x 2,048, 128) a whole
+// layer of width 2,048 took 83 us with them and 81 apart.
+static double ft_few_us(long long blocks, int chunks, bool clustered, bool apart) {
+    if (clustered && blocks > 74 && (blocks < 200 || blocks > 232)) return 1e30;
+    auto chunk = [&](long long n) { return n <= 0 ? 0. : max(n <= (clustered ? 74 : 148) ? 0.8 : 1.15, n * 0.0052); };
+    return chunks * (blocks / 296 * chunk(296) + chunk(blocks % 296)) + (blocks - 1) / 296 * 3 + (clustered ? 2 : apart ? 4 : 3);
+}
 static FtShape ft_shape(int M, int N, int K) {
     static const struct { int width; float chunk; } widths[] = {{16, 0.6f}, {32, 0.62f}, {64, 0.75f}, {96, 1.15f}, {112, 1.27f}, {128, 1.35f}};
     const int clusters[] = {1, 4, FT_PARTS};
-    FtShape best{0, 0};
+    FtShape best{0, 0, 0};
     double least = 0;
+    auto take = [&](const FtShape& shape, double us) {
+        if (best.width && us >= least) return;
+        best = shape;
+        least = us;
+    };
+    auto chunks_of = [&](int cl) { return min((K + FT_BK - 1) / FT_BK, ft_part(K) / FT_BK * (FT_PARTS / cl)); };
+    if (M <= FT_CUT) {
+        const long long tiles = ((long long)N + FT_BM - 1) / FT_BM;
+        take({16, 1, 0}, ft_few_us(tiles, chunks_of(1), false, false));
+        take({16, FT_PARTS, 0}, ft_few_us(tiles * FT_PARTS, chunks_of(FT_PARTS), true, false));
+        for (int cl = 2; cl <= FT_PARTS; cl *= 2) take({16, cl, 1}, ft_few_us(tiles * cl, chunks_of(cl), false, true));
+        return best;
+    }
     for (const auto& w : widths) {
         if (w.width <= 64 && w.width < M) continue;          // (narrow tiles only where one holds all rows)
         const bool two = w.width <= 32;
         for (int cl : clusters) {
             const long long blocks = ((long long)N + FT_BM - 1) / FT_BM * ((M + w.width - 1) / w.width) * cl;
             const int fit = cl == 1 ? (two ? 296 : 148) : cl == 4 ? (two ? 280 : 140) : (two ? 232 : 112);
-            const int chunks = min((K + FT_BK - 1) / FT_BK, ft_part(K) / FT_BK * (FT_PARTS / cl));
-            double us = (double)((blocks + fit - 1) / fit) * (chunks * w.chunk + (two ? (cl == 1 ? 5 : 6) : (cl == 1 ? 9 : 8)));
-            us = max(us, 4.0 * N * K / 6.3e6 + 5);
-            if (best.width == 0 || us < least) {
-                best = FtShape{w.width, cl};
-                least = us;
-            }
+            const double us = (double)((blocks + fit - 1) / fit) * (chunks_of(cl) * w.chunk + (two ? (cl == 1 ? 5 : 6) : (cl == 1 ? 9 : 8)));
+            take({w.width, cl, 0}, max(us, 4.0 * N * K / 6.3e6 + 5));
         }
         if (w.width <= 64) break;                            // (the narrowest that holds all rows)
     }
     return best;
 }
+static FtShape ft_shape_or(int M, int N, int K, int width, int cluster, int apart) {
+    return width && cluster ? FtShape{width, cluster, apart} : ft_shape(M, N, K);
+}
 
 }  // namespace air
 
-// planes: scratch of 3 * M * (K up to a multiple of 64) bfloat16; null up to FT_CUT rows.  W aligned to 16 bytes, K % 4 == 0.
-// w_ready as in air_gemm_f32.  width, cluster: rows of A to a tile (16, 32, 64, 96, 112 or 128) and blocks that share a tile (1, 4 or
-// 8), for tests and measurements; 0: by ft_shape.
-AIR_API int air_gemm_f32_tc(const float* A, const float* W, const float* bias, float* C, void* planes, int M, int N, int K, int w_ready,
-                            int width, int cluster, int* status, cudaStream_t stream) {
+// How many eighths' totals of M * N numbers air_gemm_f32_tc_apart wants room for: 8 or none.
+AIR_API int air_gemm_f32_tc_parts(int M, int N, int K, int width, int cluster, int apart) {
+    using namespace air;
+    return M > 0 && N > 0 && K > 0 && ft_shape_or(M, N, K, width, cluster, apart).apart ? FT_PARTS : 0;
+}
+
+// planes: scratch of 3 * M * (K up to a multiple of 64) bfloat16; null up to FT_CUT rows.  sums: scratch of
+// air_gemm_f32_tc_parts * M * N numbers.  W aligned to 16 bytes, K % 4 == 0.
+// w_ready as in air_gemm_f32.  width, cluster, apart: rows of A to a tile (16, 32, 64, 96, 112 or 128), blocks that share a tile (1, 4
+// or 8), and whether these (2, 4 or 8, for up to FT_CUT rows in tiles of 16) leave their sums in memory, for tests and measurements; 0: by
+// ft_shape.
+AIR_API int air_gemm_f32_tc_apart(const float* A, const float* W, const float* bias, float* C, void* planes, float* sums, int M, int N,
+                                  int K, int w_ready, int width, int cluster, int apart, int* status, cudaStream_t stream) {
     using namespace air;
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 4 || ((uintptr_t)W & 15)) return AIR_ERR_BAD_ARGUMENT;
-    const FtShape shape = width && cluster ? FtShape{width, cluster} : ft_shape(M, N, K);
+    const FtShape shape = ft_shape_or(M, N, K, width, cluster, apart);
     width = shape.width;
     cluster = shape.cluster;
-    if (width < 16 || (cluster != 1 && cluster != 4 && cluster != FT_PARTS)) return AIR_ERR_BAD_ARGUMENT;
     const bool cut = M <= FT_CUT && width == 16;
+    if (width < 16 || (cluster != 1 && cluster != 4 && cluster != FT_PARTS && !(cluster == 2 && shape.apart))) return AIR_ERR_BAD_ARGUMENT;
+    if (shape.apart && (!cut || cluster == 1 || !sums || ((uintptr_t)sums & 15))) return AIR_ERR_BAD_ARGUMENT;
     if (!cut && (!planes || ((uintptr_t)planes & 15))) return AIR_ERR_BAD_ARGUMENT;
     const int Kp = (K + FT_BK - 1) / FT_BK * FT_BK;
     const long long blocks = ((long long)M * Kp / 4 + 255) / 256, rows = 3ll * M;
@@ -672,7 +768,8 @@ AIR_API int air_gemm_f32_tc(const float* A, const float* W, const float* bias, f
         if (!rc) rc = tensor_map_2d(&mx, planes, rows, Kp, width);
         if (rc) return rc;
     }
-    const FtArgs args{A, W, bias, C, M, N, K, w_ready, cluster, status};
+    const FtArgs args{A, W, bias, C, M, N, K, w_ready, cluster, status, sums};
+    if (shape.apart) return ft_launch<16, true>(mw, mx, args, stream);
     switch (width) {
         case 16: return ft_launch<16>(mw, mx, args, stream);
         case 32: return ft_launch<32>(mw, mx, args, stream);
@@ -682,6 +779,17 @@ AIR_API int air_gemm_f32_tc(const float* A, const float* W, const float* bias, f
         case 128: return ft_launch<128>(mw, mx, args, stream);
         default: return AIR_ERR_BAD_ARGUMENT;
     }
+}
+
+// The same without that room.
+AIR_API int air_gemm_f32_tc(const float* A, const float* W, const float* bias, float* C, void* planes, int M, int N, int K, int w_ready,
+                            int width, int cluster, int* status, cudaStream_t stream) {
+    using namespace air;
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0) return AIR_ERR_BAD_ARGUMENT;
+    const FtShape shape = ft_shape_or(M, N, K, width, cluster, 0);
+    return air_gemm_f32_tc_apart(A, W, bias, C, planes, nullptr, M, N, K, w_ready, shape.width, shape.apart ? FT_PARTS : shape.cluster, 0,
+                                 status, stream);
 }
 
 AIR_API int air_trace_set_gemm_f32_tc(unsigned long long* buffer) { return air::set_trace_here(buffer); }

@@ -32,7 +32,8 @@ _SIGNATURES = {
     "air_silu_mul": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "air_convert": [c_void_p, c_int, c_void_p, c_int, c_longlong, c_void_p],
     "air_gemm_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
-    "air_gemm_f32_tc": [c_void_p] * 5 + [c_int] * 6 + [c_void_p, c_void_p],
+    "air_gemm_f32_tc_apart": [c_void_p] * 6 + [c_int] * 7 + [c_void_p, c_void_p],
+    "air_gemm_f32_tc_parts": [c_int] * 6,
     "air_paged_attention_ref": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p,
                                 c_int, c_void_p, c_int, c_void_p],
@@ -435,7 +436,10 @@ def convert(src, out):
 def f32_on_tensor_cores(w) -> bool:
     """Whether a product with the float32 matrix w goes to the tensor cores (gemm_f32_tc.cu): by the matrix alone, so that a
     row's result does not depend on how many rows there are.  Below these sizes a product of a row or two is latency (1,024 x
-    1,024: 3.8 us by multiply-adds, 5.7 there; 4,096 x 1,024: 4.9 and 8.1; 1,024 x 4,096: 9.8 and 9.8)."""
+    1,024: 3.8 us by multiply-adds, 5.7 there; 4,096 x 1,024: 4.9 and 8.1).  Above them one product loses, that of one single row by
+    a matrix of a few thousand outputs (2,048 x 2,048: 6.2 and 6.9; 4,096 x 2,048: 7.7 and 8.9; 4,608 x 3,584: 12.8 and 14.4), for the sake of
+    the bits that the row has among others; a layer's four products of one row gain (width 2,048: the layer 87 -> 82 us, 3,584:
+    203 -> 176), and two rows gain in each (2,048 x 2,048: 9 and 6.8)."""
     N, K = w.shape
     return K % 4 == 0 and K >= 2048 and N >= 1024 and w.data_ptr() % 16 == 0
 
@@ -443,11 +447,12 @@ def f32_on_tensor_cores(w) -> bool:
 F32_CUT_ROWS = 8      # up to so many rows the product's own blocks cut the rows into planes
 
 
-def gemm_f32(a, w, bias, out, w_ready=False, status=None, shape=(0, 0)):
+def gemm_f32(a, w, bias, out, w_ready=False, status=None, shape=(0, 0, 0)):
     """out[M, N] = a[M, K] @ w[N, K]^T + bias, all float32: large matrices on the tensor cores with every number as three
     bfloat16 numbers that add up to it, others by multiply-adds.  w_ready: w was complete before the launch ahead
     of this one was made (a model's weights), so that it may be read while that one still runs.  status [1] int32: 4 where a wait
-    inside the kernel ran out.  shape: a tile's rows of a and the blocks that share a tile, for tests (0, 0: the kernel's own choice)."""
+    inside the kernel ran out.  shape: a tile's rows of a, the blocks that share a tile, and whether these leave their sums in
+    memory (up to F32_CUT_ROWS rows), for tests (zeros: the kernel's own choice)."""
     M, K = a.shape
     N = w.shape[0]
     _req(a, "a", (torch.float32,))
@@ -457,9 +462,13 @@ def gemm_f32(a, w, bias, out, w_ready=False, status=None, shape=(0, 0)):
     _req(out, "out", (torch.float32,), (M, N))
     if f32_on_tensor_cores(w):
         planes = None if M <= F32_CUT_ROWS else empty((3, M, -(-K // 64) * 64), torch.bfloat16, a.device)
-        width, cluster = shape
-        _check(_get("air_gemm_f32_tc")(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), _ptr(planes), M, N, K,
-                                       1 if w_ready else 0, width, cluster, _ptr(status), _stream()), "gemm_f32")
+        width, cluster, apart = (*shape, 0)[:3]
+        parts = _get("air_gemm_f32_tc_parts")(M, N, K, width, cluster, apart) if M <= F32_CUT_ROWS else 0
+        sums = empty((parts, M, N), torch.float32, a.device) if parts else None
+        _check(_get("air_gemm_f32_tc_apart")(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), _ptr(planes), _ptr(sums), M, N, K,
+                                             1 if w_ready else 0, width, cluster, apart, _ptr(status), _stream()), "gemm_f32")
+        global launches
+        launches += (planes is not None) + (sums is not None)
         return out
     _check(_get("air_gemm_f32")(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K,
                               1 if w_ready else 0, _stream()), "gemm_f32")

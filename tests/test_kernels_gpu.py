@@ -339,6 +339,32 @@ def test_gemm_f32_on_the_tensor_cores(N, K):
     assert status.item() == 0
 
 
+@pytest.mark.parametrize("N,K", [(1024, 2048), (1031, 2052), (1100, 3076), (2050, 4160), (4608, 3584), (16384, 2048)])
+def test_gemm_f32_on_the_tensor_cores_with_the_sums_of_a_tiles_blocks_in_memory(N, K):
+    """Up to eight rows: two, four or eight blocks to a tile that leave the eighths' totals in memory give the bits of one block, and
+    write none of the rows and columns beyond; eighths of k without numbers are not read."""
+    from air_b200.csrc import ops as o
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    w, b = torch.randn(N, K, generator=g, device="cuda") * 0.02, torch.randn(N, generator=g, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for M in (1, 2, 5, 8):
+        a, shifted = torch.randn(M, K, generator=g, device="cuda"), torch.empty(M * K + 1, device="cuda")[1:].view(M, K)
+        one = torch.empty(M, N, device="cuda")
+        o.gemm_f32(a, w, b, one, status=status, shape=(16, 1))
+        for blocks in (2, 4, 8):
+            out = torch.full((M + 1, N), 7.0, device="cuda")
+            junk = torch.full((8, M, N), math.nan, device="cuda")      # (what the totals' memory holds before)
+            del junk
+            o.gemm_f32(a, w, b, out[:M], status=status, shape=(16, blocks, 1))
+            assert torch.equal(out[:M], one) and (out[M] == 7).all(), (M, blocks)
+            o.gemm_f32(shifted.copy_(a), w, None, out[:M], w_ready=True, status=status, shape=(16, blocks, 1))
+            assert ((out[:M] + b - one).abs() <= 2.0 ** -22 * (one.abs() + b.abs() + 1)).all()
+        chosen = torch.empty(M, N, device="cuda")
+        o.gemm_f32(a, w, b, chosen, status=status)
+        assert torch.equal(chosen, one), M
+    assert status.item() == 0
+
+
 @pytest.mark.parametrize("M", [3, 20, 200])
 def test_gemm_f32_on_the_tensor_cores_with_infinities_nan_and_the_largest_numbers(M):
     """What multiply-adds give: infinities, NaN and finite sums of numbers that are infinite as bfloat16; other rows and columns
@@ -385,7 +411,7 @@ def test_gemm_f32_on_the_tensor_cores_with_small_numbers(M, small, large):
         assert rms <= limit + 2.0 ** -149 / want.abs().mean().item(), rms
 
 
-@pytest.mark.parametrize("M,shape", [(1, (0, 0)), (5, (16, 1)), (20, (0, 0)), (20, (32, 4)), (45, (64, 8)), (200, (0, 0)), (130, (112, 8)), (130, (96, 1)),
+@pytest.mark.parametrize("M,shape", [(1, (0, 0)), (5, (16, 1)), (5, (16, 4, 1)), (8, (16, 8, 1)), (20, (0, 0)), (20, (32, 4)), (45, (64, 8)), (200, (0, 0)), (130, (112, 8)), (130, (96, 1)),
                                      (261, (128, 1))])
 def test_gemm_f32_on_the_tensor_cores_works_out_again_in_the_order_of_the_multiply_adds(M, shape):
     """Finite sums of numbers that are infinite as bfloat16 have gemm_f32.cu's bits, every one of them and in every shape of the
