@@ -411,6 +411,59 @@ def test_gemm_f32_on_the_tensor_cores_with_small_numbers(M, small, large):
         assert rms <= limit + 2.0 ** -149 / want.abs().mean().item(), rms
 
 
+def bfloat16_planes(x):
+    """Three numbers of bfloat16 that add up to float32 x, in 64 bits."""
+    first = x.bfloat16().float()
+    second = (x - first).bfloat16().float()
+    return [p.double() for p in (first, second, x - first - second)]
+
+
+SIX = [(0, 0), (0, 1), (1, 0), (1, 1), (0, 2), (2, 0)]      # (plane of the row, plane of the matrix) that the kernel multiplies
+
+
+@pytest.mark.parametrize("M,shape", [(512, (0, 0)), (512, (96, 4)), (512, (112, 1)), (64, (0, 0)), (32, (0, 0)), (16, (16, 8)), (8, (0, 0)), (8, (16, 1)),
+                                     (8, (16, 2, 1))])
+def test_gemm_f32_on_the_tensor_cores_takes_all_six_products(M, shape):
+    """Rows with a single number each, at every k of a chunk and in every eighth: a result is one product, of which the three
+    products that are left out are 2^-24 and the last addition, truncated in the tensor cores, 2^-23.  Without any one of the six
+    products the largest error here is above four times that."""
+    N, K, bound = 1024, 2048, 1.5 * 2.0 ** -23
+    g = torch.Generator(device="cuda").manual_seed(M)
+    w, b = torch.randn(N, K, generator=g, device="cuda"), torch.zeros(N, device="cuda")
+    for first in range(0, 512, M):
+        m = torch.arange(first, first + M, device="cuda")
+        at = m // 64 * (K // 8) + m // 64 % 4 * 64 + m % 64
+        a = torch.zeros(M, K, device="cuda")
+        a[torch.arange(M), at] = torch.randn(M, generator=g, device="cuda")
+        out = torch.empty(M, N, device="cuda")
+        ops().gemm_f32(a, w, b, out, shape=shape)
+        want = a.double() @ w.double().T
+        assert ((out.double() - want).abs() <= bound * want.abs()).all(), first
+    x, y = a.gather(1, at[:, None]), w.T[at]
+    xs, ys = bfloat16_planes(x), bfloat16_planes(y)
+    for left_out in SIX:
+        rest = sum(xs[i] * ys[j] for i, j in SIX if (i, j) != left_out)
+        assert ((rest - want).abs() / want.abs()).max() > 4 * bound, left_out
+    assert ((sum(xs[i] * ys[j] for i, j in SIX) - want).abs() <= 2.0 ** -24 * want.abs()).all()
+
+
+@pytest.mark.parametrize("M", [1, 8, 16, 64, 300])
+@pytest.mark.parametrize("K,limit", [(2048, 1.2e-7), (18944, 2.4e-7)])
+def test_gemm_f32_on_the_tensor_cores_errs_less_than_the_multiply_adds(M, K, limit):
+    """The 2-norm of the error on normal numbers (7.4e-8 and 1.8e-7 where the kernel was measured).  Without any one of the six
+    products it would be above twice the limit."""
+    N = 1024
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    a, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    out, want = torch.empty(M, N, device="cuda"), a.double() @ w.double().T
+    ops().gemm_f32(a, w, None, out)
+    assert ((out.double() - want).norm() / want.norm()).item() < limit
+    xs, ys = bfloat16_planes(a), bfloat16_planes(w)
+    for left_out in SIX:
+        rest = sum(xs[i] @ ys[j].T for i, j in SIX if (i, j) != left_out)
+        assert ((rest - want).norm() / want.norm()).item() > 2 * limit, left_out
+
+
 @pytest.mark.parametrize("M,shape", [(1, (0, 0)), (5, (16, 1)), (5, (16, 4, 1)), (8, (16, 8, 1)), (20, (0, 0)), (20, (32, 4)), (45, (64, 8)), (200, (0, 0)), (130, (112, 8)), (130, (96, 1)),
                                      (261, (128, 1))])
 def test_gemm_f32_on_the_tensor_cores_works_out_again_in_the_order_of_the_multiply_adds(M, shape):
