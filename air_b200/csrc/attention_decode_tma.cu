@@ -60,7 +60,8 @@ struct FreshQkv {
 // merge, the output product and the norm, and those blocks ask for their share of these ranges into L2.
 // Short requests for L2 only: beyond some 24 MB nothing was gained (the products behind take what L2 and an SM's copies
 // deliver, 8.7 TB/s over all SMs, wherever the weights lie) and the next layer's were delayed.  A step of one token, 8
-// layers of width 2,048, us: nothing asked 361.6, 8 MB 359.6, 20 MB 348.4, 40 MB 351.4, 60 MB 355.5, 100 MB 369.0.
+// layers of width 2,048, us: nothing asked 361.6, 8 MB 359.6, 20 MB 348.4, 40 MB 351.4, 60 MB 355.5, 100 MB 369.0.  Other widths, and
+// where nothing is asked: ops.asked_ahead.
 struct Ahead {
     const uint8_t* at[AHEAD];
     unsigned pieces[AHEAD];

@@ -1620,6 +1620,23 @@ def decode_attention_fresh_ok(qkv, table, cache, head_dim) -> bool:
 AHEAD_BYTES = 24 << 20     # of what lies behind, that blocks of the attention without keys ask into L2 (attention_decode_tma.cu)
 
 
+def asked_ahead(tensors):
+    """[address, bytes, address, bytes] of what the blocks without keys ask for: of up to two tensors, in their order, AHEAD_BYTES
+    together.  Nothing where these do not hold the first one: the product right behind gains little from part of its matrix, and
+    the one after it, which gains most, would get nothing.  Measured, a decoder layer in a chain of layers, us without and with 24 MB
+    asked for, 1 or 2 requests of 40 to 100 tokens / 4 of 300: width 2,048 (8 MB of output matrix) 41.9 / 43.4 -> 40.3 / 41.8, 1,536
+    39.0 / 42.2 -> 38.8 / 41.4, 2,560 51.9 / 52.9 -> 51.9 / 53.0, 3,072 (19 MB) 52.5 / 54.6 -> 52.6 / 54.4; 3,584 (26 MB) 89.1 / 90.3 -> 89.6 /
+    91.1 and 8 of 60 90.4 -> 91.3, 4,096 (34 MB) 85.7 / 87.5 -> 86.1 / 87.3, 5,120 102.0 / 104.0 -> 102.2 / 103.5; from 32 requests on the same either way."""
+    tensors, left, asked = tensors[:2], AHEAD_BYTES, []
+    if tensors and tensors[0].numel() * tensors[0].element_size() > left:
+        tensors = ()
+    for w in tensors:
+        n = min(left, w.numel() * w.element_size()) if w.is_contiguous() else 0
+        asked += [w.data_ptr(), n]
+        left -= n
+    return asked + [None, 0] * (2 - len(asked) // 2)
+
+
 def decode_attention_fresh(qkv, bias, table, cache, block_table, token_seq, positions, out, heads, window, scale,
                            write_kv=True, splits=None, status=None, ahead=()):
     """bfloat16 attention for one query token per request, straight from the q/k/v product: qkv float32
@@ -1648,17 +1665,11 @@ def decode_attention_fresh(qkv, bias, table, cache, block_table, token_seq, posi
     if splits > 1:
         po = empty(T * H * splits * d, torch.float32, qkv.device)
         pm = empty(T * H * splits * 2, torch.float32, qkv.device)
-    asked, left = [], AHEAD_BYTES
-    for w in ahead[:2]:
-        n = min(left, w.numel() * w.element_size()) if w.is_contiguous() else 0
-        asked += [w.data_ptr(), n]
-        left -= n
-    asked += [None, 0] * (2 - len(asked) // 2)
     _check(_get("air_decode_attention_tma_fresh_ahead")(
         qkv.data_ptr(), parts, _ptr(bias), table.data_ptr(), 1 if write_kv else 0, cache.data_ptr(), cache.shape[0],
         block_table.data_ptr(), block_table.shape[1], token_seq.data_ptr(), positions.data_ptr(), out.data_ptr(),
         _ptr(po), _ptr(pm), T, H, K, d, P, int(window or 0), float(scale), splits, _ptr(status),
-        *asked, _stream()), "decode_attention_tma")
+        *asked_ahead(ahead), _stream()), "decode_attention_tma")
     if splits > 1:
         global launches
         launches += 1

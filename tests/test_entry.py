@@ -42,6 +42,19 @@ def test_functions_that_c_programs_call_keep_their_arguments():
     assert lib.air_decode_combine(None, None, None, None, 1, 1, 7, 2, None) == 100001
 
 
+def test_what_the_attention_asks_for_ahead():
+    """Up to 24 MB of two tensors in their order; nothing where the first alone is larger, and never beyond a tensor's end."""
+    of = lambda mb: torch.empty(mb << 20, dtype=torch.uint8)
+    small, half, large = of(8), of(16), of(25)
+    assert ops.asked_ahead(()) == [None, 0, None, 0]
+    assert ops.asked_ahead((small,)) == [small.data_ptr(), 8 << 20, None, 0]
+    assert ops.asked_ahead((small, large)) == [small.data_ptr(), 8 << 20, large.data_ptr(), 16 << 20]
+    assert ops.asked_ahead((half, small)) == [half.data_ptr(), 16 << 20, small.data_ptr(), 8 << 20]
+    assert ops.asked_ahead((large, small)) == [None, 0, None, 0]
+    across = half.view(4, -1).t()
+    assert ops.asked_ahead((across, small)) == [across.data_ptr(), 0, small.data_ptr(), 8 << 20]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("D,splits", [(64, 1), (128, 7), (256, 32)])
 def test_the_merge_alone(D, splits):
