@@ -58,13 +58,17 @@ class RoutedExperts(FeedForward):
     grouped product (which also takes the experts' bounds from the device): there the experts' outputs are rounded to
     bfloat16 before they are added up in 32-bit."""
 
-    # Rows per expert from which the library takes over from ops.grouped_gemm, and how many times as many the stream of weights
-    # holds (144 rows).  From WIDE_ROWS on its tiles are of 128 slots: an expert's matrix then goes through the SMs once or twice
-    # instead of two or three times.  Measured, a mixture of 16 experts on the device, us, library / tiles of 64 / tiles of 128: width
-    # 2,048, 38 rows per expert 145 with either tile, 64 rows 196 / 163 / 159, 88 rows 213 / 187 / 175, 125 rows 229 / 214 / 206, 150 rows
-    # 231 / 241 / 230, 188 rows 248 / 257 / 250; width 4,096, 50 rows - / 374 / 381, 64 rows 469 / 390 / 394, 88 rows 501 / 458 / 427, 125
-    # rows 551 / 542 / 499, 150 rows 557 / 624 / 572, 188 rows 643 / 729 / 704.
-    LIBRARY_ROWS, STREAM_HOLDS, WIDE_ROWS = 64, 2.25, 64
+    # Rows per expert (in the mean) from which the library takes over from ops.grouped_gemm, and how many times as many the stream of
+    # weights holds (130 rows).  From WIDE_ROWS on its tiles are of 128 slots: an expert's matrix then goes through the SMs once instead of two
+    # times, until most experts have more rows than such a tile.  Measured, a mixture without a shared expert on the device, us, library /
+    # tiles of 64 / tiles of 128, even loads: 16 experts of 2,048 at width 2,048, 64 rows per expert 139 / 113 / 111, 80 143 / 127 / 115, 112
+    # 149 / 129 / 121, 128 154 / 143 / 135, 130 141 / - / 133, 136 141 / 143 / 152, 140 141 / 145 / 152; 16 of 3,584 at 4,096, 64 rows 360 / 291 / 291, 128 451 /
+    # 408 / 354, 130 383 / - / 334, 134 385 / - / 365, 140 350 / 401 / 362; 64 experts of 768 at 2,048 (8 to a token), 64 rows 203 / 162 / 156, 112 225 / 199 / 184, 128 229 / 213 /
+    # 217, 132 211 / - / 219, 140 219 / 229 / 229; 128 of them, 64 rows 348 / 293 / 291, 112 420 / 401 / 361, 132 377 / - / 399, 140 387 / 434 / 434; 64 of 1,536 at 4,096 (4 to a
+    # token), 64 rows 573 / 489 / 477, 80 590 / 561 / 492, 128 721 / 743 / 647, 140 584 / 750 / 672.  Uneven loads (one expert with five to
+    # ten times the mean): 64 of 768, 64 rows 207 / 168 / 176, 100 221 / 188 / 192, 140 227 / 219 / 221; 64 of 1,536, 64 rows 596 / 488 /
+    # 500, 80 627 / 514 / 510, 128 774 / 789 / 655.
+    LIBRARY_ROWS, STREAM_HOLDS, WIDE_ROWS = 64, 2.03, 64
 
     graph_safe = True
 
@@ -176,8 +180,7 @@ class RoutedExperts(FeedForward):
         start, pair_of_slot = ints[:n + 1], ints[n + 1:n + 1 + pairs]
         tiles, num_tiles = ints[n + 1 + pairs:-1].view(-1, 2), ints[-1:]
         streams = ops.expert_stream_ok(x, self.gate_up, self.block, self.gated) and ops.expert_stream_ok(x, self.down, 0, False)
-        most = self.LIBRARY_ROWS * (self.STREAM_HOLDS if streams else 1) * n
-        by_library = x.dtype == torch.bfloat16 and pairs >= most and E % 16 == 0 and F % 16 == 0
+        by_library = x.dtype == torch.bfloat16 and self._for_the_library(pairs, streams) and E % 16 == 0 and F % 16 == 0
         streams = streams and not by_library
         tile_rows = ops.GROUP_WIDE if streams and pairs >= self.WIDE_ROWS * n else ops.GROUP_TILE
         ops.moe_sort(expert, n, start, pair_of_slot, tiles, num_tiles, tile_rows=tile_rows)
@@ -210,6 +213,11 @@ class RoutedExperts(FeedForward):
         if self.shared is None:
             return y
         return GatedSum(y, self.shared.forward(x, ctx), gate)
+
+    def _for_the_library(self, pairs, streams):
+        """Whether so many (token, choice) pairs are more than this package's own products hold."""
+        most = self.LIBRARY_ROWS * self.experts
+        return pairs > self.STREAM_HOLDS * most if streams else pairs >= most
 
     def _parts(self, T):
         """Parts of k of the second product: halves in a step of few rows, where they are 8 steps of the ring or more.  A step of

@@ -152,3 +152,16 @@ def test_an_expanded_portion_reads_pages_that_the_request_still_holds(window, pa
         assert lo + ahead <= first, "every key that a query sees is gathered"
         assert all(seq.pages[0][key // page] >= 0 for key in range(lo + ahead, lo + count)), (pos0, lo, ahead)
         cache.trim("r")
+
+
+@pytest.mark.parametrize("experts", [2, 16, 128])
+def test_where_the_library_takes_the_experts_products(experts):
+    """The stream of weights holds about as many rows per expert (in the mean) as a tile has slots; where it does not take the sizes, the
+    library begins at half of that."""
+    from air_b200.csrc import ops
+    from air_b200.parts.experts import RoutedExperts
+    from air_b200.parts.spec import PartSpec
+    part = RoutedExperts(PartSpec("routed_experts", dict(hidden=64, experts=experts, top=2, intermediate=128)))
+    at = ops.GROUP_WIDE * experts
+    assert [part._for_the_library(p, True) for p in (1, at - 1, at, at + at // 32)] == [False, False, False, True]
+    assert [part._for_the_library(p, False) for p in (1, at // 2 - 1, at // 2)] == [False, False, True]
