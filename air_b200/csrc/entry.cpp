@@ -90,11 +90,13 @@ PyObject* require(PyObject*, PyObject* const* args, Py_ssize_t n, PyObject* name
     return PyObject_Vectorcall(say_why, args, (size_t)n, names);
 }
 
-// ops.empty(shape, dtype, device): torch.empty for a tuple of sizes or a number of elements.
+// ops.empty(shape, dtype, device): torch.empty for a tuple of sizes or a number of elements; other forms go to torch itself.
+PyObject* any_empty = nullptr;
+
 PyObject* empty(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 3 || !(PyTuple_Check(args[0]) || PyLong_Check(args[0])) || !THPDtype_Check(args[1]) || !THPDevice_Check(args[2]))
-        return PyErr_Format(PyExc_TypeError, "empty(a tuple of sizes or a number, a dtype, a device)");
+        return PyObject_Vectorcall(any_empty, args, (size_t)n, nullptr);
     c10::SmallVector<int64_t, 5> sizes;
     if (PyLong_Check(args[0])) sizes.push_back(PyLong_AsLongLong(args[0]));
     else
@@ -110,10 +112,10 @@ PyObject* empty(PyObject*, PyObject* const* args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-PyObject* set_say_why(PyObject*, PyObject* f) {
-    Py_XDECREF(say_why);
+template <PyObject** F> PyObject* set(PyObject*, PyObject* f) {
+    Py_XDECREF(*F);
     Py_INCREF(f);
-    say_why = f;
+    *F = f;
     Py_RETURN_NONE;
 }
 
@@ -127,7 +129,8 @@ PyMethodDef methods[] = {
     AIR_ENTRIES
     {"require", (PyCFunction)(void (*)(void))require, METH_FASTCALL | METH_KEYWORDS, nullptr},
     {"empty", (PyCFunction)(void (*)(void))empty, METH_FASTCALL, nullptr},
-    {"set_say_why", set_say_why, METH_O, nullptr},
+    {"set_say_why", set<&say_why>, METH_O, nullptr},
+    {"set_any_empty", set<&any_empty>, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "air_b200_entry", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -235,11 +235,16 @@ def _req(*args, **kwargs):
     return _req(*args, **kwargs)
 
 
+def _any_empty(shape, dtype, device):
+    return torch.empty(shape, dtype=dtype, device=device)
+
+
 def empty(shape, dtype, device):
     """torch.empty, by the library's own function from the first call on."""
     global empty
     if not torch.cuda.is_available():
-        return torch.empty(shape, dtype=dtype, device=device)
+        return _any_empty(shape, dtype, device)
+    build.entry().set_any_empty(_any_empty)
     empty = build.entry().empty
     return empty(shape, dtype, device)
 

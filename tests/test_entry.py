@@ -111,6 +111,33 @@ def test_a_tensor_is_checked_as_in_python():
         assert said[0] == said[1]
 
 
+def test_new_tensors_of_every_form_that_torch_takes():
+    """Sizes as a list, a device by its name: what the library's own function does not read goes to torch (no device is needed)."""
+    entry = build.entry()
+    entry.set_any_empty(ops._any_empty)
+    for shape, device in (((2, 3), "cpu"), ([2, 3], "cpu"), ([4], torch.device("cpu")), ((2, 0), torch.device("cpu")), (5, "cpu")):
+        a, b = entry.empty(shape, torch.bfloat16, device), torch.empty(shape, dtype=torch.bfloat16, device=device)
+        assert a.shape == b.shape and a.dtype == b.dtype and a.device == b.device
+    for wrong in ((), ((2, 3), torch.float32), ((2, 3), 7, "cpu"), ("x", torch.float32, "cpu"), ((2, "x"), torch.float32, torch.device("cpu"))):
+        with pytest.raises(TypeError):
+            entry.empty(*wrong)
+
+
+@pytest.mark.gpu
+def test_a_runtime_whose_device_is_a_name():
+    """Parts of a runtime that was given its device as a text, as torch takes it."""
+    from types import SimpleNamespace
+    from air_b200.parts.base import Runtime
+    from air_b200.parts.embedding import TokenEmbedding
+    from air_b200.parts.spec import PartSpec
+    table = torch.randn(7, 8, device="cuda").bfloat16()
+    part = TokenEmbedding(PartSpec("tokens", {"hidden": 8, "vocab": 7}), "t")
+    part.load({"t": table}, Runtime("cuda", torch.bfloat16))
+    ctx = SimpleNamespace(num_tokens=2, token_ids=torch.tensor([3, 6], dtype=torch.int32, device="cuda"), status=None, last_token=None)
+    (h,) = part.forward(ctx, ())
+    assert torch.equal(h, table[[3, 6]].float())
+
+
 @pytest.mark.gpu
 def test_new_tensors_and_launches():
     dev = torch.device("cuda:0")
