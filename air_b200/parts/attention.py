@@ -318,7 +318,7 @@ class Attention(TiledAttention, Mixer):
             out = ops.empty((T, H, d), rt.dtype, x.device)
             ops.decode_attention_fresh(qkv, self.bias, table, pages.kv, bt, ctx.token_seq, ctx.positions, out, H,
                                        self.window, self.scale, write_kv=owns_cache, status=ctx.status,
-                                       ahead=(self.o.weight, *self.behind))
+                                       ahead=(self.o.weight, *self.behind()))
             return self._project(out.view(T, H * d), ctx)
         if isinstance(x, PreNormed):
             raise ops.KernelError("attention: rows without their norm's scale reached a road that does not apply it")

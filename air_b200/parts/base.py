@@ -394,9 +394,10 @@ class RowFilter(Part):
 
 
 class Mixer(Part):
-    # Weights that the parts behind this one read in a step of few rows, in that order (the block knows them): a kernel with
-    # memory to spare may ask for them ahead of time.
-    behind: Tuple[torch.Tensor, ...] = ()
+    def behind(self) -> Tuple[torch.Tensor, ...]:
+        """Weights that the parts behind this one read in a step of few rows, in that order (the block knows them and puts a function
+        of its own here): a kernel with memory to spare may ask for them ahead of time."""
+        return ()
 
     def cache_needs(self) -> Tuple[CacheNeed, ...]:
         return ()

@@ -82,7 +82,7 @@ class PreNormBlock(Block):
     def load(self, tensors, rt):
         super().load(tensors, rt)
         if self.feed_forward is not None:
-            self.mixer.behind = self.feed_forward.streams()
+            self.mixer.behind = self.feed_forward.streams
         if self.residual_scale != 1.0:
             import torch
             self.scale = torch.full((self.spec.part("mixer_norm")["size"],), self.residual_scale, dtype=torch.float32,

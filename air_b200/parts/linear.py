@@ -50,7 +50,6 @@ class Linear:
     def __init__(self, weight: torch.Tensor, status: Optional[torch.Tensor] = None, gate_up_block: int = 0):
         assert weight.dim() == 2
         self.weight = weight
-        self.transposed = weight.t()             # (a view, as the library's product wants it)
         self.status = status
         self.out_features, self.in_features = weight.shape
         self.gate_up_block = gate_up_block       # > 0: rows are blocks of gate rows and up rows in turn
@@ -130,7 +129,7 @@ class Linear:
     def add_into(self, x: torch.Tensor, residual: torch.Tensor) -> None:
         """residual += x W^T, the sum taken in 32-bit in the library product's epilogue (the product is not
         rounded to 16 bits first, and is not written and read again by the norm that follows)."""
-        torch.addmm(residual, x, self.transposed, out_dtype=torch.float32, out=residual)
+        torch.addmm(residual, x, self.weight.t(), out_dtype=torch.float32, out=residual)
 
     def __call__(self, x: torch.Tensor, out_dtype: torch.dtype, bias=None) -> torch.Tensor:
         w = self.weight
@@ -148,4 +147,4 @@ class Linear:
             raise ops.KernelError("Linear: a bias with 16-bit weights is added by the consumer's kernel")
         if not x.is_cuda:
             raise ops.KernelError("Linear: input must be a CUDA tensor")
-        return torch.mm(x, self.transposed, out_dtype=out_dtype)
+        return torch.mm(x, w.t(), out_dtype=out_dtype)

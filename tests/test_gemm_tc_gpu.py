@@ -204,3 +204,22 @@ def test_complete_sums_by_clusters_along_k(N, K, scaled):
         kept = out if kept is None else kept
         assert close(out, want[:T], K) and torch.equal(out, kept[:T]), T
     assert status.item() == 0
+
+
+@pytest.mark.parametrize("M", [8, 200])
+def test_a_product_reads_the_weights_that_it_has_now(M):
+    """A matrix that a program has put in another's place, or whose memory it has replaced, after the product was made."""
+    from air_b200.parts.linear import Linear
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, first, second, third = rand(M, 256), rand(384, 256), rand(384, 256), rand(384, 256)
+    product = Linear(first.clone())
+    check = lambda w: close(product.f32(x), x.double().cpu() @ w.double().cpu().T, 256)
+    assert check(first)
+    product.weight = second.clone()
+    assert check(second)
+    product.weight.data = third.clone()
+    assert check(third)
+    total = torch.ones(M, 384, device="cuda")
+    product.add_into(x, total)
+    assert close(total - 1, x.double().cpu() @ third.double().cpu().T, 256)
