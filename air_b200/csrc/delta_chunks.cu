@@ -27,7 +27,7 @@
 //                              numbers arrive by the copy engine, in two runs of bytes, while this one's are used.
 //
 // Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 193 (prepare
-// 46, scan 147); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 98 (24 and 73).  Which portions come here:
+// 46, scan 147); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 102 (29 and 73).  Which portions come here:
 // parts/recurrent.py (least).
 //
 // Errors against 64 bits (2-norm of the difference over that of the result, 2,048 tokens), token by token and here: one decay per
@@ -84,7 +84,8 @@ struct DeltaChunkArgs {
 __device__ __forceinline__ float softplus_1(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 
 // (four blocks to an SM: a block is a chain of short phases between barriers.  With three 49.7 us for 128 chunks of 16 heads, 51.7 with
-// a decay per channel and 94 chunks; with four 45.7 and 48.5 for a few spilled registers; five 45.3 and 57.5)
+// a decay per channel and 94 chunks; with four 45.7 and 48.5 for a few spilled registers; five 45.3 and 57.5.  Gated linear attention, 16
+// heads, 300, 777, 1,200 and 2,048 tokens: three 13.2, 29.4, 39.2 and 64.2, four 13.5, 29.1, 37.1 and 59.5)
 template <int DP, int MODE>
 __global__ void __launch_bounds__(256, DP <= 128 ? 4 : 2) delta_chunk_prepare_kernel(const DeltaChunkArgs p) {
     constexpr int ld = DP + 4, PER = DP / 32;

@@ -385,8 +385,8 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 }
 
 // Blocks that share a tile of complete sums, by what a product takes, us: a block's copies (a step of k is 16 KB at 65 GB/s) or
-// the whole matrix at 6.5 TB/s, whichever is longer, and the exchange.  Every block has an SM to itself and eight steps of k or
-// more; clusters of four do not fit on all SMs (a cluster stands in one GPC).
+// the whole matrix at 6.5 TB/s, whichever is longer, and the exchange.  Every block has an SM to itself and eight steps of k in the
+// mean (the last one may have fewer); clusters of four do not fit on all SMs (a cluster stands in one GPC).
 static int ts_joined_parts(int n_tiles, int k_tiles, int sms) {
     int best = 1;
     double least = 0.95 * max(k_tiles * 0.25, n_tiles * k_tiles * 0.0025);

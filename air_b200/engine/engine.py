@@ -44,7 +44,7 @@ class EngineConfig:
     src/runtime/backend.cpp:538-556).  max_requests: live requests (state slots).  AIR:
     KvPolicy.page_tokens (include/air/execution.hpp:103-105) and SchedulerConfig.max_active_requests
     (include/air/serving.hpp:46-62).  keep_float32: matrices that the checkpoint stores in 32 bits stay
-    so in a bfloat16 engine (and run the CUDA-core product) instead of being rounded to bfloat16."""
+    so in a bfloat16 engine (and run the 32-bit products) instead of being rounded to bfloat16."""
     dtype: torch.dtype = torch.bfloat16
     page_tokens: int = 64
     max_tokens: Optional[int] = 8192

@@ -135,7 +135,7 @@ class RoutedExperts(FeedForward):
         # The router and the shared expert's gate are one product with 32-bit sums.  In a bfloat16 engine its operands
         # are the stored 16-bit weights and the stream's rows as the other products read them: their products are
         # exact in 32 bits, so the tensor cores' 32-bit accumulation is the 32-bit router (rows of zeros fill the matrix
-        # up to a multiple of 8, which those kernels want).  A float32 engine runs the CUDA-core product.
+        # up to a multiple of 8, which those kernels want).  A float32 engine runs the 32-bit product.
         w = torch.cat([r.to(rt.dtype) for r in rows], dim=0)
         if not rt.is_fp32 and w.shape[0] % 8:
             w = torch.cat([w, torch.zeros((8 - w.shape[0] % 8, w.shape[1]), dtype=w.dtype, device=w.device)], dim=0)

@@ -11,8 +11,8 @@ and float16).  In a bfloat16 engine a tensor stored in 16 bits is kept as bfloat
 rounded to it), integer tables become int32, and a tensor stored in 32 bits stays in 32 bits
 where its part computes with it in 32 bits (``TensorSpec.wide``: norm weights, biases, router
 weights).  A matrix that feeds the tensor cores is another matter: kept in 32 bits it would run
-the CUDA-core product at a few percent of the speed, so a float32-stored operand of a matrix
-product is rounded to bfloat16 (to nearest even), as AIR executes float32, float16 and bfloat16
+the 32-bit products, at half the speed for a few rows (twice the bytes) and a tenth for a prompt
+(six products for one), so a float32-stored operand of a matrix product is rounded to bfloat16 (to nearest even), as AIR executes float32, float16 and bfloat16
 checkpoints through one path (src/reference/tensor_reader.cpp:251-255), unless the caller asks
 for ``keep_float32``.  Either way the load says what it did: ``LoadReport`` lists the rounded and
 the kept tensors, and the engine keeps it (``Engine.load_report``).
@@ -109,7 +109,7 @@ class LoadReport:
         out = []
         if self.rounded:
             out.append(f"{len(self.rounded)} tensors stored in float32 or float16 were rounded to bfloat16 "
-                       f"(first: {self.rounded[0]}); keep_float32 keeps float32 ones, at the CUDA-core product's speed")
+                       f"(first: {self.rounded[0]}); keep_float32 keeps float32 ones, at the 32-bit products' speed")
         if self.kept_float32:
             out.append(f"{len(self.kept_float32)} tensors stay in float32 (first: {self.kept_float32[0]})")
         return "; ".join(out)

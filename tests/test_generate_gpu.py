@@ -376,7 +376,7 @@ def test_sizes_that_the_kernels_refuse_are_unsupported_with_exit_code_3(tmp_path
 def test_a_float32_checkpoint_in_the_bfloat16_engine_runs_the_tensor_core_products(tmp_path):
     """A checkpoint stored in float32, loaded by the bfloat16 engine: matrices are rounded to bfloat16 at load
     (and the load says so), so every product runs the kernels of the bfloat16 path; keep_float32 keeps them and
-    runs the CUDA-core product; both agree with the plain implementation on the rounded weights."""
+    runs the 32-bit products; both agree with the plain implementation on the rounded weights."""
     from air_b200.engine.batch import Entry
     from air_b200.engine.engine import Engine, EngineConfig, write_random_model
     folder = str(tmp_path / "m")
