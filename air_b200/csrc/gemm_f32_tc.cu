@@ -90,7 +90,8 @@ __device__ __forceinline__ void ft_less(float& x, float& y, uint32_t p) {
         : "+f"(x), "+f"(y) : "r"(p));
 }
 // Two neighbouring numbers times FT_SCALE as three pairs of bfloat16, the first in the low half.  (The factor costs 300 rows by
-// 16,384 x 2,048 138.5 -> 140.8 us, few rows nothing; as two multiplications one row lost 2 % as well.)
+// 16,384 x 2,048 142.8 -> 145.5 us, few rows nothing; as two multiplications one row lost 2 % as well.  Sums taken from tensor
+// memory 32 columns at a time instead of 8 bring it back to 143.2.)
 constexpr float FT_SCALE = 0x1p24f, FT_UNSCALE = 0x1p-48f;      // (of a number, of a product of two)
 __device__ __forceinline__ void ft_split(float x, float y, uint32_t (&p)[3]) {
     asm("{\n\t.reg .b64 v, f;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 f, {%2, %2};\n\tmul.rn.f32x2 v, v, f;\n\tmov.b64 {%0, %1}, v;\n\t}"
@@ -103,6 +104,12 @@ __device__ __forceinline__ void ft_split(float x, float y, uint32_t (&p)[3]) {
             ft_less(x, y, p[i]);
         }
     }
+}
+
+// a += x, b += y, in one instruction.
+__device__ __forceinline__ void ft_add(float& a, float& b, uint32_t x, uint32_t y) {
+    asm("{\n\t.reg .b64 u, v;\n\tmov.b64 u, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tadd.rn.f32x2 u, u, v;\n\tmov.b64 {%0, %1}, u;\n\t}"
+        : "+f"(a), "+f"(b) : "r"(x), "r"(y));
 }
 
 // Waits with a whole warp, every lane for a barrier of its own choice; one try where all are there already.
@@ -136,12 +143,26 @@ __device__ __forceinline__ void ft_store_planes(uint32_t taddr, const uint32_t (
                  "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
-__device__ __forceinline__ void ft_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
-                 "tcgen05.wait::ld.sync.aligned;"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
+// 8, 16, 24 or 32 columns with one wait, which stands in the same statement so that nothing is read ahead of it.
+#define FT_R8(r, i) "=r"(r[i]), "=r"(r[i + 1]), "=r"(r[i + 2]), "=r"(r[i + 3]), "=r"(r[i + 4]), "=r"(r[i + 5]), "=r"(r[i + 6]), "=r"(r[i + 7])
+#define FT_LD "tcgen05.ld.sync.aligned.32x32b."
+#define FT_LD_WAIT "tcgen05.wait::ld.sync.aligned;"
+__device__ __forceinline__ void ft_load(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile(FT_LD "x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t" FT_LD_WAIT : FT_R8(r, 0) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void ft_load(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(FT_LD "x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t" FT_LD_WAIT
+                 : FT_R8(r, 0), FT_R8(r, 8) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void ft_load(uint32_t taddr, uint32_t (&r)[24]) {
+    asm volatile(FT_LD "x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%24];\n\t"
+                 FT_LD "x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%25];\n\t" FT_LD_WAIT
+                 : FT_R8(r, 0), FT_R8(r, 8), FT_R8(r, 16) : "r"(taddr), "r"(taddr + 16) : "memory");
+}
+__device__ __forceinline__ void ft_load(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(FT_LD "x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, "
+                 "%22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t" FT_LD_WAIT
+                 : FT_R8(r, 0), FT_R8(r, 8), FT_R8(r, 16), FT_R8(r, 24) : "r"(taddr) : "memory");
 }
 
 // The results of rows m_lo .. m_hi - 1 and columns n0 .. n0 + 127 that are not finite, by multiply-adds from memory in the order of
@@ -414,23 +435,16 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (!ft_wait(&d_full[buf], c >> 1 & 1, abort_flag)) return false;
             tc_fence_after();
             const uint32_t from = tmem + 2 * FT_A_COLS + buf * NT + half * HALF + lanes;
-            if constexpr (HALF % 16) {
+            auto add = [&](auto first, auto columns) {      // (one wait for as many as there are registers)
+                uint32_t v[decltype(columns)::value];
+                ft_load(from + decltype(first)::value, v);
 #pragma unroll
-                for (int i = 0; i < HALF; i += 8) {
-                    uint32_t v[8];
-                    ft_ld8(from + i, v);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) total[i + e] += __uint_as_float(v[e]);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < HALF; i += 16) {
-                    uint32_t v[16];
-                    tmem_ld16(from + i, v);
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) total[i + e] += __uint_as_float(v[e]);
-                }
-            }
+                for (int e = 0; e < decltype(columns)::value; e += 2)
+                    ft_add(total[decltype(first)::value + e], total[decltype(first)::value + e + 1], v[e], v[e + 1]);
+            };
+            constexpr int AT_ONCE = HALF < 32 ? HALF : 32;
+            add(std::integral_constant<int, 0>(), std::integral_constant<int, AT_ONCE>());
+            if constexpr (HALF > AT_ONCE) add(std::integral_constant<int, AT_ONCE>(), std::integral_constant<int, HALF - AT_ONCE>());
             tc_fence_before();
             if constexpr (APART) {
                 if (--left > 0 && c + 1 < chunks) return true;
