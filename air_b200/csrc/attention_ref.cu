@@ -314,8 +314,9 @@ __device__ __forceinline__ void ref_rows(const RefArgs& a, float* smem, int t, i
 }
 
 // A block takes `per_block` rows of the batch for one head: runs of consecutive tokens of a request among them together.
-template <int D, bool SHARED>
-__global__ void __launch_bounds__(ATT_WARPS * 32, SHARED ? 3 : 1) paged_attention_f32_kernel(const RefArgs a, int per_block) {
+// ROOM: how many blocks are to find registers on an SM (0: the compiler takes as many as it likes).
+template <int D, bool SHARED, int ROOM>
+__global__ void __launch_bounds__(ATT_WARPS * 32, ROOM) paged_attention_f32_kernel(const RefArgs a, int per_block) {
     extern __shared__ __align__(16) float smem[];
     pdl_enter(TR_ATT_REF);
     const int end = min(a.T, (int)(blockIdx.x + 1) * per_block);
@@ -349,16 +350,25 @@ AIR_API int air_paged_attention_ref(const void* q, int q_f32, const void* cache,
         // As many rows to a block, up to REF_QUERIES, as leave a block for every SM.  Measured, us, against the kernel above: 300
         // rows of a prompt, 16 heads of 128: 473 -> 63; 512 rows behind 500: 3,315 -> 247; 4 single tokens over 1,000 keys, 28
         // heads: 317 -> 32; one over 4,000: 1,217 -> 99; 64 over 2,000: 2,409 -> 488.
-        // Blocks of several rows are many and each waits for its own reads, its shared-memory loads and its chains of sums, one
-        // warp to a scheduler: with the values in the keys' memory three blocks share an SM instead of one (300 rows 101 -> 63, 512
-        // 401 -> 247, 64 single tokens 744 -> 488).  A block of one row keeps both, so that the next keys arrive meanwhile.
+        // A block waits for its own reads, its shared-memory loads and its chains of sums, one warp to a scheduler.  Where there are
+        // more blocks than SMs hold at a time (two, or as many as their memory allows), the values take the keys' memory and three
+        // share an SM (300 rows 101 -> 63, 512 401 -> 247, 64 single tokens over 2,000 744 -> 488); else a block keeps both, so that
+        // the next keys arrive meanwhile.  Measured, us, both and values in the keys' memory: heads of 128 (one block of both to an SM),
+        // 128 blocks of 2,000 keys 49 and 55, 224 95 and 73, 192 of 1,000 50 and 37; heads of 96 (two), 256 blocks of 1,000 keys 37 and 45,
+        // 192 in runs of three 104 and 108, 608 of a prompt of 300 60 and 52; of 64 (two), 256 of 1,000 35 and 39, 400 of a portion 102 and 67.
+        // Sizes other than 128 have two forms with both: 142 registers where every block has an SM (128 blocks of 1,000 keys, heads of
+        // 64: 30.2 us, 31.7 with 194), 194 where two share one (256: 39.5, 34.9).
         const int per_block = (int)min((long long)air::REF_QUERIES, max(1ll, (long long)T * H / 148));
         const air::RefArgs args{(const float*)q, (const float*)cache, block_table, max_blocks, token_seq, positions, (float*)out,
                                 gate, T, H, K, d, dv, P, window, scale, softcap, mask_mode, sink, latent, db};
-        const bool shared = per_block > 1;
+        const long long blocks = (long long)((T + per_block - 1) / per_block) * H;
+        const int resident = (int)min((size_t)2, (size_t)(228 * 1024) / (air::RefPlaces{d, dv, false}.bytes() + 1024));
+        const bool shared = blocks > 148 * resident;
         const size_t smem = air::RefPlaces{d, dv, shared}.bytes();
-        auto kernel = d == 128 && dv == 128 ? (shared ? air::paged_attention_f32_kernel<128, true> : air::paged_attention_f32_kernel<128, false>)
-                                            : (shared ? air::paged_attention_f32_kernel<0, true> : air::paged_attention_f32_kernel<0, false>);
+        auto kernel = d == 128 && dv == 128 ? (shared ? air::paged_attention_f32_kernel<128, true, 3> : air::paged_attention_f32_kernel<128, false, 1>)
+                      : shared              ? air::paged_attention_f32_kernel<0, true, 3>
+                      : blocks > 148        ? air::paged_attention_f32_kernel<0, false, 1>
+                                            : air::paged_attention_f32_kernel<0, false, 0>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return (int)e;

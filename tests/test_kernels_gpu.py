@@ -511,6 +511,25 @@ def test_gemm_f32_with_a_matrix_that_the_launches_ahead_write(M):
             assert torch.equal(out, a.float() @ b.float().T)
 
 
+@pytest.mark.parametrize("H,K,d,per_sm", [(28, 4, 128, 1), (20, 4, 112, 1), (32, 8, 96, 2), (16, 2, 80, 2), (16, 16, 64, 2), (8, 8, 32, 2)])
+def test_float32_attention_with_values_in_the_keys_memory(H, K, d, per_sm):
+    """Batches on either side of the numbers of blocks from which two share an SM and from which the values take the keys' memory: the
+    bits of rows alone, for single tokens and for runs of consecutive ones."""
+    most = 148 * per_sm
+    for lens, q_lens in (([70 + 9 * i for i in range(most // H)], [1] * (most // H)), ([40 + i for i in range(most // H + 1)], [1] * (most // H + 1)),
+                         ([33 * (i % 5) + 30 for i in range(64)], [1] * 64), ([300, 91, 260], [250, 91, 17])):
+        pages = sum(-(-n // 64) for n in lens) + 2
+        q, cache, bt, positions, seq_of, _, _ = paged_case(H, K, d, 64, lens, q_lens, "float32", seed=d, num_pages=pages)
+        args = [dev(x) for x in (cache, bt)]
+        out = torch.empty(len(positions), H, d, device="cuda")
+        ops().paged_attention_ref(dev(q), *args, dev(seq_of), dev(positions), out, 0, d ** -0.5)
+        for t in range(0, len(positions), max(1, len(positions) // 12)):
+            one = torch.empty(1, H, d, device="cuda")
+            ops().paged_attention_ref(dev(q[t:t + 1]), *args, dev(seq_of[t:t + 1]), dev(positions[t:t + 1]), one, 0, d ** -0.5)
+            assert torch.equal(one[0], out[t]), (len(lens), t)
+
+
+
 @pytest.mark.parametrize("H,K,d,P", [(6, 2, 48, 16), (8, 2, 128, 64), (12, 1, 20, 48), (16, 16, 16, 16)])
 @pytest.mark.parametrize("window,chunk", [(0, None), (21, None), (0, 50)])
 def test_float32_attention_of_rows_together_is_that_of_rows_alone(H, K, d, P, window, chunk):
