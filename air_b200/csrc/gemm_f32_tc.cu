@@ -84,25 +84,30 @@ __host__ __device__ constexpr int ft_smem(int nt) {
 // k of an eighth: whole chunks
 __host__ __device__ __forceinline__ int ft_part(int K) { return ((K + FT_PARTS - 1) / FT_PARTS + FT_BK - 1) / FT_BK * FT_BK; }
 
-// x -= the low half of p, y -= the high half (bfloat16 each).
-__device__ __forceinline__ void ft_less(float& x, float& y, uint32_t p) {
-    asm("{\n\t.reg .b16 l, h, m;\n\tmov.b16 m, 0xBF80;\n\tmov.b32 {l, h}, %2;\n\tfma.rn.f32.bf16 %0, l, m, %0;\n\tfma.rn.f32.bf16 %1, h, m, %1;\n\t}"
-        : "+f"(x), "+f"(y) : "r"(p));
+// x -= the low half of p, y -= the high half (bfloat16 each): by two operations that take bfloat16 numbers as they are, or TOGETHER by one on
+// both, which wants them widened (64 rows by 11,008 x 4,096 53.4 -> 51.4 us, 300 by 16,384 x 2,048 143.5 -> 143.0; where two blocks share an SM
+// that is slower: 17 rows 45.2, 12 rows 44.0 -> 45.6).
+template <bool TOGETHER> __device__ __forceinline__ void ft_less(float& x, float& y, uint32_t p) {
+    if constexpr (TOGETHER)
+        asm("{\n\t.reg .b64 v, w;\n\t.reg .b32 l, h;\n\tshl.b32 l, %2, 16;\n\tand.b32 h, %2, 0xffff0000;\n\tmov.b64 v, {%0, %1};\n\t"
+            "mov.b64 w, {l, h};\n\tsub.rn.f32x2 v, v, w;\n\tmov.b64 {%0, %1}, v;\n\t}"
+            : "+f"(x), "+f"(y) : "r"(p));
+    else
+        asm("{\n\t.reg .b16 l, h, m;\n\tmov.b16 m, 0xBF80;\n\tmov.b32 {l, h}, %2;\n\tfma.rn.f32.bf16 %0, l, m, %0;\n\tfma.rn.f32.bf16 %1, h, m, %1;\n\t}"
+            : "+f"(x), "+f"(y) : "r"(p));
 }
 // Two neighbouring numbers times FT_SCALE as three pairs of bfloat16, the first in the low half.  (The factor costs 300 rows by
 // 16,384 x 2,048 142.8 -> 145.5 us, few rows nothing; as two multiplications one row lost 2 % as well.  Sums taken from tensor
-// memory 32 columns at a time instead of 8 bring it back to 143.2.)
+// memory 32 columns at a time instead of 8, and ft_less, bring it back to 143.0; 17 to 32 rows keep a loss of 2 to 4 %.)
 constexpr float FT_SCALE = 0x1p24f, FT_UNSCALE = 0x1p-48f;      // (of a number, of a product of two)
-__device__ __forceinline__ void ft_split(float x, float y, uint32_t (&p)[3]) {
+template <bool TOGETHER = false> __device__ __forceinline__ void ft_split(float x, float y, uint32_t (&p)[3]) {
     asm("{\n\t.reg .b64 v, f;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 f, {%2, %2};\n\tmul.rn.f32x2 v, v, f;\n\tmov.b64 {%0, %1}, v;\n\t}"
         : "+f"(x), "+f"(y) : "f"(FT_SCALE));
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const __nv_bfloat162 b = __floats2bfloat162_rn(x, y);
         p[i] = *reinterpret_cast<const uint32_t*>(&b);
-        if (i < 2) {
-            ft_less(x, y, p[i]);
-        }
+        if (i < 2) ft_less<TOGETHER>(x, y, p[i]);
     }
 }
 
@@ -486,8 +491,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     float v[4];
                     load4(row + (((4 * k + j) ^ (r & 7)) << 2), v);
                     uint32_t lo[3], hi[3];
-                    ft_split(v[0], v[1], lo);
-                    ft_split(v[2], v[3], hi);
+                    ft_split<(NT > 32)>(v[0], v[1], lo);
+                    ft_split<(NT > 32)>(v[2], v[3], hi);
 #pragma unroll
                     for (int i = 0; i < 3; ++i) {
                         p[i][2 * j] = lo[i];
