@@ -23,12 +23,18 @@
 //                              as a result of one product they are the left operand of the next without a move (the
 //                              instruction's k may run in any order that both operands share).  Every 32-bit operand enters as
 //                              two TF32 numbers, hi + lo, and every product as lo hi + hi lo + hi hi, which keeps the
-//                              operands to 2^-23: what is left out is of the order of 32-bit rounding.  The next chunk's
+//                              operands to 2^-23: what is left out is of the order of 32-bit rounding.  The next chunks'
 //                              numbers arrive by the copy engine, in two runs of bytes, while this one's are used.
 //
-// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 193 (prepare
-// 46, scan 147); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 102 (29 and 73).  Which portions come here:
+// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 152 (prepare
+// 46, scan 106); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 84 (29 and 54).  Which portions come here:
 // parts/recurrent.py (least).
+//
+// What bounds the scan is the chain from chunk to chunk: three products of 24 instructions each that a warp issues at 10 cycles an
+// instruction, the cutting of 64 numbers into halves, two barriers: 0.83 us a chunk, 0.69 for gated linear attention, which has two
+// products.  Half of the warps hold the state and do nothing that the next chunk does not wait for; the sums across warps that give U, and
+// the outputs, are the other half's, the latter a chunk behind.  (All of it in four warps: 1.15 us a chunk, 148 and 74 us for the two
+// sizes above; the state handed to the other half for q S through shared memory: 136 and 70; barriers in memory instead of bar.sync: 177.)
 //
 // Errors against 64 bits (2-norm of the difference over that of the result, 2,048 tokens), token by token and here: one decay per
 // head, outputs 1.98e-7 and 1.95e-7, states 1.56e-7 and 1.58e-7; gated linear attention 1.60e-7 and 1.60e-7, 1.40e-7 and 1.10e-7; decays
@@ -44,7 +50,7 @@
 namespace air {
 
 constexpr int DC = 16;              // tokens of a chunk, and columns of a block of the scan
-constexpr int DC_RLD = 40, DC_ULD = 24;      // strides of rows in shared memory: four rows fall into different banks
+constexpr int DC_RLD = 24, DC_ULD = 20;      // strides of rows in shared memory: four rows of 8 numbers, eight of 4, fall into different banks
 constexpr float DC_FLOOR = -110.f;   // (e^-110 is 0 in 32 bits; differences of the logarithms' sums stay numbers)
 
 // What a chunk and head leave in the scratch memory, DP the channels filled up to 32, 64, 128 or 256 (zeros), in floats:
@@ -315,42 +321,128 @@ __device__ __forceinline__ Two two_of(float x) {
     const uint32_t hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
     return Two{hi, __float_as_uint(x - __uint_as_float(hi))};
 }
-// c += a b; with k in the order that the accumulators have: a holds (row g, k 2t), (g + 8, 2t), (g, 2t + 1), (g + 8, 2t + 1), b
-// holds (k 2t, column g), (2t + 1, g)
-__device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-                 "{%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// c = a b (FRESH) or c += a b; with k in the order that the accumulators have: a holds (row g, k 2t), (g + 8, 2t), (g, 2t + 1),
+// (g + 8, 2t + 1), b holds (k 2t, column g), (2t + 1, g)
+template <bool FRESH>
+__device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (FRESH)        // (zeros as an operand of their own: no register has to be cleared)
+        asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                     "{%10, %10, %10, %10};"
+                     : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+    else
+        asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                     "{%0, %1, %2, %3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// The three products of numbers as halves, for N tiles side by side: low += lo hi + hi lo, high = hi hi.  (A product waits 24 cycles
+// for the sum that it adds to, one to a sum of its own 12.)
+template <int N>
+__device__ __forceinline__ void mma_two(bool fresh, float (&low)[N][4], float (&high)[N][4], const Two (&a)[4], const Two (&b)[N][2]) {
+#pragma unroll
+    for (int x = 0; x < N; ++x) {
+        if (fresh) mma_tf32<true>(low[x], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[x][0].hi, b[x][1].hi);
+        else mma_tf32<false>(low[x], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[x][0].hi, b[x][1].hi);
+    }
+#pragma unroll
+    for (int x = 0; x < N; ++x) mma_tf32<true>(high[x], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].hi, b[x][1].hi);
+#pragma unroll
+    for (int x = 0; x < N; ++x) mma_tf32<false>(low[x], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].lo, b[x][1].lo);
+}
+// Two numbers at a time: the same sums as one by one.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    asm("{\n\t.reg .b64 u, v;\n\tmov.b64 u, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tadd.rn.f32x2 u, u, v;\n\tmov.b64 {%0, %1}, u;\n\t}"
+        : "+f"(a.x), "+f"(a.y) : "f"(b.x), "f"(b.y));
+    return a;
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+    asm("{\n\t.reg .b64 u, v;\n\tmov.b64 u, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tsub.rn.f32x2 u, u, v;\n\tmov.b64 {%0, %1}, u;\n\t}"
+        : "+f"(a.x), "+f"(a.y) : "f"(b.x), "f"(b.y));
+    return a;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    asm("{\n\t.reg .b64 u, v, w;\n\tmov.b64 u, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 w, {%4, %5};\n\t"
+        "fma.rn.f32x2 u, u, v, w;\n\tmov.b64 {%0, %1}, u;\n\t}"
+        : "+f"(a.x), "+f"(a.y) : "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return a;
+}
+__device__ __forceinline__ void two_of_pair(Two& a, Two& b, float2 v) {
+    a.hi = (__float_as_uint(v.x) + 0x1000u) & 0xffffe000u;
+    b.hi = (__float_as_uint(v.y) + 0x1000u) & 0xffffe000u;
+    const float2 rest = sub2(v, make_float2(__uint_as_float(a.hi), __uint_as_float(b.hi)));
+    a.lo = __float_as_uint(rest.x);
+    b.lo = __float_as_uint(rest.y);
 }
 __device__ __forceinline__ void two_pair(Two (&b)[2], const float* p) {
-    const float2 v = *reinterpret_cast<const float2*>(p);
-    b[0] = two_of(v.x);
-    b[1] = two_of(v.y);
+    two_of_pair(b[0], b[1], *reinterpret_cast<const float2*>(p));
 }
 
-constexpr int DC_WARPS = 4;         // one per scheduler: the products follow one another in the tensor pipe as fast as it takes them,
-                                    // and the fewer warps share the channels, the fewer sums cross between them
-constexpr int DC_STAGES = 2;
+// One warp per scheduler holds the state: the fewer warps share the channels, the fewer sums cross between them (with eight 111 us where
+// four take 106: what crosses shared memory doubles).  As many help.
+constexpr int DC_WARPS = 4, DC_THREADS = 2 * DC_WARPS * 32;
+constexpr int DC_STAGES = 6;        // chunks under way at most
 
-// A warp holds NJ tiles of 8 channels of the state, transposed: S[j] is (column g or g + 8 of the block) x (channels 8 j + 2 t,
-// 8 j + 2 t + 1), g = lane / 4, t = lane % 4.
-template <int DP, int MODE>
-__global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const DeltaChunkArgs p) {
-    constexpr int NJ = DP / (8 * DC_WARPS);
+// The scan's two barriers: the holders arrive at SUMS and wait at READY, the helpers the other way round.
+enum { DC_SUMS = 1, DC_READY };
+template <int ID> __device__ __forceinline__ void dc_sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(DC_THREADS) : "memory"); }
+template <int ID> __device__ __forceinline__ void dc_arrive() { asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(DC_THREADS) : "memory"); }
+
+// Shared memory of a block of the scan, in floats, behind its `stages` buffers.
+template <int DP, int MODE> struct DeltaScan {
+    static constexpr bool GLA = MODE == CHUNK_GLA;
+    static constexpr int BUF = DeltaChunk<DP, MODE>::Y + DC * DC;    // a chunk's numbers and 16 columns of Y
+    static constexpr int OUTS = GLA ? 1 : 3;                         // (what a helper reads behind SUMS of the next chunk)
+    static constexpr int OUT = 0;                                    // [OUTS][warps][16 tokens][DC_ULD columns]: q S over a warp's channels
+    static constexpr int SUMS = OUT + OUTS * DC_WARPS * DC * DC_ULD;    // [warps][16 columns][DC_RLD]: W S over a warp's channels
+    static constexpr int U = SUMS + (GLA ? 0 : DC_WARPS * DC * DC_RLD); // [2][16 columns][DC_ULD]: U transposed
+    static constexpr int TWO = U + (GLA ? 0 : 2 * DC * DC_ULD);      // [2][16 columns][8 tokens][hi, lo]: the same, cut
+    static constexpr int END = TWO + (GLA ? 0 : 2 * DC * DC);
+    static constexpr size_t bytes(int stages) { return sizeof(float) * (size_t)(stages * BUF + END); }
+};
+
+// 16 rows by NJ tiles of 8 channels times the state's columns: what the tensor cores cut off instead of rounding is kept small, since a
+// large product is summed from zero and added up in 32 bits and the small ones have sums of their own.
+template <int NJ>
+__device__ __forceinline__ void rows_by_state(float2 (&sum)[2][2], const Two (&a)[NJ][4], const Two (&b)[NJ][2][2]) {
+    float low[2][4];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+        float high[2][4];
+        mma_two<2>(j == 0, low, high, a[j], b[j]);
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float2 v = make_float2(high[x][2 * e], high[x][2 * e + 1]);
+                sum[x][e] = j ? add2(sum[x][e], v) : v;
+            }
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) sum[x][e] = add2(sum[x][e], make_float2(low[x][2 * e], low[x][2 * e + 1]));
+}
+
+// DC_WARPS warps hold the state.  Such a warp holds NJ tiles of 8 channels of it, transposed: S[j] is (column g or g + 8 of the block) x
+// (channels 8 j + 2 t, 8 j + 2 t + 1), g = lane / 4, t = lane % 4.  It multiplies W with it, then q while the four helping warps add up
+// the holders' W S to U, then takes U into the state.  The helpers complete a chunk's outputs while the holders are at the next one.
+// (A warp that has given up a wait goes on through all chunks without waiting: nobody is left at a barrier.)
+template <int DP, int MODE, bool ALONE>
+__global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_kernel(const DeltaChunkArgs p, int stages) {
+    constexpr int NJ = DP / (8 * DC_WARPS), GROUP = NJ < 4 ? NJ : 4;
+    constexpr bool GLA = MODE == CHUNK_GLA, EARLY = ALONE && NJ <= 4, AHEAD = EARLY && !GLA;
     using Place = DeltaChunk<DP, MODE>;
-    constexpr int STAGES = DC_STAGES, BUF = Place::Y + DC * DC;      // floats of a buffer: the chunk's, and 16 columns of Y
-    constexpr int RG = Place::ROWS / 8;      // tiles of 8 rows of W and q
+    using Scan = DeltaScan<DP, MODE>;
+    constexpr int BUF = Scan::BUF;
     extern __shared__ __align__(16) float smem[];
-    __shared__ __align__(8) uint64_t full[STAGES];
+    __shared__ __align__(8) uint64_t full[DC_STAGES];
     __shared__ int gave_up;
-    float* red = smem + STAGES * BUF;       // [warps][16 columns][DC_RLD]: 32 sums over a warp's channels
-    float* UT = red + DC_WARPS * DC * DC_RLD;   // [16 columns][DC_ULD]: U transposed
-    float* OT = UT + DC * DC_ULD;           // the same of o's first part
+    float* const rest = smem + stages * BUF;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t2 = 2 * (lane & 3);
+    const bool holder = warp < DC_WARPS;
     if (tid == 0) {
-        for (int i = 0; i < STAGES; ++i) mbar_init(&full[i], 1);
+        for (int i = 0; i < DC_STAGES; ++i) mbar_init(&full[i], 1);
         gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -361,176 +453,241 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_kernel(const D
     const int row0 = por[0], tokens = por[1], slot = por[2], chunk0 = por[3];
     if (slot < 0) return;
     const int chunks = (tokens + DC - 1) / DC;
-    auto stage = [&](int i) {               // (one thread)
+    auto bring = [&](int i, int stage) {               // (one thread)
         const float* src = p.scratch + ((size_t)(chunk0 + i) * p.H + h) * p.stride;
-        float* dst = smem + (i % STAGES) * BUF;
-        uint64_t* bar = &full[i % STAGES];
-        mbar_expect_tx(bar, BUF * 4);
-        bulk_load(dst, src, Place::Y * 4, bar);
-        bulk_load(dst + Place::Y, src + Place::Y + col0 * DC, DC * DC * 4, bar);
+        float* dst = smem + stage * BUF;
+        mbar_expect_tx(&full[stage], BUF * 4);
+        bulk_load(dst, src, Place::Y * 4, &full[stage]);
+        bulk_load(dst + Place::Y, src + Place::Y + col0 * DC, DC * DC * 4, &full[stage]);
     };
     if (tid == 0)
-        for (int i = 0; i < min(STAGES - 1, chunks); ++i) stage(i);
-    const int r0 = warp * 8 * NJ;
-    float* st = p.state + ((size_t)slot * p.H + h) * p.d * p.dv;
-    float S[NJ][4];
-#pragma unroll
-    for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int r = r0 + 8 * j + t2 + (e & 1), c = col0 + g + 8 * (e >> 1);
-            S[j][e] = r < p.d && c < p.dv ? st[(size_t)r * p.dv + c] : 0.f;
-        }
-    // places that do not change from chunk to chunk
-    const int rows_at = g * DP + t2, swap = dc_key_place(g, 0);      // (of rows 8 j + g: the tile does not matter)
-    float* mine = red + (warp * DC + g) * DC_RLD + t2;
-    const int sum_c = tid >> 3, sum_t = 4 * (tid & 7);               // the four sums that this thread completes: column, rows
-    const float* sum_from = red + sum_c * DC_RLD + sum_t - (MODE == CHUNK_GLA && sum_t >= DC ? DC : 0);
-    float* sum_to = (sum_t < DC ? UT : OT - DC) + sum_c * DC_ULD + sum_t;
-    const int t0 = 8 * (warp & 1);                                   // warps 0 and 1: the tokens whose o they finish
-    float* out = p.out + ((size_t)(row0 + t0 + t2) * p.H + h) * p.dv + col0 + g;
-    const size_t out_row = (size_t)p.H * p.dv;
-    for (int i = 0; i < chunks; ++i) {
-        const float* buf = smem + (i % STAGES) * BUF;
-        const bool ok = mbar_wait(&full[i % STAGES], (i / STAGES) & 1, &gave_up);
-        // this chunk's numbers are there and everybody is done with the chunk before it
-        if (__syncthreads_or(!ok)) {
-            for (int x = 0; x < 32; ++x) __nanosleep(2000);      // (a copy on its way may still land)
-            if (tid == 0 && p.status) atomicExch(p.status, 9);
-            return;
-        }
-        if (tid == 0 && i + STAGES - 1 < chunks) stage(i + STAGES - 1);
-        // (the tensor cores cut sums off instead of rounding them: a large product is summed from zero and added up in 32 bits, the
-        // small ones have sums of their own, and so has what is added to the state)
-        float acc[RG][4], low[RG][4];
-#pragma unroll
-        for (int x = 0; x < RG; ++x)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[x][e] = low[x][e] = 0.f;
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-            const Two a[4] = {two_of(S[j][0]), two_of(S[j][2]), two_of(S[j][1]), two_of(S[j][3])};
-            const float* at = buf + rows_at + dc_row_place(g, r0 + 8 * j);
-            Two b[RG][2];
-#pragma unroll
-            for (int x = 0; x < RG; ++x) two_pair(b[x], at + 8 * x * DP);
-            // (the sums in turn: a product does not wait for the one before it)
-#pragma unroll
-            for (int x = 0; x < RG; ++x) mma_tf32(low[x], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[x][0].hi, b[x][1].hi);
-#pragma unroll
-            for (int x = 0; x < RG; ++x) mma_tf32(low[x], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].lo, b[x][1].lo);
-#pragma unroll
-            for (int x = 0; x < RG; ++x) {
-                float part[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_tf32(part, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[x][0].hi, b[x][1].hi);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) acc[x][e] += part[e];
-            }
-        }
-#pragma unroll
-        for (int x = 0; x < RG; ++x) {
-            *reinterpret_cast<float2*>(mine + 8 * x) = make_float2(acc[x][0] + low[x][0], acc[x][1] + low[x][1]);
-            *reinterpret_cast<float2*>(mine + 8 * DC_RLD + 8 * x) = make_float2(acc[x][2] + low[x][2], acc[x][3] + low[x][3]);
-        }
-        __syncthreads();
-        {   // the warps' sums in order: U = Y - W S (rows 0 .. 15 of 32), o's first part (the others)
-            float v[DC_WARPS][4];
-            if (MODE != CHUNK_GLA || sum_t >= DC)
-#pragma unroll
-                for (int w = 0; w < DC_WARPS; ++w) load4(sum_from + w * DC * DC_RLD, v[w]);
-            float y[4] = {0.f, 0.f, 0.f, 0.f};
-            if (sum_t < DC) load4(buf + Place::Y + sum_c * DC + sum_t, y);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (MODE != CHUNK_GLA || sum_t >= DC) {                   // (gated linear attention: u is v)
-                    const float sum = (v[0][e] + v[1][e]) + (v[2][e] + v[3][e]);
-                    y[e] = sum_t < DC ? y[e] - sum : sum;
-                }
-            }
-            if (i + 1 == chunks && sum_t < DC) {      // (of no token: nothing, also beside a state of infinities)
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (i * DC + sum_t + e >= tokens) y[e] = 0.f;
-            }
-            store4(sum_to, y);
-        }
-        __syncthreads();
-        Two u[2][4];                         // U transposed, tokens 0 .. 7 and 8 .. 15
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-            Two lo[2], hi[2];
-            two_pair(lo, UT + g * DC_ULD + 8 * x + t2);
-            two_pair(hi, UT + (g + 8) * DC_ULD + 8 * x + t2);
-            u[x][0] = lo[0]; u[x][1] = hi[0]; u[x][2] = lo[1]; u[x][3] = hi[1];
-        }
-        float more[2][NJ][4], less[NJ][4], o[4] = {0.f, 0.f, 0.f, 0.f}, o_low[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int i = 0; i < min(stages, chunks); ++i) bring(i, i);
+    bool ok = true;
+    int stage = 0, phase = 0, slot_out = 0;
+    if (holder) {
+        const int r0 = warp * 8 * NJ;
+        float* st = p.state + ((size_t)slot * p.H + h) * p.d * p.dv;
+        float2 S[NJ][2];                     // [column g, g + 8] (channels t2, t2 + 1)
 #pragma unroll
         for (int j = 0; j < NJ; ++j)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) more[0][j][e] = more[1][j][e] = less[j][e] = 0.f;
+            for (int e = 0; e < 4; ++e) {
+                const int r = r0 + 8 * j + t2 + (e & 1), c = col0 + g + 8 * (e >> 1);
+                (e & 1 ? S[j][e >> 1].y : S[j][e >> 1].x) = r < p.d && c < p.dv ? st[(size_t)r * p.dv + c] : 0.f;
+            }
+        const int swap = dc_key_place(g, 0);             // (of rows 8 j + g: the tile does not matter)
+        float* const sums_to = rest + Scan::SUMS + (warp * DC + g) * DC_RLD + t2;
+        float* const out_to = rest + Scan::OUT + (warp * DC + t2) * DC_ULD + g;
+        auto rows = [&](Two (&b)[NJ][2][2], const float* buf, int first) {           // of W or q: rows g and 8 + g
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-            Two k[NJ][2], w[2];
+            for (int j = 0; j < NJ; ++j) {
+                const float* at = buf + (first + g) * DP + t2 + dc_row_place(g, r0 + 8 * j);
+                two_pair(b[j][0], at);
+                two_pair(b[j][1], at + 8 * DP);
+            }
+        };
+        Two b[NJ][2][2];
+        ok = mbar_wait(&full[0], 0, &gave_up);
+        if constexpr (AHEAD) rows(b, smem, 0);
+        for (int i = 0; i < chunks; ++i) {
+            const float* buf = smem + stage * BUF;
+            if (++stage == stages) {
+                stage = 0;
+                phase ^= 1;
+            }
+            // (the next chunk's numbers are there by now, as a rule)
+            const bool there = i + 1 == chunks || mbar_try_wait(&full[stage], phase);
+            float2 sum[2][2];
+            Two a[NJ][4];
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                two_of_pair(a[j][0], a[j][2], S[j][0]);
+                two_of_pair(a[j][1], a[j][3], S[j][1]);
+            }
+            Two c[NJ][2][2];                     // (what is cut ahead of a product is cut between the one before it)
+            if constexpr (EARLY) rows(c, buf, Place::ROWS - DC);
+            if constexpr (!GLA) {
+                if constexpr (!AHEAD) rows(b, buf, 0);
+                rows_by_state(sum, a, b);
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) *reinterpret_cast<float2*>(sums_to + 8 * e * DC_RLD + 8 * x) = sum[x][e];
+                dc_arrive<DC_SUMS>();
+            }
+            if constexpr (!EARLY) rows(c, buf, Place::ROWS - DC);
+            Two k[2][GROUP][2], u[2][4];         // keys; U transposed, tokens 0 .. 7 and 8 .. 15
+            auto keys = [&](int j0) {
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int j = 0; j < GROUP; ++j)
+                        two_pair(k[x][j], buf + Place::KEYS + (r0 + 8 * (j0 + j) + g) * DC + ((8 * x) ^ swap) + t2);
+            };
+            if constexpr (EARLY) keys(0);
+            rows_by_state(sum, a, c);
+            if constexpr (!EARLY) keys(0);
+            if constexpr (GLA) {                 // (u is v; the helpers are done with the last chunk's sums)
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        two_of_pair(u[x][e], u[x][2 + e], *reinterpret_cast<const float2*>(buf + Place::Y + (g + 8 * e) * DC + 8 * x + t2));
+                if (i > 0) dc_sync<DC_READY>();
+            }
+            float* const to = out_to + slot_out * DC_WARPS * DC * DC_ULD;
+            if (++slot_out == Scan::OUTS) slot_out = 0;
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    to[8 * x * DC_ULD + 8 * e] = sum[x][e].x;
+                    to[(8 * x + 1) * DC_ULD + 8 * e] = sum[x][e].y;
+                }
+            if constexpr (GLA) dc_arrive<DC_SUMS>();
+            else {
+                dc_sync<DC_READY>();
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const uint4 z = *reinterpret_cast<const uint4*>(rest + Scan::TWO + x * DC * DC + (g + 8 * e) * DC + 2 * t2);
+                        u[x][e] = Two{z.x, z.y};
+                        u[x][2 + e] = Two{z.z, z.w};
+                    }
+            }
+            if (!there && ok) ok = mbar_wait(&full[stage], phase, &gave_up);
+            if constexpr (AHEAD) rows(b, smem + stage * BUF, 0);     // (between the products; of no chunk: what lies there, unused)
+#pragma unroll
+            for (int j0 = 0; j0 < NJ; j0 += GROUP) {
+                if (j0) keys(j0);
+                float more[2][GROUP][4], less[GROUP][4];
+#pragma unroll
+                for (int x = 0; x < 2; ++x) mma_two<GROUP>(x == 0, less, more[x], u[x], k[x]);
+#pragma unroll
+                for (int j = 0; j < GROUP; ++j) {
+                    const float2 left = *reinterpret_cast<const float2*>(buf + Place::LAST + r0 + 8 * (j0 + j) + t2);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const float2 x = make_float2(more[0][j][2 * e], more[0][j][2 * e + 1]), y = make_float2(more[1][j][2 * e], more[1][j][2 * e + 1]);
+                        S[j0 + j][e] = fma2(S[j0 + j][e], left, add2(x, add2(y, make_float2(less[j][2 * e], less[j][2 * e + 1]))));
+                    }
+                }
+            }
+        }
+        if constexpr (!GLA) dc_arrive<DC_SUMS>();      // (the last chunk's q S)
+        __syncthreads();
+        if (!gave_up) {
 #pragma unroll
             for (int j = 0; j < NJ; ++j)
-                two_pair(k[j], buf + Place::KEYS + (r0 + 8 * j + g) * DC + ((8 * x) ^ swap) + t2);
-            if (warp == 1 && x == 0) {       // o of tokens 8 .. 15: what tokens 0 .. 7 add, among the state's products
-                two_pair(w, buf + Place::P + (8 + g) * DC + swap + t2);
-                mma_tf32(o_low, u[0][0].lo, u[0][1].lo, u[0][2].lo, u[0][3].lo, w[0].hi, w[1].hi);
-            }
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) mma_tf32(less[j], u[x][0].lo, u[x][1].lo, u[x][2].lo, u[x][3].lo, k[j][0].hi, k[j][1].hi);
-            if (warp == 1 && x == 0) mma_tf32(o_low, u[0][0].hi, u[0][1].hi, u[0][2].hi, u[0][3].hi, w[0].lo, w[1].lo);
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) mma_tf32(less[j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].lo, k[j][1].lo);
-            if (warp == 1 && x == 0) mma_tf32(o, u[0][0].hi, u[0][1].hi, u[0][2].hi, u[0][3].hi, w[0].hi, w[1].hi);
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) mma_tf32(more[x][j], u[x][0].hi, u[x][1].hi, u[x][2].hi, u[x][3].hi, k[j][0].hi, k[j][1].hi);
+                for (int e = 0; e < 4; ++e) {
+                    const int r = r0 + 8 * j + t2 + (e & 1), c = col0 + g + 8 * (e >> 1);
+                    if (r < p.d && c < p.dv) st[(size_t)r * p.dv + c] = e & 1 ? S[j][e >> 1].y : S[j][e >> 1].x;
+                }
         }
+    } else {
+        const int mine = warp - DC_WARPS;
+        // the numbers of U that this thread completes, a column's tokens u_t and u_t + 1, and the outputs: a token and its mirror image
+        // (17 products in all)
+        const int u_c = 4 * mine + ((lane >> 2) & 3), u_t = 2 * (lane & 3) + 8 * (lane >> 4);
+        const int o_c = lane & 15, o_t = mine + 4 * (lane >> 4);
+        const float* const sums_from = rest + Scan::SUMS + u_c * DC_RLD + u_t;
+        float* const out = p.out + ((size_t)row0 * p.H + h) * p.dv + col0 + o_c;
+        const size_t out_row = (size_t)p.H * p.dv;
+        const bool in = col0 + o_c < p.dv;
+        float pa[DC / 2], pb[DC];                // of p: what the two tokens take of those up to them
+        auto rows_of_p = [&](const float* buf) {
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-            const float2 w = *reinterpret_cast<const float2*>(buf + Place::LAST + r0 + 8 * j + t2);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) S[j][e] = fmaf(S[j][e], e & 1 ? w.y : w.x, more[0][j][e] + (more[1][j][e] + less[j][e]));
-        }
-        if (warp < 2) {
-            float* to = out + (size_t)i * DC * out_row;
-            const float2 o_a = *reinterpret_cast<const float2*>(OT + g * DC_ULD + t0 + t2);
-            const float2 o_b = *reinterpret_cast<const float2*>(OT + (g + 8) * DC_ULD + t0 + t2);
-            const float first[4] = {o_a.x, o_a.y, o_b.x, o_b.y};
-            // what the eight tokens add to one another on the CUDA cores: only those up to a token itself, since a product with the
-            // zeros of p above the diagonal would carry a later token's infinity or NaN into this one's o
-            float pu[2][8], uu[2][8];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const float* row = buf + Place::P + (t0 + t2 + e) * DC + dc_key_place(t0 + t2 + e, t0);
-                const float* col = UT + (g + 8 * e) * DC_ULD + t0;
-                load4(row, *reinterpret_cast<float(*)[4]>(&pu[e][0]));
-                load4(row + 4, *reinterpret_cast<float(*)[4]>(&pu[e][4]));
-                load4(col, *reinterpret_cast<float(*)[4]>(&uu[e][0]));
-                load4(col + 4, *reinterpret_cast<float(*)[4]>(&uu[e][4]));
+            for (int s = 0; s < DC; s += 4) {
+                if (s < DC / 2) load4(buf + Place::P + o_t * DC + dc_key_place(o_t, s), *reinterpret_cast<float(*)[4]>(&pa[s]));
+                load4(buf + Place::P + (DC - 1 - o_t) * DC + dc_key_place(DC - 1 - o_t, s), *reinterpret_cast<float(*)[4]>(&pb[s]));
             }
+        };
+        // What the chunk's tokens add to one another, on the CUDA cores: only those up to a token itself, since a product with the
+        // zeros of p above the diagonal would carry a later token's infinity or NaN into this one's o.
+        auto outputs = [&](int i, const float* u_at) {
+            const float* sums_of = rest + Scan::OUT + slot_out * DC_WARPS * DC * DC_ULD + o_c;
+            if (++slot_out == Scan::OUTS) slot_out = 0;
+            float u[DC], va[DC_WARPS], vb[DC_WARPS];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float sum = o[e] + o_low[e];
+            for (int s = 0; s < DC; s += 4) load4(u_at + s, *reinterpret_cast<float(*)[4]>(&u[s]));
 #pragma unroll
-                for (int s = 0; s < 8; ++s)
-                    if (s <= t2 + (e & 1)) sum = fmaf(pu[e & 1][s], uu[e >> 1][s], sum);
-                o[e] = first[e] + sum;
+            for (int w = 0; w < DC_WARPS; ++w) {
+                va[w] = sums_of[(w * DC + o_t) * DC_ULD];
+                vb[w] = sums_of[(w * DC + DC - 1 - o_t) * DC_ULD];
             }
+            float o_a = 0.f, o_b = 0.f, late = 0.f;
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (i * DC + t0 + t2 + (e & 1) < tokens && col0 + g + 8 * (e >> 1) < p.dv)
-                    to[(e & 1) * out_row + 8 * (e >> 1)] = o[e];
+            for (int s = 0; s < DC / 2; ++s) {
+                if (s <= o_t) o_a = fmaf(pa[s], u[s], o_a);
+                o_b = fmaf(pb[s], u[s], o_b);
+                if (s < DC / 2 - o_t) late = fmaf(pb[DC / 2 + s], u[DC / 2 + s], late);
+            }
+            if (!in || !ok) return;
+            if (i * DC + o_t < tokens) out[(size_t)(i * DC + o_t) * out_row] = ((va[0] + va[1]) + (va[2] + va[3])) + o_a;
+            if (i * DC + DC - 1 - o_t < tokens) out[(size_t)(i * DC + DC - 1 - o_t) * out_row] = ((vb[0] + vb[1]) + (vb[2] + vb[3])) + (o_b + late);
+        };
+        for (int i = 0; i < chunks; ++i) {
+            const float* buf = smem + stage * BUF;
+            if (ok) ok = mbar_wait(&full[stage], phase, &gave_up);
+            float2 y = *reinterpret_cast<const float2*>(buf + Place::Y + u_c * DC + u_t);
+            dc_sync<DC_SUMS>();
+            if constexpr (!GLA) {
+                float2 v[DC_WARPS];
+#pragma unroll
+                for (int w = 0; w < DC_WARPS; ++w) v[w] = *reinterpret_cast<const float2*>(sums_from + w * DC * DC_RLD);
+                y = sub2(y, add2(add2(v[0], v[1]), add2(v[2], v[3])));
+                if (i * DC + u_t >= tokens) y.x = 0.f;       // (of no token: nothing, also beside a state of infinities)
+                if (i * DC + u_t + 1 >= tokens) y.y = 0.f;
+                Two one, two;
+                two_of_pair(one, two, y);
+                *reinterpret_cast<uint4*>(rest + Scan::TWO + (u_t >> 3) * DC * DC + u_c * DC + 2 * (u_t & 7)) = make_uint4(one.hi, one.lo, two.hi, two.lo);
+                *reinterpret_cast<float2*>(rest + Scan::U + (i & 1) * DC * DC_ULD + u_c * DC_ULD + u_t) = y;
+                dc_arrive<DC_READY>();
+            }
+            // everybody is done with the chunk before this one: its buffer may be filled again
+            if (tid == DC_WARPS * 32 && i > 0 && i - 1 + stages < chunks) bring(i - 1 + stages, stage ? stage - 1 : stages - 1);
+            if constexpr (GLA) {
+                rows_of_p(buf);
+                outputs(i, buf + Place::Y + o_c * DC);
+                if (i + 1 < chunks) dc_arrive<DC_READY>();
+            } else {
+                if (i > 0) outputs(i - 1, rest + Scan::U + ((i - 1) & 1) * DC * DC_ULD + o_c * DC_ULD);
+                rows_of_p(buf);
+            }
+            if (++stage == stages) {
+                stage = 0;
+                phase ^= 1;
+            }
         }
+        if constexpr (!GLA) {
+            dc_sync<DC_SUMS>();
+            outputs(chunks - 1, rest + Scan::U + ((chunks - 1) & 1) * DC * DC_ULD + o_c * DC_ULD);
+        }
+        __syncthreads();
     }
-#pragma unroll
-    for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int r = r0 + 8 * j + t2 + (e & 1), c = col0 + g + 8 * (e >> 1);
-            if (r < p.d && c < p.dv) st[(size_t)r * p.dv + c] = S[j][e];
-        }
+    if (gave_up) {
+        for (int x = 0; x < 32; ++x) __nanosleep(2000);      // (a copy on its way may still land)
+        if (tid == 0 && p.status) atomicExch(p.status, 9);
+    }
+}
+
+template <int DP, int MODE, bool ALONE>
+static int launch_delta_scan(const DeltaChunkArgs& a, dim3 grid, size_t room, size_t least, cudaStream_t stream) {
+    using Scan = DeltaScan<DP, MODE>;
+    int stages = DC_STAGES;
+    while (stages > 2 && Scan::bytes(stages) > room) --stages;
+    const size_t smem = max(Scan::bytes(stages), least);
+    auto kernel = delta_chunk_scan_kernel<DP, MODE, ALONE>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(DC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    return launch_counted(cfg, kernel, a, stages);
 }
 
 template <int DP, int MODE>
@@ -545,22 +702,18 @@ static int launch_delta_chunks(const DeltaChunkArgs& args, int N, int L, cudaStr
     }
     int rc = launch(delta_chunk_prepare_kernel<DP, MODE>, dim3(N, a.H), 256, smem1, stream, a);
     if (rc) return rc;
-    size_t smem2 = sizeof(float) * (DC_STAGES * (DeltaChunk<DP, MODE>::Y + DC * DC) + DC_WARPS * DC * DC_RLD + 2 * DC * DC_ULD);
     const dim3 grid(a.dvp / DC, a.H, L);
     // (as for the scan token by token: the blocks start when their predecessor has ended, and spread over the SMs)
     int sms = 148, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long blocks = (long long)grid.x * grid.y * grid.z;
-    if (blocks <= sms && smem2 < 120 * 1024) smem2 = 120 * 1024;
-    cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
-    if (e != cudaSuccess) return (int)e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(DC_WARPS * 32);
-    cfg.dynamicSmemBytes = smem2;
-    cfg.stream = stream;
-    return launch_counted(cfg, delta_chunk_scan_kernel<DP, MODE>, a);
+    // Where every block has an SM to itself, or only one block's memory fits, a warp has the registers to cut what its next product
+    // reads between the instructions of the one before, and as many chunks are under way as memory holds; else two blocks share an SM.
+    // (32 heads of 128 x 128, 256 blocks, 2,048 tokens: 192 us; with one block to an SM they would take two rounds of 106.)
+    if constexpr (DP <= 128)
+        if (blocks > sms) return launch_delta_scan<DP, MODE, false>(a, grid, 113 * 1024, 0, stream);
+    return launch_delta_scan<DP, MODE, true>(a, grid, 226 * 1024, blocks <= sms ? 120 * 1024 : 0, stream);
 }
 
 }  // namespace air

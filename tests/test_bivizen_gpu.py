@@ -276,6 +276,37 @@ def test_chunks_carry_infinities_and_nans_as_token_by_token_does(what, value, mo
         assert torch.isfinite(got[1][0][:at]).all(), "nothing runs backwards"
 
 
+@pytest.mark.parametrize("mode", ["delta", "gla", "channel"])
+@pytest.mark.parametrize("H,d,dv", [(12, 32, 40), (10, 64, 64), (8, 128, 128), (4, 256, 96), (12, 100, 17)])
+def test_chunks_of_many_portions_are_those_of_each_alone(H, d, dv, mode):
+    """Portions from one token to more chunks than are under way at a time, in a batch of more blocks than there are SMs and one by
+    one (blocks that share an SM, and blocks that have one to themselves): the same bits, outputs and states."""
+    from air_b200.csrc import ops
+    counts = [1, 16, 17, 97, 113, 15, 130]
+    which = {"delta": ops.SCAN_DELTA, "gla": ops.SCAN_GLA, "channel": ops.SCAN_CHANNEL_DELTA}[mode]
+    per, T, L = (H if mode == "delta" else H * d), sum(counts), len(counts)
+    assert L * H * -(-dv // 16) > 148 >= H * -(-dv // 16)
+    g = torch.Generator(device=DEV).manual_seed(d)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    q, k, v, z, b, S0 = rand(T, H * d), rand(T, H * d), rand(T, H * dv), rand(T, per), rand(T, H), rand(L, H, d, dv)
+    more = dict(tau=8.0) if mode == "gla" else dict(beta=b, a_log=rand(H) / 2, dt_bias=rand(per))
+    start = np.concatenate([[0], np.cumsum(counts)])
+    table = lambda rows: torch.tensor(np.array(rows), dtype=torch.int32, device=DEV)
+    portions, chunks = [], []
+    for i, n in enumerate(counts):
+        portions.append((start[i], n, i, len(chunks)))
+        chunks += [(start[i] + a, min(ops.DELTA_CHUNK, n - a)) for a in range(0, n, ops.DELTA_CHUNK)]
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got = []
+    for tables in ([portions], [[row] for row in portions]):
+        S, o = S0.clone(), torch.full((T, H, dv), 9.0, device=DEV)
+        for rows in tables:
+            ops.delta_portions(q, k, v, z, S, o, table(rows), table(chunks), d ** -0.5, mode=which, status=status, **more)
+        got.append((o, S))
+    assert int(status) == 0
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 def test_gated_norm_feed_forward_activation_and_scaled_sum():
     from air_b200.csrc import ops
     rng = np.random.default_rng(5)
