@@ -504,7 +504,7 @@ grouped_attention_tc_kernel(const void* __restrict__ q_any, int q_f32, const __n
     }
 }
 
-constexpr int GC_SPLITS = 64;
+constexpr int GC_SPLITS = 64, GC_COLUMNS = 4;      // of a thread at a time
 
 template <typename T>
 __global__ void __launch_bounds__(128)
@@ -513,44 +513,73 @@ grouped_combine_kernel(const float* __restrict__ part, const int* __restrict__ t
                        const TurnBack turn) {
     __shared__ float row[1024];
     pdl_enter(TR_ATT_GROUPED);
-    const int t = blockIdx.x, h = blockIdx.y;
+    const int t = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31;
     if (token_seq[t] < 0) return;
-    // A split's weight once per block, then a thread's columns through all splits with their loads side by side: 17 us for 256
-    // rows of 9 splits of 512 when every thread worked out every split's weight between its loads.
+    // A split's weight once per block, then a thread's columns through all splits with their loads side by side, eight splits at a time;
+    // a split that saw no key has left nothing to add and is not read.  (256 rows of 9 splits of 512: 17 us when every thread worked
+    // out every split's weight between its loads, 8 when the splits behind the first eight came one by one.)
     __shared__ float weight[GC_SPLITS];
     const float* p = part + ((size_t)t * H + h) * splits * (dv + 2);
-    float m = sink ? sink[h] : -INFINITY, own = -INFINITY;
-    for (int s = threadIdx.x & 31; s < splits; s += 32) own = fmaxf(own, p[(size_t)s * (dv + 2) + dv]);
+    float m = sink ? sink[h] : -INFINITY, ms[GC_SPLITS / 32], ls[GC_SPLITS / 32], own = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < GC_SPLITS / 32; ++i) {
+        const int s = lane + 32 * i;
+        ms[i] = s < splits ? p[(size_t)s * (dv + 2) + dv] : -INFINITY;
+        ls[i] = s < splits ? p[(size_t)s * (dv + 2) + dv + 1] : 0.f;
+        own = fmaxf(own, ms[i]);
+    }
+    for (int s = GC_SPLITS + lane; s < splits; s += 32) own = fmaxf(own, p[(size_t)s * (dv + 2) + dv]);
     m = fmaxf(m, warp_max(own));
     float mine = 0.f;
-    for (int s = threadIdx.x & 31; s < splits; s += 32) {
-        const float ms = p[(size_t)s * (dv + 2) + dv];
-        const float w = ms != -INFINITY ? expf(ms - m) : 0.f;
-        mine = fmaf(p[(size_t)s * (dv + 2) + dv + 1], w, mine);
-        if (threadIdx.x < 32 && s < GC_SPLITS) weight[s] = w;
+#pragma unroll
+    for (int i = 0; i < GC_SPLITS / 32; ++i) {
+        const float w = ms[i] != -INFINITY ? expf(ms[i] - m) : 0.f;
+        mine = fmaf(ls[i], w, mine);
+        if (threadIdx.x < 32) weight[lane + 32 * i] = w;
+    }
+    for (int s = GC_SPLITS + lane; s < splits; s += 32) {
+        const float far = p[(size_t)s * (dv + 2) + dv];
+        mine = fmaf(p[(size_t)s * (dv + 2) + dv + 1], far != -INFINITY ? expf(far - m) : 0.f, mine);
     }
     const float total = warp_sum(mine) + (sink ? expf(sink[h] - m) : 0.f);
     const float inv = 1.f / total;
     __syncthreads();
-    for (int c = threadIdx.x; c < dv; c += blockDim.x) {
-        float o = 0.f;
-#pragma unroll 8
-        for (int s = 0; s < min(splits, GC_SPLITS); ++s) {
-            const float w = weight[s];
-            const float v = p[(size_t)s * (dv + 2) + c];
-            if (w != 0.f) o = fmaf(v, w, o);          // (a split that saw no key has left nothing to add)
+    for (int c0 = threadIdx.x; c0 < dv; c0 += 128 * GC_COLUMNS) {
+        float sum[GC_COLUMNS];
+#pragma unroll
+        for (int i = 0; i < GC_COLUMNS; ++i) sum[i] = 0.f;
+        for (int s0 = 0; s0 < min(splits, GC_SPLITS); s0 += 8) {
+            float w[8], v[8][GC_COLUMNS];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                w[s] = weight[s0 + s];                     // (0 from `splits` on)
+#pragma unroll
+                for (int i = 0; i < GC_COLUMNS; ++i)
+                    v[s][i] = w[s] != 0.f && c0 + 128 * i < dv ? p[(size_t)(s0 + s) * (dv + 2) + c0 + 128 * i] : 0.f;
+            }
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+#pragma unroll
+                for (int i = 0; i < GC_COLUMNS; ++i)
+                    if (w[s] != 0.f) sum[i] = fmaf(v[s][i], w[s], sum[i]);
         }
-        for (int s = GC_SPLITS; s < splits; ++s) {
-            const float ms = p[(size_t)s * (dv + 2) + dv];
-            if (ms != -INFINITY) o += p[(size_t)s * (dv + 2) + c] * expf(ms - m);
+#pragma unroll
+        for (int i = 0; i < GC_COLUMNS; ++i) {
+            const int c = c0 + 128 * i;
+            if (c >= dv) break;
+            float o = sum[i];
+            for (int s = GC_SPLITS; s < splits; ++s) {
+                const float far = p[(size_t)s * (dv + 2) + dv];
+                if (far != -INFINITY) o += p[(size_t)s * (dv + 2) + c] * expf(far - m);
+            }
+            if (turn.freq) {
+                row[c] = o * inv;
+                continue;
+            }
+            // (a gate per output element: the logits' sigmoid multiplies as the row is written)
+            const float g = gate ? 1.f / (1.f + expf(-gate[(size_t)t * ldg + h * dv + c])) : 1.f;
+            out[((size_t)t * H + h) * dv + c] = from_float<T>(o * inv * g);
         }
-        if (turn.freq) {
-            row[c] = o * inv;
-            continue;
-        }
-        // (a gate per output element: the logits' sigmoid multiplies as the row is written)
-        const float g = gate ? 1.f / (1.f + expf(-gate[(size_t)t * ldg + h * dv + c])) : 1.f;
-        out[((size_t)t * H + h) * dv + c] = from_float<T>(o * inv * g);
     }
     if (!turn.freq) return;
     __syncthreads();         // the whole row first, then its elements turned back in pairs
@@ -640,6 +669,15 @@ AIR_API int air_grouped_attention(const void* q, int q_f32, const void* cache, i
                            H, dv, splits, gate, ldg, turn);
     });
     return 0;
+}
+
+// The merge alone, bfloat16 out (for attention_latent.cu).
+AIR_API int air_grouped_combine(const float* part, const int* token_seq, const float* sink, void* out, int T, int H, int dv, int splits,
+                                const float* gate, int ldg, const double* turn_freq, int turn_rot, int turn_pairing,
+                                const int* positions, cudaStream_t stream) {
+    const air::TurnBack turn{turn_freq, turn_rot, turn_pairing, positions};
+    return air::launch(air::grouped_combine_kernel<__nv_bfloat16>, dim3(T, H), 128, 0, stream, part, token_seq, sink, (__nv_bfloat16*)out, H,
+                       dv, splits, gate, ldg, turn);
 }
 
 AIR_API int air_trace_set_attention_grouped(unsigned long long* buffer) { return air::set_trace_here(buffer); }

@@ -106,6 +106,9 @@ _SIGNATURES = {
     "air_glu": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_void_p],
     "air_scaled_norm": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_int,
                         c_void_p, c_int, c_void_p, c_int, c_int, c_float, c_void_p],
+    "air_latent_attention": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                             c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_int, c_int,
+                             c_void_p, c_void_p],
     "air_table_update": [c_void_p, c_void_p, c_int, c_int, c_void_p],
     "air_decode_attention": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                              c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
@@ -557,7 +560,7 @@ def grouped_attention_ok(cache_dtype, d, dv) -> bool:
 
 
 def grouped_attention(q, cache, block_table, token_seq, positions, out, window, scale, kv_heads=1, page_tokens=None,
-                      chunk=None, sink=None, latent=False, splits=None, softcap=0.0, gate=None, turn=None, bias=None):
+                      chunk=None, sink=None, latent=False, splits=None, softcap=0.0, gate=None, turn=None, bias=None, status=None):
     """paged_attention_ref's arithmetic and arguments (32-bit, any batch, window or chunk, sink, latent rows, bias), by the
     kernel in which a block serves all query heads of a key/value head and the keys of a token are split over
     `splits` blocks (default: enough to fill the device); needs grouped_attention_ok(cache.dtype, d, dv).  gate (float32
@@ -593,6 +596,21 @@ def grouped_attention(q, cache, block_table, token_seq, positions, out, window, 
     if window and chunk:
         raise KernelError("grouped_attention: a window or a chunk, not both")
     J = H // G
+    if (latent and splits is None and bias is None and q.dtype == torch.float32 and cache.dtype == torch.bfloat16 and d % 64 == 0 and d <= 576
+            and dv % 128 == 0 and dv <= 512 and (P % 64 == 0 if P >= 64 else P >= 8 and 64 % P == 0)):
+        # rows that the tcgen05 kernel takes (attention_latent.cu): up to 32 heads to a block, a block to an SM.  (At most 24 parts of a
+        # token's keys, us with 16, 24 and 32: one token at 32 heads over 4,096 keys 21.7, 17.6, 18.0, over 8,191 27.0, 22.9, 19.3; four
+        # tokens over 1,000 13.5, 13.9, 16.0, over 4,096 22.1, 18.8, 22.5)
+        splits = max(1, min(24, 148 // (T * (1 if H <= 16 else -(-H // 32)))))
+        part = empty((T, H, splits, dv + 2), torch.float32, q.device)
+        _check(_get("air_latent_attention")(
+            q.data_ptr(), cache.data_ptr(), cache.shape[0], block_table.data_ptr(), block_table.shape[1], token_seq.data_ptr(),
+            positions.data_ptr(), part.data_ptr(), out.data_ptr(), T, H, d, dv, P, int(chunk or window or 0), float(scale),
+            1 if chunk else 0, _ptr(sink), splits, float(softcap or 0.0), gp, ldg, *_turn(turn, dv), _ptr(status), _stream()),
+            "latent_attention")
+        global launches
+        launches += 1
+        return out
     if splits is None:
         # float32: always the same number, so that a row's sums do not depend on what else is in the batch;
         # bfloat16: as many as fill the device
@@ -606,7 +624,6 @@ def grouped_attention(q, cache, block_table, token_seq, positions, out, window, 
         block_table.shape[1], token_seq.data_ptr(), positions.data_ptr(), part.data_ptr(), out.data_ptr(), T, H, G, d,
         dv, P, int(chunk or window or 0), float(scale), 1 if chunk else 0, _ptr(sink), 1 if latent else 0, int(splits),
         float(softcap or 0.0), gp, ldg, *_turn(turn, dv), *_distance_bias(bias, H), _stream()), "grouped_attention")
-    global launches
     launches += 1
     return out
 

@@ -84,7 +84,7 @@ class PortionAttention:
             if ops.grouped_attention_ok(cache.dtype, q.shape[2], out.shape[2]):
                 ops.grouped_attention(q, cache, bt, token_seq, ctx.positions, out, self.window, self.scale,
                                       kv_heads=kv_heads, page_tokens=page_tokens, chunk=self.chunk, sink=sinks,
-                                      latent=latent, softcap=softcap, gate=gate, turn=turn, bias=bias)
+                                      latent=latent, softcap=softcap, gate=gate, turn=turn, bias=bias, status=ctx.status)
                 return
             ops.paged_attention_ref(q, cache, bt, token_seq, ctx.positions, out, self.window, self.scale,
                                     kv_heads=kv_heads, page_tokens=page_tokens, chunk=self.chunk, sink=sinks,

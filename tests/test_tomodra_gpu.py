@@ -753,6 +753,72 @@ def test_expert_stream_in_wide_tiles(T, top, n, E, F):
             assert (outs[1][2][c, t].double() - want).abs().max() <= 0.01 * want.abs().max()
 
 
+@pytest.mark.parametrize("H,d,dv,P", [(16, 576, 512, 64), (32, 576, 512, 64), (40, 576, 512, 16), (3, 320, 256, 128), (17, 128, 128, 32), (20, 192, 128, 8)])
+@pytest.mark.parametrize("kind", ["plain", "window", "chunk", "cap", "sink", "rising"])
+def test_single_tokens_over_latents_on_the_tensor_cores(H, d, dv, P, kind):
+    """Contexts around a tile's edges, from one key to more tiles than there are parts, in one batch with a padded row: against 64-bit
+    attention over the seen rows, with NaN in every row of the pages that no token sees, scores that rise from tile to tile (the reference
+    maximum moves), and steps captured in a graph."""
+    from air_b200.csrc import ops
+    contexts = [0, 62, 63, 64, 127, 128, 700, 1700, 2600]
+    T, rot, scale = len(contexts) + 1, d - dv, (dv + 32) ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(H + d)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    need = [-(-(c + 1) // P) for c in contexts]
+    order = torch.randperm(sum(need) + 3, generator=torch.Generator().manual_seed(d))
+    rows = torch.full((sum(need) + 3, P, d), float("nan"), device="cuda", dtype=torch.bfloat16)
+    table = torch.full((T, max(need)), -1, dtype=torch.int32)
+    q, past, at = rand(T, H, d) * 1.5, [], 0
+    for i, (c, k) in enumerate(zip(contexts, need)):
+        table[i, :k] = order[at:at + k].int()
+        at += k
+        x = rand(c + 1, d)
+        if kind == "rising":            # keys along the first head's query, longer and longer
+            x = x * 0.2 + q[i, 0] / q[i, 0].norm() * torch.linspace(0, 60, c + 1, device="cuda")[:, None]
+        past.append(x.bfloat16())
+        full = torch.full((k * P, d), float("nan"), device="cuda", dtype=torch.bfloat16)
+        full[:c + 1] = past[-1]
+        rows[table[i, :k].long().cuda()] = full.view(k, P, d)
+    window, chunk = (100 if kind == "window" else None), (96 if kind == "chunk" else None)
+    if window or chunk:                 # what no token sees may hold anything, ahead of the first key too
+        for i, c in enumerate(contexts):
+            lo = max(0, c - window + 1) if window else c - c % chunk
+            for key in range(lo):
+                rows[table[i, key // P], key % P] = float("nan")
+    sink = rand(H) if kind == "sink" else None
+    cap = 20.0 if kind == "cap" else 0.0
+    seq = torch.tensor(list(range(len(contexts))) + [-1], dtype=torch.int32, device="cuda")
+    pos = torch.tensor(contexts + [0], dtype=torch.int32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.full((T, H, dv), 7.0, device="cuda", dtype=torch.bfloat16)
+    table = table.cuda()
+    call = lambda: ops.grouped_attention(q, rows, table, seq, pos, out, window, scale, latent=True, chunk=chunk, sink=sink, softcap=cap,
+                                         status=status)
+    call()
+    first = out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    out.fill_(7.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert status.item() == 0 and torch.equal(out, first)
+    assert (out[-1] == 7.0).all(), "a padded row is not touched"
+    for i, c in enumerate(contexts):
+        lo = max(0, c - window + 1) if window else c - c % chunk if chunk else 0
+        keys = past[i][lo:].double()
+        s = q[i].double() @ keys.t() * scale
+        s = cap * torch.tanh(s / cap) if cap else s
+        if sink is not None:
+            s = torch.cat([s, sink.double()[:, None]], dim=1)
+        p = torch.softmax(s, dim=1)[:, :keys.shape[0]]
+        want = p @ keys[:, :dv]
+        # (the output's rounding to 8 bits, 2^-8 of a number at most; queries and weights as two such halves each, to 2^-16 of what they are
+        # multiplied with)
+        bound = 2.0 ** -8 * want.abs() + 2.0 ** -16 * (p @ keys[:, :dv].abs()) + 2.0 ** -16 * (q[i].double().abs() @ keys.abs().t() * scale).max() * keys.abs().max()
+        assert ((first[i].double() - want).abs() <= bound).all(), (i, float(((first[i].double() - want).abs() / bound).max()))
+
+
 def test_a_rows_experts_do_not_depend_on_the_rows_beside_it():
     """A mixture in bfloat16: a row's planes are the same, bit for bit, in every step of up to 64 rows, and in every longer one on
     the stream of weights; their sums are those of the 64-bit experts."""
