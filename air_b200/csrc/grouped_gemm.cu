@@ -347,6 +347,76 @@ grouped_gemm_tc_kernel(const GroupedArgs p) {
     }
 }
 
+// A product per head over a step's few rows (bfloat16, no lists) whose matrices no kernel writes, in one go: a block has GH_BN rows of W_g and up
+// to GH_ROWS rows of A, all of k, in shared memory.  The kernel above is a chain of K / 32 stages, each a round trip that three others
+// hide in part.  Here W is asked for at once, while the kernel ahead is still running, and the rows of A when that one has ended; the
+// products are W's rows as the instruction's 16 rows by 8 rows of A, in the order of k as above (the same bits).
+// Measured, us, the kernel above and this one: 32 heads of 512 x 128 (out x in), 1, 8, 16, 20 and 32 rows 4.2 and 2.6, 4.3 and 2.8, 4.7 and 3.6, 4.9 and
+// 4.4, 5.2 and 5.1; 128 x 512, 8, 32 and 64 rows 7.4 and 3.3, 8.0 and 6.0, 9.0 and 7.2; 16 heads of 192 x 1,024, 8 and 64 rows 12.4 and 4.1, 15.1 and
+// 12.9.  From some 24 rows on a k below 256 is a short chain above and its tiles of 64 rows serve all of them.
+constexpr int GH_BN = 32, GH_ROWS = 32, GH_MOST_K = 1024;
+struct HeadsArgs {
+    const __nv_bfloat16* A; long long lda, a_group_stride;
+    const __nv_bfloat16* W; long long w_group_stride;
+    void* out; long long ldo, o_group_stride; int out_f32;
+    int rows, N, K;
+    const float* o_scale; int o_scale_ld;
+};
+__global__ void __launch_bounds__(128) heads_gemm_kernel(const HeadsArgs p) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    const int ld = p.K + 8, pieces = p.K / 8;                // (rows 16 bytes apart in the banks)
+    __nv_bfloat16* sw = reinterpret_cast<__nv_bfloat16*>(smem_raw);
+    __nv_bfloat16* sa = sw + GH_BN * ld;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = blockIdx.z, n0 = blockIdx.x * GH_BN, t0 = blockIdx.y * GH_ROWS;
+    const int rows = min(GH_ROWS, p.rows - t0);
+    pdl_trigger();
+    const __nv_bfloat16* W = p.W + (size_t)g * p.w_group_stride + (size_t)n0 * p.K;
+    for (int r = warp; r < GH_BN; r += 4)
+        for (int c = lane; c < pieces; c += 32) cp_async16(sw + r * ld + c * 8, W + (size_t)r * p.K + c * 8, n0 + r < p.N);
+    pdl_wait();
+    trace_point(TR_GROUPED_GEMM);
+    const __nv_bfloat16* A = p.A + (size_t)t0 * p.lda + (size_t)g * p.a_group_stride;
+    const int up = (rows + 7) / 8 * 8;                       // (rows of zeros up to whole eights)
+    for (int r = warp; r < up; r += 4)
+        for (int c = lane; c < pieces; c += 32)
+            cp_async16(sa + r * ld + c * 8, A + (size_t)(r < rows ? r : 0) * p.lda + c * 8, r < rows);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    // warps 0 and 2 take W's first 16 rows, 1 and 3 the others; eights of A's rows go round between the two
+    const uint32_t w_at = (uint32_t)__cvta_generic_to_shared(sw + ((warp & 1) * 16 + (lane & 15)) * ld + (lane >> 4) * 8);
+    const int gq = lane >> 2, tq = lane & 3, n = n0 + (warp & 1) * 16 + gq;
+    for (int e = warp >> 1; e * 8 < rows; e += 2) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint32_t a_at = (uint32_t)__cvta_generic_to_shared(sa + (e * 8 + (lane & 7)) * ld + (lane >> 3) * 8);
+        int k = 0;
+#pragma unroll 4
+        for (; k + 32 <= p.K; k += 32) {
+            uint32_t w0[4], w1[4], b[4];
+            ldmatrix_x4(w0, w_at + k * 2);
+            ldmatrix_x4(w1, w_at + k * 2 + 32);
+            ldmatrix_x4(b, a_at + k * 2);
+            mma_bf16_16816(acc, w0[0], w0[1], w0[2], w0[3], b[0], b[1]);
+            mma_bf16_16816(acc, w1[0], w1[1], w1[2], w1[3], b[2], b[3]);
+        }
+        if (k < p.K) {
+            uint32_t w0[4], b[4];
+            ldmatrix_x4(w0, w_at + k * 2);
+            ldmatrix_x4(b, a_at + k * 2 - (lane >> 4) * 32);      // (the second half's addresses are the first's: not used)
+            mma_bf16_16816(acc, w0[0], w0[1], w0[2], w0[3], b[0], b[1]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = e * 8 + 2 * tq + (i & 1), col = n + 8 * (i >> 1);
+            if (row >= rows || col >= p.N) continue;
+            const long long at = (t0 + row) * p.ldo + (long long)g * p.o_group_stride + col;
+            const float v = acc[i] * (p.o_scale ? p.o_scale[(long long)(t0 + row) * p.o_scale_ld + g] : 1.f);
+            if (p.out_f32) ((float*)p.out)[at] = v;
+            else ((__nv_bfloat16*)p.out)[at] = __float2bfloat16_rn(v);
+        }
+    }
+}
+
 }  // namespace air
 
 AIR_API int air_grouped_gemm(const void* A, long long lda, long long a_group_stride, const int* a_index, int a_div,
@@ -387,6 +457,26 @@ AIR_API int air_grouped_gemm(const void* A, long long lda, long long a_group_str
         return air::launch(air::grouped_gemm_kernel<TT, 0>, grid, 256, 0, stream, p);
     });
     return 0;
+}
+
+// C_g [rows, N] = A_g W_g^T per head g for up to 64 rows: A's row r at r * lda + g * a_group_stride, C's at r * ldo + g * o_group_stride, times
+// o_scale[r * o_scale_ld + g] (or null); K a multiple of 16 up to 1,024, W [groups, N, K].  W is read ahead of the kernel's wait for its
+// predecessor: no kernel may be writing it.
+AIR_API int air_heads_gemm(const void* A, long long lda, long long a_group_stride, const void* W, void* out, long long ldo,
+                           long long o_group_stride, int out_f32, int rows, int groups, int N, int K, const float* o_scale, int o_scale_ld,
+                           cudaStream_t stream) {
+    using namespace air;
+    if (rows <= 0 || N <= 0 || groups <= 0) return 0;
+    if (rows > 2 * GH_ROWS || K <= 0 || K % 16 || K > GH_MOST_K || lda % 8 || a_group_stride % 8 || (((uintptr_t)A | (uintptr_t)W) & 15) || groups > 65535)
+        return AIR_ERR_BAD_ARGUMENT;
+    const size_t smem = (size_t)(GH_BN + min(GH_ROWS, (rows + 7) / 8 * 8)) * (K + 8) * 2;
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(heads_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    const HeadsArgs h{(const __nv_bfloat16*)A, lda, a_group_stride, (const __nv_bfloat16*)W, (long long)N * K, out, ldo, o_group_stride,
+                      out_f32, rows, N, K, o_scale, o_scale_ld};
+    return launch(heads_gemm_kernel, dim3((N + GH_BN - 1) / GH_BN, (rows + GH_ROWS - 1) / GH_ROWS, groups), 128, smem, stream, h);
 }
 
 AIR_API int air_trace_set_grouped_gemm(unsigned long long* buffer) { return air::set_trace_here(buffer); }

@@ -109,6 +109,8 @@ _SIGNATURES = {
     "air_latent_attention": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                              c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_int, c_int,
                              c_void_p, c_void_p],
+    "air_heads_gemm": [c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_longlong, c_longlong, c_int, c_int, c_int, c_int, c_int,
+                       c_void_p, c_int, c_void_p],
     "air_table_update": [c_void_p, c_void_p, c_int, c_int, c_void_p],
     "air_decode_attention": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                              c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
@@ -1028,14 +1030,15 @@ def moe_sort(expert, experts, start, pair_of_slot, tiles, num_tiles, tile_rows=G
 def grouped_gemm(a, w, out, n, k, *, lda, ldo, groups, a_group_stride=0, o_group_stride=0, a_index=None, a_div=1,
                  a_scale=None, a_local=False, o_index=None, o_div=1, o_part_stride=0, o_local=False, start=None,
                  rows_per_group=0, tiles=None, num_tiles=None, silu_mul=False, gate_block=0, o_scale=None, o_scale_ld=0,
-                 relu2=False, act=(1.0, 0.0, 0.0)):
+                 relu2=False, act=(1.0, 0.0, 0.0), w_ready=False):
     """out rows = a rows @ w[g]^T for every group g (w [groups, n (2n with silu_mul), k]); see grouped_gemm.cu for how
     rows are found.  Strides in elements.  out is float32 or of a's type; with silu_mul out = silu(gate) * linear, the
     rows of w[g] being blocks of gate_block gate rows and as many linear rows in turn (0: all gate rows first); act =
     (alpha, limit, shift) is then the gated activation as gemm_tc describes it (default: SiLU).
     o_scale float32: the row written for slot s is multiplied, in 32-bit, by o_scale[o_index[s]], or without o_index by
     o_scale[row * o_scale_ld + g] (row: the row of out, inside the group where o_local).  relu2: out = max(product, 0)^2
-    in a's type."""
+    in a's type.  w_ready: w was there long before (no kernel of this stream may still be writing it): a product per head over
+    few rows then asks for it ahead of its turn, the same bits (heads_gemm_kernel)."""
     if relu2 and (silu_mul or out.dtype != a.dtype):
         raise KernelError("grouped_gemm: the squared relu is written in the input's type, and is not gated")
     _req(a, "a", _FLOATS)
@@ -1051,6 +1054,14 @@ def grouped_gemm(a, w, out, n, k, *, lda, ldo, groups, a_group_stride=0, o_group
         _req(a_scale, "a_scale", (torch.float32,))
     if o_scale is not None:
         _req(o_scale, "o_scale", (torch.float32,))
+    if (w_ready and a.dtype == torch.bfloat16 and a_local and o_local and not (silu_mul or relu2) and start is None and a_index is None
+            and o_index is None and 0 < rows_per_group <= (64 if k >= 256 else 24) and k % 16 == 0 and k <= 1024 and lda % 8 == 0
+            and a_group_stride % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
+        _check(_get("air_heads_gemm")(
+            a.data_ptr(), int(lda), int(a_group_stride), w.data_ptr(), out.data_ptr(), int(ldo), int(o_group_stride),
+            1 if out.dtype == torch.float32 else 0, int(rows_per_group), int(groups), int(n), int(k), _ptr(o_scale), int(o_scale_ld),
+            _stream()), "heads_gemm")
+        return out
     _check(_get("air_grouped_gemm")(
         a.data_ptr(), int(lda), int(a_group_stride), _ptr(a_index), int(a_div), 1 if a_local else 0, _ptr(a_scale),
         w.data_ptr(), w.shape[1] * w.shape[2], out.data_ptr(), int(ldo), int(o_group_stride), _ptr(o_index), int(o_div),

@@ -233,11 +233,11 @@ class LatentAttention(PortionAttention, Mixer):
         out = ops.empty((T, H, dv), rt.dtype, dev)
         if rows:
             ops.grouped_gemm(q_plain, self.uk_t, q_full, R, d, lda=H * d, ldo=H * (R + rot), groups=H, a_group_stride=d,
-                             o_group_stride=R + rot, a_local=True, o_local=True, rows_per_group=rows)
+                             o_group_stride=R + rot, a_local=True, o_local=True, rows_per_group=rows, w_ready=True)
             summed = ops.empty((T, H, R), rt.dtype, dev)
             self.attend(q_full, latent.rows, bt, ctx, summed, latent=True)
             ops.grouped_gemm(summed, self.uv, out, dv, R, lda=H * R, ldo=H * dv, groups=H, a_group_stride=R,
-                             o_group_stride=dv, a_local=True, o_local=True, rows_per_group=rows, o_scale=gate, o_scale_ld=H)
+                             o_group_stride=dv, a_local=True, o_local=True, rows_per_group=rows, o_scale=gate, o_scale_ld=H, w_ready=True)
         if expanded:      # (behind the other roads' products, which write all of the leading rows)
             self._attend_expanded(plan, q_plain, q_rot, latent, bt, ctx, out)
             if gate is not None:

@@ -753,6 +753,31 @@ def test_expert_stream_in_wide_tiles(T, top, n, E, F):
             assert (outs[1][2][c, t].double() - want).abs().max() <= 0.01 * want.abs().max()
 
 
+@pytest.mark.parametrize("T", [1, 7, 8, 9, 24, 25, 33, 64, 65])
+@pytest.mark.parametrize("H,N,K", [(3, 512, 128), (5, 128, 512), (2, 33, 1024), (4, 72, 80), (1, 31, 16), (2, 64, 272)])
+def test_products_per_head_of_few_rows(H, N, K, T):
+    """Matrices that are read ahead of time, rows around eights and around the lines of the dispatch, rows of W that are not whole tiles, k
+    that is no whole step of 32: the bits of the grouped product, and the 64-bit product's numbers; bands of wider rows, scales."""
+    from air_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w, scale = rand(T, H * K + 8).bfloat16(), rand(H, N, K).bfloat16(), rand(T, H + 1)
+    for dtype, kw in ((torch.float32, {}), (torch.bfloat16, dict(o_scale=scale, o_scale_ld=H + 1))):
+        outs = []
+        for ready in (False, True):
+            out = torch.full((T, H * N + 3), 9.0, device="cuda", dtype=dtype)
+            ops.grouped_gemm(x, w, out, N, K, lda=H * K + 8, ldo=H * N + 3, groups=H, a_group_stride=K, o_group_stride=N, a_local=True,
+                             o_local=True, rows_per_group=T, w_ready=ready, **kw)
+            outs.append(out)
+        assert torch.equal(*outs) and (outs[1][:, H * N:] == 9.0).all()
+        want = torch.einsum("thk,hnk->thn", x[:, :H * K].view(T, H, K).double(), w.double())
+        want = want * scale[:, :H, None].double() if kw else want
+        most = torch.einsum("thk,hnk->thn", x[:, :H * K].view(T, H, K).double().abs(), w.double().abs()) * (scale[:, :H, None].double().abs() if kw else 1)
+        # (32-bit sums of exact products, and the output's rounding to 8 bits)
+        bound = K * 2.0 ** -24 * most + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)
+        assert ((outs[1][:, :H * N].view(T, H, N).double() - want).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("H,d,dv,P", [(16, 576, 512, 64), (32, 576, 512, 64), (40, 576, 512, 16), (3, 320, 256, 128), (17, 128, 128, 32), (20, 192, 128, 8)])
 @pytest.mark.parametrize("kind", ["plain", "window", "chunk", "cap", "sink", "rising"])
 def test_single_tokens_over_latents_on_the_tensor_cores(H, d, dv, P, kind):
