@@ -111,6 +111,8 @@ _SIGNATURES = {
                              c_void_p, c_void_p],
     "air_heads_gemm": [c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_longlong, c_longlong, c_int, c_int, c_int, c_int, c_int,
                        c_void_p, c_int, c_void_p],
+    "air_attention_f32_single": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                                 c_int, c_int, c_int, c_float, c_float, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
     "air_table_update": [c_void_p, c_void_p, c_int, c_int, c_void_p],
     "air_decode_attention": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                              c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
@@ -486,7 +488,7 @@ def gemm_f32(a, w, bias, out, w_ready=False, status=None, shape=(0, 0, 0)):
 
 
 def paged_attention_ref(q, cache, block_table, token_seq, positions, out, window, scale, softcap=0.0, gate=None,
-                        kv_heads=None, page_tokens=None, chunk=None, sink=None, latent=False, bias=None):
+                        kv_heads=None, page_tokens=None, chunk=None, sink=None, latent=False, bias=None, single=False, status=None):
     """Causal attention over the pages with 32-bit arithmetic, for any batch.  q [T, H, d], out [T, H, dv].
     cache [page, 2, K, P, d] where dv == d; where keys and values differ in size a page is flat: the keys
     [K, P, d], then the values [K, P, dv], and kv_heads and page_tokens say what K and P are.  score = scale * q.k,
@@ -495,7 +497,8 @@ def paged_attention_ref(q, cache, block_table, token_seq, positions, out, window
     those from p - p % chunk on.  sink (float32 [H]): one more term exp(sink[h]) in the softmax's denominator.
     latent: cache [page, P, d] holds one row per token that every head reads as its key and whose first dv elements
     it reads as its value; q may then be float32 whatever the cache's type.  bias (float32 [H, n]): a score gets
-    bias[h, min(p - key's position, n - 1)]."""
+    bias[h, min(p - key's position, n - 1)].  single: the caller knows that hardly any rows are consecutive tokens of a request (a step
+    of single next tokens): heads that share a key/value head then go together (attention_f32.cu), the same bits."""
     T, H, d = q.shape
     dv = out.shape[2]
     _req(q, "q", _FLOATS)
@@ -528,6 +531,13 @@ def paged_attention_ref(q, cache, block_table, token_seq, positions, out, window
         raise KernelError("paged_attention_ref: a window or a chunk, not both")
     if d > 640 or dv > 640:
         raise KernelError(f"head sizes {d} and {dv}: the 32-bit attention kernel takes up to 640")
+    if (single and not latent and cache.dtype == torch.float32 and H % K == 0 and H > K and T <= 65535 and d <= 128 and dv <= 128 and d % 4 == 0 and dv % 4 == 0
+            and cache.data_ptr() % 16 == 0):
+        _check(_get("air_attention_f32_single")(
+            q.data_ptr(), cache.data_ptr(), block_table.data_ptr(), block_table.shape[1], token_seq.data_ptr(), positions.data_ptr(),
+            out.data_ptr(), _ptr(gate), T, H, K, d, dv, P, int(chunk or window or 0), float(scale), float(softcap or 0.0), 1 if chunk else 0,
+            _ptr(sink), *_distance_bias(bias, H), _ptr(status), _stream()), "attention_f32_single")
+        return out
     _check(_get("air_paged_attention_ref")(
         q.data_ptr(), 1 if q.dtype == torch.float32 else 0, cache.data_ptr(), _DT[cache.dtype], block_table.data_ptr(),
         block_table.shape[1], token_seq.data_ptr(), positions.data_ptr(), out.data_ptr(), _ptr(gate), T, H, K, d, dv, P,

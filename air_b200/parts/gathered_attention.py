@@ -88,7 +88,7 @@ class PortionAttention:
                 return
             ops.paged_attention_ref(q, cache, bt, token_seq, ctx.positions, out, self.window, self.scale,
                                     kv_heads=kv_heads, page_tokens=page_tokens, chunk=self.chunk, sink=sinks,
-                                    latent=latent, softcap=softcap, bias=bias)
+                                    latent=latent, softcap=softcap, bias=bias, single=ctx.all_decode, status=ctx.status)
             if turn is not None:
                 ops.turn_heads(out, *turn, ctx.positions, token_seq, back=True)
             if gate is not None:

@@ -554,6 +554,42 @@ def test_float32_attention_of_rows_together_is_that_of_rows_alone(H, K, d, P, wi
         assert np.abs(out.cpu().numpy() - want).max() < 2e-6 * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("H,K,d,dv,P", [(28, 4, 128, 128, 64), (16, 4, 128, 128, 48), (40, 2, 128, 128, 32), (6, 2, 48, 64, 16),
+                                        (33, 3, 4, 128, 64), (12, 1, 128, 20, 7)])
+@pytest.mark.parametrize("window,chunk", [(0, None), (77, None), (0, 50)])
+@pytest.mark.parametrize("n", [1, 5, 70])
+def test_float32_attention_of_single_tokens(H, K, d, dv, P, window, chunk, n):
+    """Heads that share keys together (few requests: a head or a few to a block; many: up to eight): the bits of the kernel of a head
+    by itself, over contexts on either side of a block of 32 keys and of the four chains, with rows of padding, unseen rows that hold
+    NaN, a sink, a softcap, a gate and a bias; and captured."""
+    gen = torch.Generator().manual_seed(H + d + n)
+    contexts = [[0], [31, 32, 127, 128, 500], [(37 * i) % 300 for i in range(n)]][(n > 1) + (n > 5)]
+    per = max(contexts) // P + 1
+    pages = torch.randperm(n * per, generator=gen).int().view(n, per)
+    cache = torch.randn(n * per, K * P * (d + dv), generator=gen)
+    for i, c in enumerate(contexts):                      # (what no row sees)
+        page = cache[pages[i, c // P]]
+        page[:K * P * d].view(K, P, d)[:, c % P + 1:] = float("nan")
+        page[K * P * d:].view(K, P, dv)[:, c % P + 1:] = float("nan")
+    q, gate, sink, bias = (torch.randn(s, generator=gen).cuda() for s in ((n + 2, H, d), (n + 2, H), (H,), (H, 40)))
+    seq_of = torch.tensor(list(range(n)) + [-1, -1], dtype=torch.int32).cuda()
+    positions = torch.tensor(contexts + [0, 0], dtype=torch.int32).cuda()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    cache, pages = cache.cuda(), pages.cuda()
+    for more in (dict(), dict(sink=sink, softcap=3.0, gate=gate, bias=bias)):
+        args = (q, cache, pages, seq_of, positions)
+        more = dict(more, kv_heads=K, page_tokens=P, chunk=chunk)
+        want, out, captured = (torch.full((n + 2, H, dv), 7.0, device="cuda") for _ in range(3))
+        ops().paged_attention_ref(*args, want, window, d ** -0.5, **more)
+        ops().paged_attention_ref(*args, out, window, d ** -0.5, single=True, status=status, **more)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            ops().paged_attention_ref(*args, captured, window, d ** -0.5, single=True, status=status, **more)
+        graph.replay()
+        assert torch.isfinite(out).all() and torch.equal(out, want) and torch.equal(captured, want)
+        assert (out[n:] == 7.0).all() and int(status) == 0
+
+
 @pytest.mark.parametrize("far", [0, 15, 16, 17, 63, 64, 300, 447])
 def test_attention_finds_one_far_key_among_hundreds(far):
     """One key is made to match the query so that its score stands out: the output must be that
