@@ -38,7 +38,7 @@
 namespace air {
 
 constexpr int TS_BK = 64;
-constexpr int TS_THREADS = 192;
+
 
 enum { TS_F32 = 0, TS_BF16 = 1, TS_SILU = 2, TS_PARTIAL = 3, TS_RELU2 = 4,   // as in gemm_tc.cu
        TS_JOINED = 5 };
@@ -59,15 +59,20 @@ struct TsArgs {
     float act_alpha, act_limit, act_shift;
 };
 
+// Warps that issue products, each into accumulators of its own: one needs 0.2 us for a step of k, four products and a commit.
+__host__ __device__ constexpr int ts_issuers(int halves) { return halves == 1 ? 2 : 1; }
+__host__ __device__ constexpr int ts_threads(int halves) { return 160 + 32 * ts_issuers(halves); }
+// (a stage always belongs to the same issuer)
 __host__ __device__ constexpr int ts_stages(int nt, int halves) {
-    return 196 * 1024 / ((halves * 128 + nt) * TS_BK * 2) > 24 ? 24 : 196 * 1024 / ((halves * 128 + nt) * TS_BK * 2);
+    const int fit = 196 * 1024 / ((halves * 128 + nt) * TS_BK * 2);
+    return (fit > 24 ? 24 : fit) / ts_issuers(halves) * ts_issuers(halves);
 }
 __host__ __device__ constexpr int ts_tmem_cols(int nt, int halves) {
-    return 2 * halves * nt < 32 ? 32 : 2 * halves * nt;      // 32, 64, 128 or 256: a power of two
+    return 2 * halves * nt * ts_issuers(halves);             // 64, 128 or 256: a power of two
 }
 
 template <int NT>
-__device__ __forceinline__ void ts_load_row(uint32_t taddr, float (&v)[NT]) {
+__device__ __forceinline__ void ts_load_part(uint32_t taddr, float (&v)[NT]) {
     if constexpr (NT == 16) {
         uint32_t r[16];
         tmem_ld16(taddr, r);
@@ -84,8 +89,20 @@ __device__ __forceinline__ void ts_load_row(uint32_t taddr, float (&v)[NT]) {
     }
 }
 
+// A row's sums, of the issuers' accumulators; of one alone, which the only step of k went to, where there are no more steps.
+template <int NT, int ISSUERS>
+__device__ __forceinline__ void ts_load_row(uint32_t taddr, float (&v)[NT], int steps, int before) {
+    ts_load_part<NT>(taddr + (ISSUERS > 1 && steps == 1 ? before % ISSUERS * NT : 0), v);
+    if (ISSUERS > 1 && steps > 1) {
+        float more[NT];
+        ts_load_part<NT>(taddr + NT, more);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) v[t] += more[t];
+    }
+}
+
 template <int NT, int EPI, int HALVES>
-__global__ void __launch_bounds__(TS_THREADS, 1)
+__global__ void __launch_bounds__(ts_threads(HALVES), 1)
 gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                      const TsArgs args) {
     constexpr bool PAIRED = EPI == TS_SILU && HALVES == 1;      // 64 gate rows and 64 up rows to a tile
@@ -95,7 +112,8 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     constexpr int STAGE_W = HALVES * HALF_W;
     constexpr int STAGE_X = NT * TS_BK * 2;
     constexpr int STAGES = ts_stages(NT, HALVES);
-    constexpr int ACC_COLS = HALVES * NT;
+    constexpr int ISSUERS = ts_issuers(HALVES);
+    constexpr int ACC_COLS = HALVES * NT * ISSUERS;
     constexpr int TMEM_COLS = ts_tmem_cols(NT, HALVES);
     constexpr int TILE_N = HALVES * 128;               // rows of W per tile
     extern __shared__ uint8_t smem_raw[];
@@ -119,7 +137,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     };
 
     pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int n_tiles = (args.N + TILE_N - 1) / TILE_N;
     const int k_tiles = (args.K + TS_BK - 1) / TS_BK;
     const int k_per = (k_tiles + args.splits - 1) / args.splits;
@@ -131,7 +149,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             mbar_init(&empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_full[i], ISSUERS);
             mbar_init(&acc_empty[i], 4);
         }
         *abort_flag = 0;
@@ -183,12 +201,14 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 }
             }
         }
-    } else if (warp == 1) {
-        // ---------------------------------------------------- MMA issuer: the warp runs together, an
-        // elected lane issues (see gemm_tc.cu)
+    } else if (warp == 1 || warp > 5) {
+        // ---------------------------------------------------- MMA issuers: each warp runs together, an
+        // elected lane issues (see gemm_tc.cu).  Two of them take the stages in turn, each always the same ones: a wait by parity
+        // could not tell a round of a stage from the one two later, were a stage to go from one to the other.
         constexpr uint32_t idesc = umma_idesc(128, NT);
         const uint64_t dw0 = umma_desc(smem_u32(sw)), dx0 = umma_desc(smem_u32(sx));
-        uint32_t stage = 0, phase = 0, it = 0;
+        const int issuer = warp == 1 ? 0 : warp - 5;
+        uint32_t before = 0, it = 0;                      // steps of k in the tiles so far
         bool ok = true;
         for (int tile = blockIdx.x; tile < total && ok && !*abort_flag; tile += gridDim.x, ++it) {
             const int split = tile % args.splits;
@@ -197,8 +217,10 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag));
             if (!ok) break;
             tc_fence_after();
-            const uint32_t d = tmem_base + acc * ACC_COLS;
-            for (int kt = k_begin; kt < k_end; ++kt) {
+            const uint32_t d = tmem_base + acc * ACC_COLS + issuer * NT;
+            const int skip = (issuer + before) % ISSUERS;  // (1 - before, 0 - before: the same modulo two)
+            uint32_t stage = (before + skip) % STAGES, phase = (before + skip) / STAGES & 1;
+            for (int kt = k_begin + skip; kt < k_end; kt += ISSUERS) {
                 // (a stage that is already there costs one try; the bounded loop only where the issuer has to wait)
                 if (!mbar_try_wait(&full[stage], phase)) ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag));
                 if (!ok) break;
@@ -210,13 +232,14 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     for (int k = 0; k < TS_BK / 16; ++k)
 #pragma unroll
                         for (int hf = 0; hf < HALVES; ++hf)
-                            umma_bf16(d + hf * NT, dw + (uint64_t)(hf * (HALF_W >> 4)) + 2 * k, dx + 2 * k, idesc,
-                                      (kt > k_begin || k > 0) ? 1u : 0u);
+                            umma_bf16(d + hf * ISSUERS * NT, dw + (uint64_t)(hf * (HALF_W >> 4)) + 2 * k, dx + 2 * k, idesc,
+                                      (kt >= k_begin + ISSUERS || k > 0) ? 1u : 0u);
                     umma_commit(&empty[stage]);
                 }
                 __syncwarp();
-                if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                if ((stage += ISSUERS) >= STAGES) { stage -= STAGES; phase ^= 1; }
             }
+            before += k_end - k_begin;
             if (ok && elect_one()) umma_commit(&acc_full[acc]);
             __syncwarp();
         }
@@ -245,11 +268,14 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
         uint32_t it = 0;
+        int done = 0;                                     // steps of k in the tiles so far
         // (PAIRED: the four warps meet at a barrier twice per tile, so all of them go through all tiles, also when a wait has
         // run out: one that left would keep the others there for good)
         for (int tile = blockIdx.x; tile < total && (PAIRED || !*abort_flag); tile += gridDim.x, ++it) {
             const int split = tile % args.splits;
             const int n0 = (tile / args.splits) * TILE_N;
+            const int steps = min(k_tiles, (split + 1) * k_per) - split * k_per, before = done;
+            done += steps;
             const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
             bool ok = mbar_wait(&acc_full[acc], acc_phase, abort_flag);
             if constexpr (PAIRED) ok = __all_sync(0xffffffffu, ok);
@@ -258,13 +284,13 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
             if constexpr (JOINED) {
                 float v[NT];
-                ts_load_row<NT>(taddr, v);
+                ts_load_row<NT, ISSUERS>(taddr, v, steps, before);
                 float* mine = (float*)smem;               // [NT][128]: every copy has landed and every product is done
 #pragma unroll
                 for (int t = 0; t < NT; ++t) mine[t * 128 + r] = v[t];
             } else if constexpr (PAIRED) {
                 float v[NT];
-                if (ok) ts_load_row<NT>(taddr, v);
+                if (ok) ts_load_row<NT, ISSUERS>(taddr, v, steps, before);
                 if (args.ss) {
 #pragma unroll
                     for (int t = 0; t < NT; ++t) v[t] *= row_scale[t];
@@ -285,8 +311,8 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 asm volatile("bar.sync 1, 128;" ::: "memory");      // (read before the next tile's are written)
             } else if constexpr (EPI == TS_SILU) {
                 float gate[NT], up[NT];
-                ts_load_row<NT>(taddr, gate);
-                ts_load_row<NT>(taddr + NT, up);
+                ts_load_row<NT, ISSUERS>(taddr, gate, steps, before);
+                ts_load_row<NT, ISSUERS>(taddr + ISSUERS * NT, up, steps, before);
                 if (args.ss) {
 #pragma unroll
                     for (int t = 0; t < NT; ++t) { gate[t] *= row_scale[t]; up[t] *= row_scale[t]; }
@@ -305,7 +331,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 #pragma unroll
                 for (int hf = 0; hf < HALVES; ++hf) {
                     float v[NT];
-                    ts_load_row<NT>(taddr + hf * NT, v);
+                    ts_load_row<NT, ISSUERS>(taddr + hf * ISSUERS * NT, v, steps, before);
                     if (args.ss) {
 #pragma unroll
                         for (int t = 0; t < NT; ++t) v[t] *= row_scale[t];
@@ -355,7 +381,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     if constexpr (JOINED) {
         cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
         cluster.sync();
-        if (warp >= 2) {                                  // the parts in order; the tokens are shared out among the blocks
+        if (warp >= 2 && warp < 6) {                      // the parts in order; the tokens are shared out among the blocks
             // (a warp takes a token's 128 features at once, a lane four of them)
             const int col = (int)blockIdx.x / args.splits * TILE_N + 4 * lane;
             const bool whole = args.N % 4 == 0;
@@ -422,7 +448,7 @@ static int ts_launch(const CUtensorMap& mw, const CUtensorMap& mx, const TsArgs&
     if constexpr (EPI == TS_JOINED) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(blocks);
-        cfg.blockDim = dim3(TS_THREADS);
+        cfg.blockDim = dim3(ts_threads(HALVES));
         cfg.dynamicSmemBytes = request;
         cfg.stream = stream;
         cudaLaunchAttribute attr[2];
@@ -435,7 +461,7 @@ static int ts_launch(const CUtensorMap& mw, const CUtensorMap& mx, const TsArgs&
         cfg.numAttrs = pdl_enabled() ? 2 : 1;
         return launch_counted(cfg, kernel, mw, mx, args);
     }
-    return launch(kernel, blocks, TS_THREADS, request, stream, mw, mx, args);
+    return launch(kernel, blocks, ts_threads(HALVES), request, stream, mw, mx, args);
 }
 
 template <int NT, int HALVES>
