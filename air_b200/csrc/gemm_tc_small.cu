@@ -9,9 +9,9 @@
 // per block.  Here a k step takes the time of reading 128 x 16 weights from shared memory (about
 // 32 cycles).
 //
-// One persistent block per SM, 192 threads, as in gemm_tc.cu: warp 0 issues TMA loads (a tile of
+// One persistent block per SM, 192 or 224 threads, as in gemm_tc.cu: warp 0 issues TMA loads (a tile of
 // HALVES x 128 rows of W and the NT-row tile of X per stage, 128-byte swizzle, no multicast), warp 1
-// issues tcgen05.mma (M 128, N NT, K 16; per k step one per half of the W tile, sharing the tile of
+// (and warp 6, in turn, where a step is 16 KB) issues tcgen05.mma (M 128, N NT, K 16; per k step one per half of the W tile, sharing the tile of
 // X) into one of two sets of accumulators, warps 2-5 read a finished accumulator (thread = output
 // feature, columns = tokens) and write the result, coalesced over the features.
 //   EPI_F32 / EPI_BF16  store C
@@ -19,7 +19,7 @@
 //                       by the 128 rows of the up projection for the same outputs: silu(gate) * up
 //   EPI_SILU, HALVES 1  the same with 64 gate rows and the 64 up rows for the same outputs in one tile of 128 (two copies a
 //                       stage): twice as many tiles, for matrices whose tiles of 256 leave more than half of the SMs idle.
-//                       The up half's warps hand their sums to the gate half's through shared memory
+//                       The sums go through shared memory, where a thread finds a gate's and its up's
 //   EPI_RELU2           store max(C, 0)^2 as bfloat16 (the hidden layer of a feed-forward without a gate)
 //   EPI_F32, joined     matrices of few tiles, whose sums are wanted complete: a cluster of two or four blocks shares a tile, a part
 //                       of the k range each, and adds the parts up, in order, through one another's shared memory.  A block's
@@ -71,34 +71,29 @@ __host__ __device__ constexpr int ts_tmem_cols(int nt, int halves) {
     return 2 * halves * nt * ts_issuers(halves);             // 64, 128 or 256: a power of two
 }
 
-template <int NT>
-__device__ __forceinline__ void ts_load_part(uint32_t taddr, float (&v)[NT]) {
-    if constexpr (NT == 16) {
-        uint32_t r[16];
-        tmem_ld16(taddr, r);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-    } else {
-#pragma unroll
-        for (int c = 0; c < NT; c += 32) {
-            uint32_t r[32];
-            tmem_ld32(taddr + c, r);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[c + i] = __uint_as_float(r[i]);
-        }
-    }
+template <int N>
+__device__ __forceinline__ void ts_ask(uint32_t taddr, uint32_t (&r)[N]) {
+    static_assert(N == 4 || N == 8, "columns of tensor memory at a time");
+    if constexpr (N == 4)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr) : "memory");
 }
-
-// A row's sums, of the issuers' accumulators; of one alone, which the only step of k went to, where there are no more steps.
-template <int NT, int ISSUERS>
-__device__ __forceinline__ void ts_load_row(uint32_t taddr, float (&v)[NT], int steps, int before) {
-    ts_load_part<NT>(taddr + (ISSUERS > 1 && steps == 1 ? before % ISSUERS * NT : 0), v);
-    if (ISSUERS > 1 && steps > 1) {
-        float more[NT];
-        ts_load_part<NT>(taddr + NT, more);
+// The sums of N tokens for this thread's feature, of the issuers' accumulators (of one alone, which the only step of k went to,
+// where there are no more steps).  taddr: the first token's column of the first accumulator.
+template <int NT, int ISSUERS, int N>
+__device__ __forceinline__ void ts_sums(uint32_t taddr, int steps, int before, float (&v)[N]) {
+    uint32_t a[N], b[N];
+    __syncwarp();
+    const bool both = ISSUERS > 1 && steps > 1;
+    ts_ask<N>(taddr + (ISSUERS > 1 && steps == 1 ? before % ISSUERS * NT : 0), a);
+    if (both) ts_ask<N>(taddr + NT, b);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int t = 0; t < NT; ++t) v[t] += more[t];
-    }
+    for (int i = 0; i < N; ++i) v[i] = both ? __uint_as_float(a[i]) + __uint_as_float(b[i]) : __uint_as_float(a[i]);
 }
 
 template <int NT, int EPI, int HALVES>
@@ -128,7 +123,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     float* row_scale = (float*)(tmem_slot + 2);       // [NT]
-    float* ups = row_scale + NT;                       // PAIRED: [NT][64]
+    float* pairs = row_scale + NT;                     // PAIRED: [NT][128], a tile's sums
     // where a tile's rows of W lie (PAIRED: its gate rows; the up rows are 128 further on)
     auto row_of = [](int tile) { return PAIRED ? tile / 2 * 256 + tile % 2 * 64 : tile * TILE_N; };
     auto load_w = [&](int stage, int k, int n0) {
@@ -282,79 +277,76 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             else if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
+            // Loops over a few tokens at a time, as far as there are tokens: this code runs once or twice per launch, from cold
+            // instruction caches, and its length is what it costs.  All tokens at once, one after the other in the code, against this, us
+            // a decoder layer of width 2,048: 1 token 55 -> 53, 24 tokens 64.5 -> 60.1, 50 tokens 79 -> 66.
             if constexpr (JOINED) {
-                float v[NT];
-                ts_load_row<NT, ISSUERS>(taddr, v, steps, before);
                 float* mine = (float*)smem;               // [NT][128]: every copy has landed and every product is done
+#pragma unroll 1
+                for (int t = 0; t < args.T; t += 8) {
+                    float v[8];
+                    ts_sums<NT, ISSUERS, 8>(taddr + t, steps, before, v);
 #pragma unroll
-                for (int t = 0; t < NT; ++t) mine[t * 128 + r] = v[t];
-            } else if constexpr (PAIRED) {
-                float v[NT];
-                if (ok) ts_load_row<NT, ISSUERS>(taddr, v, steps, before);
-                if (args.ss) {
-#pragma unroll
-                    for (int t = 0; t < NT; ++t) v[t] *= row_scale[t];
+                    for (int i = 0; i < 8; ++i) mine[(t + i) * 128 + r] = v[i];
                 }
-                if (ok && r >= 64) {
+            } else if constexpr (PAIRED) {
+                if (ok) {
+#pragma unroll 1
+                    for (int t = 0; t < args.T; t += 8) {
+                        float v[8];
+                        ts_sums<NT, ISSUERS, 8>(taddr + t, steps, before, v);
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) ups[t * 64 + r - 64] = v[t];
+                        for (int i = 0; i < 8; ++i) pairs[(t + i) * 128 + r] = args.ss ? v[i] * row_scale[t + i] : v[i];
+                    }
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (ok && r < 64) {
-                    __nv_bfloat16* out = (__nv_bfloat16*)args.out + (size_t)(tile / args.splits) * 64 + r;
-#pragma unroll
-                    for (int t = 0; t < NT; ++t)
-                        if (t < args.T)
-                            out[(size_t)t * (args.N / 2)] = __float2bfloat16_rn(
-                                gated_activation(v[t], ups[t * 64 + r], args.act_alpha, args.act_limit, args.act_shift));
+                if (ok) {
+                    __nv_bfloat16* out = (__nv_bfloat16*)args.out + (size_t)(tile / args.splits) * 64 + (r & 63);
+#pragma unroll 2
+                    for (int t = r >> 6; t < args.T; t += 2)
+                        out[(size_t)t * (args.N / 2)] = __float2bfloat16_rn(
+                            gated_activation(pairs[t * 128 + (r & 63)], pairs[t * 128 + 64 + (r & 63)], args.act_alpha, args.act_limit, args.act_shift));
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");      // (read before the next tile's are written)
             } else if constexpr (EPI == TS_SILU) {
-                float gate[NT], up[NT];
-                ts_load_row<NT, ISSUERS>(taddr, gate, steps, before);
-                ts_load_row<NT, ISSUERS>(taddr + ISSUERS * NT, up, steps, before);
-                if (args.ss) {
-#pragma unroll
-                    for (int t = 0; t < NT; ++t) { gate[t] *= row_scale[t]; up[t] *= row_scale[t]; }
-                }
                 const int col = n0 / 2 + r;
-                if (col < args.N / 2) {
-                    __nv_bfloat16* out = (__nv_bfloat16*)args.out + col;
+#pragma unroll 1
+                for (int t = 0; t < args.T; t += 4) {
+                    float gate[4], up[4];
+                    ts_sums<NT, ISSUERS, 4>(taddr + t, steps, before, gate);
+                    ts_sums<NT, ISSUERS, 4>(taddr + ISSUERS * NT + t, steps, before, up);
+                    if (col < args.N / 2) {
+                        __nv_bfloat16* out = (__nv_bfloat16*)args.out + (size_t)t * (args.N / 2) + col;
 #pragma unroll
-                    for (int t = 0; t < NT; ++t)
-                        if (t < args.T) {
-                            out[(size_t)t * (args.N / 2)] = __float2bfloat16_rn(
-                                gated_activation(gate[t], up[t], args.act_alpha, args.act_limit, args.act_shift));
+                        for (int i = 0; i < 4; ++i) {
+                            const float scale = args.ss ? row_scale[t + i] : 1.f;
+                            if (t + i < args.T)
+                                out[(size_t)i * (args.N / 2)] = __float2bfloat16_rn(
+                                    gated_activation(gate[i] * scale, up[i] * scale, args.act_alpha, args.act_limit, args.act_shift));
                         }
+                    }
                 }
             } else {
-#pragma unroll
-                for (int hf = 0; hf < HALVES; ++hf) {
-                    float v[NT];
-                    ts_load_row<NT, ISSUERS>(taddr + hf * ISSUERS * NT, v, steps, before);
-                    if (args.ss) {
-#pragma unroll
-                        for (int t = 0; t < NT; ++t) v[t] *= row_scale[t];
-                    }
+#pragma unroll 1
+                for (int at = 0; at < HALVES * NT; at += 8) {
+                    const int hf = at / NT, t = at % NT;
+                    if (t >= args.T) continue;
+                    float v[8];
+                    ts_sums<NT, ISSUERS, 8>(taddr + hf * ISSUERS * NT + t, steps, before, v);
                     const int col = n0 + hf * 128 + r;
                     if (col < args.N) {
-                        if constexpr (EPI == TS_BF16) {
-                            __nv_bfloat16* out = (__nv_bfloat16*)args.out + col;
 #pragma unroll
-                            for (int t = 0; t < NT; ++t)
-                                if (t < args.T) out[(size_t)t * args.N] = __float2bfloat16_rn(v[t]);
-                        } else if constexpr (EPI == TS_RELU2) {
-                            __nv_bfloat16* out = (__nv_bfloat16*)args.out + col;
-#pragma unroll
-                            for (int t = 0; t < NT; ++t) {
-                                const float r = fmaxf(v[t], 0.f);
-                                if (t < args.T) out[(size_t)t * args.N] = __float2bfloat16_rn(r * r);
+                        for (int i = 0; i < 8; ++i) {
+                            if (t + i >= args.T) break;
+                            if (args.ss) v[i] *= row_scale[t + i];
+                            if constexpr (EPI == TS_BF16) {
+                                ((__nv_bfloat16*)args.out)[(size_t)(t + i) * args.N + col] = __float2bfloat16_rn(v[i]);
+                            } else if constexpr (EPI == TS_RELU2) {
+                                const float x = fmaxf(v[i], 0.f);
+                                ((__nv_bfloat16*)args.out)[(size_t)(t + i) * args.N + col] = __float2bfloat16_rn(x * x);
+                            } else {
+                                ((float*)args.out)[((size_t)split * args.T + t + i) * args.N + col] = v[i];
                             }
-                        } else {
-                            float* out = (float*)args.out + (size_t)split * args.T * args.N + col;
-#pragma unroll
-                            for (int t = 0; t < NT; ++t)
-                                if (t < args.T) out[(size_t)t * args.N] = v[t];
                         }
                     }
                 }
@@ -440,7 +432,7 @@ static int ts_launch(const CUtensorMap& mw, const CUtensorMap& mx, const TsArgs&
     // always more than half of an SM's shared memory, so that two blocks never share an SM (and its
     // tensor memory)
     const size_t smem = 1024 + (size_t)STAGES * (HALVES * 128 + NT) * TS_BK * 2 + 16 * STAGES + 256 + 4 * NT +
-                        (EPI == TS_SILU && HALVES == 1 ? 256 * NT : 0);
+                        (EPI == TS_SILU && HALVES == 1 ? 512 * NT : 0);
     const size_t request = smem < 120 * 1024 ? 120 * 1024 : smem;
     auto kernel = gemm_tc_small_kernel<NT, EPI, HALVES>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)request);
