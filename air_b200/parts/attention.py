@@ -186,7 +186,8 @@ class TiledAttention:
         d = self.head_dim
         if not self.fast_attention(ctx, kv.shape[3]):
             return ops.paged_attention_ref(q, kv, bt, ctx.token_seq, ctx.positions, out, self.window, self.scale,
-                                           softcap=self.softcap, single=ctx.all_decode, status=ctx.status)
+                                           softcap=self.softcap, single=getattr(ctx, "all_decode", False),
+                                           status=getattr(ctx, "status", None))
         if ctx.all_decode:
             return ops.decode_attention(q, kv, bt, ctx.token_seq, ctx.positions, out, self.window, self.scale,
                                         softcap=self.softcap)

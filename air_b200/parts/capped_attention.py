@@ -127,5 +127,6 @@ class CappedAttention(TiledAttention, Mixer):
                 ops.head_gate(out, gate, ctx.token_seq)
         else:
             ops.paged_attention_ref(q, kv, bt, ctx.token_seq, ctx.positions, out, self.window, self.scale,
-                                    softcap=self.softcap, gate=gate, kv_heads=G, page_tokens=P, single=ctx.all_decode, status=ctx.status)
+                                    softcap=self.softcap, gate=gate, kv_heads=G, page_tokens=P, single=getattr(ctx, "all_decode", False),
+                                    status=getattr(ctx, "status", None))
         return self.o.f32_sums(out.view(T, H * dv))

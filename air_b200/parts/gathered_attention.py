@@ -84,11 +84,13 @@ class PortionAttention:
             if ops.grouped_attention_ok(cache.dtype, q.shape[2], out.shape[2]):
                 ops.grouped_attention(q, cache, bt, token_seq, ctx.positions, out, self.window, self.scale,
                                       kv_heads=kv_heads, page_tokens=page_tokens, chunk=self.chunk, sink=sinks,
-                                      latent=latent, softcap=softcap, gate=gate, turn=turn, bias=bias, status=ctx.status)
+                                      latent=latent, softcap=softcap, gate=gate, turn=turn, bias=bias,
+                                      status=getattr(ctx, "status", None))
                 return
             ops.paged_attention_ref(q, cache, bt, token_seq, ctx.positions, out, self.window, self.scale,
                                     kv_heads=kv_heads, page_tokens=page_tokens, chunk=self.chunk, sink=sinks,
-                                    latent=latent, softcap=softcap, bias=bias, single=ctx.all_decode, status=ctx.status)
+                                    latent=latent, softcap=softcap, bias=bias, single=getattr(ctx, "all_decode", False),
+                                    status=getattr(ctx, "status", None))
             if turn is not None:
                 ops.turn_heads(out, *turn, ctx.positions, token_seq, back=True)
             if gate is not None:
