@@ -1210,3 +1210,39 @@ def test_prefill_attention_tc_finds_one_far_key(far, n, cut):
     for t in range(16):
         for h in range(H):
             assert np.abs(got[t, h] - vs[0][far, h * K // H]).max() < 2e-2
+
+
+@pytest.mark.parametrize("K", [8, 64, 72, 192, 200, 648, 1160])
+@pytest.mark.parametrize("T", [1, 8, 16, 17, 33, 64])
+def test_products_of_few_rows_with_two_issuing_warps(K, T):
+    """Tiles of one step of k and of odd numbers of them, several tiles to a block (a block's steps then begin with either warp), every
+    epilogue.  A sum of K terms is off by at most K 2^-23 of the sum of their magnitudes (an addition of the tensor cores may cut off a
+    last place); a bfloat16 result is off by another 2^-8 of itself."""
+    o = ops()
+    gen = torch.Generator(device="cuda").manual_seed(K + T)
+    for N, blocks in ((256, 0), (256, 3), (1280, 3), (1280, 0), (130 * 4, 2)):
+        x, w = (torch.randn(s, device="cuda", generator=gen).bfloat16() for s in ((T, K), (N, K)))
+        want, off = x.double() @ w.double().T, (x.double().abs() @ w.double().abs().T) * K * 2.0 ** -23
+        for bn in (128, 256):
+            out = o.gemm_tc(x, w, torch.full((T, N), 7.0, device="cuda"), bn, o.EPI_F32, max_blocks=blocks)
+            assert ((out - want).abs() <= off).all()
+            for splits in (2, 3):
+                k_tiles = -(-K // 64)
+                if splits > k_tiles or (splits - 1) * -(-k_tiles // splits) >= k_tiles:
+                    continue
+                out = o.gemm_tc(x, w, torch.full((splits, T, N), 7.0, device="cuda"), bn, o.EPI_PARTIAL, splits=splits, max_blocks=blocks)
+                assert ((out.double().sum(0) - want).abs() <= off).all()
+            out = o.gemm_tc(x, w, torch.full((T, N), 7.0, dtype=torch.bfloat16, device="cuda"), bn, o.EPI_BF16, max_blocks=blocks)
+            assert ((out - want).abs() <= off + 2.0 ** -8 * want.abs()).all()
+            out = o.gemm_tc(x, w, torch.full((T, N), 7.0, dtype=torch.bfloat16, device="cuda"), bn, o.EPI_RELU2, max_blocks=blocks)
+            y = want.clamp(min=0)
+            assert ((out - y * y).abs() <= 2 * (y + off) * off + 2.0 ** -8 * y * y).all()
+        if N % 256 == 0:
+            ss, eps = torch.rand(2, T, device="cuda", generator=gen) * K, 1e-6
+            for more, scale in ((dict(), torch.ones(T, 1, device="cuda")), (dict(row_ss=ss, eps=eps), (ss.double().sum(0) / K + eps).rsqrt()[:, None])):
+                out = o.gemm_tc(x, w, torch.full((T, N // 2), 7.0, dtype=torch.bfloat16, device="cuda"), 256, o.EPI_SILU, max_blocks=blocks, **more)
+                (g, u), (dg, du) = ((v * scale).view(T, N // 256, 2, 128).permute(2, 0, 1, 3).reshape(2, T, N // 2) for v in (want, off))
+                silu = g / (1 + torch.exp(-g))
+                # (the slope of x / (1 + e^-x) is at most 1.1; the function and the scale themselves: 2^-19 of the result)
+                bound = 1.1 * dg * (u.abs() + du) + silu.abs() * du + (2.0 ** -8 + 2.0 ** -19) * (silu * u).abs() + 1e-30
+                assert ((out - silu * u).abs() <= bound).all()
