@@ -23,7 +23,7 @@
 //   EPI_RELU2           store max(C, 0)^2 as bfloat16 (the hidden layer of a feed-forward without a gate)
 //   EPI_F32, joined     matrices of few tiles, whose sums are wanted complete: a cluster of two or four blocks shares a tile, a part
 //                       of the k range each, and adds the parts up, in order, through one another's shared memory.  A block's
-//                       copies bring 65 GB/s whatever the tile, so 53 tiles leave half of the memory's rate unused:
+//                       steps pass at some 65 GB/s whatever the tile, so 53 tiles leave half of the memory's rate unused:
 //                       8 rows by 6,720 x 4,096 (two blocks) 16.4 -> 13.5 us, by 4,096 x 4,096 (four) 15.2 -> 10.0, by 3,648 x
 //                       2,048 (four) 8.7 -> 6.7, 64 rows by 6,720 x 4,096 18.4 -> 15.6.  Tiles of 64 or 32 rows: 20 and 29.
 //   EPI_PARTIAL         the k range is split over `splits` blocks; each writes C[split][T][N] (float32)
