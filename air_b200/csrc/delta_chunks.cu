@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
     const int h = blockIdx.y, col0 = blockIdx.x * DC;
     const int* por = p.portions + 4 * blockIdx.z;
     const int row0 = por[0], tokens = por[1], slot = por[2], chunk0 = por[3];
-    if (slot < 0) return;
+    if (slot < 0 || tokens <= 0) return;     // (no chunk: nothing to wait for, to add or to write)
     const int chunks = (tokens + DC - 1) / DC;
     auto bring = [&](int i, int stage) {               // (one thread)
         const float* src = p.scratch + ((size_t)(chunk0 + i) * p.H + h) * p.stride;

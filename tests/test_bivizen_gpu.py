@@ -307,6 +307,37 @@ def test_chunks_of_many_portions_are_those_of_each_alone(H, d, dv, mode):
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("mode", ["delta", "gla", "channel"])
+@pytest.mark.parametrize("H,d,dv", [(2, 64, 40), (12, 128, 128), (4, 256, 96)])
+def test_portions_of_no_token_leave_everything_as_it_is(H, d, dv, mode):
+    """Portions of no token with a slot of their own, ahead of, between and behind others: their states stay, nothing is written
+    ahead of the outputs or in another portion's rows, no wait runs out, and the others have the bits that they have by themselves."""
+    from air_b200.csrc import ops
+    counts = [0, 17, 0, 33, 0]
+    which = {"delta": ops.SCAN_DELTA, "gla": ops.SCAN_GLA, "channel": ops.SCAN_CHANNEL_DELTA}[mode]
+    per, T, L = (H if mode == "delta" else H * d), sum(counts), len(counts)
+    g = torch.Generator(device=DEV).manual_seed(d)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    q, k, v, z, b, S0 = rand(T, H * d), rand(T, H * d), rand(T, H * dv), rand(T, per), rand(T, H), rand(L, H, d, dv)
+    more = dict(tau=8.0) if mode == "gla" else dict(beta=b, a_log=rand(H) / 2, dt_bias=rand(per))
+    start = np.concatenate([[0], np.cumsum(counts)])
+    table = lambda rows: torch.tensor(np.array(rows), dtype=torch.int32, device=DEV)
+    portions, chunks = [], []
+    for i, n in enumerate(counts):
+        portions.append((start[i], n, i, len(chunks)))
+        chunks += [(start[i] + a, min(ops.DELTA_CHUNK, n - a)) for a in range(0, n, ops.DELTA_CHUNK)]
+    got = []
+    for rows in (portions, [row for row in portions if row[1]]):
+        status, S = torch.zeros(1, dtype=torch.int32, device=DEV), S0.clone()
+        room = torch.full((32 + T, H, dv), 9.0, device=DEV)       # (rows ahead of the outputs, and behind them)
+        ops.delta_portions(q, k, v, z, S, room[16:16 + T], table(rows), table(chunks), d ** -0.5, mode=which, status=status, **more)
+        assert int(status) == 0
+        assert (room[:16] == 9.0).all() and (room[16 + T:] == 9.0).all()
+        assert all(torch.equal(S[i], S0[i]) for i, n in enumerate(counts) if not n)
+        got.append((room, S))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 def test_gated_norm_feed_forward_activation_and_scaled_sum():
     from air_b200.csrc import ops
     rng = np.random.default_rng(5)
