@@ -318,7 +318,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_cache, const
         for (int it = 0; it < n_tiles; ++it) {
             const int stage = it % DT_STAGES;
             // (a warp whose wait ran out goes on without work, so that it still meets the others at the barrier below)
-            if (alive && !mbar_wait(&full[stage], (it / DT_STAGES) & 1, abort_flag)) alive = false;
+            if (alive) alive = __all_sync(0xffffffffu, mbar_wait(&full[stage], (it / DT_STAGES) & 1, abort_flag));
             if (patch && begin + it == own_tile) {
                 // the token's own k and v: into their row of the tile (what the copy brought there is older)
                 const int row = pos - own_tile * DT_TILE;

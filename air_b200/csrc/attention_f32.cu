@@ -225,8 +225,7 @@ __global__ void __launch_bounds__(FS_THREADS, 2) attention_f32_single_kernel(con
                 add_values(values[y % 2]);
             }
         };
-        bool ok = n == 0 || mbar_wait(&full[0], 0, &gave_up);
-        ok = __all_sync(0xffffffffu, ok);
+        bool ok = n == 0 || __all_sync(0xffffffffu, mbar_wait(&full[0], 0, &gave_up));
         if (n > 0 && ok)
 #pragma unroll 8
             for (int x = 0; x < d; x += 4) score(here, x, s);

@@ -276,9 +276,12 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attention_kernel(const _
         // group g's part of O: numbers 128 g + row of the values, every head's upper and lower sums
         const uint32_t o_at = lane_at + O_COL + group * 2 * HN;
         const bool holder = group < a.dv / 128;
-        bool ok = true;                                      // (a warp that has given up a wait goes on: nobody is left at a barrier)
+        // A thread that has given up a wait goes on without waiting, and its warp together: nobody is left at a barrier.  (A vote of the
+        // warp on every wait instead: 1 to 4 % of the whole.)
+        bool ok = true;
         for (int j = 0; j < n; ++j) {
             if (ok) ok = mbar_wait(&s_full[j & 1], (j >> 1) & 1, abort_flag);
+            __syncwarp();
             tc_fence_after();
             float s[NH];
             bool over = false;
@@ -326,6 +329,7 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attention_kernel(const _
             }
             // O's step j - 1 has ended: P may be written again, and O rescaled
             if (j > 0 && ok) ok = mbar_wait(pv_done, (j - 1) & 1, abort_flag);
+            __syncwarp();
             if (any && j > 0 && holder) {
                 tc_fence_after();
 #pragma unroll
@@ -364,7 +368,7 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attention_kernel(const _
             __syncwarp();
             if (lane == 0) mbar_arrive(p_ready);
         }
-        if (n > 0 && ok) ok = mbar_wait(pv_done, (n - 1) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok && (n == 0 || mbar_wait(pv_done, (n - 1) & 1, abort_flag)));
         const float total = across<NH, true>(sum, lane);
         if ((lane & 15) < NH) wide[quarter * HN + h1 + (lane & 15)] = total;
         asm volatile("bar.sync 1, %0;" ::"n"(WIDTH) : "memory");

@@ -140,7 +140,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_cache, const __
 
         for (int it = 0; it < n_tiles; ++it) {
             const int stage = it % PF_STAGES;
-            if (!mbar_wait(&full[stage], (it / PF_STAGES) & 1, abort_flag)) break;
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], (it / PF_STAGES) & 1, abort_flag))) break;
             const int kbase = (tile0 + it) * PF_TILE;
             if (active && kbase <= last && kbase + PF_TILE - 1 >= lo) {
                 const uint32_t kt = smem_u32(smem + stage * STAGE_BYTES);

@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
             }
         };
         Two b[NJ][2][2];
-        ok = mbar_wait(&full[0], 0, &gave_up);
+        ok = __all_sync(0xffffffffu, mbar_wait(&full[0], 0, &gave_up));
         if constexpr (AHEAD) rows(b, smem, 0);
         for (int i = 0; i < chunks; ++i) {
             const float* buf = smem + stage * BUF;
@@ -557,6 +557,7 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
                     }
             }
             if (!there && ok) ok = mbar_wait(&full[stage], phase, &gave_up);
+            __syncwarp();
             if constexpr (AHEAD) rows(b, smem + stage * BUF, 0);     // (between the products; of no chunk: what lies there, unused)
 #pragma unroll
             for (int j0 = 0; j0 < NJ; j0 += GROUP) {
@@ -631,6 +632,7 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
         for (int i = 0; i < chunks; ++i) {
             const float* buf = smem + stage * BUF;
             if (ok) ok = mbar_wait(&full[stage], phase, &gave_up);
+            __syncwarp();
             float2 y = *reinterpret_cast<const float2*>(buf + Place::Y + u_c * DC + u_t);
             dc_sync<DC_SUMS>();
             if constexpr (!GLA) {

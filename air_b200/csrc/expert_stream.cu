@@ -215,9 +215,9 @@ expert_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             }
-            const bool ok = mbar_wait(&acc_full[acc], acc_phase, abort_flag);
+            const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_phase, abort_flag));
             if constexpr (EPI == 0) {
-                if (!__all_sync(0xffffffffu, ok)) continue;
+                if (!ok) continue;
             } else if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);

@@ -219,7 +219,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int mn = tile / args.splits;
             const int m0 = (mn % m_tiles) * TILE_M + half * TC_BM, n0 = (mn / m_tiles) * BN;
             const uint32_t acc = it % NACC, acc_phase = (it / NACC) & 1;
-            if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag)) break;
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_phase, abort_flag))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = m0 + quarter * 32 + lane;
             const bool warp_has_rows = m0 + quarter * 32 < args.M;

@@ -277,9 +277,8 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             const int steps = min(k_tiles, (split + 1) * k_per) - split * k_per, before = done;
             done += steps;
             const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-            bool ok = mbar_wait(&acc_full[acc], acc_phase, abort_flag);
-            if constexpr (PAIRED) ok = __all_sync(0xffffffffu, ok);
-            else if (!ok) break;
+            const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_phase, abort_flag));
+            if (!PAIRED && !ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
             // Loops over a few tokens at a time, as far as there are tokens: this code runs once or twice per launch, from cold

@@ -33,7 +33,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 // Waits for the phase with the given parity; gives up after SPIN_LIMIT tries or when another
-// role has given up.  Returns false on giving up.
+// role has given up.  Returns false on giving up.  A thread's own answer: a warp whose threads go on together (products, reads of
+// tensor memory, barriers) votes on it, or some of them would stand at an instruction that wants all.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
     for (uint32_t i = 0; i < SPIN_LIMIT; ++i) {
         if (mbar_try_wait(bar, parity)) return true;

@@ -42,6 +42,49 @@ def test_functions_that_c_programs_call_keep_their_arguments():
     assert lib.air_decode_combine(None, None, None, None, 1, 1, 7, 2, None) == 100001
 
 
+def waits(source):
+    """Of every bounded wait on a barrier in memory: its line, what stands ahead of the blocks around it, its statement up to it, and what
+    follows the statement."""
+    source = re.sub(r"//[^\n]*", "", source)
+    around, depth, begin = [], 0, 0
+    for m in re.finditer(r"[(){};]|\bmbar_wait\(", source):
+        c, at = m.group(), m.start()
+        if c == "mbar_wait(":
+            yield source.count("\n", 0, at) + 1, [opening for opening, _ in around], source[begin:at], source[source.index(";", at) + 1:].lstrip()
+        if c.endswith("("):
+            depth += 1
+        elif c == ")":
+            depth -= 1
+        elif c == "{":
+            around.append((source[begin:at], depth))
+            depth, begin = 0, at + 1
+        elif c == "}":
+            depth, begin = around.pop()[1], at + 1
+        elif depth == 0:
+            begin = at + 1
+
+
+def test_a_warp_goes_on_together_behind_a_wait():
+    """A wait that runs out answers each thread by itself.  Products, reads of tensor memory and barriers of a block want whole warps:
+    every wait is voted on, or made by one thread, or the warp comes together behind it and nothing is left out by those whose wait ran
+    out.  (elementwise.cu: each thread chooses where it reads its own numbers.)"""
+    one = re.compile(r"(lane|tid|threadIdx\.x) == 0( &&|\))|elect_one\(\)")
+    voted, together, alone, left = 0, 0, 0, []
+    for path in sorted(glob.glob(os.path.join(build.HERE, "*.cu"))):
+        with open(path) as f:
+            source = f.read()
+        for line, around, statement, behind in waits(source):
+            if re.search(r"__all_sync\(0xffffffffu,[^;]*$|__syncthreads_or\(!$", statement):
+                voted += 1
+            elif re.search(r"\bok = $", statement) and behind.startswith("__syncwarp();"):
+                together += 1
+            elif any(one.search(opening) for opening in around + [statement]):
+                alone += 1
+            elif os.path.basename(path) != "elementwise.cu":
+                left.append(f"{os.path.basename(path)}:{line}")
+    assert not left and voted > 20 and alone > 5, (left, voted, together, alone)
+
+
 def test_what_the_attention_asks_for_ahead():
     """Up to 24 MB of two tensors in their order; nothing where the first alone is larger, and never beyond a tensor's end."""
     of = lambda mb: torch.empty(mb << 20, dtype=torch.uint8)
