@@ -608,9 +608,11 @@ def grouped_attention(q, cache, block_table, token_seq, positions, out, window, 
     if window and chunk:
         raise KernelError("grouped_attention: a window or a chunk, not both")
     J = H // G
-    if (latent and splits is None and bias is None and q.dtype == torch.float32 and cache.dtype == torch.bfloat16 and d % 64 == 0 and d <= 576
-            and dv % 128 == 0 and dv <= 512 and (P % 64 == 0 if P >= 64 else P >= 8 and 64 % P == 0)):
-        # rows that the tcgen05 kernel takes (attention_latent.cu): up to 32 heads to a block, a block to an SM.  (At most 24 parts of a
+    if (latent and T and splits is None and bias is None and q.dtype == torch.float32 and cache.dtype == torch.bfloat16 and d % 64 == 0 and d <= 576
+            and dv % 128 == 0 and dv <= 512 and (P % 64 == 0 if P >= 64 else P >= 8 and 64 % P == 0) and q.data_ptr() % 16 == 0
+            and cache.shape[0] * P < 1 << 31):
+        # rows that the tcgen05 kernel takes (attention_latent.cu; it reads the queries by 16 bytes, and numbers the cache's rows in 31
+        # bits): up to 32 heads to a block, a block to an SM.  (At most 24 parts of a
         # token's keys, us with 16, 24 and 32: one token at 32 heads over 4,096 keys 21.7, 17.6, 18.0, over 8,191 27.0, 22.9, 19.3; four
         # tokens over 1,000 13.5, 13.9, 16.0, over 4,096 22.1, 18.8, 22.5)
         splits = max(1, min(24, 148 // (T * (1 if H <= 16 else -(-H // 32)))))

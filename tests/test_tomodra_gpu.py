@@ -844,6 +844,31 @@ def test_single_tokens_over_latents_on_the_tensor_cores(H, d, dv, P, kind):
         assert ((first[i].double() - want).abs() <= bound).all(), (i, float(((first[i].double() - want).abs() / bound).max()))
 
 
+@pytest.mark.parametrize("H,d,dv", [(16, 576, 512), (3, 320, 256), (20, 128, 128)])
+def test_latent_queries_on_any_boundary(H, d, dv):
+    """Queries that do not begin on 16 bytes take the kernels that read them by less, a batch of no token takes none."""
+    from air_b200.csrc import ops
+    contexts = [0, 70, 300]
+    T, P = len(contexts), 64
+    g = torch.Generator(device="cuda").manual_seed(d)
+    rows = torch.randn(T * 5, P, d, generator=g, device="cuda").bfloat16()
+    table = torch.arange(T * 5, dtype=torch.int32, device="cuda").view(T, 5)
+    seq, pos = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in (list(range(T)), contexts))
+    numbers = torch.randn(T, H, d, generator=g, device="cuda")
+    outs = []
+    for shift in (0, 2, 1):                     # (floats: boundaries of 16, 8 and 4 bytes)
+        room = torch.empty(T * H * d + 4, device="cuda")
+        q = room[shift:shift + T * H * d].view(T, H, d).copy_(numbers)
+        assert q.data_ptr() % 16 == 4 * shift
+        out = torch.full((T, H, dv), 7.0, device="cuda", dtype=torch.bfloat16)
+        ops.grouped_attention(q, rows, table, seq, pos, out, None, d ** -0.5, latent=True)
+        outs.append(out.double())
+    for other in outs[1:]:                      # (two roundings to 8 bits, and as two halves of 8 bits what is multiplied)
+        assert ((other - outs[0]).abs() <= 2.0 ** -7 * outs[0].abs() + 2.0 ** -12).all()
+    none = torch.empty((0, H, dv), device="cuda", dtype=torch.bfloat16)
+    ops.grouped_attention(numbers[:0], rows, table, seq[:0], pos[:0], none, None, d ** -0.5, latent=True)
+
+
 def test_a_rows_experts_do_not_depend_on_the_rows_beside_it():
     """A mixture in bfloat16: a row's planes are the same, bit for bit, in every step of up to 64 rows, and in every longer one on
     the stream of weights; their sums are those of the 64-bit experts."""
