@@ -1066,9 +1066,9 @@ def grouped_gemm(a, w, out, n, k, *, lda, ldo, groups, a_group_stride=0, o_group
         _req(a_scale, "a_scale", (torch.float32,))
     if o_scale is not None:
         _req(o_scale, "o_scale", (torch.float32,))
-    if (w_ready and a.dtype == torch.bfloat16 and a_local and o_local and not (silu_mul or relu2) and start is None and a_index is None
-            and o_index is None and 0 < rows_per_group <= (64 if k >= 256 else 24) and k % 16 == 0 and k <= 1024 and lda % 8 == 0
-            and a_group_stride % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
+    if (w_ready and a.dtype == torch.bfloat16 and a_local and o_local and not (silu_mul or relu2) and start is None and tiles is None
+            and a_index is None and a_scale is None and o_index is None and k % 16 == 0 and lda % 8 == 0 and a_group_stride % 8 == 0
+            and 0 < rows_per_group <= (64 if k >= 256 else 24) and k <= 1024 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
         _check(_get("air_heads_gemm")(
             a.data_ptr(), int(lda), int(a_group_stride), w.data_ptr(), out.data_ptr(), int(ldo), int(o_group_stride),
             1 if out.dtype == torch.float32 else 0, int(rows_per_group), int(groups), int(n), int(k), _ptr(o_scale), int(o_scale_ld),

@@ -778,6 +778,20 @@ def test_products_per_head_of_few_rows(H, N, K, T):
         assert ((outs[1][:, :H * N].view(T, H, N).double() - want).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("ready", [False, True])
+def test_products_per_head_refuse_what_they_do_not_read(ready):
+    """A scale of A's rows without a list of them, and tiles without their starts, are refused whether or not W was there before."""
+    from air_b200.csrc import ops
+    H, N, K, T = 2, 64, 128, 4
+    x, w = (torch.randn(*s, device="cuda").bfloat16() for s in ((T, H * K), (H, N, K)))
+    out, scale, tiles = torch.zeros(T, H * N, device="cuda"), torch.ones(T, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+    for more in (dict(a_scale=scale), dict(tiles=tiles, num_tiles=tiles)):
+        with pytest.raises(ops.KernelError):
+            ops.grouped_gemm(x, w, out, N, K, lda=H * K, ldo=H * N, groups=H, a_group_stride=K, o_group_stride=N, a_local=True, o_local=True,
+                             rows_per_group=T, w_ready=ready, **more)
+    assert (out == 0).all()
+
+
 @pytest.mark.parametrize("H,d,dv,P", [(16, 576, 512, 64), (32, 576, 512, 64), (40, 576, 512, 16), (3, 320, 256, 128), (17, 128, 128, 32), (20, 192, 128, 8)])
 @pytest.mark.parametrize("kind", ["plain", "window", "chunk", "cap", "sink", "rising"])
 def test_single_tokens_over_latents_on_the_tensor_cores(H, d, dv, P, kind):
