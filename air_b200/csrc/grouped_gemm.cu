@@ -353,7 +353,8 @@ grouped_gemm_tc_kernel(const GroupedArgs p) {
 // products are W's rows as the instruction's 16 rows by 8 rows of A, in the order of k as above (the same bits).
 // Measured, us, the kernel above and this one: 32 heads of 512 x 128 (out x in), 1, 8, 16, 20 and 32 rows 4.2 and 2.6, 4.3 and 2.8, 4.7 and 3.6, 4.9 and
 // 4.4, 5.2 and 5.1; 128 x 512, 8, 32 and 64 rows 7.4 and 3.3, 8.0 and 6.0, 9.0 and 7.2; 16 heads of 192 x 1,024, 8 and 64 rows 12.4 and 4.1, 15.1 and
-// 12.9.  From some 24 rows on a k below 256 is a short chain above and its tiles of 64 rows serve all of them.
+// 12.9.  From some 24 rows on a k below 256 is a short chain above and its tiles of 64 rows serve all of them; many heads of many rows are more
+// rounds of these blocks than the chain above is long (64 heads of 192 x 1,024, 64 rows 24.4 and 33.3): ops.heads_at_once.
 constexpr int GH_BN = 32, GH_ROWS = 32, GH_MOST_K = 1024;
 struct HeadsArgs {
     const __nv_bfloat16* A; long long lda, a_group_stride;

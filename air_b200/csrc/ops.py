@@ -1039,6 +1039,29 @@ def moe_sort(expert, experts, start, pair_of_slot, tiles, num_tiles, tile_rows=G
                                 pair_of_slot.data_ptr(), tiles.data_ptr(), num_tiles.data_ptr(), _stream()), "moe_sort")
 
 
+def heads_at_once(rows: int, groups: int, n: int, k: int) -> bool:
+    """Whether heads_gemm_kernel takes products per head of that many rows: by how many rounds of the SMs its blocks need, each of 32 rows
+    of W and up to 32 of A in shared memory.  The grouped kernel is a chain through k that hardly grows with the number of heads, and
+    reads W once for 64 rows; this one is ahead while its rounds are few and full.  us, the grouped kernel and this one, by heads x [n, k],
+    rows and rounds: more than 32 rows 48 x [128, 512] 64 0.9 9.0 / 6.5; 64 heads 1.2 9.6 / 11.7, 48 rows 9.0 / 8.5; 96 heads 1.7 14.4 / 12.3; 128
+    heads, 48 rows 2.3 13.5 / 13.4, 64 rows 15.1 / 17.9; 16 x [192, 1024] 1.3 14.0 / 10.9, 32 heads 2.6 15.0 / 16.6.  Up to 32: 160 x [128, 512] 32
+    1.4 14.7 / 12.3; 64 x [192, 1024] 2.6 20.1 / 17.4, 128 heads 5.2 27 / 34; 128 x [256, 256] 1.2 10.0 / 10.3; 96 x [512, 256] 1.7 13.7 /
+    13.0.  Up to 16: 160 x [512, 256] 2.2 14.2 / 12.4; 160 x [192, 1024] 3.2 22.9 / 22.3; 96 x [512, 64] 0.6 6.6 / 5.5, 128 heads 0.9 6.7 / 7.5."""
+    if not 0 < rows <= (64 if k >= 256 else 24) or k > 1024:
+        return False
+    block = (32 + min(32, -(-rows // 8) * 8)) * (k + 8) * 2 + 1024
+    rounds = groups * -(-n // 32) * -(-rows // 32) / (148 * min(16, 228 * 1024 // block))
+    if k < 128:
+        return rounds <= (0.7 if rows <= 16 else 0.35)
+    if rows <= 16:
+        return rounds <= (4.0 if k > 512 else 2.5)
+    if rows <= 32:
+        return rounds <= (3.0 if k > 512 else 2.0) and (k > 256 or not 1.0 < rounds < 1.6)
+    if rows <= 48:
+        return rounds <= (2.5 if 256 < k <= 512 else 2.0)
+    return rounds <= 2.0 and (k > 512 or not 1.0 < rounds < 1.6)
+
+
 def grouped_gemm(a, w, out, n, k, *, lda, ldo, groups, a_group_stride=0, o_group_stride=0, a_index=None, a_div=1,
                  a_scale=None, a_local=False, o_index=None, o_div=1, o_part_stride=0, o_local=False, start=None,
                  rows_per_group=0, tiles=None, num_tiles=None, silu_mul=False, gate_block=0, o_scale=None, o_scale_ld=0,
@@ -1068,7 +1091,7 @@ def grouped_gemm(a, w, out, n, k, *, lda, ldo, groups, a_group_stride=0, o_group
         _req(o_scale, "o_scale", (torch.float32,))
     if (w_ready and a.dtype == torch.bfloat16 and a_local and o_local and not (silu_mul or relu2) and start is None and tiles is None
             and a_index is None and a_scale is None and o_index is None and k % 16 == 0 and lda % 8 == 0 and a_group_stride % 8 == 0
-            and 0 < rows_per_group <= (64 if k >= 256 else 24) and k <= 1024 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
+            and heads_at_once(rows_per_group, groups, n, k) and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
         _check(_get("air_heads_gemm")(
             a.data_ptr(), int(lda), int(a_group_stride), w.data_ptr(), out.data_ptr(), int(ldo), int(o_group_stride),
             1 if out.dtype == torch.float32 else 0, int(rows_per_group), int(groups), int(n), int(k), _ptr(o_scale), int(o_scale_ld),

@@ -778,6 +778,23 @@ def test_products_per_head_of_few_rows(H, N, K, T):
         assert ((outs[1][:, :H * N].view(T, H, N).double() - want).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("H,N,K,rows", [(160, 128, 512, (32, 33)), (128, 128, 512, (32, 48, 49)), (32, 192, 1024, (16, 32, 33)), (96, 512, 64, (16, 17)),
+                                        (128, 256, 256, (16, 24, 33))])
+def test_products_of_many_heads_on_either_side_of_their_line(H, N, K, rows):
+    """More blocks than the SMs take at once, on both sides of the rule's lines: the grouped product's bits."""
+    from air_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(H + N)
+    w = torch.randn(H, N, K, generator=g, device="cuda").bfloat16()
+    assert len({ops.heads_at_once(T, H, N, K) for T in rows}) == 2
+    for T in rows:
+        x, outs = torch.randn(T, H * K, generator=g, device="cuda").bfloat16(), []
+        for ready in (False, True):
+            outs.append(torch.full((T, H * N), 9.0, device="cuda"))
+            ops.grouped_gemm(x, w, outs[-1], N, K, lda=H * K, ldo=H * N, groups=H, a_group_stride=K, o_group_stride=N, a_local=True, o_local=True,
+                             rows_per_group=T, w_ready=ready)
+        assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("ready", [False, True])
 def test_products_per_head_refuse_what_they_do_not_read(ready):
     """A scale of A's rows without a list of them, and tiles without their starts, are refused whether or not W was there before."""
