@@ -15,7 +15,7 @@
 // q, out: [T, H, d]; cache, block_table, token_seq, positions, window, mask_mode, softcap, sink, gate, bias as in attention_ref.cu.
 // Every wait on an mbarrier is bounded; on giving up the block sets *status = 5.
 //
-// Measured, us, that kernel -> this one (28 heads of 128 in groups of seven): 4 requests over 40 keys 6.1 -> 6.4, over 1,000 26.5 -> 14.4,
+// Measured, us, that kernel -> this one (28 heads of 128 in groups of seven): 4 requests over 40 keys 6.1 -> 6.1, over 1,000 26.5 -> 14.4,
 // over 2,000 49 -> 24; 8 over 2,000 73 -> 31; 64 over 2,000 552 -> 191; one over 4,000 94 -> 37.  16 heads in groups of four: 8 over 2,000
 // 49 -> 24; 64 over 1,000 201 -> 88.  16 heads of 64 in pairs: 8 over 1,000 30 -> 16, 16 over 100 7.8 -> 7.1.  From 5 to 100 keys they
 // differ by no more than 0.3.
@@ -261,7 +261,6 @@ __global__ void __launch_bounds__(FS_THREADS, 2) attention_f32_single_kernel(con
         }
     }
     cluster.sync();                              // (from here on each reads its own memory only)
-    cluster.sync();
     for (int x = tid; x < (nh - chain + FS_CHAINS - 1) / FS_CHAINS * dv; x += (int)blockDim.x) {
         const int i = x / dv, c = x % dv, h = h0 + i * FS_CHAINS + chain;
         const float* from = smem + places.results() + i * FS_CHAINS * (dv + 4);
