@@ -15,10 +15,11 @@
 // q, out: [T, H, d]; cache, block_table, token_seq, positions, window, mask_mode, softcap, sink, gate, bias as in attention_ref.cu.
 // Every wait on an mbarrier is bounded; on giving up the block sets *status = 5.
 //
-// Measured, us, that kernel -> this one (28 heads of 128 in groups of seven): 4 requests over 40 keys 6.1 -> 6.1, over 1,000 26.5 -> 14.4,
-// over 2,000 49 -> 24; 8 over 2,000 73 -> 31; 64 over 2,000 552 -> 191; one over 4,000 94 -> 37.  16 heads in groups of four: 8 over 2,000
-// 49 -> 24; 64 over 1,000 201 -> 88.  16 heads of 64 in pairs: 8 over 1,000 30 -> 16, 16 over 100 7.8 -> 7.1.  From 5 to 100 keys they
-// differ by no more than 0.3.
+// Measured, us, that kernel -> this one (28 heads of 128 in groups of seven): 4 requests over 40 keys 6.1 -> 5.8, over 1,000 26 -> 14.0; 8 over
+// 1,000 39 -> 17.9; 64 over 40 36 -> 19.0, over 1,000 288 -> 104; one over 2,000 48 -> 20.6, over 8,000 181 -> 66.  16 heads in groups of four: 64 over
+// 1,000 200 -> 86.  16 heads of 64 in pairs: 8 over 1,000 30 -> 15.8, 64 over 100 34 -> 22.  Up to eight requests over 5 to 100 keys differ by
+// no more than 0.4, but for 40 and 48 heads in groups of five and six, 6 over 40: 6.6 -> 7.4 and 7.7.  32 heads of 128 in pairs, 64 over 100: 52 -> 60.
+// (With blocks that stay although their chain has no keys: 64 over 40, 28 heads 25.7; 40 heads in groups of five 45 instead of 30.)
 #include "common.cuh"
 #include "tma.cuh"
 
@@ -33,18 +34,20 @@ struct SingleArgs {
     const float* q; const float* cache; const int* block_table; int max_blocks; const int* token_seq; const int* positions;
     float* out; const float* gate; int H, K, d, dv, P, window; float scale, softcap; int mask_mode; const float* sink;
     DistanceBias bias;
-    int heads, stages;            // heads of a block, places of the ring
+    int heads, stages, leave;     // heads of a block, places of the ring, whether blocks without keys leave
     int* status;
 };
-// Shared memory, in floats: the heads' queries, their weights of a block of keys, their results, then per stage 32 keys (rows of d + 4) and
-// 32 values.
+// Shared memory, in floats: the heads' queries, their weights of a block of keys, per stage 32 keys (rows of d + 4) and 32 values, then the
+// results of the heads that this block merges (a share of them, a place for every chain: up to three more than heads).
 struct SinglePlaces {
     int d, dv;
     __host__ __device__ int stage() const { return 32 * (d + 4) + 32 * dv; }
     __host__ __device__ int weights() const { return FS_HEADS * d; }
-    __host__ __device__ int results() const { return weights() + FS_HEADS * 32; }
-    __host__ __device__ int ring() const { return results() + FS_HEADS * (dv + 4); }
-    __host__ __device__ size_t bytes(int stages) const { return sizeof(float) * (size_t)(ring() + stages * stage()); }
+    __host__ __device__ int ring() const { return weights() + FS_HEADS * 32; }
+    __host__ __device__ int results(int stages) const { return ring() + stages * stage(); }
+    __host__ __device__ size_t bytes(int heads, int stages) const {
+        return sizeof(float) * (size_t)(results(stages) + (heads + FS_CHAINS - 1) * (dv + 4));
+    }
 };
 
 // A warp per head of the block, and two that bring.  D: the size of keys and values where it is known, else 0.
@@ -74,7 +77,11 @@ __global__ void __launch_bounds__(FS_THREADS, 2) attention_f32_single_kernel(con
     if (seq < 0) return;                         // padding: the same for the whole cluster
     const int pos = a.positions[t];
     const int lo = a.window > 0 ? (a.mask_mode == 1 ? pos - pos % a.window : max(0, pos - a.window + 1)) : 0;
-    const int first = (lo / 32 / FS_CHAINS) * FS_CHAINS + chain, n = first * 32 > pos ? 0 : (pos / 32 - first) / FS_CHAINS + 1;
+    const int base = (lo / 32 / FS_CHAINS) * FS_CHAINS, first = base + chain;
+    // Where blocks wait for SMs, one whose chain has no keys leaves (the cluster's barriers wait for those that have not left): the others
+    // merge without it, and nobody writes into its memory.
+    if (a.leave && chain > pos / 32 - base) return;
+    const int n = first * 32 > pos ? 0 : (pos / 32 - first) / FS_CHAINS + 1;
     float* ring = smem + places.ring();
     float m = -INFINITY, l = 0.f, acc[4] = {};   // of this warp's head: lane x holds numbers 4x..4x+3 of its weighted values
     cluster.barrier_arrive();
@@ -251,9 +258,10 @@ __global__ void __launch_bounds__(FS_THREADS, 2) attention_f32_single_kernel(con
             here = there;
         }
     }
-    cluster.barrier_wait();                      // (all four have begun: their memory may be written)
+    cluster.barrier_wait();                      // (all that stay have begun: their memory may be written)
+    const int chains = a.leave ? min(FS_CHAINS, pos / 32 - lo / 32 / FS_CHAINS * FS_CHAINS + 1) : FS_CHAINS;
     if (warp < nh) {
-        float* results = cluster.map_shared_rank(smem + places.results(), warp % FS_CHAINS) + (warp / FS_CHAINS * FS_CHAINS + chain) * (dv + 4);
+        float* results = cluster.map_shared_rank(smem + places.results(a.stages), warp % chains) + (warp / chains * chains + chain) * (dv + 4);
         if (lane * 4 < dv) *(float4*)(results + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
         if (lane == 0) {
             results[dv] = m;
@@ -261,16 +269,16 @@ __global__ void __launch_bounds__(FS_THREADS, 2) attention_f32_single_kernel(con
         }
     }
     cluster.sync();                              // (from here on each reads its own memory only)
-    for (int x = tid; x < (nh - chain + FS_CHAINS - 1) / FS_CHAINS * dv; x += (int)blockDim.x) {
-        const int i = x / dv, c = x % dv, h = h0 + i * FS_CHAINS + chain;
-        const float* from = smem + places.results() + i * FS_CHAINS * (dv + 4);
+    for (int x = tid; x < (nh - chain + chains - 1) / chains * dv; x += (int)blockDim.x) {
+        const int i = x / dv, c = x % dv, h = h0 + i * chains + chain;
+        const float* from = smem + places.results(a.stages) + i * chains * (dv + 4);
         float mm = a.sink ? a.sink[h] : -INFINITY, mw[FS_CHAINS], lw[FS_CHAINS], aw[FS_CHAINS];
 #pragma unroll
         for (int w = 0; w < FS_CHAINS; ++w) {
             const float* head = from + w * (dv + 4);
-            mw[w] = head[dv];
-            lw[w] = head[dv + 1];
-            aw[w] = head[c];
+            mw[w] = w < chains ? head[dv] : -INFINITY;
+            lw[w] = w < chains ? head[dv + 1] : 0.f;
+            aw[w] = w < chains ? head[c] : 0.f;
         }
 #pragma unroll
         for (int w = 0; w < FS_CHAINS; ++w) mm = fmaxf(mm, mw[w]);
@@ -292,6 +300,12 @@ __global__ void __launch_bounds__(FS_THREADS, 2) attention_f32_single_kernel(con
 
 }  // namespace air
 
+// A head to a block, for any batch (attention_ref.cu).
+extern "C" int air_paged_attention_ref(const void* q, int q_f32, const void* cache, int dtype, const int* block_table, int max_blocks,
+                                       const int* token_seq, const int* positions, void* out, const float* gate, int T, int H, int K, int d,
+                                       int dv, int P, int window, float scale, float softcap, int mask_mode, const float* sink, int latent,
+                                       const float* bias, int bias_n, cudaStream_t stream);
+
 // Every row of the batch as a token by itself, for a float32 cache [page, K, P, d] keys then [K, P, dv] values on a 16-byte boundary, d and dv
 // multiples of 4 up to 128, H a multiple of K.
 AIR_API int air_attention_f32_single(const float* q, const float* cache, const int* block_table, int max_blocks, const int* token_seq,
@@ -305,7 +319,7 @@ AIR_API int air_attention_f32_single(const float* q, const float* cache, const i
         return AIR_ERR_BAD_ARGUMENT;
     const int G = H / K;
     SingleArgs a{q, cache, block_table, max_blocks, token_seq, positions, out, gate, H, K, d, dv, P, window, scale, softcap, mask_mode, sink,
-                 DistanceBias{bias, bias_n}, 0, 0, status};
+                 DistanceBias{bias, bias_n}, 0, 0, 0, status};
     // As even shares of a group's heads as blocks of up to eight allow; fewer heads to a block where SMs would be idle (one request over
     // 2,000 keys, 28 heads in groups of seven: 29.7 us with seven to a block, 21.2 with one).
     const int idle = (int)max(1ll, min((long long)G, 128ll / ((long long)FS_CHAINS * K * T)));
@@ -313,15 +327,22 @@ AIR_API int air_attention_f32_single(const float* q, const float* cache, const i
     a.heads = (G + most - 1) / most;
     const int shares = (G + a.heads - 1) / a.heads;
     const SinglePlaces places{d, dv};
-    // Blocks that all find an SM look far ahead; beyond, as many share one as there are, and as registers, 96 a thread, allow (512 blocks
-    // of 1,000 keys, 16 heads of 64 in pairs: 32 us with three to an SM, 20 with four; 1,024 of 2,000 keys, seven heads: 238 with room for
-    // three of which registers let two in, 191 with room for two).
+    // Blocks that all find an SM look far ahead; beyond, as many share one as there are, as registers, five warps to a scheduler, allow and as
+    // two places of each find room (512 blocks of 1,000 keys, 16 heads of 64 in pairs: 32 us with three to an SM, 20 with four; 1,024 of 2,000
+    // keys, seven heads: 238 with room for three of which registers let two in, 191 with room for two).
     const long long blocks = (long long)FS_CHAINS * K * shares * T;
-    const int resident = (int)min((blocks + 147) / 148, (long long)min(4, 680 / ((a.heads + 2) * 32)));
+    const int fit = (int)min((long long)min(4, 20 / (a.heads + 2)), 227 * 1024ll / (long long)(places.bytes(a.heads, 2) + 1280));
+    // (heads in pairs gain little by reading keys once: not a second round of the SMs for a few blocks.  16 pairs of 128, 8 requests, 512
+    // blocks where 444 fit, over 100 and 1,000 keys: 11.9 and 48 us, one head to a block 8.3 and 42; 24 requests 23 and 28, here and there)
+    if (G == 2 && fit < 4 && blocks > 148ll * fit && 2 * blocks < 3 * 148ll * fit)
+        return air_paged_attention_ref(q, 1, cache, AIR_F32, block_table, max_blocks, token_seq, positions, out, gate, T, H, K, d, dv, P, window,
+                                       scale, softcap, mask_mode, sink, 0, bias, bias_n, stream);
+    const int resident = (int)min((blocks + 147) / 148, (long long)fit);
+    a.leave = blocks > 148ll * resident;
     const size_t room = (resident == 1 ? 200 : 226 / resident - 1) * 1024;
     a.stages = FS_MOST_STAGES;
-    while (a.stages > 2 && places.bytes(a.stages) > room) --a.stages;
-    const size_t smem = places.bytes(a.stages);
+    while (a.stages > 2 && places.bytes(a.heads, a.stages) > room) --a.stages;
+    const size_t smem = places.bytes(a.heads, a.stages);
     auto kernel = d == FS_D && dv == FS_D ? attention_f32_single_kernel<FS_D> : attention_f32_single_kernel<0>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;

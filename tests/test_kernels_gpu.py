@@ -590,6 +590,22 @@ def test_float32_attention_of_single_tokens(H, K, d, dv, P, window, chunk, n):
         assert (out[n:] == 7.0).all() and int(status) == 0
 
 
+@pytest.mark.parametrize("T", [6, 8, 10, 12, 40])
+def test_float32_attention_of_pairs_of_heads(T):
+    """Sixteen pairs of heads of 128: fewer blocks than the SMs take at once, a few more (a head by itself then), and many more, of which
+    those without keys leave: the bits of the kernel of a head by itself."""
+    H, K, d, P = 32, 16, 128, 32
+    gen = torch.Generator().manual_seed(T)
+    contexts = [(29 * i) % 200 for i in range(T)]
+    cache, pages = torch.randn(T * 7, 2, K, P, d, generator=gen).cuda(), torch.randperm(T * 7, generator=gen).int().view(T, 7).cuda()
+    q, positions, seq_of = torch.randn(T, H, d, generator=gen).cuda(), torch.tensor(contexts, dtype=torch.int32).cuda(), torch.arange(T, dtype=torch.int32).cuda()
+    outs = []
+    for single in (False, True):
+        outs.append(torch.full((T, H, d), 7.0, device="cuda"))
+        ops().paged_attention_ref(q, cache, pages, seq_of, positions, outs[-1], 0, d ** -0.5, single=single)
+    assert torch.isfinite(outs[0]).all() and torch.equal(*outs)
+
+
 @pytest.mark.parametrize("far", [0, 15, 16, 17, 63, 64, 300, 447])
 def test_attention_finds_one_far_key_among_hundreds(far):
     """One key is made to match the query so that its score stands out: the output must be that
