@@ -403,25 +403,67 @@ template <int DP, int MODE> struct DeltaScan {
 
 // 16 rows by NJ tiles of 8 channels times the state's columns: what the tensor cores cut off instead of rounding is kept small, since a
 // large product is summed from zero and added up in 32 bits and the small ones have sums of their own.
+template <int N>
+__device__ __forceinline__ void add_tile(float2 (&sum)[N][2], float (&low)[N][4], int j, const Two (&a)[4], const Two (&b)[N][2]) {
+    float high[N][4];
+    mma_two<N>(j == 0, low, high, a, b);
+#pragma unroll
+    for (int x = 0; x < N; ++x)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float2 v = make_float2(high[x][2 * e], high[x][2 * e + 1]);
+            sum[x][e] = j ? add2(sum[x][e], v) : v;
+        }
+}
+template <int N> __device__ __forceinline__ void add_low(float2 (&sum)[N][2], const float (&low)[N][4]) {
+#pragma unroll
+    for (int x = 0; x < N; ++x)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) sum[x][e] = add2(sum[x][e], make_float2(low[x][2 * e], low[x][2 * e + 1]));
+}
 template <int NJ>
 __device__ __forceinline__ void rows_by_state(float2 (&sum)[2][2], const Two (&a)[NJ][4], const Two (&b)[NJ][2][2]) {
     float low[2][4];
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-        float high[2][4];
-        mma_two<2>(j == 0, low, high, a[j], b[j]);
+    for (int j = 0; j < NJ; ++j) add_tile(sum, low, j, a[j], b[j]);
+    add_low(sum, low);
+}
+
+// U's numbers of a column and two tokens: Y less the four warps' W S.
+__device__ __forceinline__ float2 less_sums(float2 y, const float* from) {
+    float2 v[DC_WARPS];
 #pragma unroll
-        for (int x = 0; x < 2; ++x)
+    for (int w = 0; w < DC_WARPS; ++w) v[w] = *reinterpret_cast<const float2*>(from + w * DC * DC_RLD);
+    return sub2(y, add2(add2(v[0], v[1]), add2(v[2], v[3])));
+}
+// Of p: what token t (0 .. 7) and its mirror image 15 - t take of the tokens up to them (17 products in all).
+__device__ __forceinline__ void rows_of_p(float (&pa)[DC / 2], float (&pb)[DC], const float* p, int t) {
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const float2 v = make_float2(high[x][2 * e], high[x][2 * e + 1]);
-                sum[x][e] = j ? add2(sum[x][e], v) : v;
-            }
+    for (int s = 0; s < DC; s += 4) {
+        if (s < DC / 2) load4(p + t * DC + dc_key_place(t, s), *reinterpret_cast<float(*)[4]>(&pa[s]));
+        load4(p + (DC - 1 - t) * DC + dc_key_place(DC - 1 - t, s), *reinterpret_cast<float(*)[4]>(&pb[s]));
     }
+}
+// The outputs of these two tokens in a column: q S (the warps' sums [warps][16][DC_ULD], at the column) and what the chunk's tokens add to
+// one another, on the CUDA cores: only those up to a token itself, since a product with the zeros of p above the diagonal would carry a
+// later token's infinity or NaN into this one's o.
+__device__ __forceinline__ float2 outputs_of(const float (&pa)[DC / 2], const float (&pb)[DC], const float* u_at, const float* sums, int t) {
+    float u[DC], va[DC_WARPS], vb[DC_WARPS];
 #pragma unroll
-    for (int x = 0; x < 2; ++x)
+    for (int s = 0; s < DC; s += 4) load4(u_at + s, *reinterpret_cast<float(*)[4]>(&u[s]));
 #pragma unroll
-        for (int e = 0; e < 2; ++e) sum[x][e] = add2(sum[x][e], make_float2(low[x][2 * e], low[x][2 * e + 1]));
+    for (int w = 0; w < DC_WARPS; ++w) {
+        va[w] = sums[(w * DC + t) * DC_ULD];
+        vb[w] = sums[(w * DC + DC - 1 - t) * DC_ULD];
+    }
+    float o_a = 0.f, o_b = 0.f, late = 0.f;
+#pragma unroll
+    for (int s = 0; s < DC / 2; ++s) {
+        if (s <= t) o_a = fmaf(pa[s], u[s], o_a);
+        o_b = fmaf(pb[s], u[s], o_b);
+        if (s < DC / 2 - t) late = fmaf(pb[DC / 2 + s], u[DC / 2 + s], late);
+    }
+    return make_float2(((va[0] + va[1]) + (va[2] + va[3])) + o_a, ((vb[0] + vb[1]) + (vb[2] + vb[3])) + (o_b + late));
 }
 
 // DC_WARPS warps hold the state.  Such a warp holds NJ tiles of 8 channels of it, transposed: S[j] is (column g or g + 8 of the block) x
@@ -431,7 +473,7 @@ __device__ __forceinline__ void rows_by_state(float2 (&sum)[2][2], const Two (&a
 template <int DP, int MODE, bool ALONE>
 __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_kernel(const DeltaChunkArgs p, int stages) {
     constexpr int NJ = DP / (8 * DC_WARPS), GROUP = NJ < 4 ? NJ : 4;
-    constexpr bool GLA = MODE == CHUNK_GLA, EARLY = ALONE && NJ <= 4, AHEAD = EARLY && !GLA;
+    constexpr bool GLA = MODE == CHUNK_GLA, EARLY = ALONE && NJ <= 4, AHEAD = EARLY && !GLA, BY_TILE = GLA && !ALONE && NJ > 4;
     using Place = DeltaChunk<DP, MODE>;
     using Scan = DeltaScan<DP, MODE>;
     constexpr int BUF = Scan::BUF;
@@ -499,11 +541,12 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
             const bool there = i + 1 == chunks || mbar_try_wait(&full[stage], phase);
             float2 sum[2][2];
             Two a[NJ][4];
+            if constexpr (!BY_TILE)
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-                two_of_pair(a[j][0], a[j][2], S[j][0]);
-                two_of_pair(a[j][1], a[j][3], S[j][1]);
-            }
+                for (int j = 0; j < NJ; ++j) {
+                    two_of_pair(a[j][0], a[j][2], S[j][0]);
+                    two_of_pair(a[j][1], a[j][3], S[j][1]);
+                }
             Two c[NJ][2][2];                     // (what is cut ahead of a product is cut between the one before it)
             if constexpr (EARLY) rows(c, buf, Place::ROWS - DC);
             if constexpr (!GLA) {
@@ -515,7 +558,7 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
                     for (int e = 0; e < 2; ++e) *reinterpret_cast<float2*>(sums_to + 8 * e * DC_RLD + 8 * x) = sum[x][e];
                 dc_arrive<DC_SUMS>();
             }
-            if constexpr (!EARLY) rows(c, buf, Place::ROWS - DC);
+            if constexpr (!EARLY && !BY_TILE) rows(c, buf, Place::ROWS - DC);
             Two k[2][GROUP][2], u[2][4];         // keys; U transposed, tokens 0 .. 7 and 8 .. 15
             auto keys = [&](int j0) {
 #pragma unroll
@@ -525,7 +568,22 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
                         two_pair(k[x][j], buf + Place::KEYS + (r0 + 8 * (j0 + j) + g) * DC + ((8 * x) ^ swap) + t2);
             };
             if constexpr (EARLY) keys(0);
-            rows_by_state(sum, a, c);
+            if constexpr (BY_TILE) {             // (as many registers as two blocks to an SM have)
+                float low[2][4];
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) {
+                    Two at[4], q[2][2];
+                    two_of_pair(at[0], at[2], S[j][0]);
+                    two_of_pair(at[1], at[3], S[j][1]);
+                    const float* row = buf + g * DP + t2 + dc_row_place(g, r0 + 8 * j);
+                    two_pair(q[0], row);
+                    two_pair(q[1], row + 8 * DP);
+                    add_tile(sum, low, j, at, q);
+                }
+                add_low(sum, low);
+            } else {
+                rows_by_state(sum, a, c);
+            }
             if constexpr (!EARLY) keys(0);
             if constexpr (GLA) {                 // (u is v; the helpers are done with the last chunk's sums)
 #pragma unroll
@@ -590,44 +648,20 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
     } else {
         const int mine = warp - DC_WARPS;
         // the numbers of U that this thread completes, a column's tokens u_t and u_t + 1, and the outputs: a token and its mirror image
-        // (17 products in all)
         const int u_c = 4 * mine + ((lane >> 2) & 3), u_t = 2 * (lane & 3) + 8 * (lane >> 4);
         const int o_c = lane & 15, o_t = mine + 4 * (lane >> 4);
         const float* const sums_from = rest + Scan::SUMS + u_c * DC_RLD + u_t;
         float* const out = p.out + ((size_t)row0 * p.H + h) * p.dv + col0 + o_c;
         const size_t out_row = (size_t)p.H * p.dv;
         const bool in = col0 + o_c < p.dv;
-        float pa[DC / 2], pb[DC];                // of p: what the two tokens take of those up to them
-        auto rows_of_p = [&](const float* buf) {
-#pragma unroll
-            for (int s = 0; s < DC; s += 4) {
-                if (s < DC / 2) load4(buf + Place::P + o_t * DC + dc_key_place(o_t, s), *reinterpret_cast<float(*)[4]>(&pa[s]));
-                load4(buf + Place::P + (DC - 1 - o_t) * DC + dc_key_place(DC - 1 - o_t, s), *reinterpret_cast<float(*)[4]>(&pb[s]));
-            }
-        };
-        // What the chunk's tokens add to one another, on the CUDA cores: only those up to a token itself, since a product with the
-        // zeros of p above the diagonal would carry a later token's infinity or NaN into this one's o.
+        float pa[DC / 2], pb[DC];
         auto outputs = [&](int i, const float* u_at) {
             const float* sums_of = rest + Scan::OUT + slot_out * DC_WARPS * DC * DC_ULD + o_c;
             if (++slot_out == Scan::OUTS) slot_out = 0;
-            float u[DC], va[DC_WARPS], vb[DC_WARPS];
-#pragma unroll
-            for (int s = 0; s < DC; s += 4) load4(u_at + s, *reinterpret_cast<float(*)[4]>(&u[s]));
-#pragma unroll
-            for (int w = 0; w < DC_WARPS; ++w) {
-                va[w] = sums_of[(w * DC + o_t) * DC_ULD];
-                vb[w] = sums_of[(w * DC + DC - 1 - o_t) * DC_ULD];
-            }
-            float o_a = 0.f, o_b = 0.f, late = 0.f;
-#pragma unroll
-            for (int s = 0; s < DC / 2; ++s) {
-                if (s <= o_t) o_a = fmaf(pa[s], u[s], o_a);
-                o_b = fmaf(pb[s], u[s], o_b);
-                if (s < DC / 2 - o_t) late = fmaf(pb[DC / 2 + s], u[DC / 2 + s], late);
-            }
+            const float2 o = outputs_of(pa, pb, u_at, sums_of, o_t);
             if (!in || !ok) return;
-            if (i * DC + o_t < tokens) out[(size_t)(i * DC + o_t) * out_row] = ((va[0] + va[1]) + (va[2] + va[3])) + o_a;
-            if (i * DC + DC - 1 - o_t < tokens) out[(size_t)(i * DC + DC - 1 - o_t) * out_row] = ((vb[0] + vb[1]) + (vb[2] + vb[3])) + (o_b + late);
+            if (i * DC + o_t < tokens) out[(size_t)(i * DC + o_t) * out_row] = o.x;
+            if (i * DC + DC - 1 - o_t < tokens) out[(size_t)(i * DC + DC - 1 - o_t) * out_row] = o.y;
         };
         for (int i = 0; i < chunks; ++i) {
             const float* buf = smem + stage * BUF;
@@ -636,10 +670,7 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
             float2 y = *reinterpret_cast<const float2*>(buf + Place::Y + u_c * DC + u_t);
             dc_sync<DC_SUMS>();
             if constexpr (!GLA) {
-                float2 v[DC_WARPS];
-#pragma unroll
-                for (int w = 0; w < DC_WARPS; ++w) v[w] = *reinterpret_cast<const float2*>(sums_from + w * DC * DC_RLD);
-                y = sub2(y, add2(add2(v[0], v[1]), add2(v[2], v[3])));
+                y = less_sums(y, sums_from);
                 if (i * DC + u_t >= tokens) y.x = 0.f;       // (of no token: nothing, also beside a state of infinities)
                 if (i * DC + u_t + 1 >= tokens) y.y = 0.f;
                 Two one, two;
@@ -651,12 +682,12 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
             // everybody is done with the chunk before this one: its buffer may be filled again
             if (tid == DC_WARPS * 32 && i > 0 && i - 1 + stages < chunks) bring(i - 1 + stages, stage ? stage - 1 : stages - 1);
             if constexpr (GLA) {
-                rows_of_p(buf);
+                rows_of_p(pa, pb, buf + Place::P, o_t);
                 outputs(i, buf + Place::Y + o_c * DC);
                 if (i + 1 < chunks) dc_arrive<DC_READY>();
             } else {
                 if (i > 0) outputs(i - 1, rest + Scan::U + ((i - 1) & 1) * DC * DC_ULD + o_c * DC_ULD);
-                rows_of_p(buf);
+                rows_of_p(pa, pb, buf + Place::P, o_t);
             }
             if (++stage == stages) {
                 stage = 0;
@@ -675,6 +706,148 @@ __global__ void __launch_bounds__(DC_THREADS, ALONE ? 1 : 2) delta_chunk_scan_ke
     }
 }
 
+// The same scan in four warps, for more blocks than the SMs hold of the other's (launch_delta_chunks says where).  What counts then is not the
+// chain but how many of them an SM has: half the threads, one chunk ahead instead of five, nothing cut ahead of its use, three to
+// eight blocks to an SM.  Every number is summed as above and in the same order, a chunk's outputs with the chunk: the same bits.
+template <int DP, int MODE> struct DeltaTogether {
+    static constexpr bool GLA = MODE == CHUNK_GLA;
+    static constexpr int BUF = DeltaScan<DP, MODE>::BUF;
+    static constexpr int OUT = 0, SUMS = OUT + DC_WARPS * DC * DC_ULD, U = SUMS + (GLA ? 0 : DC_WARPS * DC * DC_RLD), END = U + (GLA ? 0 : DC * DC_ULD);
+    static constexpr size_t bytes = sizeof(float) * (size_t)(2 * BUF + END);
+};
+template <int DP, int MODE>
+__global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_scan_together_kernel(const DeltaChunkArgs p) {
+    constexpr int NJ = DP / (8 * DC_WARPS), GROUP = NJ < 4 ? NJ : 4, RG = DeltaChunk<DP, MODE>::ROWS / 8;
+    constexpr bool GLA = MODE == CHUNK_GLA;
+    using Place = DeltaChunk<DP, MODE>;
+    using Scan = DeltaTogether<DP, MODE>;
+    constexpr int BUF = Scan::BUF;
+    extern __shared__ __align__(16) float smem[];
+    __shared__ __align__(8) uint64_t full[2];
+    __shared__ int gave_up;
+    float* const rest = smem + 2 * BUF;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t2 = 2 * (lane & 3);
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) mbar_init(&full[i], 1);
+        gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pdl_enter(TR_SCAN);
+    const int h = blockIdx.y, col0 = blockIdx.x * DC;
+    const int* por = p.portions + 4 * blockIdx.z;
+    const int row0 = por[0], tokens = por[1], slot = por[2], chunk0 = por[3];
+    if (slot < 0 || tokens <= 0) return;
+    const int chunks = (tokens + DC - 1) / DC;
+    auto bring = [&](int i) {               // (one thread)
+        const float* src = p.scratch + ((size_t)(chunk0 + i) * p.H + h) * p.stride;
+        float* dst = smem + (i & 1) * BUF;
+        mbar_expect_tx(&full[i & 1], BUF * 4);
+        bulk_load(dst, src, Place::Y * 4, &full[i & 1]);
+        bulk_load(dst + Place::Y, src + Place::Y + col0 * DC, DC * DC * 4, &full[i & 1]);
+    };
+    if (tid == 0) bring(0);
+    const int r0 = warp * 8 * NJ;
+    float* st = p.state + ((size_t)slot * p.H + h) * p.d * p.dv;
+    float2 S[NJ][2];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = r0 + 8 * j + t2 + (e & 1), c = col0 + g + 8 * (e >> 1);
+            (e & 1 ? S[j][e >> 1].y : S[j][e >> 1].x) = r < p.d && c < p.dv ? st[(size_t)r * p.dv + c] : 0.f;
+        }
+    const int swap = dc_key_place(g, 0);
+    const int u_c = 4 * warp + ((lane >> 2) & 3), u_t = 2 * (lane & 3) + 8 * (lane >> 4);
+    const int o_c = lane & 15, o_t = warp + 4 * (lane >> 4);
+    float* const out = p.out + ((size_t)row0 * p.H + h) * p.dv + col0 + o_c;
+    const size_t out_row = (size_t)p.H * p.dv;
+    for (int i = 0; i < chunks; ++i) {
+        const float* buf = smem + (i & 1) * BUF;
+        // this chunk's numbers are there and everybody is done with the chunk before it
+        if (__syncthreads_or(!mbar_wait(&full[i & 1], (i >> 1) & 1, &gave_up))) {
+            for (int x = 0; x < 32; ++x) __nanosleep(2000);      // (a copy on its way may still land)
+            if (tid == 0 && p.status) atomicExch(p.status, 9);
+            return;
+        }
+        if (tid == 0 && i + 1 < chunks) bring(i + 1);
+        float2 sum[RG][2];
+        float low[RG][4];
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            Two a[4], b[RG][2];
+            two_of_pair(a[0], a[2], S[j][0]);
+            two_of_pair(a[1], a[3], S[j][1]);
+            const float* at = buf + g * DP + t2 + dc_row_place(g, r0 + 8 * j);
+#pragma unroll
+            for (int x = 0; x < RG; ++x) two_pair(b[x], at + 8 * x * DP);
+            add_tile(sum, low, j, a, b);
+        }
+        add_low(sum, low);
+#pragma unroll
+        for (int x = 0; x < RG; ++x)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (x < RG - 2) {                // W's rows, then q's
+                    *reinterpret_cast<float2*>(rest + Scan::SUMS + (warp * DC + g + 8 * e) * DC_RLD + 8 * x + t2) = sum[x][e];
+                } else {
+                    float* to = rest + Scan::OUT + (warp * DC + 8 * (x - (RG - 2)) + t2) * DC_ULD + g + 8 * e;
+                    to[0] = sum[x][e].x;
+                    to[DC_ULD] = sum[x][e].y;
+                }
+            }
+        __syncthreads();
+        if constexpr (!GLA) {
+            float2 y = less_sums(*reinterpret_cast<const float2*>(buf + Place::Y + u_c * DC + u_t), rest + Scan::SUMS + u_c * DC_RLD + u_t);
+            if (i * DC + u_t >= tokens) y.x = 0.f;       // (of no token: nothing, also beside a state of infinities)
+            if (i * DC + u_t + 1 >= tokens) y.y = 0.f;
+            *reinterpret_cast<float2*>(rest + Scan::U + u_c * DC_ULD + u_t) = y;
+            __syncthreads();
+        }
+        const float* const U = GLA ? buf + Place::Y : rest + Scan::U;
+        constexpr int ULD = GLA ? DC : DC_ULD;
+        Two u[2][4];                         // U transposed, tokens 0 .. 7 and 8 .. 15
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) two_of_pair(u[x][e], u[x][2 + e], *reinterpret_cast<const float2*>(U + (g + 8 * e) * ULD + 8 * x + t2));
+#pragma unroll
+        for (int j0 = 0; j0 < NJ; j0 += GROUP) {
+            float more[2][GROUP][4], less[GROUP][4];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                Two k[GROUP][2];
+#pragma unroll
+                for (int j = 0; j < GROUP; ++j) two_pair(k[j], buf + Place::KEYS + (r0 + 8 * (j0 + j) + g) * DC + ((8 * x) ^ swap) + t2);
+                mma_two<GROUP>(x == 0, less, more[x], u[x], k);
+            }
+#pragma unroll
+            for (int j = 0; j < GROUP; ++j) {
+                const float2 left = *reinterpret_cast<const float2*>(buf + Place::LAST + r0 + 8 * (j0 + j) + t2);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float2 x = make_float2(more[0][j][2 * e], more[0][j][2 * e + 1]), y = make_float2(more[1][j][2 * e], more[1][j][2 * e + 1]);
+                    S[j0 + j][e] = fma2(S[j0 + j][e], left, add2(x, add2(y, make_float2(less[j][2 * e], less[j][2 * e + 1]))));
+                }
+            }
+        }
+        float pa[DC / 2], pb[DC];
+        rows_of_p(pa, pb, buf + Place::P, o_t);
+        const float2 o = outputs_of(pa, pb, U + o_c * ULD, rest + Scan::OUT + o_c, o_t);
+        if (col0 + o_c < p.dv) {
+            if (i * DC + o_t < tokens) out[(size_t)(i * DC + o_t) * out_row] = o.x;
+            if (i * DC + DC - 1 - o_t < tokens) out[(size_t)(i * DC + DC - 1 - o_t) * out_row] = o.y;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = r0 + 8 * j + t2 + (e & 1), c = col0 + g + 8 * (e >> 1);
+            if (r < p.d && c < p.dv) st[(size_t)r * p.dv + c] = e & 1 ? S[j][e >> 1].y : S[j][e >> 1].x;
+        }
+}
+
 template <int DP, int MODE, bool ALONE>
 static int launch_delta_scan(const DeltaChunkArgs& a, dim3 grid, size_t room, size_t least, cudaStream_t stream) {
     using Scan = DeltaScan<DP, MODE>;
@@ -690,6 +863,19 @@ static int launch_delta_scan(const DeltaChunkArgs& a, dim3 grid, size_t room, si
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     return launch_counted(cfg, kernel, a, stages);
+}
+
+template <int DP, int MODE> static int launch_delta_together(const DeltaChunkArgs& a, dim3 grid, cudaStream_t stream) {
+    const size_t smem = DeltaTogether<DP, MODE>::bytes;
+    auto kernel = delta_chunk_scan_together_kernel<DP, MODE>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(DC_WARPS * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    return launch_counted(cfg, kernel, a);
 }
 
 template <int DP, int MODE>
@@ -710,10 +896,18 @@ static int launch_delta_chunks(const DeltaChunkArgs& args, int N, int L, cudaStr
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long blocks = (long long)grid.x * grid.y * grid.z;
-    // Where every block has an SM to itself, or only one block's memory fits, a warp has the registers to cut what its next product
-    // reads between the instructions of the one before, and as many chunks are under way as memory holds; else two blocks share an SM.
-    // (32 heads of 128 x 128, 256 blocks, 2,048 tokens: 192 us; with one block to an SM they would take two rounds of 106.)
+    // Where every block has an SM to itself a warp has the registers to cut what its next product reads between the instructions of the one
+    // before, and as many chunks are under way as memory holds; else two blocks share an SM, except where a delta rule's rows of 256 leave
+    // no registers for that.  (32 heads of 128 x 128, 256 blocks, 2,048 tokens: 192 us; with one block to an SM they would take two rounds of
+    // 106.  Gated linear attention, heads of 256 x 256, two to an SM and one, us with the preparation: 16 heads, 300 tokens 69.3 and 72, 32 heads,
+    // 1,000 tokens 342 and 359, 8 portions of 33 tokens 166 and 205.)
+    // More blocks than that, and an SM is kept busy by four warps of each of three to eight: delta rule, two to an SM and these, heads of 64 x 128,
+    // 512 blocks 3, 7 and 13 chunks long 22.7 / 20.6, 32.2 / 30.5 and 47.5 / 45.8, 4,096 of 7 172 / 152; heads of 128, 512 of 3, 7 and 63 chunks
+    // 25.0 / 24.7, 47.1 / 48.5 and 240 / 248 (gated linear attention 22.6 / 20.8, 38.8 / 37.4, 184 / 195), 1,024 of 7 67.6 / 65.7, 4,096 of 3 108 /
+    // 98; heads of 256, 4,096 of 13 656 / 734.
     if constexpr (DP <= 128)
+        if (blocks > 2 * sms && (DP <= 64 || blocks > 4 * sms || N <= 4 * L)) return launch_delta_together<DP, MODE>(a, grid, stream);
+    if constexpr (DP <= 128 || MODE == CHUNK_GLA)
         if (blocks > sms) return launch_delta_scan<DP, MODE, false>(a, grid, 113 * 1024, 0, stream);
     return launch_delta_scan<DP, MODE, true>(a, grid, 226 * 1024, blocks <= sms ? 120 * 1024 : 0, stream);
 }

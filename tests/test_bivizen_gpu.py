@@ -308,6 +308,39 @@ def test_chunks_of_many_portions_are_those_of_each_alone(H, d, dv, mode):
 
 
 @pytest.mark.parametrize("mode", ["delta", "gla", "channel"])
+@pytest.mark.parametrize("H,d,dv", [(48, 32, 24), (24, 64, 64), (29, 50, 65), (12, 128, 128), (9, 256, 256)])
+@pytest.mark.parametrize("counts", [(1, 16, 17, 97, 113, 15, 130), (33, 1, 16, 40, 17, 2, 31)])
+def test_chunks_in_more_blocks_than_find_room(counts, H, d, dv, mode):
+    """Several blocks of four warps to an SM, or two of eight, against a block by itself: the same bits, outputs and states, also of
+    what an infinity and a NaN reach."""
+    from air_b200.csrc import ops
+    which = {"delta": ops.SCAN_DELTA, "gla": ops.SCAN_GLA, "channel": ops.SCAN_CHANNEL_DELTA}[mode]
+    per, T, L = (H if mode == "delta" else H * d), sum(counts), len(counts)
+    assert L * H * -(-dv // 16) > 4 * 148 and H * -(-dv // 16) <= 148
+    g = torch.Generator(device=DEV).manual_seed(d)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    q, k, v, z, b, S0 = rand(T, H * d), rand(T, H * d), rand(T, H * dv), rand(T, per), rand(T, H), rand(L, H, d, dv)
+    v[counts[0] + 5, 0], v[counts[0] + counts[1] + 3, dv] = float("inf"), float("nan")
+    more = dict(tau=8.0) if mode == "gla" else dict(beta=b, a_log=rand(H) / 2, dt_bias=rand(per))
+    start = np.concatenate([[0], np.cumsum(counts)])
+    table = lambda rows: torch.tensor(np.array(rows), dtype=torch.int32, device=DEV)
+    portions, chunks = [], []
+    for i, n in enumerate(counts):
+        portions.append((start[i], n, i, len(chunks)))
+        chunks += [(start[i] + a, min(ops.DELTA_CHUNK, n - a)) for a in range(0, n, ops.DELTA_CHUNK)]
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got = []
+    for tables in ([portions], [[row] for row in portions]):
+        S, o = S0.clone(), torch.full((T, H, dv), 9.0, device=DEV)
+        for rows in tables:
+            ops.delta_portions(q, k, v, z, S, o, table(rows), table(chunks), d ** -0.5, mode=which, status=status, **more)
+        got.append((o, S))
+    assert int(status) == 0
+    for a, b in zip(*got):
+        assert ((a == b) | (a.isnan() & b.isnan())).all() and a.isnan().any()
+
+
+@pytest.mark.parametrize("mode", ["delta", "gla", "channel"])
 @pytest.mark.parametrize("H,d,dv", [(2, 64, 40), (12, 128, 128), (4, 256, 96)])
 def test_portions_of_no_token_leave_everything_as_it_is(H, d, dv, mode):
     """Portions of no token with a slot of their own, ahead of, between and behind others: their states stay, nothing is written
