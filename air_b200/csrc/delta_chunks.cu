@@ -313,14 +313,7 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 4 : 2) delta_chunk_prepare_ke
     }
 }
 
-// A 32-bit number as two TF32 numbers: the instruction reads the upper 19 bits of an operand.  The upper one is rounded, so that
-// the lower one has 12 bits and a sign of its own, and what it loses is 2^-23 of x at most, to either side.  (Where rounding
-// carries a NaN's bits into the sign, x - hi is a NaN all the same.)
 struct Two { uint32_t hi, lo; };
-__device__ __forceinline__ Two two_of(float x) {
-    const uint32_t hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    return Two{hi, __float_as_uint(x - __uint_as_float(hi))};
-}
 // c = a b (FRESH) or c += a b; with k in the order that the accumulators have: a holds (row g, k 2t), (g + 8, 2t), (g, 2t + 1),
 // (g + 8, 2t + 1), b holds (k 2t, column g), (2t + 1, g)
 template <bool FRESH>
@@ -367,6 +360,9 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
         : "+f"(a.x), "+f"(a.y) : "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
     return a;
 }
+// A 32-bit number as two TF32 numbers, for a pair of them: the instruction reads the upper 19 bits of an operand.  The upper one is rounded,
+// so that the lower one has 12 bits and a sign of its own, and what it loses is 2^-23 of x at most, to either side.  (Where rounding
+// carries a NaN's bits into the sign, x - hi is a NaN all the same.)
 __device__ __forceinline__ void two_of_pair(Two& a, Two& b, float2 v) {
     a.hi = (__float_as_uint(v.x) + 0x1000u) & 0xffffe000u;
     b.hi = (__float_as_uint(v.y) + 0x1000u) & 0xffffe000u;
