@@ -316,9 +316,12 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 const int col = n0 / 2 + r;
 #pragma unroll 1
                 for (int t = 0; t < args.T; t += 4) {
-                    float gate[4], up[4];
-                    ts_sums<NT, ISSUERS, 4>(taddr + t, steps, before, gate);
-                    ts_sums<NT, ISSUERS, 4>(taddr + ISSUERS * NT + t, steps, before, up);
+                    static_assert(ISSUERS == 1, "gate and up in tiles of 256 rows");
+                    uint32_t gate[4], up[4];
+                    __syncwarp();
+                    ts_ask<4>(taddr + t, gate);
+                    ts_ask<4>(taddr + NT + t, up);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (col < args.N / 2) {
                         __nv_bfloat16* out = (__nv_bfloat16*)args.out + (size_t)t * (args.N / 2) + col;
 #pragma unroll
@@ -326,7 +329,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                             const float scale = args.ss ? row_scale[t + i] : 1.f;
                             if (t + i < args.T)
                                 out[(size_t)i * (args.N / 2)] = __float2bfloat16_rn(
-                                    gated_activation(gate[i] * scale, up[i] * scale, args.act_alpha, args.act_limit, args.act_shift));
+                                    gated_activation(__uint_as_float(gate[i]) * scale, __uint_as_float(up[i]) * scale, args.act_alpha, args.act_limit, args.act_shift));
                         }
                     }
                 }
