@@ -615,7 +615,10 @@ def grouped_attention(q, cache, block_table, token_seq, positions, out, window, 
         # bits): up to 32 heads to a block, a block to an SM.  (At most 24 parts of a
         # token's keys, us with 16, 24 and 32: one token at 32 heads over 4,096 keys 21.7, 17.6, 18.0, over 8,191 27.0, 22.9, 19.3; four
         # tokens over 1,000 13.5, 13.9, 16.0, over 4,096 22.1, 18.8, 22.5)
-        splits = max(1, min(24, 148 // (T * (1 if H <= 16 else -(-H // 32)))))
+        # (Up to 8 heads and 8 tokens: some SMs are left without a block, where the merge's few blocks stand ready.  148 and 133 blocks, 4 heads,
+        # 8 tokens over 30, 1,000, 4,000 and 8,000 keys: rows of 128 10.7 / 8.7, 11.2 / 9.6, 14.5 / 12.5, 19.2 / 17.9, of 576 12.3 / 10.3, 12.9 /
+        # 11.4, 18.4 / 16.5, 25.5 / 26.1; 16 heads, rows of 576 12.4 / 11.7, 13.5 / 12.8, 18.7 / 17.9, 26.5 / 27.8; 12 tokens, 8,000 keys 36.2 / 37.2)
+        splits = max(1, min(24, (133 if H <= 8 and T <= 8 else 148) // (T * (1 if H <= 16 else -(-H // 32)))))
         part = empty((T, H, splits, dv + 2), torch.float32, q.device)
         _check(_get("air_latent_attention")(
             q.data_ptr(), cache.data_ptr(), cache.shape[0], block_table.data_ptr(), block_table.shape[1], token_seq.data_ptr(),

@@ -875,11 +875,11 @@ def test_single_tokens_over_latents_on_the_tensor_cores(H, d, dv, P, kind):
         assert ((first[i].double() - want).abs() <= bound).all(), (i, float(((first[i].double() - want).abs() / bound).max()))
 
 
-@pytest.mark.parametrize("H,d,dv", [(16, 576, 512), (3, 320, 256), (20, 128, 128)])
-def test_latent_queries_on_any_boundary(H, d, dv):
+@pytest.mark.parametrize("H,d,dv", [(16, 576, 512), (3, 320, 256), (20, 128, 128), (8, 576, 512)])
+@pytest.mark.parametrize("contexts", [[0, 70, 300], [0, 5, 63, 64, 65, 200, 299, 319]])
+def test_latent_queries_on_any_boundary(contexts, H, d, dv):
     """Queries that do not begin on 16 bytes take the kernels that read them by less, a batch of no token takes none."""
     from air_b200.csrc import ops
-    contexts = [0, 70, 300]
     T, P = len(contexts), 64
     g = torch.Generator(device="cuda").manual_seed(d)
     rows = torch.randn(T * 5, P, d, generator=g, device="cuda").bfloat16()
