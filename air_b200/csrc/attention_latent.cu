@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attention_kernel(const _
             }
             // O's step j - 1 has ended: P may be written again, and O rescaled
             if (j > 0 && ok) ok = mbar_wait(pv_done, (j - 1) & 1, abort_flag);
-            __syncwarp();
             if (any && j > 0 && holder) {
+                __syncwarp();
                 tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < 2 * HN; c += 16) {

@@ -76,7 +76,7 @@ def test_a_warp_goes_on_together_behind_a_wait():
         for line, around, statement, behind in waits(source):
             if re.search(r"__all_sync\(0xffffffffu,[^;]*$|__syncthreads_or\(!$", statement):
                 voted += 1
-            elif re.search(r"\bok = $", statement) and behind.startswith("__syncwarp();"):
+            elif re.search(r"\bok = $", statement) and re.match(r"(if \([^{;]*\) \{\s*)?__syncwarp\(\);", behind):
                 together += 1
             elif any(one.search(opening) for opening in around + [statement]):
                 alone += 1
