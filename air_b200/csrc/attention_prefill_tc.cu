@@ -389,7 +389,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         bool ok = true;
         for (int it = 0; it < me.n && ok; ++it) {
             const int b = it & 1;
-            ok = __all_sync(0xffffffffu, mbar_wait(&my_s_full[b], (it >> 1) & 1, abort_flag));
+            ok = mbar_wait(&my_s_full[b], (it >> 1) & 1, abort_flag);
             if (!ok) break;
             tc_fence_after();
             uint32_t sv[AT_BN];
@@ -476,12 +476,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             // issue).  Looking at its barrier all the same, every time, keeps the parity that a wait
             // sees at most one phase behind: a wait by parity cannot tell a phase from the one two later.
             if (it >= 2) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&my_pv_done[b], ((it >> 1) - 1) & 1, abort_flag));
+                ok = mbar_wait(&my_pv_done[b], ((it >> 1) - 1) & 1, abort_flag);
                 if (!ok) break;
             }
             if (it >= 1 && __any_sync(0xffffffffu, move)) {
                 // O must be rescaled: every product issued so far (up to tile it-1) has to be complete
-                ok = __all_sync(0xffffffffu, mbar_wait(&my_pv_done[b ^ 1], ((it - 1) >> 1) & 1, abort_flag));
+                ok = mbar_wait(&my_pv_done[b ^ 1], ((it - 1) >> 1) & 1, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll
@@ -500,8 +500,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             __syncwarp();
             if (lane == 0) mbar_arrive(&my_p_ready[b]);
         }
-        if (ok && me.n >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&my_pv_done[me.n & 1], ((me.n - 2) >> 1) & 1, abort_flag));
-        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&my_pv_done[(me.n - 1) & 1], ((me.n - 1) >> 1) & 1, abort_flag));
+        if (ok && me.n >= 2) ok = mbar_wait(&my_pv_done[me.n & 1], ((me.n - 2) >> 1) & 1, abort_flag);
+        if (ok) ok = mbar_wait(&my_pv_done[(me.n - 1) & 1], ((me.n - 1) >> 1) & 1, abort_flag);
         if (ok) {
             // The rows leave through the row tile's own Q tile in shared memory, which no product reads any more:
             // thread r puts its row there in 16-byte chunks (chunk c at place c ^ r of the row: no two lanes of a
