@@ -26,12 +26,14 @@
 //                              operands to 2^-23: what is left out is of the order of 32-bit rounding.  The next chunks'
 //                              numbers arrive by the copy engine, in two runs of bytes, while this one's are used.
 //
-// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 152 (prepare
-// 46, scan 106); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 84 (29 and 54).  Which portions come here:
+// delta_chunk_scan_together_kernel   the same in half the threads, for many blocks.
+//
+// Measured, us, against the scan token by token: 2,048 tokens, 16 heads of 128 x 128, one decay per head 432 -> 149 (prepare
+// 46, scan 102); gated linear attention, 777 tokens, 16 heads of 128 x 256, 189 -> 83 (29 and 53).  Which portions come here:
 // parts/recurrent.py (least).
 //
 // What bounds the scan is the chain from chunk to chunk: three products of 24 instructions each that a warp issues at 10 cycles an
-// instruction, the cutting of 64 numbers into halves, two barriers: 0.83 us a chunk, 0.69 for gated linear attention, which has two
+// instruction, the cutting of 64 numbers into halves, two barriers: 0.80 us a chunk, 0.69 for gated linear attention, which has two
 // products.  Half of the warps hold the state and do nothing that the next chunk does not wait for; the sums across warps that give U, and
 // the outputs, are the other half's, the latter a chunk behind.  (All of it in four warps: 1.15 us a chunk, 148 and 74 us for the two
 // sizes above; the state handed to the other half for q S through shared memory: 136 and 70; barriers in memory instead of bar.sync: 177.)
@@ -895,7 +897,7 @@ static int launch_delta_chunks(const DeltaChunkArgs& args, int N, int L, cudaStr
     // Where every block has an SM to itself a warp has the registers to cut what its next product reads between the instructions of the one
     // before, and as many chunks are under way as memory holds; else two blocks share an SM, except where a delta rule's rows of 256 leave
     // no registers for that.  (32 heads of 128 x 128, 256 blocks, 2,048 tokens: 192 us; with one block to an SM they would take two rounds of
-    // 106.  Gated linear attention, heads of 256 x 256, two to an SM and one, us with the preparation: 16 heads, 300 tokens 69.3 and 72, 32 heads,
+    // 102.  Gated linear attention, heads of 256 x 256, two to an SM and one, us with the preparation: 16 heads, 300 tokens 69.3 and 72, 32 heads,
     // 1,000 tokens 342 and 359, 8 portions of 33 tokens 166 and 205.)
     // More blocks than that, and an SM is kept busy by four warps of each of three to eight: delta rule, two to an SM and these, heads of 64 x 128,
     // 512 blocks 3, 7 and 13 chunks long 22.7 / 20.6, 32.2 / 30.5 and 47.5 / 45.8, 4,096 of 7 172 / 152; heads of 128, 512 of 3, 7 and 63 chunks
