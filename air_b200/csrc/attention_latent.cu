@@ -23,7 +23,9 @@
 // the queries are what an SM holds), against 1.1 that an SM's copies of the tile take; and 9 us in front of the first and behind the last.
 // Measured with the merge, rows of 576 (values 512), 32 heads, us, grouped_attention_tc_kernel and this one: 8 tokens over 100 keys 17.6 and 14.4,
 // 1,000 23.8 and 16.4, 4,096 48.3 and 22.9 (its keys at the copy rate: 5.8), 8,000 74.6 and 32.4; 32 tokens over 4,096 149.9 and 55.1 (23); one
-// over 8,191 48.3 and 22.9; 16 heads: 8 tokens over 4,096 36.0 and 19.7.  Scores in a thread per key (32 heads each, on two of four schedulers): 40.1
+// over 8,191 48.3 and 22.9; 16 heads: 8 tokens over 4,096 36.0 and 19.7.  Shorter rows, 32 heads, 32 tokens over 4,000: of 128 (values 128) 65.5 and
+// 31.7, 192 (128) 70.8 and 33.3, 256 (256) 80.0 and 37.7, 384 (256) 115 and 44, 512 (512) 131 and 50; 4 heads, 8 over 4,000, rows of 128 19.9 and 12.5; of
+// 655 sizes only rows of 128 have slower ones, 8 tokens by up to 20 heads over few keys (10.7 and 11.6 the worst).  Scores in a thread per key (32 heads each, on two of four schedulers): 40.1
 // instead of 22.9; rows to be zeroed one after the other by one warp: 29.5.
 #include "common.cuh"
 #include "umma.cuh"
